@@ -108,6 +108,7 @@ struct bfgFac_s {
   bool arena32Ready = false, arenaDfReady = false;
   DevBuf srcPerm, tgtPerm;
   DevBuf items, contribs, rowSeg, segStart, segContrib0, segBase;
+  DevBuf rowExp;                    // FP64 apply: scale codes, 32 rows per contribution
   DevBuf ws, xbuf;
   DevBuf hx128, hy128, hx64, hy64;  // staging of the host-operand apply
   // pipelined host-operand applies (bfgFacApplyHostAsync): two staging
@@ -588,7 +589,32 @@ void buildApply(bfgFac f) {
   upload(f->segContrib0, p.segContrib0, s, "apply program");
   upload(f->segBase, p.segBase, s, "apply program");
   f->stageItem0 = p.stageItem0;
+  // the FP64 apply's row scales: here, once, and not in the applies, so that
+  // these launch and allocate nothing for it (a pass over the factors: 0.6 ms
+  // for 3.3 GB)
+  ck(f->rowExp.ensure(std::max<size_t>(1, p.contribs.size()) * bfg::kItemRows * sizeof(int16_t)),
+     "apply program");
+  ck(bfg::launchRowExp(f->items.as<bfg::ApplyItem>(), (int64_t)p.items.size(),
+                       f->contribs.as<bfg::ApplyContrib>(), f->arena64.as<double2>(),
+                       f->rowExp.as<int16_t>(), s),
+     "apply program");
   ck(cudaStreamSynchronize(s), "apply program");
+}
+
+// one stage of the FP64 and FP32 applies
+cudaError_t launchStage(bfgFac f, size_t st, double2 const *arena, double2 const *X, int64_t ldx,
+                        double2 *W, int64_t R) {
+  int64_t const a = f->stageItem0[st], b = f->stageItem0[st + 1];
+  return bfg::launchApplyStageFixed(f->items.as<bfg::ApplyItem>() + a, b - a,
+                                    f->contribs.as<bfg::ApplyContrib>(), f->rowExp.as<int16_t>(),
+                                    arena, X, ldx, W, R, f->ctx->stream);
+}
+cudaError_t launchStage(bfgFac f, size_t st, float2 const *arena, float2 const *X, int64_t ldx,
+                        float2 *W, int64_t R) {
+  int64_t const a = f->stageItem0[st], b = f->stageItem0[st + 1];
+  return bfg::launchApplyStage(f->items.as<bfg::ApplyItem>() + a, b - a,
+                               f->contribs.as<bfg::ApplyContrib>(), arena, X, ldx, W, R,
+                               f->ctx->stream);
 }
 
 void fillStats(bfgFac f) {
@@ -635,10 +661,7 @@ void runApply(bfgFac f, T2 const *arena, T2 const *X, int64_t ldx, int64_t R, T2
   }
   size_t const nStages = f->stageItem0.size() - 1;
   for (size_t st = 0; st < nStages; ++st) {
-    int64_t a = f->stageItem0[st], b = f->stageItem0[st + 1];
-    ck(bfg::launchApplyStage<T2>(f->items.as<bfg::ApplyItem>() + a, b - a,
-                                 f->contribs.as<bfg::ApplyContrib>(), arena, Xt, ldxt, W, R, s),
-       "apply stage");
+    ck(launchStage(f, st, arena, Xt, ldxt, W, R), "apply stage");
     mark();
   }
   ck(bfg::launchApplyReduce<T2>(f->rowSeg.as<int32_t>(), f->segStart.as<int64_t>(),
@@ -989,13 +1012,8 @@ bfgStatus noAllocApplyFp64(bfgFac f, double2 const *X, int64_t ldx, int64_t R, d
       ldxt = R;
     }
     size_t const nStages = f->stageItem0.size() - 1;
-    for (size_t st = 0; st < nStages; ++st) {
-      int64_t a = f->stageItem0[st], b = f->stageItem0[st + 1];
-      ck(bfg::launchApplyStage<double2>(f->items.as<bfg::ApplyItem>() + a, b - a,
-                                        f->contribs.as<bfg::ApplyContrib>(),
-                                        f->arena64.as<double2>(), Xt, ldxt, W, R, s),
-         "apply stage");
-    }
+    for (size_t st = 0; st < nStages; ++st)
+      ck(launchStage(f, st, f->arena64.as<double2>(), Xt, ldxt, W, R), "apply stage");
     ck(bfg::launchApplyReduce<double2>(
            f->rowSeg.as<int32_t>(), f->segStart.as<int64_t>(), f->segContrib0.as<int64_t>(),
            f->segBase.as<int64_t>(), W, R, Y, ldy, p.numRows,

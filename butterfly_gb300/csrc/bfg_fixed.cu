@@ -1,0 +1,559 @@
+// FP64 apply of the butterfly factors (complex128 factors and vectors) with
+// the products formed exactly from fixed-point parts: integer digits on the
+// tensor cores for several right-hand sides (bfg_fixed.cuh), 28-bit halves on
+// the integer units for one.  GB300's FP64 units (2 FMAs a clock and SM) made
+// the plain form 3 to 40 times slower than HBM delivers the factors.  Same
+// apply program and workspace as the other precisions
+// (mat_block_dense.c:512-572, mat_product.c:211-245): one item = up to 32
+// output rows of one block row, summing its blocks in order; no atomics on
+// results, reproducible bit for bit.  Scales: one per (block row piece, row)
+// of the factors, computed once when the factors are stored (rowExpKernel),
+// and one per right-hand side of the input rows in hand, found as they are
+// read.  Rows that fixed point does not cover (NaN, infinities, subnormals,
+// products beyond the exponent range) are multiplied in plain FP64 by the
+// same kernels.
+//
+// Measured (GB300; microseconds an apply; before: the FP64-unit kernels):
+//   32,768 points, k = 256, 6.0e7 entries   R = 1: 526 -> 350
+//     R = 2..4: 4,000 -> 515   R = 8: 4,018 -> 870   R = 16: 7,650 -> 1,650
+//     R = 64: 27,950 -> 6,200
+//   65,536 points, k = 512, 2.1e8 entries   R = 1: 1,583 -> 912
+// Error against extended precision on the same blocks: 4,096 points at
+// tolerance 1e-8, R = 1 4.4e-16 -> 2.0e-16, R = 2 1.1e-15 -> 2.1e-16, R = 9
+// 6.4e-16 -> 2.2e-16; 1,500 points at the reference's settings 2.0e-15 ->
+// 1.9e-15, 5.5e-15 -> 1.9e-15, 3.7e-15 -> 2.2e-15.
+//
+// Why not `tcgen05` for the digits: a lane forms an entry's digits from the
+// 16 bytes it loaded, in the registers `mma.sync` reads them from; `tcgen05`
+// needs them in shared memory, and precomputed in HBM they would be 28 bytes
+// an entry beside the stored 16.
+//
+// Complex to real: A (16 rows x 16) holds row m = Re a_m0, Im a_m0, Re a_m1,
+// ...; B's rows 2c, 2c+1 are (Re x, -Im x) in the column of Re y and
+// (Im x, Re x) in that of Im y.  In the fragment layouts of m16n8k16 a lane
+// (g = lane / 4, t = lane % 4) holds the entries (g, t), (g + 8, t),
+// (g, t + 4), (g + 8, t + 4) of A, one register each, and the results of rows
+// g and g + 8 in columns 2t, 2t + 1: one complex value each.
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "bfg_device.cuh"
+#include "bfg_fixed.cuh"
+#include "bfg_kernels.cuh"
+
+namespace bfg {
+namespace {
+
+static_assert(kItemRows == 32, "two 16-row MMA tiles per item");
+
+// Row scales of every contribution of every item: rowExp[32 (contribution) +
+// row].  One CTA per item, the warps split a contribution's columns.  HBM
+// bound: reads the stored factors once.
+__global__ void __launch_bounds__(256) rowExpKernel(ApplyItem const *__restrict__ items,
+                                                    ApplyContrib const *__restrict__ contribs,
+                                                    double2 const *__restrict__ arena,
+                                                    int16_t *__restrict__ rowExp) {
+  __shared__ int red[8][32];
+  int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  ApplyItem const it = items[blockIdx.x];
+  for (int c = 0; c < it.nContrib; ++c) {
+    ApplyContrib const cb = contribs[it.contrib0 + c];
+    double2 const *a = arena + cb.aOff + lane;
+    int code = 0;
+    if (lane < it.rows)
+      for (int j = warp; j < cb.n; j += 8) code = max(code, fixCode(a[(int64_t)j * cb.lda]));
+    red[warp][lane] = code;
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+      for (int w = 1; w < 8; ++w) code = max(code, red[w][lane]);
+      rowExp[(it.contrib0 + c) * 32 + lane] = (int16_t)fixScaleOf(code);
+    }
+    __syncthreads();
+  }
+}
+
+constexpr int kFixWarps = 4, kFixThreads = 32 * kFixWarps;
+
+// What a warp of an item's CTA works on: rows 16 mt .. of the item and every
+// ks-th k-step from kp on (two warps a row tile for items of more than 16
+// rows, else all four on the one tile).
+struct FixRole {
+  int mt, kp, ks;
+  int row0, row1;   // the lane's two rows (clamped into the item)
+  __device__ __forceinline__ FixRole(int rows, int warp, int lane) {
+    bool const two = rows > 16;
+    mt = two ? warp & 1 : 0;
+    kp = two ? warp >> 1 : warp;
+    ks = two ? kFixWarps / 2 : kFixWarps;
+    row0 = min(16 * mt + (lane >> 2), rows - 1);
+    row1 = min(16 * mt + (lane >> 2) + 8, rows - 1);
+  }
+};
+
+// The chunk being fetched: columns [j0, j0 + n) of contribution c of an item.
+struct FixCursor {
+  int c = 0, j0 = 0, n = 0;
+  int ea0 = 1023, ea1 = 1023;   // scales of the lane's rows
+  int eaMin = 1023, eaMax = 1023;
+  double2 const *a = nullptr;   // item row 0, chunk column 0
+  double2 const *x = nullptr;   // chunk row 0, right-hand side 0 of the tile
+  int64_t lda = 0, xld = 0;
+};
+
+// the lane's four entries of k-step st; columns past the end re-read the last
+// one (against zero inputs)
+__device__ __forceinline__ void fixLoadA(double2 (&av)[4], FixCursor const &k, FixRole const &role,
+                                         int st, int lane) {
+  int64_t const c0 = (int64_t)min(8 * st + (lane & 3), k.n - 1) * k.lda;
+  int64_t const c1 = (int64_t)min(8 * st + (lane & 3) + 4, k.n - 1) * k.lda;
+  av[0] = k.a[c0 + role.row0];
+  av[1] = k.a[c0 + role.row1];
+  av[2] = k.a[c1 + role.row0];
+  av[3] = k.a[c1 + role.row1];
+}
+
+__device__ __forceinline__ void fixNextBlock(FixCursor &k, ApplyItem const &it, ApplyContrib &cb,
+                                             ApplyContrib const *__restrict__ contribs,
+                                             int16_t const *__restrict__ rowExp,
+                                             double2 const *arena, double2 const *X, int64_t ldx,
+                                             double2 const *W, int64_t ldw, int64_t r0,
+                                             FixRole const &role, int lane) {
+  cb = contribs[it.contrib0 + k.c];
+  int16_t const *e = rowExp + (it.contrib0 + k.c) * 32;
+  k.ea0 = e[role.row0];
+  k.ea1 = e[role.row1];
+  int const mine = e[min(lane, it.rows - 1)];
+  k.eaMin = __reduce_min_sync(0xffffffffu, mine);
+  k.eaMax = __reduce_max_sync(0xffffffffu, mine);
+  k.lda = cb.lda;
+  k.xld = cb.inIsX ? ldx : ldw;
+  k.x = (cb.inIsX ? X + cb.inRow * ldx : W + cb.inRow * ldw) + r0;
+  k.a = arena + cb.aOff;
+}
+
+// Several right-hand sides: one CTA of 4 warps per (item, tile of 4 NT
+// right-hand sides).  A block's columns are walked in chunks of 128 / NT: the
+// chunk's input rows (fetched a chunk ahead, into registers) are split into
+// digits in shared memory in the B fragments' order, the factor entries
+// (fetched a k-step ahead) in the registers of the lane that loaded them.
+// The digit sums are flushed into FP64 accumulators at the end of a block,
+// after fixMaxSteps k-steps and when a chunk's inputs pass their scale by more
+// than a binade; the chunk after a flush sets the scale.  The warps that share rows
+// add their FP64 sums at the end, in order.
+// Bound by instruction issue and latency, not by the tensor pipe (30 % busy at
+// 16 right-hand sides): splitting the entries and the inputs takes about 45
+// instructions each.  Wider CTAs (8 warps on 128 rows, 8 right-hand sides a
+// tile, the next step split under the MMAs) were slower: 2,330 against 1,650
+// us at 32,768 points and 16 right-hand sides.
+template <int NT>
+__global__ void __launch_bounds__(kFixThreads, NT == 1 ? 3 : 2) fixTileKernel(
+    ApplyItem const *__restrict__ items, ApplyContrib const *__restrict__ contribs,
+    int16_t const *__restrict__ rowExp, double2 const *__restrict__ arena, double2 const *X,
+    int64_t ldx, double2 *W, int64_t R, unsigned tiles) {
+  constexpr int RT = 4 * NT, KC = 128 / NT, D = kFixDigits;
+  // chunks of 32 columns flush less often with room for growth
+  constexpr int kGrow = NT == 4 ? 1 : 0;
+  static_assert(KC / 8 / (kFixWarps / 2) <= fixMaxSteps(kGrow), "a chunk between flushes");
+  // B fragments: word ((st D + digit) NT + n tile) 64 + 2 lane + register
+  __shared__ __align__(16) uint32_t sB[(KC / 8) * D * NT * 64];
+  __shared__ int sMax[2][RT];
+  static_assert(sizeof(sB) >= kFixWarps * NT * 4 * 32 * sizeof(double), "partial sums");
+  int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t = lane & 3;
+  int const q = tid % RT, colX = tid / RT;   // the input entries this thread splits
+  // the tiles of an item run side by side and read its blocks from HBM once
+  ApplyItem const it = items[blockIdx.x / tiles];
+  int64_t const r0 = (int64_t)(blockIdx.x % tiles) * RT;
+  int const nr = (R - r0) < RT ? (int)(R - r0) : RT;
+  FixRole const role(it.rows, warp, lane);
+
+  double acc[NT][4];   // (row0 re, im, row1 re, im) of right-hand side 4 nt + t
+  float sum[NT][kFixSums][4];
+#pragma unroll
+  for (int u = 0; u < NT; ++u)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      acc[u][r] = 0.0;
+#pragma unroll
+      for (int s = 0; s < kFixSums; ++s) sum[u][s][r] = 0.f;
+    }
+
+  FixCursor k;
+  ApplyContrib cb{};
+  double2 av[4], xv[4];
+  auto fetch = [&](int buf) {
+    if (k.j0 == 0) {
+      fixNextBlock(k, it, cb, contribs, rowExp, arena, X, ldx, W, R, r0, role, lane);
+    } else {
+      k.a += KC * k.lda;
+      k.x += KC * k.xld;
+    }
+    k.n = min(KC, cb.n - k.j0);
+    int code = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      int const col = colX + i * (kFixThreads / RT);
+      xv[i] = (q < nr && col < k.n) ? k.x[col * k.xld + q] : make_double2(0.0, 0.0);
+    }
+    fixLoadA(av, k, role, role.kp, lane);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) code = max(code, fixCode(xv[i]));
+#pragma unroll
+    for (int o = RT; o < 32; o *= 2) code = max(code, __shfl_xor_sync(0xffffffffu, code, o));
+    if (lane < RT && code) atomicMax(&sMax[buf][q], code);   // order does not matter
+  };
+  if (tid < 2 * RT) sMax[tid / RT][tid % RT] = 0;
+  __syncthreads();
+
+  int buf = 0, steps = 0;   // k-steps summed since the last flush (any warp's most)
+  int code = 0;             // lane l: scale code of right-hand side l
+  int ea0 = 1023, ea1 = 1023;
+  auto flush = [&]() {
+#pragma unroll
+    for (int u = 0; u < NT; ++u) {
+      int const ex = fixScaleOf(__shfl_sync(0xffffffffu, code, 4 * u + t));
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        int v[kFixSums];
+#pragma unroll
+        for (int s = 0; s < kFixSums; ++s) {
+          v[s] = __float2int_rn(sum[u][s][r]);
+          sum[u][s][r] = 0.f;
+        }
+        int64_t const V = ((int64_t)v[0] << 40) + ((int64_t)v[1] << 32) + ((int64_t)v[2] << 24) +
+                          ((int64_t)v[3] << 16) + ((int64_t)v[4] << 8) +
+                          (v[5] + ((v[6] + (v[7] >> 8) + 128) >> 8));
+        acc[u][r] = fma((double)V, fixScale((r < 2 ? ea0 : ea1) + ex), acc[u][r]);
+      }
+    }
+    steps = 0;
+  };
+  if (it.nContrib > 0) fetch(0);
+  while (k.c < it.nContrib) {
+    __syncthreads();
+    int const cm = lane < RT ? sMax[buf][lane] : 0;
+    bool const first = k.j0 == 0;
+    // a scale stays until an entry passes it by more than kGrow binades.
+    // Every warp holds the same codes and row scales, so these decisions are
+    // the same in the whole CTA.
+    int const mySteps = (KC / 8 + role.ks - 1) / role.ks;
+    bool const grown = code == 0 ? cm != 0 : cm > code + kGrow || cm >= kFixSpecial;
+    if (steps > 0 && (first || steps + mySteps > fixMaxSteps(kGrow) || __any_sync(0xffffffffu, grown)))
+      flush();
+    if (steps == 0) code = cm;
+    ea0 = k.ea0;
+    ea1 = k.ea1;
+    int const ex = fixScaleOf(code);
+    bool const plain = !__all_sync(0xffffffffu, fixCovers(k.eaMin, k.eaMax, ex));
+    int const exq = __shfl_sync(0xffffffffu, ex, q);
+    if (tid < RT) sMax[buf ^ 1][tid] = 0;   // read by every warp a chunk ago
+    if (!plain) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        int const col = colX + i * (kFixThreads / RT);
+        uint32_t d[D];
+        fixSplit<kGrow>(xv[i], exq, d);
+        // column col = 8 st + c8: lane t = c8 % 4, register c8 / 4; result
+        // columns 2 (q % 4) and 2 (q % 4) + 1 of n tile q / 4
+        uint32_t *w = sB + ((col >> 3) * D * NT + (q >> 2)) * 64 +
+                      2 * (8 * (q & 3) + (col & 3)) + ((col >> 2) & 1);
+#pragma unroll
+        for (int j = 0; j < D; ++j, w += NT * 64) {
+          w[0] = d[j] ^ 0x80000000u;                   // (Re x, -Im x)
+          w[8] = __byte_perm(d[j], 0, 0x1032);         // (Im x, Re x)
+        }
+      }
+    }
+    __syncthreads();
+    int const nSteps = (k.n + 7) >> 3;
+    if (!plain) {
+#pragma unroll 1
+      for (int st = role.kp; st < nSteps; st += role.ks) {
+        uint32_t d[4][D];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) fixSplit(av[e], e & 1 ? ea1 : ea0, d[e]);
+        if (st + role.ks < nSteps) fixLoadA(av, k, role, st + role.ks, lane);
+        uint2 const *b = reinterpret_cast<uint2 const *>(sB) + st * D * NT * 32 + lane;
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+          uint2 bv[NT];
+#pragma unroll
+          for (int u = 0; u < NT; ++u) bv[u] = b[(j * NT + u) * 32];
+#pragma unroll
+          for (int i = 0; i < D && i + j < kFixSums; ++i)
+#pragma unroll
+            for (int u = 0; u < NT; ++u)
+              fixMma(sum[u][i + j], d[0][i], d[1][i], d[2][i], d[3][i], bv[u].x, bv[u].y);
+        }
+      }
+      steps += mySteps;
+    } else {
+      for (int st = role.kp; st < nSteps; st += role.ks)
+        for (int col = 8 * st; col < min(8 * st + 8, k.n); ++col) {
+          double2 const a0 = k.a[col * k.lda + role.row0], a1 = k.a[col * k.lda + role.row1];
+#pragma unroll
+          for (int u = 0; u < NT; ++u)
+            if (4 * u + t < nr) {
+              double2 const x = k.x[col * k.xld + 4 * u + t];
+              cmacc(acc[u][0], acc[u][1], a0, x);
+              cmacc(acc[u][2], acc[u][3], a1, x);
+            }
+        }
+    }
+    k.j0 += KC;
+    if (k.j0 >= cb.n) {
+      k.j0 = 0;
+      ++k.c;
+    }
+    buf ^= 1;
+    if (k.c < it.nContrib) fetch(buf);
+  }
+  if (steps > 0) flush();
+  __syncthreads();
+  double *const part = reinterpret_cast<double *>(sB);   // [warp][u][r][lane]
+#pragma unroll
+  for (int u = 0; u < NT; ++u)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) part[((warp * NT + u) * 4 + r) * 32 + lane] = acc[u][r];
+  __syncthreads();
+  if (role.kp != 0) return;
+  int const warpStep = kFixWarps / role.ks;   // warps of one row tile
+#pragma unroll
+  for (int u = 0; u < NT; ++u) {
+    for (int w = 1; w < role.ks; ++w)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        acc[u][r] += part[(((warp + w * warpStep) * NT + u) * 4 + r) * 32 + lane];
+    int const rhs = 4 * u + t, row = 16 * role.mt + (lane >> 2);
+    if (rhs < nr) {
+      double2 *out = W + (it.outRow + row) * R + r0 + rhs;
+      if (row < it.rows) out[0] = make_double2(acc[u][0], acc[u][1]);
+      if (row + 8 < it.rows) out[8 * R] = make_double2(acc[u][2], acc[u][3]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// One right-hand side.  A matrix tile of 8 columns would be nearly empty, so
+// the products are formed from two 28-bit halves on the integer units
+// instead: t (the scaled entry, |t| <= 2^55) = hi 2^28 + lo, and
+//   t t' = 2^56 hi hi' + 2^28 (hi lo' + lo hi') + lo lo',
+// each sum carried in 64 bits without rounding: 16 widening multiply-adds a
+// complex entry (32 lanes of them a clock and SM, against 2 FP64 FMAs).
+//
+// One CTA of 4 warps per item, lane = row.  A block's columns are walked in
+// passes of at most 120: the pass's input rows are brought to one scale in
+// shared memory, warp w multiplies columns w, w + 4, ..., splitting its factor
+// entries in registers with the next three columns' loads in flight, and the
+// warps' integer sums are added exactly before two threads a row turn them
+// into FP64: one rounding a pass.  The next pass's input rows and first
+// entries are fetched while a pass is multiplied, so a pass costs two
+// barriers and no exposed latency.
+// ---------------------------------------------------------------------------
+constexpr int kGemvCols = 120, kGemvAhead = 3, kGemvWarps = 4;
+static_assert(kGemvCols <= 127, "4 products of 2^54 a column below 2^63");
+static_assert(kGemvCols <= 32 * kGemvWarps, "one input row per thread");
+static_assert(kGemvCols % (kGemvWarps * kGemvAhead) == 0, "whole batches of columns");
+
+// (hi, lo) of v at scale E, rounded: |hi| <= 2^27, |lo| <= 2^27
+__device__ __forceinline__ int2 fixHalves(double v, int E) {
+  uint32_t const h = (uint32_t)__double2hiint(v), l = (uint32_t)__double2loint(v);
+  uint32_t const mh = (h & 0xFFFFFu) | 0x100000u, sh = (uint32_t)E - ((h >> 20) & 0x7FFu);
+  int32_t const s = (int32_t)h >> 31;
+  // twice t, truncated (its last bit rounds lo); shr.u64 gives 0 from 64 on
+  uint64_t y = ((uint64_t)__funnelshift_l(l, mh, 3) << 32) | (l << 3);
+  asm("shr.u64 %0, %0, %1;" : "+l"(y) : "r"(sh));
+  uint64_t const u = (y ^ (uint64_t)(int64_t)s) + (uint32_t)((1 << 28) - s);
+  uint32_t const ul = (uint32_t)u, uh = (uint32_t)(u >> 32);
+  return make_int2((int32_t)__funnelshift_r(ul, uh, 29),
+                   ((int32_t)(ul & 0x1FFFFFFFu) - ((1 << 28) - 1)) >> 1);
+}
+__device__ __forceinline__ int4 fixHalves(double2 v, int E) {
+  int2 const a = fixHalves(v.x, E), b = fixHalves(v.y, E);
+  return make_int4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void fixMad(int64_t &acc, int32_t a, int32_t b) {
+  acc += (int64_t)a * b;
+}
+
+__global__ void __launch_bounds__(32 * kGemvWarps, 6)
+fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restrict__ contribs,
+              int16_t const *__restrict__ rowExp, double2 const *__restrict__ arena,
+              double2 const *X, int64_t ldx, double2 *W) {
+  constexpr int S = kGemvWarps, U = kGemvAhead, KC = kGemvCols;
+  __shared__ int4 sx[KC];
+  __shared__ int sMax[2][S];
+  // sums of the real part (high, mixed, low) and of the imaginary part
+  __shared__ int64_t part[6][S][32];
+  int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  ApplyItem const it = items[blockIdx.x];
+  bool const active = lane < it.rows;
+  double acc = 0.0;   // the last two warps: real and imaginary part of row lane
+  double spr = 0.0, spi = 0.0;   // plain FP64 sums of this lane's columns
+  bool anySpecial = false;
+
+  // the pass being fetched: columns [j0, j0 + n) of contribution c
+  int c = 0, j0 = 0, n = 0, last = 0, ea = 1023;
+  double2 const *a = nullptr, *x = nullptr;
+  int64_t step = 0, xs = 0, lda = 0;
+  ApplyContrib cb{};
+  double2 av[U], xv;
+  auto fetch = [&](int buf) {
+    if (j0 == 0) {
+      cb = contribs[it.contrib0 + c];
+      ea = active ? rowExp[(it.contrib0 + c) * 32 + lane] : 1023;
+      lda = cb.lda;
+      step = (int64_t)S * lda;
+      xs = cb.inIsX ? ldx : 1;
+      x = cb.inIsX ? X + cb.inRow * ldx : W + cb.inRow;
+      a = arena + cb.aOff + (active ? lane : 0);   // inactive lanes re-read row 0
+    } else {
+      x += KC * xs;
+      a += KC * lda;
+    }
+    n = min(KC, cb.n - j0);
+    xv = tid < n ? x[(int64_t)tid * xs] : make_double2(0.0, 0.0);
+    // this warp's columns warp, warp + 4, ... in whole batches: a column past
+    // the end re-reads the last one (or column 0) against a zero input
+    last = (n - 1 - warp) / S;
+    double2 const *aw = a + (n > warp ? warp * lda : 0);
+#pragma unroll
+    for (int u = 0; u < U; ++u) av[u] = aw[min(u, last) * step];
+    int const code = __reduce_max_sync(0xffffffffu, fixCode(xv));
+    if (lane == 0) sMax[buf][warp] = code;
+  };
+  int buf = 0;
+  if (it.nContrib > 0) fetch(0);
+  while (c < it.nContrib) {
+    __syncthreads();
+    int code = sMax[buf][0];
+#pragma unroll
+    for (int w = 1; w < S; ++w) code = max(code, sMax[buf][w]);
+    int const ex = fixScaleOf(code);
+    // the same in every warp: all hold the scales of the same 32 rows
+    bool const special = !__all_sync(0xffffffffu, fixCovers(ea, ea, ex));
+    if (!special && tid < KC) sx[tid] = tid < n ? fixHalves(xv, ex) : make_int4(0, 0, 0, 0);
+    __syncthreads();
+    int64_t hr = 0, mr = 0, lr = 0, hi = 0, mi = 0, li = 0;
+    int const eaNow = ea;
+    if (!special) {
+      double2 const *aw = a + (n > warp ? warp * lda : 0);
+      int4 const *xw = sx + warp;
+#pragma unroll 1
+      for (int i = 0; i <= last; i += U, xw += U * S) {
+        double2 nv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) nv[u] = aw[min(i + U + u, last) * step];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          int4 const f = fixHalves(av[u], eaNow), y = xw[u * S];
+          int const nh = -f.z, nl = -f.w;
+          fixMad(hr, f.x, y.x);
+          fixMad(hi, f.x, y.z);
+          fixMad(mr, f.x, y.y);
+          fixMad(mi, f.x, y.w);
+          fixMad(lr, f.y, y.y);
+          fixMad(li, f.y, y.w);
+          fixMad(hr, nh, y.z);
+          fixMad(hi, f.z, y.x);
+          fixMad(mr, f.y, y.x);
+          fixMad(mi, f.y, y.z);
+          fixMad(lr, nl, y.w);
+          fixMad(li, f.w, y.y);
+          fixMad(mr, nh, y.w);
+          fixMad(mi, f.z, y.y);
+          fixMad(mr, nl, y.z);
+          fixMad(mi, f.w, y.x);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) av[u] = nv[u];
+      }
+      part[0][warp][lane] = hr;
+      part[1][warp][lane] = mr;
+      part[2][warp][lane] = lr;
+      part[3][warp][lane] = hi;
+      part[4][warp][lane] = mi;
+      part[5][warp][lane] = li;
+    } else {
+      anySpecial = true;
+      for (int j = warp; j < n; j += S) cmacc(spr, spi, a[j * lda], x[j * xs]);
+    }
+    j0 += KC;
+    if (j0 >= cb.n) {
+      j0 = 0;
+      ++c;
+    }
+    buf ^= 1;
+    if (c < it.nContrib) fetch(buf);
+    if (!special) {
+      __syncthreads();
+      if (warp >= S - 2) {
+        int const q = 3 * (warp - (S - 2));
+        int64_t h = 0, m = 0, l = 0;
+#pragma unroll
+        for (int w = 0; w < S; ++w) {
+          h += part[q][w][lane];
+          m += part[q + 1][w][lane];
+          l += part[q + 2][w][lane];
+        }
+        m += l >> 28;
+        h += m >> 28;
+        int const e = eaNow + ex;
+        acc = fma((double)h, fixScale(e),
+                  fma((double)(int)(m & 0xFFFFFFF), fixScale(e) * 0x1.0p-28, acc));
+      }
+    }
+  }
+  // rare: add the plain FP64 sums of the warps, in order
+  if (anySpecial) {
+    __syncthreads();
+    double *const p = reinterpret_cast<double *>(part);
+    p[warp * 32 + lane] = spr;
+    p[(S + warp) * 32 + lane] = spi;
+    __syncthreads();
+    if (warp >= S - 2)
+      for (int w = 0; w < S; ++w) acc += p[((warp - (S - 2)) * S + w) * 32 + lane];
+  }
+  if (warp >= S - 2 && active) reinterpret_cast<double *>(W + it.outRow + lane)[warp - (S - 2)] = acc;
+}
+
+template <int NT>
+cudaError_t launchTile(ApplyItem const *items, int64_t nItems, ApplyContrib const *contribs,
+                       int16_t const *rowExp, double2 const *arena, double2 const *X, int64_t ldx,
+                       double2 *W, int64_t R, cudaStream_t stream) {
+  int64_t const tiles = (R + 4 * NT - 1) / (4 * NT);
+  if (tiles > 0x7fffffff / nItems) return cudaErrorInvalidConfiguration;
+  fixTileKernel<NT><<<(unsigned)(nItems * tiles), kFixThreads, 0, stream>>>(
+      items, contribs, rowExp, arena, X, ldx, W, R, (unsigned)tiles);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launchRowExp(ApplyItem const *items, int64_t nItems, ApplyContrib const *contribs,
+                         double2 const *arena, int16_t *rowExp, cudaStream_t stream) {
+  if (nItems == 0) return cudaSuccess;
+  rowExpKernel<<<(unsigned)nItems, 256, 0, stream>>>(items, contribs, arena, rowExp);
+  return cudaGetLastError();
+}
+
+cudaError_t launchApplyStageFixed(ApplyItem const *items, int64_t nItems,
+                                  ApplyContrib const *contribs, int16_t const *rowExp,
+                                  double2 const *arena, double2 const *X, int64_t ldx, double2 *W,
+                                  int64_t R, cudaStream_t stream) {
+  if (nItems == 0) return cudaSuccess;
+  if (R == 1) {
+    fixGemvKernel<<<(unsigned)nItems, 32 * kGemvWarps, 0, stream>>>(items, contribs, rowExp, arena,
+                                                                    X, ldx, W);
+    return cudaGetLastError();
+  }
+  // the narrowest tile that holds the right-hand sides: a tile's empty
+  // columns cost as much as full ones (32,768 points: 515 us with 4 columns,
+  // 870 with 8, 1,650 with 16, whatever part of them is used)
+  if (R <= 4) return launchTile<1>(items, nItems, contribs, rowExp, arena, X, ldx, W, R, stream);
+  if (R <= 8) return launchTile<2>(items, nItems, contribs, rowExp, arena, X, ldx, W, R, stream);
+  return launchTile<4>(items, nItems, contribs, rowExp, arena, X, ldx, W, R, stream);
+}
+
+}  // namespace bfg

@@ -8,9 +8,9 @@
 //                          (helm2.c:321-365) plus the pseudo-inverse
 //                          least-squares solve (mat_dense_complex.c:1768-1849)
 //                          by a one-sided Jacobi SVD (details at the kernel).
-//  * applyGemvKernel /     one stage of the staged apply (single / many RHS),
-//    applyTileKernel       each item a row chunk of one block row summing its
-//                          blocks in order; no atomics, so results are
+//  * applyGemvKernel /     one stage of the staged FP32 apply (single / many
+//    applyTileKernel       RHS), each item a row chunk of one block row summing
+//                          its blocks in order; no atomics, so results are
 //                          reproducible bit for bit.
 //  * applyReduceKernel     sums the per-product outputs into Y in a fixed
 //                          order (the reference's block-dense accumulation,
@@ -786,20 +786,11 @@ __device__ __forceinline__ void load2(float2 const *p, float2 &a, float2 &b) {
   a = make_float2(v.x, v.y);
   b = make_float2(v.z, v.w);
 }
-__device__ __forceinline__ void load2(double2 const *p, double2 &a, double2 &b) {
-  a = p[0];
-  b = p[1];
-}
 
-// Asynchronous global -> shared copies (LDGSTS) of one complex entry; the
-// 16-byte form bypasses L1 (stored blocks are read once per launch).
+// Asynchronous global -> shared copies (LDGSTS) of one complex entry
 __device__ __forceinline__ void cpAsyncEntry(float2 *dst, float2 const *src) {
   unsigned const d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cpAsyncEntry(double2 *dst, double2 const *src) {
-  unsigned const d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cpAsyncCommit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -1198,11 +1189,11 @@ cudaError_t launchC64ToC128(float2 const *a, int64_t lda, int64_t rows, int64_t 
   return cudaGetLastError();
 }
 
-template <typename T2>
 cudaError_t launchApplyStage(ApplyItem const *items, int64_t nItems,
-                             ApplyContrib const *contribs, T2 const *arena,
-                             T2 const *X, int64_t ldx, T2 *W, int64_t R,
+                             ApplyContrib const *contribs, float2 const *arena,
+                             float2 const *X, int64_t ldx, float2 *W, int64_t R,
                              cudaStream_t stream) {
+  using T2 = float2;
   if (nItems == 0) return cudaSuccess;
   if (R == 1) {
     applyGemvKernel<T2><<<(unsigned)nItems, 32 * kGemvWarps, 0, stream>>>(items, contribs,
@@ -1258,12 +1249,6 @@ cudaError_t launchGatherRows(T2 const *X, int64_t ldx, int64_t const *perm,
   return cudaGetLastError();
 }
 
-template cudaError_t launchApplyStage<double2>(ApplyItem const *, int64_t, ApplyContrib const *,
-                                               double2 const *, double2 const *, int64_t,
-                                               double2 *, int64_t, cudaStream_t);
-template cudaError_t launchApplyStage<float2>(ApplyItem const *, int64_t, ApplyContrib const *,
-                                              float2 const *, float2 const *, int64_t, float2 *,
-                                              int64_t, cudaStream_t);
 template cudaError_t launchApplyReduce<double2>(int32_t const *, int64_t const *, int64_t const *,
                                                 int64_t const *, double2 const *, int64_t,
                                                 double2 *, int64_t, int64_t, int64_t const *,

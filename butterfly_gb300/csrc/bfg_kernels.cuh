@@ -139,12 +139,20 @@ cudaError_t launchC128ToC64(double2 const *a, int64_t lda, int64_t rows, int64_t
 cudaError_t launchC64ToC128(float2 const *a, int64_t lda, int64_t rows, int64_t cols,
                             double2 *b, int64_t ldb, cudaStream_t stream);
 
-// Apply: one stage of items, element type T2 (double2 or float2).
-template <typename T2>
+// FP32 apply: one stage of items.
 cudaError_t launchApplyStage(ApplyItem const *items, int64_t nItems,
-                             ApplyContrib const *contribs, T2 const *arena,
-                             T2 const *X, int64_t ldx, T2 *W, int64_t R,
+                             ApplyContrib const *contribs, float2 const *arena,
+                             float2 const *X, int64_t ldx, float2 *W, int64_t R,
                              cudaStream_t stream);
+
+// FP64 apply (bfg_fixed.cu): the factors' row scales, kItemRows per
+// contribution of the program, and one stage of items
+cudaError_t launchRowExp(ApplyItem const *items, int64_t nItems, ApplyContrib const *contribs,
+                         double2 const *arena, int16_t *rowExp, cudaStream_t stream);
+cudaError_t launchApplyStageFixed(ApplyItem const *items, int64_t nItems,
+                                  ApplyContrib const *contribs, int16_t const *rowExp,
+                                  double2 const *arena, double2 const *X, int64_t ldx, double2 *W,
+                                  int64_t R, cudaStream_t stream);
 
 // W row-major with leading dimension R, or (wTile > 0) tile-major: panel t
 // of wTile columns at W + t wTileStride, leading dimension wTile

@@ -1,0 +1,105 @@
+"""The FP64 apply's fixed-point products (bfg_fixed.cu) against extended
+precision, evaluated from the factorization's own stored blocks.
+
+Every block is dense here (no split below depth 1), so a row's error bound is
+known: a part of an entry is off by at most 2^-55 of its row's largest part
+(2^-54 of the largest input, whose scale may start a binade high), a complex
+product has two such real products a part, and each FP64 rounding of a sum is
+below 2^-53 of the sum of moduli.  Together less than
+2^-51 n max|a_i| max|x| a block of n columns."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import butterfly_gb300 as B  # noqa: E402
+
+LD = np.clongdouble
+
+
+def _dense_blocks(fac):
+    """(row offset, column offset, block) of every block of an all-dense plan."""
+    tab, ent = fac.blocks()
+    lines = [ln.split() for ln in fac.describe().splitlines()]
+    assert lines[0][0] == "BD" and all(ln[0] == "DC" for ln in lines[3:])
+    ro, co = [int(v) for v in lines[1][1:]], [int(v) for v in lines[2][1:]]
+    out, nc = [], len(co) - 1
+    for b, (kind, m, n, off) in enumerate(tab):
+        assert kind == 3
+        out.append((ro[b // nc], co[b % nc], ent[off:off + m * n].reshape(n, m).T))
+    return out
+
+
+def _problem(m, n):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    fac = B.FacHelm2.make_multilevel(
+        B.Helm2(9.0), B.Quadtree(B.uniform_square_points(n, m), leaf_size=4096),
+        B.Quadtree(B.curve_points("circle", m), leaf_size=4096), context=B.default_context(0))
+    return fac, _dense_blocks(fac)
+
+
+def _exact_and_bound(fac, blocks, X):
+    Y = np.zeros((fac.shape[0], X.shape[1]), LD)
+    bound = np.zeros(Y.shape, np.longdouble)
+    for r, c, A in blocks:
+        m, n = A.shape
+        x = X[c:c + n].astype(LD)
+        Y[r:r + m] += A.astype(LD) @ x
+        bound[r:r + m] += (2.0 ** -51 * n * np.abs(A).max(1).astype(np.longdouble)[:, None]
+                           * np.abs(x).max(0)[None, :])
+    return Y, bound
+
+
+def _apply(fac, X):
+    return fac.apply(torch.from_numpy(X).cuda()).cpu().numpy()
+
+
+# quarters of the points land in a block, so these put block rows and columns
+# on both sides of the 16-row tiles, the 32-row items, and the 8-, 32-, 64-,
+# 120- and 128-column steps, chunks and passes
+@pytest.mark.parametrize("m,n", [(4, 4), (9, 31), (66, 33), (131, 127), (130, 257), (70, 485),
+                                 (257, 515), (40, 2101)])
+def test_fixed_point_error_is_within_its_bound(m, n):
+    fac, blocks = _problem(m, n)
+    X = B.Rng(n).complex_randn(n * 33).reshape(n, 33)
+    X *= np.exp(B.Rng(m).complex_randn(n).real * 3.0)[:, None]   # rows of unlike size
+    Y, bound = _exact_and_bound(fac, blocks, X)
+    for R in (1, 2, 4, 5, 8, 9, 16, 17, 33):
+        y = _apply(fac, X[:, :R].copy())
+        err = np.abs(y.astype(LD) - Y[:, :R])
+        assert np.all(err <= bound[:, :R]), (R, float((err / bound[:, :R]).max()))
+
+
+def test_scales_are_exact_and_ranges_fall_back():
+    fac, blocks = _problem(90, 300)
+    X = B.Rng(1).complex_randn(300 * 9).reshape(300, 9)
+    for R in (1, 3, 9):
+        y = _apply(fac, X[:, :R].copy())
+        for s in (-600.0, 600.0):     # a power of two changes exponents only
+            assert np.array_equal(_apply(fac, X[:, :R] * 2.0 ** s), y * 2.0 ** s)
+        # right-hand sides of unlike size side by side keep their own scale
+        w = 2.0 ** (40.0 * (np.arange(R) - R // 2))
+        assert np.array_equal(_apply(fac, X[:, :R] * w), y * w)
+        assert not np.any(_apply(fac, np.zeros((300, R), complex)))
+        # below the fixed-point range: plain FP64 sums
+        Y, bound = _exact_and_bound(fac, blocks, X[:, :R])
+        tiny = _apply(fac, X[:, :R] * 2.0 ** -1010) * 2.0 ** 1000 * 2.0 ** 10
+        assert np.all(np.abs(tiny.astype(LD) - Y) <= bound + np.abs(Y).max() * 2.0 ** -40)
+
+
+@pytest.mark.parametrize("R", [1, 2, 7, 16])
+def test_infinities_and_nans_reach_the_rows_they_meet(R):
+    fac, blocks = _problem(90, 300)
+    X = B.Rng(2).complex_randn(300 * R).reshape(300, R)
+    clean = _apply(fac, X.copy())
+    Y, bound = _exact_and_bound(fac, blocks, X)
+    for bad in (complex(np.inf, 0.0), complex(0.0, -np.inf), complex(np.nan, 1.0)):
+        Z = X.copy()
+        Z[17, R // 2] = bad
+        y = _apply(fac, Z)
+        assert not np.any(np.isfinite(y[:, R // 2]))
+        others = np.arange(R) != R // 2
+        assert np.all(np.abs(y[:, others].astype(LD) - Y[:, others]) <= bound[:, others])
+    assert np.array_equal(_apply(fac, X.copy()), clean)
