@@ -711,16 +711,16 @@ void ensureArenaDf(bfgFac f) {
   f->arenaDfReady = true;
 }
 
-// the double-float apply: input split (and gathered) into the X buffer,
-// stages on double-float rows, final sum into complex128 Y.  Same launch
-// count as runApply (the split stands in for its gather; without
-// BFG_APPLY_ORIGINAL_ORDER it is timed with the first stage).
-void runApplyDf(bfgFac f, double2 const *X, int64_t ldx, int64_t R, double2 *Y, int64_t ldy,
-                uint32_t flags, std::vector<cudaEvent_t> *events) {
+// the double-float apply of one right-hand side: input split (and gathered)
+// into the X buffer, stages on double-float rows, final sum into complex128
+// Y.  Same launch count as runApply (the split stands in for its gather;
+// without BFG_APPLY_ORIGINAL_ORDER it is timed with the first stage).
+void runApplyDf(bfgFac f, double2 const *X, int64_t ldx, double2 *Y, int64_t ldy, uint32_t flags,
+                std::vector<cudaEvent_t> *events) {
   cudaStream_t s = f->ctx->stream;
   bfg::ApplyProgram const &p = f->prog;
-  ck(f->ws.ensure((size_t)std::max<int64_t>(1, p.wsRows) * R * sizeof(float4)), "workspace");
-  ck(f->xbuf.ensure((size_t)std::max<int64_t>(1, p.numCols) * R * sizeof(float4)), "input buffer");
+  ck(f->ws.ensure((size_t)std::max<int64_t>(1, p.wsRows) * sizeof(float4)), "workspace");
+  ck(f->xbuf.ensure((size_t)std::max<int64_t>(1, p.numCols) * sizeof(float4)), "input buffer");
   float4 *W = f->ws.as<float4>(), *Xd = f->xbuf.as<float4>();
   size_t ev = 0;
   auto mark = [&]() {
@@ -728,7 +728,7 @@ void runApplyDf(bfgFac f, double2 const *X, int64_t ldx, int64_t R, double2 *Y, 
   };
   bool const orig = (flags & BFG_APPLY_ORIGINAL_ORDER) != 0;
   mark();
-  ck(bfg::launchGatherToDf(X, ldx, orig ? f->srcPerm.as<int64_t>() : nullptr, p.numCols, R, Xd, s),
+  ck(bfg::launchGatherToDf(X, ldx, orig ? f->srcPerm.as<int64_t>() : nullptr, p.numCols, Xd, s),
      "split X");
   if (orig) mark();
   size_t const nStages = f->stageItem0.size() - 1;
@@ -736,13 +736,13 @@ void runApplyDf(bfgFac f, double2 const *X, int64_t ldx, int64_t R, double2 *Y, 
     int64_t a = f->stageItem0[st], b = f->stageItem0[st + 1];
     ck(bfg::launchApplyStageDf(f->items.as<bfg::ApplyItem>() + a, b - a,
                                f->contribs.as<bfg::ApplyContrib>(), f->arenaDf.as<float4>(), Xd,
-                               W, R, s),
+                               W, s),
        "apply stage");
     mark();
   }
   ck(bfg::launchApplyReduceDf(f->rowSeg.as<int32_t>(), f->segStart.as<int64_t>(),
-                              f->segContrib0.as<int64_t>(), f->segBase.as<int64_t>(), W, R, Y,
-                              ldy, p.numRows, orig ? f->tgtPerm.as<int64_t>() : nullptr, s),
+                              f->segContrib0.as<int64_t>(), f->segBase.as<int64_t>(), W, Y, ldy,
+                              p.numRows, orig ? f->tgtPerm.as<int64_t>() : nullptr, s),
      "apply reduce");
   mark();
 }
@@ -943,10 +943,17 @@ bfgStatus applyDispatch(bfgFac f, bfgPrecision prec, void const *X, int64_t ldx,
     ensureArena32(f);
     runApply<float2>(f, f->arena32.as<float2>(), static_cast<float2 const *>(X), ldx, R,
                      static_cast<float2 *>(Y), ldy, flags, ev);
+  } else if (prec == BFG_PRECISION_DF64 && R > 1) {
+    // the FP64 apply's fixed-point products are both more exact than
+    // double-float ones and faster from two right-hand sides on, where those
+    // cost as much a right-hand side as for one (32,768 points: 262 us each;
+    // the FP64 apply takes 515 for 2 and 1,650 for 16)
+    if (R > 65535) ck(cudaErrorInvalidConfiguration, "apply stage");   // refused as ever
+    runApply<double2>(f, f->arena64.as<double2>(), static_cast<double2 const *>(X), ldx, R,
+                      static_cast<double2 *>(Y), ldy, flags, ev);
   } else if (prec == BFG_PRECISION_DF64) {
     ensureArenaDf(f);
-    runApplyDf(f, static_cast<double2 const *>(X), ldx, R, static_cast<double2 *>(Y), ldy, flags,
-               ev);
+    runApplyDf(f, static_cast<double2 const *>(X), ldx, static_cast<double2 *>(Y), ldy, flags, ev);
   } else if (isTcPrecision(prec)) {
     int const terms = prec == BFG_PRECISION_BF16X3 ? 3 : 2;
     ensureTc(f, terms);

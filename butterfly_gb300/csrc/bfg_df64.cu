@@ -1,10 +1,10 @@
-// Double-float ("df64") apply: the FP64 factors and vectors carried as
-// pairs of FP32 numbers (hi + lo, ~48 significant bits) and multiplied with
-// FP32 FMAs and their exact error terms.  GB300 runs FP64 at 1/64 of the
-// FP32 rate, so the plain FP64 single-vector apply is bound by its FP64
-// units (~1.2 TFLOP/s) rather than by HBM; with double-float arithmetic the
-// same 16 bytes per stored entry stream at HBM speed and the result stays
-// within ~1e-13 of FP64.  Same apply program as the other precisions
+// Double-float ("df64") apply of one right-hand side: the FP64 factors and
+// vectors carried as pairs of FP32 numbers (hi + lo, ~48 significant bits) and
+// multiplied with FP32 FMAs and their exact error terms.  The same 16 bytes
+// per stored entry as FP64, within ~1e-13 of it, and fewer instructions an
+// entry than the FP64 apply's fixed-point products (32,768 points: 262 us
+// against 350).  Several right-hand sides take the FP64 apply, which is both
+// more exact and faster there.  Same apply program as the other precisions
 // (mat_block_dense.c:512-572, mat_product.c:211-245, one item = rows of one
 // block row summing its blocks in order), no atomics, reproducible.
 //
@@ -75,28 +75,23 @@ __global__ void arenaToDfKernel(double2 const *__restrict__ a, float4 *__restric
     b[i] = dfSplit(a[i]);
 }
 
-// out (nRows x R, leading dimension R) = X rows (perm[i] or i), split
+// out[i] = X row perm[i] (or i), split
 __global__ void gatherToDfKernel(double2 const *__restrict__ X, int64_t ldx,
-                                 int64_t const *__restrict__ perm, int64_t nRows, int64_t R,
+                                 int64_t const *__restrict__ perm, int64_t nRows,
                                  float4 *__restrict__ out) {
-  int64_t const total = nRows * R;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    int64_t const i = e / R, r = e % R;
-    out[e] = dfSplit(X[(perm ? perm[i] : i) * ldx + r]);
-  }
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nRows;
+       i += (int64_t)gridDim.x * blockDim.x)
+    out[i] = dfSplit(X[(perm ? perm[i] : i) * ldx]);
 }
 
-// One CTA per (item, RHS): lane = item row, the 8 warps take every 8th
-// column with 4 entries in flight each; the warps' sums are combined in a
-// fixed order.  X and W hold double-float rows with leading dimension R.
+// One CTA per item: lane = item row, the 8 warps take every 8th column with 4
+// entries in flight each; the warps' sums are combined in a fixed order.
 __global__ void __launch_bounds__(32 * kDfWarps)
 applyGemvDfKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restrict__ contribs,
                   float4 const *__restrict__ arena, float4 const *__restrict__ X,
-                  float4 *__restrict__ W, int64_t R) {
+                  float4 *__restrict__ W) {
   __shared__ float4 part[kDfWarps][32];
   int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int64_t const r = blockIdx.y;
   ApplyItem const it = items[blockIdx.x];
   bool const active = lane < it.rows;
   float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
@@ -110,7 +105,7 @@ applyGemvDfKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__res
   for (int c = 0; c < it.nContrib; ++c) {
     ApplyContrib const cb = contribs[it.contrib0 + c];
     float4 const *a = arena + cb.aOff + lane;
-    float4 const *x = (cb.inIsX ? X : W) + cb.inRow * R + r;
+    float4 const *x = (cb.inIsX ? X : W) + cb.inRow;
     int const n = cb.n;
     int64_t const lda = cb.lda;
     constexpr int S = kDfWarps;
@@ -125,8 +120,8 @@ applyGemvDfKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__res
       } else {
         a0 = a1 = a2 = a3 = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      float4 const x0 = x[(int64_t)(j + 0 * S) * R], x1 = x[(int64_t)(j + 1 * S) * R];
-      float4 const x2 = x[(int64_t)(j + 2 * S) * R], x3 = x[(int64_t)(j + 3 * S) * R];
+      float4 const x0 = x[j + 0 * S], x1 = x[j + 1 * S];
+      float4 const x2 = x[j + 2 * S], x3 = x[j + 3 * S];
       mac(a0, x0);
       mac(a1, x1);
       mac(a2, x2);
@@ -134,7 +129,7 @@ applyGemvDfKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__res
     }
     for (; j < n; j += S) {
       float4 const a0 = active ? a[(int64_t)j * lda] : make_float4(0.f, 0.f, 0.f, 0.f);
-      mac(a0, x[(int64_t)j * R]);
+      mac(a0, x[j]);
     }
   }
   part[warp][lane] = make_float4(rh, rl, ih, il);
@@ -150,7 +145,7 @@ applyGemvDfKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__res
     float a, b, c, d;
     fastTwoSum(sh, sl, a, b);
     fastTwoSum(th, tl, c, d);
-    W[(it.outRow + lane) * R + r] = make_float4(a, b, c, d);
+    W[it.outRow + lane] = make_float4(a, b, c, d);
   }
 }
 
@@ -159,23 +154,21 @@ __global__ void applyReduceDfKernel(int32_t const *__restrict__ rowSeg,
                                     int64_t const *__restrict__ segStart,
                                     int64_t const *__restrict__ segContrib0,
                                     int64_t const *__restrict__ segBase,
-                                    float4 const *__restrict__ W, int64_t R,
-                                    double2 *__restrict__ Y, int64_t ldy, int64_t nRows,
+                                    float4 const *__restrict__ W, double2 *__restrict__ Y,
+                                    int64_t ldy, int64_t nRows,
                                     int64_t const *__restrict__ outPerm) {
-  int64_t const total = nRows * R;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    int64_t const i = e / R, r = e % R;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nRows;
+       i += (int64_t)gridDim.x * blockDim.x) {
     int const s = rowSeg[i];
     int64_t const di = i - segStart[s];
     double sr = 0, si = 0;
     for (int64_t c = segContrib0[s]; c < segContrib0[s + 1]; ++c) {
-      float4 const v = W[(segBase[c] + di) * R + r];
+      float4 const v = W[segBase[c] + di];
       sr += (double)v.x + (double)v.y;
       si += (double)v.z + (double)v.w;
     }
     int64_t const oi = outPerm ? outPerm[i] : i;
-    Y[oi * ldy + r] = make_double2(sr, si);
+    Y[oi * ldy] = make_double2(sr, si);
   }
 }
 
@@ -193,29 +186,26 @@ cudaError_t launchArenaToDf(double2 const *a64, float4 *adf, int64_t n, cudaStre
 }
 
 cudaError_t launchGatherToDf(double2 const *X, int64_t ldx, int64_t const *perm, int64_t nRows,
-                             int64_t R, float4 *out, cudaStream_t stream) {
-  if (nRows * R == 0) return cudaSuccess;
-  gatherToDfKernel<<<gridDf(nRows * R), 256, 0, stream>>>(X, ldx, perm, nRows, R, out);
+                             float4 *out, cudaStream_t stream) {
+  if (nRows == 0) return cudaSuccess;
+  gatherToDfKernel<<<gridDf(nRows), 256, 0, stream>>>(X, ldx, perm, nRows, out);
   return cudaGetLastError();
 }
 
 cudaError_t launchApplyStageDf(ApplyItem const *items, int64_t nItems,
                                ApplyContrib const *contribs, float4 const *arena,
-                               float4 const *X, float4 *W, int64_t R, cudaStream_t stream) {
+                               float4 const *X, float4 *W, cudaStream_t stream) {
   if (nItems == 0) return cudaSuccess;
-  if (R > 65535) return cudaErrorInvalidConfiguration;   // one grid row per RHS
-  dim3 grid((unsigned)nItems, (unsigned)R);
-  applyGemvDfKernel<<<grid, 32 * kDfWarps, 0, stream>>>(items, contribs, arena, X, W, R);
+  applyGemvDfKernel<<<(unsigned)nItems, 32 * kDfWarps, 0, stream>>>(items, contribs, arena, X, W);
   return cudaGetLastError();
 }
 
 cudaError_t launchApplyReduceDf(int32_t const *rowSeg, int64_t const *segStart,
                                 int64_t const *segContrib0, int64_t const *segBase,
-                                float4 const *W, int64_t R, double2 *Y, int64_t ldy,
-                                int64_t nRows, int64_t const *outPerm, cudaStream_t stream) {
-  applyReduceDfKernel<<<gridDf(nRows * R), 256, 0, stream>>>(rowSeg, segStart, segContrib0,
-                                                             segBase, W, R, Y, ldy, nRows,
-                                                             outPerm);
+                                float4 const *W, double2 *Y, int64_t ldy, int64_t nRows,
+                                int64_t const *outPerm, cudaStream_t stream) {
+  applyReduceDfKernel<<<gridDf(nRows), 256, 0, stream>>>(rowSeg, segStart, segContrib0, segBase,
+                                                         W, Y, ldy, nRows, outPerm);
   return cudaGetLastError();
 }
 
