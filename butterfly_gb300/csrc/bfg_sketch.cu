@@ -433,7 +433,18 @@ __global__ void __launch_bounds__(512) hqrKernel(HqrDesc const *__restrict__ des
 // schedule, one warp per column pair, rotation when |<x, y>| > eps sqrt(n)
 // |x| |y|; sweeps until none rotates (cap kSketchMaxSweeps).  Then the
 // squared column norms over the first rowsDot rows.
+//
+// Bound by the FP64 pipe, where a warp instruction takes 16 clocks of the SM
+// whatever its lanes do.  A rotation's angle takes about a hundred of them
+// (square roots, divisions), more than the products of a pair of 50-row
+// columns: so a round goes in three steps -- every warp's dot products, the
+// angles of up to kJacSlots pairs with one thread a pair, the rotations --
+// and the angles cost one pair's instructions for 32 pairs.  Measured: the
+// sweeps of the re-expansions 436 -> 234 ms at 65,536 points (k = 512), 762 ->
+// 416 ms for twelve problems of up to 16,384 points, 21 -> 11 ms at 4,096.
 // ---------------------------------------------------------------------------
+constexpr int kJacPer = 8, kJacSlots = 16 * kJacPer;   // pairs a warp / a CTA of 16 warps a step
+
 template <int kMode>
 __global__ void __launch_bounds__(512) sketchJacobiKernel(JacobiDesc const *__restrict__ descs,
                                                           int32_t *status) {
@@ -448,52 +459,81 @@ __global__ void __launch_bounds__(512) sketchJacobiKernel(JacobiDesc const *__re
   int const gWarp = rank * nWarps + warp, gWarps = ctas * nWarps;
   double2 *M = d.M;
   __shared__ int sRotated;
+  // pair k nWarps + w of a step: warp w's k-th; (|x|^2, |y|^2, <x, y>), then
+  // the rotation (c, s, exp(-i phi)), c = 2 for none
+  __shared__ double4 sPair[kJacSlots];
 
   int const P = nc + (nc & 1), nPairs = P / 2;
   double const tolRot = kEpsS * sqrt((double)rd);
+  // the columns of pair pr of a round (false: the bye of an odd count)
+  auto columns = [&](int round, int pr, double2 *&ci, double2 *&cj) {
+    int i, j;
+    if (pr == 0) {
+      i = round;
+      j = P - 1;
+    } else {
+      i = round + pr;
+      if (i >= P - 1) i -= P - 1;
+      j = round - pr;
+      if (j < 0) j += P - 1;
+    }
+    ci = M + (int64_t)i * LD;
+    cj = M + (int64_t)j * LD;
+    return i < nc && j < nc;
+  };
   bool converged = nc < 2;
   for (int sweep = 0; sweep < kSketchMaxSweeps && !converged; ++sweep) {
     if (tid == 0) sRotated = 0;
     __syncthreads();
     for (int round = 0; round < P - 1; ++round) {
-      for (int pr = gWarp; pr < nPairs; pr += gWarps) {
-        int i, j;
-        if (pr == 0) {
-          i = round;
-          j = P - 1;
-        } else {
-          i = (round + pr) % (P - 1);
-          j = (round - pr + (P - 1)) % (P - 1);
+      for (int pr0 = 0; pr0 < nPairs; pr0 += gWarps * kJacPer) {
+        for (int k = 0, pr = pr0 + gWarp; k < kJacPer && pr < nPairs; ++k, pr += gWarps) {
+          double2 *ci, *cj;
+          double al = 0, be = 0, gr = 0, gi = 0;
+          if (columns(round, pr, ci, cj))
+            for (int r = lane; r < rd; r += 32) {
+              double2 const x = Mem::ld(ci + r), y = Mem::ld(cj + r);
+              al = fma(x.x, x.x, fma(x.y, x.y, al));
+              be = fma(y.x, y.x, fma(y.y, y.y, be));
+              gr = fma(x.x, y.x, fma(x.y, y.y, gr));
+              gi = fma(x.x, y.y, fma(-x.y, y.x, gi));
+            }
+          // (a bye's zeros do not rotate)
+          double const v = warpSum4(al, be, gr, gi);
+          if ((lane & 7) == 0)
+            reinterpret_cast<double *>(sPair + k * nWarps + warp)[lane >> 3] = v;
         }
-        if (i >= nc || j >= nc) continue;
-        double2 *ci = M + (int64_t)i * LD, *cj = M + (int64_t)j * LD;
-        double al = 0, be = 0, gr = 0, gi = 0;
-        for (int r = lane; r < rd; r += 32) {
-          double2 const x = Mem::ld(ci + r), y = Mem::ld(cj + r);
-          al = fma(x.x, x.x, fma(x.y, x.y, al));
-          be = fma(y.x, y.x, fma(y.y, y.y, be));
-          gr = fma(x.x, y.x, fma(x.y, y.y, gr));
-          gi = fma(x.x, y.y, fma(-x.y, y.x, gi));
+        __syncthreads();
+        int const left = nPairs - pr0 - rank * nWarps;   // pairs from this CTA's first on
+        for (int q = tid; q < kJacPer * nWarps; q += nthr) {
+          if ((q / nWarps) * gWarps + q % nWarps >= left) continue;
+          double const al = sPair[q].x, be = sPair[q].y, gr = sPair[q].z, gi = sPair[q].w;
+          double4 rot = make_double4(2.0, 0.0, 0.0, 0.0);
+          double const ag = sqrt(gr * gr + gi * gi);
+          if (ag > tolRot * sqrt(al * be) && ag > 0.0) {
+            double const zeta = (be - al) / (2.0 * ag);
+            double const t = (zeta >= 0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+            double const c = 1.0 / sqrt(1.0 + t * t);
+            rot = make_double4(c, c * t, gr / ag, -gi / ag);
+            sRotated = 1;
+          }
+          sPair[q] = rot;
         }
-        al = warpSum(al);
-        be = warpSum(be);
-        gr = warpSum(gr);
-        gi = warpSum(gi);
-        double const ag = sqrt(gr * gr + gi * gi);
-        if (ag > tolRot * sqrt(al * be) && ag > 0.0) {
-          double const zeta = (be - al) / (2.0 * ag);
-          double const t = (zeta >= 0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-          double const c = 1.0 / sqrt(1.0 + t * t), s = c * t;
-          double const er = gr / ag, ei = -gi / ag;
-          __syncwarp();
+        __syncthreads();
+        for (int k = 0, pr = pr0 + gWarp; k < kJacPer && pr < nPairs; ++k, pr += gWarps) {
+          double4 const rot = sPair[k * nWarps + warp];
+          if (rot.x > 1.5) continue;
+          double const c = rot.x, s = rot.y, er = rot.z, ei = rot.w;
+          double2 *ci, *cj;
+          columns(round, pr, ci, cj);
           for (int r = lane; r < LD; r += 32) {
             double2 const x = Mem::ld(ci + r), y = Mem::ld(cj + r);
             double const ytr = y.x * er - y.y * ei, yti = y.x * ei + y.y * er;
             Mem::st(ci + r, make_double2(c * x.x - s * ytr, c * x.y - s * yti));
             Mem::st(cj + r, make_double2(s * x.x + c * ytr, s * x.y + c * yti));
           }
-          if (lane == 0) sRotated = 1;
         }
+        if (pr0 + gWarps * kJacPer < nPairs) __syncthreads();   // sPair is rewritten
       }
       Mem::sync();
     }
