@@ -214,18 +214,8 @@ __global__ void __launch_bounds__(kFixThreads, NT == 1 ? 3 : 2) fixTileKernel(
     for (int u = 0; u < NT; ++u) {
       int const ex = fixScaleOf(__shfl_sync(0xffffffffu, code, 4 * u + t));
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        int v[kFixSums];
-#pragma unroll
-        for (int s = 0; s < kFixSums; ++s) {
-          v[s] = __float2int_rn(sum[u][s][r]);
-          sum[u][s][r] = 0.f;
-        }
-        int64_t const V = ((int64_t)v[0] << 40) + ((int64_t)v[1] << 32) + ((int64_t)v[2] << 24) +
-                          ((int64_t)v[3] << 16) + ((int64_t)v[4] << 8) +
-                          (v[5] + ((v[6] + (v[7] >> 8) + 128) >> 8));
-        acc[u][r] = fma((double)V, fixScale((r < 2 ? ea0 : ea1) + ex), acc[u][r]);
-      }
+      for (int r = 0; r < 4; ++r)
+        acc[u][r] = fma((double)fixTake(sum[u], r), fixScale((r < 2 ? ea0 : ea1) + ex), acc[u][r]);
     }
     steps = 0;
   };

@@ -107,6 +107,20 @@ __device__ __forceinline__ void fixSplit(double2 v, int E, uint32_t (&d)[kFixDig
   }
 }
 
+// the exact sum put together from the digit sums' element r, in units of 2^56
+// (rounded), which are cleared
+__device__ __forceinline__ int64_t fixTake(float (&sum)[kFixSums][4], int r) {
+  int v[kFixSums];
+#pragma unroll
+  for (int s = 0; s < kFixSums; ++s) {
+    v[s] = __float2int_rn(sum[s][r]);
+    sum[s][r] = 0.f;
+  }
+  return ((int64_t)v[0] << 40) + ((int64_t)v[1] << 32) + ((int64_t)v[2] << 24) +
+         ((int64_t)v[3] << 16) + ((int64_t)v[4] << 8) +
+         (v[5] + ((v[6] + (v[7] >> 8) + 128) >> 8));
+}
+
 // D += A B, 16 x 8 x 16, halves in, FP32 sums (of integers: exact)
 __device__ __forceinline__ void fixMma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                        uint32_t a3, uint32_t b0, uint32_t b1) {

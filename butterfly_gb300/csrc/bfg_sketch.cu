@@ -12,7 +12,8 @@
 // reference's SVD spends O(p^3) on directions that the pseudo-inverse cut
 // then drops.  This path spends its work on the numerical rank instead
 // (a randomized range finder; Halko, Martinsson and Tropp, SIAM Review 53,
-// 2011, algorithms 4.1 and 5.1), in FP64 throughout:
+// 2011, algorithms 4.1 and 5.1), in FP64 precision throughout
+// (the products by exact digit sums, bfg_fixed.cuh):
 //
 //   Y  = Z_equiv Omega        Omega p x l with iid complex Gaussian entries
 //   Q  = qr(Y)                Householder (explicit Q, p x l)
@@ -42,6 +43,7 @@
 #include <vector>
 
 #include "bfg_device.cuh"
+#include "bfg_fixed.cuh"
 #include "bfg_kernels.cuh"
 
 namespace bfg {
@@ -51,7 +53,7 @@ namespace {
 constexpr double kEpsS = 2.220446049250313e-16;
 constexpr int kSketchMaxSweeps = 60;
 constexpr int kSketchCluster = 8;      // CTAs per block in cluster mode
-constexpr int kGT = 64, kGK = 16;      // GEMM tile and K chunk
+constexpr int kGM = 64, kGN = 32;      // GEMM tile
 constexpr int kFillTile = 16384;       // entries per fill CTA
 
 // one block of the randomized path, as the kernels read it (offsets in
@@ -78,6 +80,7 @@ struct GemmDesc {
   int64_t lda, ldb, ldc;
   int32_t M, N, K, opA;     // opA 0: A is M x K; 1: C = A^H B with A stored K x M
   double const *colScale;   // optional: column j of C scaled by colScale[j]
+  int16_t *rowCode, *colCode;   // scale codes of op(A)'s rows and B's columns (set at launch)
 };
 
 struct HqrDesc {
@@ -208,78 +211,191 @@ __global__ void __launch_bounds__(256) sketchFillKernel(SketchDev const *__restr
 }
 
 // ---------------------------------------------------------------------------
-// Batched complex FP64 GEMM, C = diag(rowScale) op(A) B, one 64 x 64 tile
-// per CTA (tiles of all problems in one launch).  16 x 16 threads, each a
-// 4 x 4 register tile (rows ty + 16 r, columns tx + 16 c); A and B staged
-// through shared memory in chunks of 16 along K.  GB300's FP64 units (about
-// 2 FMA per clock per SM) bound it; the staging is not the limit.
+// Batched complex FP64 GEMM, C = diag(rowScale) op(A) B diag(colScale), one
+// 64 x 32 tile per CTA (tiles of all problems in one launch), the products
+// formed from integer digits on the tensor cores (bfg_fixed.cuh).  A row of
+// op(A) and a column of B have one scale each (gemmCodeKernel, one pass over
+// the operands); a tile that meets a row or column without one (NaN,
+// infinities, subnormals) is summed in plain FP64.
+//
+// 8 warps: four 16-row tiles times two groups of 16 columns.  Per k-step of 8:
+// each thread splits two entries of A and one of B into shared memory in the
+// fragments' order -- while the MMAs of the step before run from the other
+// buffer -- and fetches the ones after.  34 MMAs of 16 x 8 x 16 per four
+// columns; the exact sums go to FP64 every fixMaxSteps k-steps.
+// Bound by the tensor pipe and by splitting the entries.  Measured, against the
+// FP64-FMA form (64 x 64 tiles, FP64 pipe 99.9 % busy): all products of the
+// 65,536-point factorization 296 -> 52 ms (the output products 225 -> 41), of
+// twelve problems of up to 16,384 points 257 -> 45 ms.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) zgemmKernel(GemmDesc const *__restrict__ descs,
-                                                   int4 const *__restrict__ tiles) {
+constexpr int kGemmStageWords = kFixDigits * (4 * 32 * 4 + 8 * 32 * 2);
+
+__device__ __forceinline__ double2 gemmA(GemmDesc const &g, int i, int k) {
+  if (i >= g.M || k >= g.K) return make_double2(0.0, 0.0);
+  return g.opA == 0 ? g.A[i + (int64_t)k * g.lda] : conjD(g.A[k + (int64_t)i * g.lda]);
+}
+__device__ __forceinline__ double2 gemmB(GemmDesc const &g, int k, int j) {
+  return (j < g.N && k < g.K) ? g.B[k + (int64_t)j * g.ldb] : make_double2(0.0, 0.0);
+}
+
+// scale codes of 64 rows of op(A) (what 0) or of 64 columns of B (what 1):
+// tile (desc, what, first row or column)
+__global__ void __launch_bounds__(256) gemmCodeKernel(GemmDesc const *__restrict__ descs,
+                                                      int4 const *__restrict__ tiles) {
   int4 const t = tiles[blockIdx.x];
   GemmDesc const g = descs[t.x];
-  int const i0 = t.y * kGT, j0 = t.z * kGT;
-  __shared__ double2 As[kGK][kGT + 1];
-  __shared__ double2 Bs[kGK][kGT + 1];
-  int const tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  double2 acc[4][4];
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc[r][c] = make_double2(0.0, 0.0);
-  for (int k0 = 0; k0 < g.K; k0 += kGK) {
-    if (g.opA == 0) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        int const i = tid & 63, kk = (tid >> 6) + 4 * q;
-        int const gi = i0 + i, gk = k0 + kk;
-        As[kk][i] = (gi < g.M && gk < g.K) ? g.A[gi + (int64_t)gk * g.lda] : make_double2(0.0, 0.0);
-      }
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        int const kk = tid & 15, i = (tid >> 4) + 16 * q;
-        int const gi = i0 + i, gk = k0 + kk;
-        As[kk][i] = (gi < g.M && gk < g.K) ? conjD(g.A[gk + (int64_t)gi * g.lda])
-                                           : make_double2(0.0, 0.0);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      int const kk = tid & 15, j = (tid >> 4) + 16 * q;
-      int const gj = j0 + j, gk = k0 + kk;
-      Bs[kk][j] = (gj < g.N && gk < g.K) ? g.B[gk + (int64_t)gj * g.ldb] : make_double2(0.0, 0.0);
-    }
+  int const tid = threadIdx.x;
+  if (t.y == 0 && g.opA == 0) {   // along the stored rows: 64 rows, 4 column slices
+    __shared__ int red[4][64];
+    int const i = t.z + (tid & 63);
+    int code = 0;
+    for (int k = tid >> 6; k < g.K; k += 4) code = max(code, fixCode(gemmA(g, i, k)));
+    red[tid >> 6][tid & 63] = code;
     __syncthreads();
-#pragma unroll 4
-    for (int kk = 0; kk < kGK; ++kk) {
-      double2 a[4], b[4];
+    if (tid < 64 && i < g.M)
+      g.rowCode[i] = (int16_t)fixScaleOf(
+          max(max(red[0][tid], red[1][tid]), max(red[2][tid], red[3][tid])));
+    return;
+  }
+  int const lane = tid & 31, n = t.y == 0 ? g.M : g.N;
+  double2 const *p = t.y == 0 ? g.A : g.B;
+  int64_t const ld = t.y == 0 ? g.lda : g.ldb;
+  for (int q = tid >> 5; q < 64 && t.z + q < n; q += 8) {   // a stored column per warp
+    int code = 0;
+    for (int k = lane; k < g.K; k += 32) code = max(code, fixCode(p[k + (t.z + q) * ld]));
+    code = __reduce_max_sync(0xffffffffu, code);
+    if (lane == 0) (t.y == 0 ? g.rowCode : g.colCode)[t.z + q] = (int16_t)fixScaleOf(code);
+  }
+}
+
+__global__ void __launch_bounds__(256, 1) zgemmKernel(GemmDesc const *__restrict__ descs,
+                                                      int4 const *__restrict__ tiles) {
+  constexpr int D = kFixDigits;
+  extern __shared__ __align__(16) uint32_t gemmSmem[];   // two stages
+  __shared__ int16_t sRow[kGM], sCol[kGN];
+  int4 const tile = tiles[blockIdx.x];
+  GemmDesc const g = descs[tile.x];
+  int const i0 = tile.y * kGM, j0 = tile.z * kGN;
+  int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t = lane & 3, gr = lane >> 2;
+  int const mt = warp & 3, nh = warp >> 2;
+  if (tid < kGM) sRow[tid] = i0 + tid < g.M ? g.rowCode[i0 + tid] : 1023;
+  if (tid >= 64 && tid < 64 + kGN) sCol[tid - 64] = j0 + tid - 64 < g.N ? g.colCode[j0 + tid - 64] : 1023;
+  __syncthreads();
+  bool covered = true;
+  for (int e = tid; e < kGM * kGN; e += 256)
+    covered = covered && fixCovers(sRow[e % kGM], sRow[e % kGM], sCol[e / kGM]);
+  bool const plain = __syncthreads_or(!covered);
+
+  // this lane's results: rows 16 mt + gr, + 8; columns 16 nh + 4 u + t
+  double acc[4][4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) a[r] = As[kk][ty + 16 * r];
+  for (int u = 0; u < 4; ++u)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) b[c] = Bs[kk][tx + 16 * c];
+    for (int r = 0; r < 4; ++r) acc[u][r] = 0.0;
+
+  if (!plain) {
+    float sum[4][kFixSums][4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
+    for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          acc[r][c].x = fma(a[r].x, b[c].x, fma(-a[r].y, b[c].y, acc[r][c].x));
-          acc[r][c].y = fma(a[r].x, b[c].y, fma(a[r].y, b[c].x, acc[r][c].y));
-        }
+      for (int s = 0; s < kFixSums; ++s)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) sum[u][s][r] = 0.f;
+    // the entries this thread splits: of A, row 16 (warp / 2) + gr + 8 h with
+    // h = warp % 2 at columns t and t + 4; of B, columns 8 (warp / 2) + gr at
+    // row t + 4 h
+    int const h = warp & 1, ra = 16 * (warp >> 1) + gr + 8 * h, cb = 8 * (warp >> 1) + gr;
+    int const ea = sRow[ra], eb = sCol[cb];
+    double2 a0, a1, b0;
+    auto fetch = [&](int k0) {
+      a0 = gemmA(g, i0 + ra, k0 + t);
+      a1 = gemmA(g, i0 + ra, k0 + t + 4);
+      b0 = gemmB(g, k0 + t + 4 * h, j0 + cb);
+    };
+    // A: word ((digit 4 + row tile) 32 + lane) 4 + register (register h of
+    // column t, 2 + h of t + 4); B: word ((digit 8 + n tile) 32 + lane) 2 +
+    // register
+    auto put = [&](uint32_t *sA) {
+      uint32_t *sB = sA + D * 4 * 32 * 4;
+      uint32_t d[D];
+      fixSplit(a0, ea, d);
+      uint32_t *p = sA + ((warp >> 1) * 32 + lane) * 4 + h;
+#pragma unroll
+      for (int q = 0; q < D; ++q) p[q * 512] = d[q];
+      fixSplit(a1, ea, d);
+#pragma unroll
+      for (int q = 0; q < D; ++q) p[q * 512 + 2] = d[q];
+      fixSplit(b0, eb, d);
+      p = sB + ((cb >> 2) * 32 + 8 * (cb & 3) + t) * 2 + h;
+#pragma unroll
+      for (int q = 0; q < D; ++q) {
+        p[q * 512] = d[q] ^ 0x80000000u;              // (Re b, -Im b)
+        p[q * 512 + 8] = __byte_perm(d[q], 0, 0x1032);   // (Im b, Re b)
+      }
+    };
+    int const ea0 = sRow[16 * mt + gr], ea1 = sRow[16 * mt + gr + 8];
+    auto flush = [&]() {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        int const ec = sCol[16 * nh + 4 * u + t];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          acc[u][r] = fma((double)fixTake(sum[u], r), fixScale((r < 2 ? ea0 : ea1) + ec), acc[u][r]);
+      }
+    };
+    fetch(0);
+    put(gemmSmem);
+    fetch(8);
+    int buf = 0, steps = 0;
+    for (int k0 = 0; k0 < g.K; k0 += 8, buf ^= 1) {
+      __syncthreads();
+      if (k0 + 8 < g.K) {
+        put(gemmSmem + (buf ^ 1) * kGemmStageWords);
+        if (k0 + 16 < g.K) fetch(k0 + 16);
+      }
+      uint4 const *sA = reinterpret_cast<uint4 const *>(gemmSmem + buf * kGemmStageWords) +
+                        mt * 32 + lane;
+      uint2 const *sB = reinterpret_cast<uint2 const *>(gemmSmem + buf * kGemmStageWords +
+                                                        D * 4 * 32 * 4) + nh * 4 * 32 + lane;
+#pragma unroll
+      for (int i = 0; i < D; ++i) {
+        uint4 const a = sA[i * 128];
+#pragma unroll
+        for (int j = 0; j < D && i + j < kFixSums; ++j)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            uint2 const b = sB[(j * 8 + u) * 32];
+            fixMma(sum[u][i + j], a.x, a.y, a.z, a.w, b.x, b.y);
+          }
+      }
+      if (++steps == fixMaxSteps(false)) {
+        flush();
+        steps = 0;
+      }
     }
-    __syncthreads();
+    if (steps > 0) flush();
+  } else {
+    for (int k = 0; k < g.K; ++k) {
+      double2 const x0 = gemmA(g, i0 + 16 * mt + gr, k), x1 = gemmA(g, i0 + 16 * mt + gr + 8, k);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        double2 const y = gemmB(g, k, j0 + 16 * nh + 4 * u + t);
+        cmacc(acc[u][0], acc[u][1], x0, y);
+        cmacc(acc[u][2], acc[u][3], x1, y);
+      }
+    }
   }
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    int const gi = i0 + ty + 16 * r;
-    if (gi >= g.M) continue;
-    double const sc = g.rowScale ? g.rowScale[gi] : 1.0;
+  for (int u = 0; u < 4; ++u) {
+    int const j = j0 + 16 * nh + 4 * u + t;
+    if (j >= g.N) continue;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      int const gj = j0 + tx + 16 * c;
-      if (gj < g.N) {
-        double const scc = g.colScale ? sc * g.colScale[gj] : sc;
-        g.C[gi + (int64_t)gj * g.ldc] = make_double2(scc * acc[r][c].x, scc * acc[r][c].y);
-      }
+    for (int r = 0; r < 2; ++r) {
+      int const i = i0 + 16 * mt + gr + 8 * r;
+      if (i >= g.M) continue;
+      double const sc = g.rowScale ? g.rowScale[i] : 1.0;
+      double const scc = g.colScale ? sc * g.colScale[j] : sc;
+      g.C[i + (int64_t)j * g.ldc] = make_double2(scc * acc[u][2 * r], scc * acc[u][2 * r + 1]);
     }
   }
 }
@@ -638,32 +754,56 @@ uint64_t splitmixHost(uint64_t x) {
 bool hqrCluster(int64_t p, int64_t l) { return p * l >= (int64_t)1 << 17; }
 bool jacobiCluster(int64_t l) { return l >= 160; }
 
-cudaError_t launchGemms(std::vector<GemmDesc> const &g, Buf &dDesc, Buf &dTiles,
-                        cudaStream_t s) {
+// device buffers of the GEMM launches, reused from one to the next
+struct GemmBufs {
+  Buf desc, tiles, code;
+};
+
+cudaError_t launchGemms(std::vector<GemmDesc> &g, GemmBufs &b, cudaStream_t s) {
   if (g.empty()) return cudaSuccess;
+  int64_t codes = 0;
+  for (GemmDesc const &d : g) codes += d.M + d.N;
+  cudaError_t e = b.code.ensure((size_t)std::max<int64_t>(1, codes) * sizeof(int16_t));
+  if (e != cudaSuccess) return e;
+  int16_t *code = static_cast<int16_t *>(b.code.p);
+  for (GemmDesc &d : g) {
+    d.rowCode = code;
+    d.colCode = code + d.M;
+    code += d.M + d.N;
+  }
+  // the scale codes' tiles, then the products': longest K first, so that the
+  // longest tiles start in the first wave
   std::vector<int4> tiles;
-  // longest K first, so that the longest tiles start in the first wave
   std::vector<int> order(g.size());
   for (size_t i = 0; i < g.size(); ++i) order[i] = (int)i;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return g[a].K > g[b].K; });
+  std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return g[a].K > g[c].K; });
   for (int i : order) {
-    int const tm = (g[i].M + kGT - 1) / kGT, tn = (g[i].N + kGT - 1) / kGT;
+    for (int a = 0; a < g[i].M; a += 64) tiles.push_back(make_int4(i, 0, a, 0));
+    for (int a = 0; a < g[i].N; a += 64) tiles.push_back(make_int4(i, 1, a, 0));
+  }
+  size_t const nCode = tiles.size();
+  for (int i : order) {
+    int const tm = (g[i].M + kGM - 1) / kGM, tn = (g[i].N + kGN - 1) / kGN;
     for (int a = 0; a < tm; ++a)
       for (int c = 0; c < tn; ++c) tiles.push_back(make_int4(i, a, c, 0));
   }
-  if (tiles.empty()) return cudaSuccess;
-  cudaError_t e = put(dDesc, g, s);
-  if (e != cudaSuccess) return e;
-  e = put(dTiles, tiles, s);
+  if (tiles.size() == nCode) return cudaSuccess;
+  if ((e = put(b.desc, g, s)) != cudaSuccess) return e;
+  if ((e = put(b.tiles, tiles, s)) != cudaSuccess) return e;
+  GemmDesc const *desc = static_cast<GemmDesc const *>(b.desc.p);
+  int4 const *dt = static_cast<int4 const *>(b.tiles.p);
+  constexpr int smem = 2 * kGemmStageWords * (int)sizeof(uint32_t);
+  e = cudaFuncSetAttribute(zgemmKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   // grids are limited to 2^31 - 1 CTAs in x; one launch per 2^30 tiles
   size_t const step = (size_t)1 << 30;
-  for (size_t t0 = 0; t0 < tiles.size(); t0 += step) {
-    size_t const cnt = std::min(step, tiles.size() - t0);
-    zgemmKernel<<<(unsigned)cnt, 256, 0, s>>>(static_cast<GemmDesc const *>(dDesc.p),
-                                              static_cast<int4 const *>(dTiles.p) + t0);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+  for (size_t t0 = 0; t0 < nCode; t0 += step) {
+    gemmCodeKernel<<<(unsigned)std::min(step, nCode - t0), 256, 0, s>>>(desc, dt + t0);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  for (size_t t0 = nCode; t0 < tiles.size(); t0 += step) {
+    zgemmKernel<<<(unsigned)std::min(step, tiles.size() - t0), 256, smem, s>>>(desc, dt + t0);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
@@ -795,7 +935,8 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
   };
   std::stable_sort(queue.begin(), queue.end(),
                    [&](Group const &a, Group const &b) { return cost(a) > cost(b); });
-  Buf scratch, dBlk, dTiles, dDesc, dHqr1, dHqr2, dJac1, dJac2, dW, dFail, dStatus;
+  GemmBufs gemmBufs;
+  Buf scratch, dBlk, dTiles, dHqr1, dHqr2, dJac1, dJac2, dW, dFail, dStatus;
   err = dStatus.ensure(sizeof(int32_t));
   if (err != cudaSuccess) return err;
   err = cudaMemsetAsync(dStatus.p, 0, sizeof(int32_t), s);
@@ -901,7 +1042,7 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
     std::vector<GemmDesc> g;
     for (auto const &b : blks)
       g.push_back(GemmDesc{S + b.oZ, S + b.oB0, S + b.oB1, nullptr, b.p, b.p, b.p, b.p, b.l, b.p, 0});
-    if ((err = launchGemms(g, dDesc, dTiles, s)) != cudaSuccess) return err;
+    if ((err = launchGemms(g, gemmBufs, s)) != cudaSuccess) return err;
     // Q = qr(Y) into B0
     mark(2);
     std::vector<HqrDesc> h1, h2;
@@ -916,7 +1057,7 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
     g.clear();
     for (auto const &b : blks)
       g.push_back(GemmDesc{S + b.oZ, S + b.oB0, S + b.oB1, nullptr, b.p, b.p, b.p, b.p, b.l, b.p, 1});
-    if ((err = launchGemms(g, dDesc, dTiles, s)) != cudaSuccess) return err;
+    if ((err = launchGemms(g, gemmBufs, s)) != cudaSuccess) return err;
     // G = Q2 R2: Q2 into B2, [R2^H ; I] into M
     mark(4);
     h1.clear();
@@ -1024,12 +1165,12 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
       rep->sumWidth += b.l;
     }
     mark(7);
-    if ((err = launchGemms(gE, dDesc, dTiles, s)) != cudaSuccess) return err;
-    if ((err = launchGemms(gF, dDesc, dTiles, s)) != cudaSuccess) return err;
-    if ((err = launchGemms(gc, dDesc, dTiles, s)) != cudaSuccess) return err;
-    if ((err = launchGemms(gd, dDesc, dTiles, s)) != cudaSuccess) return err;
-    if ((err = launchGemms(ge, dDesc, dTiles, s)) != cudaSuccess) return err;
-    if ((err = launchGemms(gx, dDesc, dTiles, s)) != cudaSuccess) return err;
+    if ((err = launchGemms(gE, gemmBufs, s)) != cudaSuccess) return err;
+    if ((err = launchGemms(gF, gemmBufs, s)) != cudaSuccess) return err;
+    if ((err = launchGemms(gc, gemmBufs, s)) != cudaSuccess) return err;
+    if ((err = launchGemms(gd, gemmBufs, s)) != cudaSuccess) return err;
+    if ((err = launchGemms(ge, gemmBufs, s)) != cudaSuccess) return err;
+    if ((err = launchGemms(gx, gemmBufs, s)) != cudaSuccess) return err;
     mark(8);
     // descriptors and scratch are reused by the next batch
     if ((err = cudaStreamSynchronize(s)) != cudaSuccess) return err;

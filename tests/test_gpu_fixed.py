@@ -103,3 +103,21 @@ def test_infinities_and_nans_reach_the_rows_they_meet(R):
         others = np.arange(R) != R // 2
         assert np.all(np.abs(y[:, others].astype(LD) - Y[:, others]) <= bound[:, others])
     assert np.array_equal(_apply(fac, X.copy()), clean)
+
+
+# ranks (and so the products' sizes) below, at and above the 32-column and
+# 64-row tiles and the 64-row flush interval of the factorization's products
+@pytest.mark.parametrize("k", [12.0, 25.0, 41.0, 60.0, 97.0])
+def test_factorization_products_match_the_full_path(k):
+    """The operators of the randomized path, whose products the digits form,
+    and of the full path, which uses none (the bound of the sketch tests)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    n = 2500
+    src, tgt = B.uniform_square_points(n, 11), B.curve_points("star", n)
+    X = torch.from_numpy(B.Rng(3).complex_randn(2 * n).reshape(n, 2)).cuda()
+    y = [B.FacHelm2.make_multilevel(B.Helm2(k), B.Quadtree(src, leaf_size=32),
+                                    B.Quadtree(tgt, leaf_size=32), rank_eps=1e-10, pinv_tol=1e-10,
+                                    sketch=s, context=B.default_context(0)).apply(X)
+         for s in (True, False)]
+    assert torch.linalg.norm(y[0] - y[1]) < 2e-9 * torch.linalg.norm(y[1])
