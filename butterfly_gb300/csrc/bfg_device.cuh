@@ -15,13 +15,21 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
+// |(dx, dy)|; the plain form where no square over- or underflows takes half
+// the FP64 instructions of hypot
+__device__ __forceinline__ double planeDistance(double dx, double dy) {
+  double const r2 = fma(dx, dx, dy * dy);
+  if (r2 > 1e-280 && r2 < 1e280) return sqrt(r2);
+  return hypot(dx, dy);
+}
+
 // Kernel value K(x_tgt, x_src) for the layer potential in kp (helm2.c:38-91;
 // matrix fills return 0 at r == 0, helm2.c:114, 159-160, 207, 255).
 __device__ __forceinline__ double2 kernelValue(KernelParams const &kp, double tx,
                                                double ty, double tnx, double tny,
                                                double sx, double sy, double snx,
                                                double sny) {
-  double const r = hypot(sx - tx, sy - ty);
+  double const r = planeDistance(sx - tx, sy - ty);
   if (r == 0.0) return make_double2(0.0, 0.0);
   double const kr = kp.k * r;
   if (kp.layerPot == kLpSingle) {

@@ -235,7 +235,7 @@ __device__ int reexpScaleExp(int eTop, int p, int32_t *clusterFlags, int rank) {
 // blocks are members[groupStart[blk] .. groupStart[blk + 1]), each of which
 // gets its own Z_shift from the one pseudo-inverse.
 template <int kMode, bool kDf>
-__global__ void __launch_bounds__(512) reexpansionKernel(
+__global__ void __launch_bounds__(512, kMode == 0 ? 2 : 1) reexpansionKernel(
     FillDesc const *__restrict__ descs, PointsDev src, KernelParams kp, int32_t cutMode,
     double cutTol, double2 *arena, double2 *scratch, int64_t const *scratchOff,
     int32_t *flags, int32_t *status, FillDesc const *__restrict__ members,

@@ -65,6 +65,7 @@ struct SketchDev {
   double k;
   uint64_t seed;
   int64_t oZ, oB0, oB1, oB2, oM, oZo, oC, oD, oTau, oSW, oFlags;
+  int64_t oT, oTo;   // unit circles: p points, and (MIDDLE) the n source points
 };
 
 struct FillTileDesc {
@@ -162,6 +163,24 @@ __device__ __forceinline__ double2 conjD(double2 a) { return make_double2(a.x, -
 // (2 pi / p) a on the check and equivalent circles, (2 pi / n) b on the
 // source-child circle of a MIDDLE block.
 // ---------------------------------------------------------------------------
+// (cos, sin) of theta_a = (2 pi / p) a of every group (blocks 0 .. nGroups-1)
+// and of (2 pi / n) b of every MIDDLE member: one sincos a point, not one for
+// both points of every entry
+__global__ void __launch_bounds__(256) sketchCircleKernel(SketchDev const *__restrict__ blks,
+                                                          int nGroups, double2 *scratch) {
+  SketchDev const b = blks[blockIdx.x];
+  bool const group = (int)blockIdx.x < nGroups;
+  if (!group && b.kind == kFirst) return;
+  int const n = group ? b.p : b.n;
+  double2 *out = scratch + (group ? b.oT : b.oTo);
+  double const scale = kTwoPiDev / (double)n;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    double s, c;
+    sincos(scale * i, &s, &c);
+    out[i] = make_double2(c, s);
+  }
+}
+
 __global__ void __launch_bounds__(256) sketchFillKernel(SketchDev const *__restrict__ blks,
                                                         FillTileDesc const *__restrict__ tiles,
                                                         PointsDev src, KernelParams kp,
@@ -170,9 +189,9 @@ __global__ void __launch_bounds__(256) sketchFillKernel(SketchDev const *__restr
   SketchDev const b = blks[t.blk];
   kp.k = b.k;
   int const p = b.p;
-  double const scaleP = kTwoPiDev / (double)p;
   bool const useSrcN = kp.layerPot == kLpPvDouble || kp.layerPot == kLpCombinedField;
   double2 *out = scratch + (t.what == 0 ? b.oZ : t.what == 1 ? b.oB0 : b.oZo);
+  double2 const *circ = scratch + b.oT, *circo = scratch + b.oTo;
   for (int q = threadIdx.x; q < t.cnt; q += blockDim.x) {
     int64_t const e = t.e0 + q;
     if (t.what == 1) {
@@ -181,30 +200,22 @@ __global__ void __launch_bounds__(256) sketchFillKernel(SketchDev const *__restr
     }
     int const i = (int)(e % p);
     int64_t const j = e / p;
-    double s, c;
-    sincos(scaleP * i, &s, &c);
-    double const tx = b.cchk[2] * c + b.cchk[0], ty = b.cchk[2] * s + b.cchk[1];
+    double2 const u = circ[i];
+    double const tx = b.cchk[2] * u.x + b.cchk[0], ty = b.cchk[2] * u.y + b.cchk[1];
     double sx, sy, snx, sny;
-    if (t.what == 0) {
-      double s2, c2;
-      sincos(scaleP * (int)j, &s2, &c2);
-      sx = b.ceq[2] * c2 + b.ceq[0];
-      sy = b.ceq[2] * s2 + b.ceq[1];
-      snx = c2;
-      sny = s2;
-    } else if (b.kind == kFirst) {
+    if (t.what == 0 || b.kind != kFirst) {
+      double2 const v = t.what == 0 ? circ[j] : circo[j];
+      double const *cc = t.what == 0 ? b.ceq : b.corig;
+      sx = cc[2] * v.x + cc[0];
+      sy = cc[2] * v.y + cc[1];
+      snx = v.x;
+      sny = v.y;
+    } else {
       int64_t const sj = b.s0 + j;
       sx = src.x[sj];
       sy = src.y[sj];
       snx = (useSrcN && src.nx) ? src.nx[sj] : 0.0;
       sny = (useSrcN && src.ny) ? src.ny[sj] : 0.0;
-    } else {
-      double s2, c2;
-      sincos((kTwoPiDev / (double)b.n) * (int)j, &s2, &c2);
-      sx = b.corig[2] * c2 + b.corig[0];
-      sy = b.corig[2] * s2 + b.corig[1];
-      snx = c2;
-      sny = s2;
     }
     out[e] = kernelValue(kp, tx, ty, 0.0, 0.0, sx, sy, snx, sny);
   }
@@ -957,8 +968,8 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
     while (q1 < queue.size()) {
       Group const &gr = queue[q1];
       int64_t const p = gr.mem[0].m, l = gr.l;
-      int64_t e = p * p + 3 * p * l + 2 * l * l + l + l + 4;
-      for (auto const &d : gr.mem) e += p * d.n + 2 * l * d.n;
+      int64_t e = p * p + 3 * p * l + 2 * l * l + l + l + 4 + p;
+      for (auto const &d : gr.mem) e += p * d.n + 2 * l * d.n + d.n;
       if (q1 > q0 && total + e > budgetEntries) break;
       FillDesc const &d0 = gr.mem[0];
       SketchDev b{};
@@ -984,6 +995,7 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
       b.oTau = o; o += l;
       b.oSW = o; o += l;
       b.oFlags = o; o += 4;
+      b.oT = o; o += p;
       for (auto const &d : gr.mem) {
         SketchDev m = b;
         m.kind = d.kind;
@@ -994,6 +1006,7 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
         m.oZo = o; o += p * d.n;
         m.oC = o; o += l * d.n;
         m.oD = o; o += l * d.n;
+        m.oTo = o; o += d.n;
         mems.push_back(m);
         memberOf.push_back(blks.size());
       }
@@ -1029,6 +1042,9 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
       addTiles(nb + i, 2, (int64_t)mems[i].p * mems[i].n);
     if ((err = put(dBlk, descs, s)) != cudaSuccess) return err;
     if ((err = put(dTiles, tiles, s)) != cudaSuccess) return err;
+    sketchCircleKernel<<<(unsigned)descs.size(), 256, 0, s>>>(static_cast<SketchDev const *>(dBlk.p),
+                                                              (int)nb, S);
+    if ((err = cudaGetLastError()) != cudaSuccess) return err;
     for (size_t t0 = 0; t0 < tiles.size(); t0 += ((size_t)1 << 30)) {
       size_t const cnt = std::min<size_t>((size_t)1 << 30, tiles.size() - t0);
       sketchFillKernel<<<(unsigned)cnt, 256, 0, s>>>(

@@ -15,11 +15,18 @@
 //                       derivative of that series.
 //   otherwise           Hankel's asymptotic expansion (A&S 9.2.5-9.2.10):
 //                       H_nu(x) ~ sqrt(2/(pi x)) (P + i Q) exp(i chi),
-//                       chi = x - (nu/2 + 1/4) pi, with the terms
-//                       t_k = t_{k-1} (4 nu^2 - (2k-1)^2) / (8 k x) summed
-//                       until they fall below 1e-17.  exp(i chi) is formed
+//                       chi = x - (nu/2 + 1/4) pi, P and Q polynomials in
+//                       1/x^2 with the coefficients
+//                       a_k = a_{k-1} (4 nu^2 - (2k-1)^2) / (8 k), as many as
+//                       lie above 1e-17 at x.  exp(i chi) is formed
 //                       from sincos(x) and the exact rotation by pi/4 or
 //                       3 pi/4, so no rounding of x - chi enters.
+//
+// GB300's FP64 pipe (2 lanes a clock and SM) bounds every kernel that
+// evaluates these, so the coefficients of both the expansion and the
+// recurrence are compile-time constants and nothing is divided: about 60
+// FP64 instructions for the expansion at x >= 100 and 200 for the recurrence,
+// against 350 and 1,300 when each term formed its own factor by division.
 //
 // The same source compiles for the host (tests) and the device (kernels).
 #pragma once
@@ -37,7 +44,7 @@ namespace bfg {
 constexpr double kPi = 3.14159265358979323846264338327950288;
 constexpr double kTwoOverPi = 0.636619772367581343075535053490057448;
 constexpr double kEulerGamma = 0.577215664901532860606512090082402431;
-constexpr double kInvSqrt2 = 0.707106781186547524400844362104849039;
+constexpr double kInvSqrtPi = 0.564189583547756286948079451560772586;
 constexpr double kSeriesMax = 0.25;
 constexpr double kAsymptoticMin = 20.0;
 
@@ -92,83 +99,112 @@ BFG_HD Bessel01 besselSeries(double x) {
 }
 
 // kSeriesMax <= x < kAsymptoticMin: Miller's algorithm + Neumann series.
+// Step N forms J_{N-1} from J_N (jn) and J_{N+1} (jn1), then its part of
+//   norm = 2 sum_{even m>=2} J_m
+//   s0   = sum_{even m>=2} (-1)^{m/2} (4/m) J_m
+//   s1   = sum_{odd  m>=3} (-1)^{(m+1)/2} 4m/(m^2-1) J_m
+struct MillerState {
+  double jn1, jn, norm, s0, s1, j1;
+};
+template <int M>
+BFG_HD void millerAdd(MillerState &s) {
+  if constexpr (M >= 2 && M % 2 == 0) {
+    constexpr double c = ((M / 2) % 2 ? -4.0 : 4.0) / M;
+    s.norm += s.jn;
+    s.s0 = fma(c, s.jn, s.s0);
+  } else if constexpr (M >= 3) {
+    constexpr double c = (((M + 1) / 2) % 2 ? -4.0 : 4.0) * M / ((double)M * M - 1.0);
+    s.s1 = fma(c, s.jn, s.s1);
+  }
+}
+template <int N>
+BFG_HD void millerStep(MillerState &s, double twoOverX) {
+  double const jm1 = fma((double)N * twoOverX, s.jn, -s.jn1);
+  s.jn1 = s.jn;
+  s.jn = jm1;
+  millerAdd<N - 1>(s);
+  if constexpr (N == 2) s.j1 = s.jn;
+  if constexpr (N > 1) millerStep<N - 1>(s, twoOverX);
+}
+
+template <int kStart>   // even, above x + 34
 BFG_HD Bessel01 besselMiller(double x) {
-  int const nStart = 2 * (int)(0.5 * (x + 36.0));   // even, > x + 34
   double const twoOverX = 2.0 / x;
-  double jn1 = 0.0;     // J_{n+1}
-  double jn = 1e-30;    // J_n, arbitrary small start at n = nStart
-  double norm = 0.0;    // 2 sum_{even n>=2} J_n
-  double s0 = 0.0;      // sum_{even n>=2} (-1)^{n/2} (4/n) J_n
-  double s1 = 0.0;      // sum_{odd  n>=3} (-1)^{(n+1)/2} 4n/(n^2-1) J_n
-  double j1 = 0.0;
-  // account for J_nStart itself (even)
-  {
-    int const n = nStart;
-    double const sgn = ((n >> 1) & 1) ? -1.0 : 1.0;
-    norm += 2.0 * jn;
-    s0 += sgn * (4.0 / n) * jn;
-  }
-  for (int n = nStart; n >= 1; --n) {
-    double const jm1 = (double)n * twoOverX * jn - jn1;   // J_{n-1}
-    jn1 = jn;
-    jn = jm1;
-    int const m = n - 1;                 // index of the value just formed
-    if (m == 0) break;
-    if ((m & 1) == 0) {
-      double const sgn = ((m >> 1) & 1) ? -1.0 : 1.0;
-      norm += 2.0 * jn;
-      s0 += sgn * (4.0 / m) * jn;
-    } else if (m == 1) {
-      j1 = jn;
-    } else {
-      double const sgn = (((m + 1) >> 1) & 1) ? -1.0 : 1.0;
-      s1 += sgn * (4.0 * m / ((double)m * m - 1.0)) * jn;
-    }
-  }
-  double const j0 = jn;
-  double const scale = 1.0 / (j0 + norm);
+  MillerState s{0.0, 1e-30, 0.0, 0.0, 0.0, 0.0};   // J_kStart: an arbitrary small start
+  millerAdd<kStart>(s);
+  millerStep<kStart>(s, twoOverX);
+  double const scale = 1.0 / fma(2.0, s.norm, s.jn);
   Bessel01 b;
-  b.j0 = j0 * scale;
-  b.j1 = j1 * scale;
+  b.j0 = s.jn * scale;
+  b.j1 = s.j1 * scale;
   double const l = log(0.5 * x) + kEulerGamma;
-  b.y0 = kTwoOverPi * (l * b.j0 - s0 * scale);
+  b.y0 = kTwoOverPi * (l * b.j0 - s.s0 * scale);
   // Y1 = (2/pi) [ -J0/x + l J1 + (-J1 + s1) ]
-  b.y1 = kTwoOverPi * (-b.j0 / x + l * b.j1 - b.j1 + s1 * scale);
+  b.y1 = kTwoOverPi * (l * b.j1 - 0.5 * twoOverX * b.j0 - b.j1 + s.s1 * scale);
   return b;
+}
+
+// a_k of order nu
+template <int kNu, int K>
+struct HankelA {
+  static constexpr double v =
+      HankelA<kNu, K - 1>::v * (4.0 * kNu * kNu - (2.0 * K - 1.0) * (2.0 * K - 1.0)) / (8.0 * K);
+};
+template <int kNu>
+struct HankelA<kNu, 0> {
+  static constexpr double v = 1.0;
+};
+// sum of a_{First + 2j} w^j, j = J .. kTerms - 1, by Horner's rule
+template <int kNu, int kFirst, int kTerms, int J = 0>
+BFG_HD double hankelPoly(double w) {
+  if constexpr (J + 1 == kTerms)
+    return HankelA<kNu, kFirst + 2 * J>::v;
+  else
+    return fma(hankelPoly<kNu, kFirst, kTerms, J + 1>(w), w, HankelA<kNu, kFirst + 2 * J>::v);
+}
+// P = sum (-1)^j a_2j / x^2j, Q = sum (-1)^j a_{2j+1} / x^{2j+1}: kTerms each
+template <bool kOrder1, int kTerms>
+BFG_HD void hankelPQ(double z, double &p0, double &q0, double &p1, double &q1) {
+  double const w = -z * z;
+  p0 = hankelPoly<0, 0, kTerms>(w);
+  q0 = z * hankelPoly<0, 1, kTerms>(w);
+  if constexpr (kOrder1) {
+    p1 = hankelPoly<1, 0, kTerms>(w);
+    q1 = z * hankelPoly<1, 1, kTerms>(w);
+  } else {
+    p1 = q1 = 0.0;
+  }
 }
 
 // x >= kAsymptoticMin: Hankel's expansion; order 1 only when kOrder1.
 template <bool kOrder1 = true>
 BFG_HD Bessel01 besselAsymptotic(double x) {
-  double const inv8x = 0.125 / x;
-  // order 0: mu = 0; order 1: mu = 4
-  double t0 = 1.0, t1 = 1.0;
-  double p0 = 1.0, q0 = 0.0, p1 = 1.0, q1 = 0.0;
-  for (int k = 1; k <= 60; ++k) {
-    double const odd = (double)(2 * k - 1);
-    double const f = inv8x / (double)k;
-    t0 *= (0.0 - odd * odd) * f;
-    if (kOrder1) t1 *= (4.0 - odd * odd) * f;
-    // k odd -> Q with sign (-1)^{(k-1)/2}; k even -> P with sign (-1)^{k/2}
-    int const r = k & 3;
-    if (r == 1) { q0 += t0; q1 += t1; }
-    else if (r == 2) { p0 -= t0; p1 -= t1; }
-    else if (r == 3) { q0 -= t0; q1 -= t1; }
-    else { p0 += t0; p1 += t1; }
-    if (fabs(t0) < 1e-17 && (!kOrder1 || fabs(t1) < 1e-17)) break;
-  }
+#if defined(__CUDA_ARCH__)
+  double const rx = rsqrt(x);
+#else
+  double const rx = 1.0 / sqrt(x);
+#endif
+  double const z = rx * rx;
+  double p0, q0, p1, q1;
+  // terms from which a_k / x^k < 1e-17 (both orders): 8 at x = 200, 10 at
+  // 100, 13 at 50, 17 at 30, 27 at 20
+  if (x >= 200.0) hankelPQ<kOrder1, 4>(z, p0, q0, p1, q1);
+  else if (x >= 100.0) hankelPQ<kOrder1, 5>(z, p0, q0, p1, q1);
+  else if (x >= 50.0) hankelPQ<kOrder1, 7>(z, p0, q0, p1, q1);
+  else if (x >= 30.0) hankelPQ<kOrder1, 9>(z, p0, q0, p1, q1);
+  else hankelPQ<kOrder1, 14>(z, p0, q0, p1, q1);
   double s, c;
   bfgSincos(x, &s, &c);
-  double const amp = sqrt(kTwoOverPi / x);
-  // chi0 = x - pi/4, chi1 = x - 3pi/4
-  double const c0 = (c + s) * kInvSqrt2, s0 = (s - c) * kInvSqrt2;
-  double const c1 = (s - c) * kInvSqrt2, s1 = -(s + c) * kInvSqrt2;
+  // sqrt(2 / (pi x)) and the 1 / sqrt(2) of the rotations by pi/4 (chi0 =
+  // x - pi/4: cos chi0 = (c + s) / sqrt 2, sin chi0 = (s - c) / sqrt 2) and
+  // 3 pi/4 (cos chi1 = sin chi0, sin chi1 = -cos chi0)
+  double const amp = kInvSqrtPi * rx, cs = amp * (c + s), sc = amp * (s - c);
   Bessel01 b;
-  b.j0 = amp * (p0 * c0 - q0 * s0);
-  b.y0 = amp * (p0 * s0 + q0 * c0);
+  b.j0 = p0 * cs - q0 * sc;
+  b.y0 = p0 * sc + q0 * cs;
   if (kOrder1) {
-    b.j1 = amp * (p1 * c1 - q1 * s1);
-    b.y1 = amp * (p1 * s1 + q1 * c1);
+    b.j1 = p1 * sc + q1 * cs;
+    b.y1 = q1 * sc - p1 * cs;
   } else {
     b.j1 = b.y1 = 0.0;
   }
@@ -179,7 +215,9 @@ BFG_HD Bessel01 besselAsymptotic(double x) {
 template <bool kOrder1 = true>
 BFG_HD Bessel01 bessel01(double x) {
   if (x >= kAsymptoticMin) return besselAsymptotic<kOrder1>(x);
-  if (x >= kSeriesMax) return besselMiller(x);
+  // one start index for the whole range: a shorter one below x = 8 saves less
+  // than the two paths cost in warps that meet both
+  if (x >= kSeriesMax) return besselMiller<56>(x);
   return besselSeries(x);
 }
 
