@@ -19,8 +19,9 @@
 //   Q  = qr(Y)                Householder (explicit Q, p x l)
 //   G  = Z_equiv^H Q          so Z_equiv ~ Q G^H
 //   G  = Q2 R2                Householder
-//   [R2^H ; I] W  ->  [T ; W] one-sided Jacobi: T = R2^H W has orthogonal
-//                             columns, sigma_a = |t_a|, W unitary
+//   [R2^H ; I] W  ->  [T ; W] one-sided Jacobi, first in FP32, then in FP64:
+//                             T = R2^H W has orthogonal columns,
+//                             sigma_a = |t_a|, W unitary
 //   Z_equiv ~ (Q T diag(1/sigma)) diag(sigma) (Q2 W)^H, hence
 //   Z_shift = Q2 (W (diag(w) (T^H (Q^H Z_orig))))
 //             with w_a = 1/sigma_a^2 for sigma_a >= cut, else 0 -- the
@@ -38,6 +39,7 @@
 #include <algorithm>
 #include <array>
 #include <map>
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <vector>
@@ -81,7 +83,9 @@ struct GemmDesc {
   int64_t lda, ldb, ldc;
   int32_t M, N, K, opA;     // opA 0: A is M x K; 1: C = A^H B with A stored K x M
   double const *colScale;   // optional: column j of C scaled by colScale[j]
-  int16_t *rowCode, *colCode;   // scale codes of op(A)'s rows and B's columns (set at launch)
+  int32_t newton = 0;       // 1: C = 3/2 I - 1/2 op(A) B instead
+  int16_t *rowCode = nullptr, *colCode = nullptr;   // scale codes of op(A)'s rows and B's
+                                                    // columns (set at launch)
 };
 
 struct HqrDesc {
@@ -405,8 +409,10 @@ __global__ void __launch_bounds__(256, 1) zgemmKernel(GemmDesc const *__restrict
       int const i = i0 + 16 * mt + gr + 8 * r;
       if (i >= g.M) continue;
       double const sc = g.rowScale ? g.rowScale[i] : 1.0;
-      double const scc = g.colScale ? sc * g.colScale[j] : sc;
-      g.C[i + (int64_t)j * g.ldc] = make_double2(scc * acc[u][2 * r], scc * acc[u][2 * r + 1]);
+      double const scc = g.newton ? -0.5 : g.colScale ? sc * g.colScale[j] : sc;
+      double2 v = make_double2(scc * acc[u][2 * r], scc * acc[u][2 * r + 1]);
+      if (g.newton && i == j) v.x += 1.5;
+      g.C[i + (int64_t)j * g.ldc] = v;
     }
   }
 }
@@ -568,7 +574,8 @@ __global__ void __launch_bounds__(512) hqrKernel(HqrDesc const *__restrict__ des
 // angles of up to kJacSlots pairs with one thread a pair, the rotations --
 // and the angles cost one pair's instructions for 32 pairs.  Measured: the
 // sweeps of the re-expansions 436 -> 234 ms at 65,536 points (k = 512), 762 ->
-// 416 ms for twelve problems of up to 16,384 points, 21 -> 11 ms at 4,096.
+// 416 ms for twelve problems of up to 16,384 points, 21 -> 11 ms at 4,096 (and
+// less again after the FP32 sweeps below).
 // ---------------------------------------------------------------------------
 constexpr int kJacPer = 8, kJacSlots = 16 * kJacPer;   // pairs a warp / a CTA of 16 warps a step
 
@@ -686,6 +693,137 @@ __global__ void __launch_bounds__(512) sketchJacobiKernel(JacobiDesc const *__re
     s2 = warpSum(s2);
     if (lane == 0) d.s2[a] = s2;
   }
+}
+
+// ---------------------------------------------------------------------------
+// The first sweeps of the Jacobi in FP32: one-sided Jacobi on [X ; I], X the
+// top half of M scaled to FP32's range, one CTA per block; M's bottom half
+// receives the rotations' product V (unitary to ~1e-5).  Two Newton-Schulz
+// steps make V unitary to FP64 (products on the tensor cores), and the FP64
+// sweeps then run on [X V ; V], whose columns are orthogonal to ~1e-6: three
+// sweeps with half their pairs rotating instead of seven or eight, at FP32's 64
+// times higher rate for the rest (mixed-precision Jacobi: Zhang, Gao and Bai,
+// SIAM J. Matrix Anal. Appl. 2022).  The FP64 sweeps' stopping rule is
+// unchanged, and so is the accuracy of what they leave.
+// [X ; I] lives in shared memory where it fits (l <= 118), else in `scr`.
+// Measured, all sweeps: 234 -> 117 ms at 65,536 points (k = 512), 416 -> 195 ms
+// for twelve problems of up to 16,384 points, 11.9 -> 6.8 ms at 4,096.
+// ---------------------------------------------------------------------------
+struct Jac32Desc {
+  double2 *M;    // 2 l x l, ld 2 l
+  float2 *scr;   // 2 l x l
+  int32_t l, pad;
+};
+constexpr int kJac32Sweeps = 12, kJac32MaxSmem = 220 * 1024;
+constexpr float kEps32 = 1.1920929e-7f;
+
+__device__ __forceinline__ float4 warpSum4f(float a, float b, float c, float d) {
+  int const lane = threadIdx.x & 31;
+  bool const hi = lane & 16, odd = lane & 8;
+  float p = hi ? c : a, q = hi ? d : b;
+  p += __shfl_xor_sync(0xffffffffu, hi ? a : c, 16);
+  q += __shfl_xor_sync(0xffffffffu, hi ? b : d, 16);
+  float v = odd ? q : p;
+  v += __shfl_xor_sync(0xffffffffu, odd ? p : q, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return make_float4(__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 8),
+                     __shfl_sync(0xffffffffu, v, 16), __shfl_sync(0xffffffffu, v, 24));
+}
+
+__global__ void __launch_bounds__(512) jac32Kernel(Jac32Desc const *__restrict__ descs,
+                                                   int32_t inShared) {
+  extern __shared__ __align__(16) float2 jac32Smem[];
+  __shared__ int sRotated, sExp;
+  Jac32Desc const d = descs[blockIdx.x];
+  int const l = d.l, LD = 2 * l;
+  int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nWarps = blockDim.x >> 5;
+  float2 *A = inShared ? jac32Smem : d.scr;
+  if (tid == 0) sExp = -100000;
+  __syncthreads();
+  int top = -100000;   // exponent of the largest part (integer work, no FP64)
+  for (int e = tid; e < l * l; e += blockDim.x) {
+    double2 const v = d.M[(int64_t)(e / l) * LD + e % l];
+    int const c = max(((__double2hiint(v.x) >> 20) & 0x7FF), ((__double2hiint(v.y) >> 20) & 0x7FF));
+    if (c) top = max(top, c - 1023);
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) atomicMax(&sExp, top);
+  __syncthreads();
+  double const scale = sExp > -100000 ? scalbn(1.0, 25 - sExp) : 1.0;
+  for (int e = tid; e < l * LD; e += blockDim.x) {
+    int const j = e / LD, r = e % LD;
+    float2 v = make_float2(r - l == j ? 1.f : 0.f, 0.f);
+    if (r < l) {
+      double2 const x = d.M[(int64_t)j * LD + r];
+      v = make_float2((float)(x.x * scale), (float)(x.y * scale));
+    }
+    A[e] = v;
+  }
+  __syncthreads();
+  int const P = l + (l & 1), nPairs = P / 2;
+  float const tolRot = kEps32 * sqrtf((float)l);
+  for (int sweep = 0; sweep < kJac32Sweeps; ++sweep) {
+    if (tid == 0) sRotated = 0;
+    __syncthreads();
+    for (int round = 0; round < P - 1; ++round) {
+      for (int pr = warp; pr < nPairs; pr += nWarps) {
+        int i, j;
+        if (pr == 0) {
+          i = round;
+          j = P - 1;
+        } else {
+          i = round + pr;
+          if (i >= P - 1) i -= P - 1;
+          j = round - pr;
+          if (j < 0) j += P - 1;
+        }
+        if (i >= l || j >= l) continue;
+        float2 *ci = A + i * LD, *cj = A + j * LD;
+        float al = 0.f, be = 0.f, gr = 0.f, gi = 0.f;
+        for (int r = lane; r < l; r += 32) {
+          float2 const x = ci[r], y = cj[r];
+          al = fmaf(x.x, x.x, fmaf(x.y, x.y, al));
+          be = fmaf(y.x, y.x, fmaf(y.y, y.y, be));
+          gr = fmaf(x.x, y.x, fmaf(x.y, y.y, gr));     // conj(x) y
+          gi = fmaf(x.x, y.y, fmaf(-x.y, y.x, gi));
+        }
+        float4 const w = warpSum4f(al, be, gr, gi);
+        float const ag = sqrtf(w.z * w.z + w.w * w.w);
+        if (!(ag > tolRot * (sqrtf(w.x) * sqrtf(w.y))) || !(ag > 0.f)) continue;
+        float const zeta = (w.y - w.x) / (2.f * ag), az = fabsf(zeta);
+        float t = az > 1e8f ? 0.5f / az : 1.f / (az + sqrtf(1.f + az * az));
+        if (zeta < 0.f) t = -t;
+        float const c = rsqrtf(1.f + t * t), s = c * t;
+        float const er = w.z / ag, ei = -w.w / ag;   // exp(-i phi)
+        for (int r = lane; r < LD; r += 32) {
+          float2 const x = ci[r], y = cj[r];
+          float const ytr = y.x * er - y.y * ei, yti = y.x * ei + y.y * er;
+          ci[r] = make_float2(c * x.x - s * ytr, c * x.y - s * yti);
+          cj[r] = make_float2(s * x.x + c * ytr, s * x.y + c * yti);
+        }
+        if (lane == 0) sRotated = 1;
+      }
+      __syncthreads();
+    }
+    bool const rotated = sRotated;
+    __syncthreads();   // the flag is cleared by the next sweep
+    if (!rotated) break;
+  }
+  for (int e = tid; e < l * l; e += blockDim.x) {
+    int64_t const o = (int64_t)(e / l) * LD + l + e % l;
+    float2 const v = A[o];
+    d.M[o] = make_double2((double)v.x, (double)v.y);
+  }
+}
+
+// M's top half = T (l x l, ld l)
+__global__ void __launch_bounds__(256) jacTopKernel(Jac32Desc const *__restrict__ descs,
+                                                    double2 const *const *__restrict__ T) {
+  Jac32Desc const d = descs[blockIdx.x];
+  double2 const *t = T[blockIdx.x];
+  for (int e = threadIdx.x; e < d.l * d.l; e += blockDim.x)
+    d.M[(int64_t)(e / d.l) * 2 * d.l + e % d.l] = t[e];
 }
 
 // pseudo-inverse weights with the reference's cut rule
@@ -947,7 +1085,7 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
   std::stable_sort(queue.begin(), queue.end(),
                    [&](Group const &a, Group const &b) { return cost(a) > cost(b); });
   GemmBufs gemmBufs;
-  Buf scratch, dBlk, dTiles, dHqr1, dHqr2, dJac1, dJac2, dW, dFail, dStatus;
+  Buf scratch, dBlk, dTiles, dJ32, dTops, dHqr1, dHqr2, dJac1, dJac2, dW, dFail, dStatus;
   err = dStatus.ensure(sizeof(int32_t));
   if (err != cudaSuccess) return err;
   err = cudaMemsetAsync(dStatus.p, 0, sizeof(int32_t), s);
@@ -1084,8 +1222,68 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
     }
     if ((err = launchHqr<1>(h1, dHqr1, s)) != cudaSuccess) return err;
     if ((err = launchHqr<2>(h2, dHqr2, s)) != cudaSuccess) return err;
-    // Jacobi on [R2^H ; I]
+    // Jacobi on [R2^H ; I]: FP32 sweeps give V (M's bottom half), two
+    // Newton-Schulz steps V <- V (3/2 I - 1/2 V^H V) by way of Z's and G's
+    // buffers, then FP64 sweeps on [R2^H V ; V]
     mark(5);
+    {
+      // by shared memory: four, two and one CTA an SM, and in global memory
+      constexpr int64_t most[4] = {55 * 1024, 110 * 1024, kJac32MaxSmem, INT64_MAX};
+      std::vector<Jac32Desc> js;
+      std::vector<double2 const *> tops;
+      size_t at[5] = {0, 0, 0, 0, 0};
+      int64_t smem[4] = {0, 0, 0, 0};
+      for (int c = 0; c < 4; ++c) {
+        for (auto const &b : blks) {
+          int64_t const bytes = 16 * (int64_t)b.l * b.l;
+          if (bytes > most[c] || (c > 0 && bytes <= most[c - 1])) continue;
+          js.push_back(Jac32Desc{S + b.oM, reinterpret_cast<float2 *>(S + b.oB1), b.l, 0});
+          tops.push_back(S + b.oZ);
+          if (c < 3) smem[c] = std::max(smem[c], bytes);
+        }
+        at[c + 1] = js.size();
+      }
+      if ((err = put(dJ32, js, s)) != cudaSuccess) return err;
+      if ((err = put(dTops, tops, s)) != cudaSuccess) return err;
+      Jac32Desc const *jd = static_cast<Jac32Desc const *>(dJ32.p);
+      err = cudaFuncSetAttribute(jac32Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kJac32MaxSmem);
+      if (err != cudaSuccess) return err;
+      for (int c = 3; c >= 0; --c) {   // the largest first
+        if (at[c + 1] == at[c]) continue;
+        jac32Kernel<<<(unsigned)(at[c + 1] - at[c]), 512, (size_t)smem[c], s>>>(jd + at[c], c < 3);
+        if ((err = cudaGetLastError()) != cudaSuccess) return err;
+      }
+      // what 0: S = 3/2 I - 1/2 V^H V; 1: V S; 2: R2^H V
+      auto products = [&](int what, bool second) {
+        g.clear();
+        for (auto const &b : blks) {
+          double2 *top = S + b.oM, *low = S + b.oM + b.l, *z = S + b.oZ, *sb = S + b.oB1;
+          int64_t const l = b.l;
+          GemmDesc d{};
+          d.M = d.N = d.K = b.l;
+          double2 *v = second ? z : low;
+          int64_t const ldv = second ? l : 2 * l;
+          if (what == 0) {
+            d.A = v; d.lda = ldv; d.B = v; d.ldb = ldv; d.C = sb; d.ldc = l; d.opA = 1; d.newton = 1;
+          } else if (what == 1) {
+            d.A = v; d.lda = ldv; d.B = sb; d.ldb = l;
+            d.C = second ? low : z; d.ldc = second ? 2 * l : l;
+          } else {
+            d.A = top; d.lda = 2 * l; d.B = low; d.ldb = 2 * l; d.C = z; d.ldc = l;
+          }
+          g.push_back(d);
+        }
+        return launchGemms(g, gemmBufs, s);
+      };
+      if ((err = products(0, false)) != cudaSuccess) return err;
+      if ((err = products(1, false)) != cudaSuccess) return err;
+      if ((err = products(0, true)) != cudaSuccess) return err;
+      if ((err = products(1, true)) != cudaSuccess) return err;
+      if ((err = products(2, false)) != cudaSuccess) return err;
+      jacTopKernel<<<(unsigned)js.size(), 256, 0, s>>>(jd, static_cast<double2 const *const *>(dTops.p));
+      if ((err = cudaGetLastError()) != cudaSuccess) return err;
+    }
     std::vector<JacobiDesc> j1, j2;
     for (auto const &b : blks) {
       JacobiDesc j{};
