@@ -67,6 +67,7 @@ struct SketchDev {
   double k;
   uint64_t seed;
   int64_t oZ, oB0, oB1, oB2, oM, oZo, oC, oD, oTau, oSW, oFlags;
+  int64_t oStep;
   int64_t oT, oTo;   // unit circles: p points, and (MIDDLE) the n source points
 };
 
@@ -92,6 +93,7 @@ struct HqrDesc {
   double2 *A;     // rows x cols, ld rows: overwritten by the reflectors and R
   double2 *Q;     // rows x cols, ld rows: receives the explicit Q
   double2 *tau;   // cols
+  double2 *step;  // 4 entries: the reflector in hand (cluster mode)
   double2 *Rt;    // optional: R^H (cols x cols, lower triangular) and the
                   // identity below it, ld = 2 cols
   int32_t rows, cols;
@@ -145,19 +147,6 @@ struct SMem {
     else __syncthreads();
   }
 };
-
-// the CTA-wide sum, the same bits in every thread (and in every CTA that
-// sums the same values)
-__device__ __forceinline__ double blockSumAll(double v, double *red) {
-  int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  v = warpSum(v);
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  double t = 0.0;
-  for (int w = 0; w < nw; ++w) t += red[w];
-  __syncthreads();
-  return t;
-}
 
 __device__ __forceinline__ double2 conjD(double2 a) { return make_double2(a.x, -a.y); }
 
@@ -421,11 +410,49 @@ __global__ void __launch_bounds__(256, 1) zgemmKernel(GemmDesc const *__restrict
 // Householder QR (LAPACK zgeqr2 / zlarfg conventions: H = I - tau v v^H,
 // v_0 = 1, H^H [alpha; x] = [beta; 0] with beta real) and the explicit Q
 // (zung2r), one block per CTA (mode 1) or per cluster of kSketchCluster
-// CTAs (mode 2).  Every CTA forms the reflector of column k itself (same
-// sums, same bits); warps across the cluster update the trailing columns;
+// CTAs (mode 2).  Half a warp updates a trailing column; the one that updates
+// column k + 1 goes on to that column's reflector (its norm, square root and
+// divisions) while the others update the rest, so a step ends at one barrier.
 // CTA 0 stores the scaled reflector of column k while the others work on
-// step k + 1, which no longer reads it, so each step ends at one barrier.
+// step k + 1, which no longer reads it.
+//
+// Bound by the FP64 pipe, where a warp instruction takes 16 clocks of the SM
+// whatever its lanes do: a column's sums and coefficients take as many as its
+// products at 60 rows, hence two columns a warp, and a reflector's scalars
+// about eighty, hence one warp instead of all 16.  Measured, both QRs of
+// a factorization: 126 -> 87 ms at 65,536 points (k = 512), 171 -> 73 ms for
+// twelve problems of up to 16,384 points, 7.0 -> 3.8 ms at 4,096.
 // ---------------------------------------------------------------------------
+// the sums of a and b over each half warp, in every lane of the half
+__device__ __forceinline__ void halfSum2(double &a, double &b) {
+  int const lane = threadIdx.x & 31;
+  bool const hi = lane & 8;
+  double v = hi ? b : a;
+  v += __shfl_xor_sync(0xffffffffu, hi ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  a = __shfl_sync(0xffffffffu, v, lane & 16);
+  b = __shfl_sync(0xffffffffu, v, (lane & 16) | 8);
+}
+
+// the reflector of [alpha; x], s = |x|^2: v = [1; sc x]
+struct Reflector {
+  double2 tau, sc;
+  double beta;
+  __device__ __forceinline__ void form(double2 alpha, double s) {
+    if (s == 0.0 && alpha.y == 0.0) {
+      tau = sc = make_double2(0.0, 0.0);
+      beta = alpha.x;
+    } else {
+      beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + s), alpha.x);
+      tau = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
+      double2 const den = make_double2(alpha.x - beta, alpha.y);   // sc = 1 / (alpha - beta)
+      double const dd = den.x * den.x + den.y * den.y;
+      sc = make_double2(den.x / dd, -den.y / dd);
+    }
+  }
+};
+
 template <int kMode>
 __global__ void __launch_bounds__(512) hqrKernel(HqrDesc const *__restrict__ descs) {
   using Mem = SMem<kMode>;
@@ -436,78 +463,97 @@ __global__ void __launch_bounds__(512) hqrKernel(HqrDesc const *__restrict__ des
   int const m = d.rows, nc = d.cols;
   int const tid = threadIdx.x, nthr = blockDim.x;
   int const lane = tid & 31, warp = tid >> 5, nWarps = nthr >> 5;
+  int const hl = lane & 15, half = lane >> 4;
   int const gWarp = rank * nWarps + warp, gWarps = ctas * nWarps;
-  __shared__ double red[32];
+  __shared__ Reflector sRef[2];   // by the step's parity
   double2 *A = d.A;
 
-  double2 prevSc = make_double2(0.0, 0.0), prevTau = make_double2(0.0, 0.0);
-  double prevBeta = 0.0;
+  if (warp == 0 && nc > 0) {   // (every CTA of a cluster: the same bits)
+    double s = 0.0;
+    for (int i = 1 + lane; i < m; i += 32) {
+      double2 const v = Mem::ld(A + i);
+      s = fma(v.x, v.x, fma(v.y, v.y, s));
+    }
+    s = warpSum(s);
+    Reflector r;
+    r.form(Mem::ld(A), s);
+    if (lane == 0) sRef[0] = r;
+    if (rank == 0 && lane == 0) Mem::st(d.tau, r.tau);
+  }
+  __syncthreads();
+  Reflector prev{};
   for (int k = 0; k < nc; ++k) {
     double2 const *col = A + (int64_t)k * m;
-    double s = 0.0;
-    for (int i = k + 1 + tid; i < m; i += nthr) {
-      double2 const v = Mem::ld(col + i);
-      s += v.x * v.x + v.y * v.y;
+    Reflector ref;
+    if (kMode == 2 && k > 0) {   // formed by the cluster's first CTA
+      double2 const *p = d.step + 2 * (k & 1);
+      ref.sc = Mem::ld(p);
+      ref.beta = Mem::ld(p + 1).x;
+      ref.tau = Mem::ld(d.tau + k);
+    } else {
+      ref = sRef[k & 1];
     }
-    s = blockSumAll(s, red);
-    double2 const alpha = Mem::ld(col + k);
     if (rank == 0 && k > 0) {
       double2 *pc = A + (int64_t)(k - 1) * m;
-      for (int i = k + tid; i < m; i += nthr) Mem::st(pc + i, cmul(prevSc, Mem::ld(pc + i)));
-      if (tid == 0) {
-        Mem::st(pc + (k - 1), make_double2(prevBeta, 0.0));
-        Mem::st(d.tau + (k - 1), prevTau);
-      }
-    }
-    double2 tau, sc;
-    double beta;
-    if (s == 0.0 && alpha.y == 0.0) {
-      tau = make_double2(0.0, 0.0);
-      sc = make_double2(0.0, 0.0);
-      beta = alpha.x;
-    } else {
-      beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + s), alpha.x);
-      tau = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
-      double2 const den = make_double2(alpha.x - beta, alpha.y);   // sc = 1 / (alpha - beta)
-      double const dd = den.x * den.x + den.y * den.y;
-      sc = make_double2(den.x / dd, -den.y / dd);
+      for (int i = k + tid; i < m; i += nthr) Mem::st(pc + i, cmul(prev.sc, Mem::ld(pc + i)));
+      if (tid == 0) Mem::st(pc + (k - 1), make_double2(prev.beta, 0.0));
     }
     // a_j -= conj(tau) v (v^H a_j) for j > k, v = [1; sc x]
-    for (int j = k + 1 + gWarp; j < nc; j += gWarps) {
-      double2 *cj = A + (int64_t)j * m;
+    for (int jb = k + 1 + 2 * gWarp; jb < nc; jb += 2 * gWarps) {
+      bool const next = jb == k + 1;            // this warp's first half has column k + 1
+      bool const on = jb + half < nc;
+      double2 *cj = A + (int64_t)(on ? jb + half : jb) * m;
       double sr = 0.0, si = 0.0;
-      for (int i = k + 1 + lane; i < m; i += 32) {
+      for (int i = k + 1 + hl; i < m; i += 16) {
         double2 const x = Mem::ld(col + i), a = Mem::ld(cj + i);
         sr = fma(x.x, a.x, fma(x.y, a.y, sr));
         si = fma(x.x, a.y, fma(-x.y, a.x, si));
       }
-      sr = warpSum(sr);
-      si = warpSum(si);
+      halfSum2(sr, si);
       double2 const akj = Mem::ld(cj + k);
-      double2 const cs = cmul(conjD(sc), make_double2(sr, si));
+      double2 const cs = cmul(conjD(ref.sc), make_double2(sr, si));
       double2 const w = make_double2(akj.x + cs.x, akj.y + cs.y);
-      double2 const tw = cmul(conjD(tau), w);
-      double2 const f = cmul(sc, tw);
+      double2 const tw = cmul(conjD(ref.tau), w);
+      double2 const f = cmul(ref.sc, tw);
       __syncwarp();
-      if (lane == 0) Mem::st(cj + k, make_double2(akj.x - tw.x, akj.y - tw.y));
-      for (int i = k + 1 + lane; i < m; i += 32) {
-        double2 const x = Mem::ld(col + i), a = Mem::ld(cj + i);
-        double2 const u = cmul(f, x);
-        Mem::st(cj + i, make_double2(a.x - u.x, a.y - u.y));
+      if (on && hl == 0) Mem::st(cj + k, make_double2(akj.x - tw.x, akj.y - tw.y));
+      double n2 = 0.0;
+      double2 alpha = make_double2(0.0, 0.0);
+      for (int i = k + 1 + hl; i < m; i += 16) {
+        double2 const x = Mem::ld(col + i);
+        double2 a = Mem::ld(cj + i);
+        a.x = fma(-f.x, x.x, fma(f.y, x.y, a.x));
+        a.y = fma(-f.x, x.y, fma(-f.y, x.x, a.y));
+        if (on) Mem::st(cj + i, a);
+        if (next) {
+          if (i == k + 1) alpha = a;
+          else n2 = fma(a.x, a.x, fma(a.y, a.y, n2));
+        }
+      }
+      if (next) {
+        double unused = 0.0;
+        halfSum2(n2, unused);
+        alpha.x = __shfl_sync(0xffffffffu, alpha.x, 0);
+        alpha.y = __shfl_sync(0xffffffffu, alpha.y, 0);
+        Reflector r;
+        r.form(alpha, n2);
+        if (lane == 0) {
+          sRef[(k + 1) & 1] = r;
+          Mem::st(d.tau + k + 1, r.tau);
+          if (kMode == 2) {
+            Mem::st(d.step + 2 * ((k + 1) & 1), r.sc);
+            Mem::st(d.step + 2 * ((k + 1) & 1) + 1, make_double2(r.beta, 0.0));
+          }
+        }
       }
     }
     Mem::sync();
-    prevSc = sc;
-    prevTau = tau;
-    prevBeta = beta;
+    prev = ref;
   }
   if (rank == 0 && nc > 0) {
     double2 *pc = A + (int64_t)(nc - 1) * m;
-    for (int i = nc + tid; i < m; i += nthr) Mem::st(pc + i, cmul(prevSc, Mem::ld(pc + i)));
-    if (tid == 0) {
-      Mem::st(pc + (nc - 1), make_double2(prevBeta, 0.0));
-      Mem::st(d.tau + (nc - 1), prevTau);
-    }
+    for (int i = nc + tid; i < m; i += nthr) Mem::st(pc + i, cmul(prev.sc, Mem::ld(pc + i)));
+    if (tid == 0) Mem::st(pc + (nc - 1), make_double2(prev.beta, 0.0));
   }
   Mem::sync();
 
@@ -536,26 +582,29 @@ __global__ void __launch_bounds__(512) hqrKernel(HqrDesc const *__restrict__ des
   for (int i = nc - 1; i >= 0; --i) {
     double2 const t = Mem::ld(d.tau + i);
     double2 const *v = A + (int64_t)i * m;
-    for (int j = i + gWarp; j < nc; j += gWarps) {
-      double2 *qj = Q + (int64_t)j * m;
+    for (int jb = i + 2 * gWarp; jb < nc; jb += 2 * gWarps) {
+      bool const on = jb + half < nc;
+      double2 *qj = Q + (int64_t)(on ? jb + half : jb) * m;
       double sr = 0.0, si = 0.0;
-      for (int r = i + 1 + lane; r < m; r += 32) {
+      for (int r = i + 1 + hl; r < m; r += 16) {
         double2 const x = Mem::ld(v + r), a = Mem::ld(qj + r);
         sr = fma(x.x, a.x, fma(x.y, a.y, sr));
         si = fma(x.x, a.y, fma(-x.y, a.x, si));
       }
-      sr = warpSum(sr);
-      si = warpSum(si);
+      halfSum2(sr, si);
       double2 const qij = Mem::ld(qj + i);
       double2 const w = make_double2(qij.x + sr, qij.y + si);
       double2 const tw = cmul(t, w);
       __syncwarp();
-      if (lane == 0) Mem::st(qj + i, make_double2(qij.x - tw.x, qij.y - tw.y));
-      for (int r = i + 1 + lane; r < m; r += 32) {
-        double2 const x = Mem::ld(v + r), a = Mem::ld(qj + r);
-        double2 const u = cmul(tw, x);
-        Mem::st(qj + r, make_double2(a.x - u.x, a.y - u.y));
-      }
+      if (on && hl == 0) Mem::st(qj + i, make_double2(qij.x - tw.x, qij.y - tw.y));
+      if (on)
+        for (int r = i + 1 + hl; r < m; r += 16) {
+          double2 const x = Mem::ld(v + r);
+          double2 q = Mem::ld(qj + r);
+          q.x = fma(-tw.x, x.x, fma(tw.y, x.y, q.x));
+          q.y = fma(-tw.x, x.y, fma(-tw.y, x.x, q.y));
+          Mem::st(qj + r, q);
+        }
     }
     Mem::sync();
   }
@@ -1106,7 +1155,7 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
     while (q1 < queue.size()) {
       Group const &gr = queue[q1];
       int64_t const p = gr.mem[0].m, l = gr.l;
-      int64_t e = p * p + 3 * p * l + 2 * l * l + l + l + 4 + p;
+      int64_t e = p * p + 3 * p * l + 2 * l * l + l + l + 8 + p;
       for (auto const &d : gr.mem) e += p * d.n + 2 * l * d.n + d.n;
       if (q1 > q0 && total + e > budgetEntries) break;
       FillDesc const &d0 = gr.mem[0];
@@ -1133,6 +1182,7 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
       b.oTau = o; o += l;
       b.oSW = o; o += l;
       b.oFlags = o; o += 4;
+      b.oStep = o; o += 4;
       b.oT = o; o += p;
       for (auto const &d : gr.mem) {
         SketchDev m = b;
@@ -1201,7 +1251,7 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
     mark(2);
     std::vector<HqrDesc> h1, h2;
     for (auto const &b : blks) {
-      HqrDesc h{S + b.oB1, S + b.oB0, S + b.oTau, nullptr, b.p, b.l};
+      HqrDesc h{S + b.oB1, S + b.oB0, S + b.oTau, S + b.oStep, nullptr, b.p, b.l};
       (hqrCluster(b.p, b.l) ? h2 : h1).push_back(h);
     }
     if ((err = launchHqr<1>(h1, dHqr1, s)) != cudaSuccess) return err;
@@ -1217,7 +1267,7 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
     h1.clear();
     h2.clear();
     for (auto const &b : blks) {
-      HqrDesc h{S + b.oB1, S + b.oB2, S + b.oTau, S + b.oM, b.p, b.l};
+      HqrDesc h{S + b.oB1, S + b.oB2, S + b.oTau, S + b.oStep, S + b.oM, b.p, b.l};
       (hqrCluster(b.p, b.l) ? h2 : h1).push_back(h);
     }
     if ((err = launchHqr<1>(h1, dHqr1, s)) != cudaSuccess) return err;
