@@ -286,12 +286,14 @@ constexpr int32_t kSketchMinRank = 128;
 // the same path at full width (l = p) for every other FIRST/MIDDLE block
 // from this rank with the relative cut and FP64 sweeps: its Jacobi runs on
 // the triangular factor of a QR of Z_equiv, which converges in fewer sweeps
-// than the one-sided Jacobi on Z_equiv itself (factorization time at
-// 65,536 / 262,144 points and of the 256-problem batch: 1.95 -> 1.12 s,
-// 34.7 -> 24.2 s, 48.3 -> 26.1 s; the same operators to rounding).  The
-// random Q stays at full width: with Q = I the QR of Z_equiv^H is not rank
-// revealing and the sweeps were slower again (24.2 -> 31.0 s)
-constexpr int32_t kQrMinRank = 32;
+// than the one-sided Jacobi on Z_equiv itself, and starts in FP32.  Below 8
+// there is nothing left to gain (factorization at 4,096 / 32,768 points and of
+// twelve problems of up to 16,384, from rank 32: 21.5, 162 and 402 ms; 24: 19.0,
+// 131, 392; 16: 15.8, 114, 386; 8: 15.8, 113, 386; the same operators to
+// rounding).  The random Q stays at full width: with Q = I the QR of
+// Z_equiv^H is not rank revealing and the sweeps were slower again.  (The
+// statistics count blocks of rank 32 and more as the randomized path's.)
+constexpr int32_t kQrMinRank = 8;
 constexpr double kSketchMaxFraction = 0.8;
 constexpr double kSketchWidthScale = 1.1;
 constexpr int32_t kSketchWidthPad = 40;
@@ -429,6 +431,7 @@ void factorize(bfgFac f) {
     full.insert(full.end(), back.begin(), back.end());
     f->stats.numSketched = rep.blocks;
     f->stats.sketchGroups = rep.groups;
+    f->stats.reexpSvds = rep.smallGroups;
     f->stats.sketchRetries = rep.retries;
     f->stats.sketchFallbacks = rep.fallbacks;
     f->stats.sketchMaxWidth = rep.maxWidth;
@@ -459,7 +462,7 @@ void factorize(bfgFac f) {
       for (auto const &m : g) lead.n = std::max(lead.n, m.n);
       route(lead, std::move(g));
     }
-    f->stats.reexpSvds = (int64_t)groups.size();
+    f->stats.reexpSvds += (int64_t)groups.size();
   }
   // largest work first, so that the longest CTAs start in the first wave
   auto cost = [](bfg::FillDesc const &lead, std::vector<bfg::FillDesc> const &mem) {

@@ -74,9 +74,13 @@ struct SketchInput {
   int32_t l;
   int32_t fullOk;
 };
+// ranks from which a block counts as one of the randomized path; the smaller
+// ones, which run the same kernels at full width, stand for the full path's
+constexpr int32_t kSketchCounted = 32;
 struct SketchReport {
-  int64_t blocks = 0;      // blocks computed by this path
+  int64_t blocks = 0;      // blocks computed by this path (of rank >= kSketchCounted)
   int64_t groups = 0;      // their distinct Z_equiv (one sketch and SVD each)
+  int64_t smallGroups = 0;   // the distinct Z_equiv of the smaller blocks
   int64_t retries = 0;     // sketches redone with a wider l
   int64_t fallbacks = 0;   // blocks handed back to the full path
   int64_t maxWidth = 0, sumWidth = 0;

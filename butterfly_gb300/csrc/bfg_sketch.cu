@@ -949,6 +949,9 @@ uint64_t splitmixHost(uint64_t x) {
 
 
 // modes of the HQR / Jacobi launches: a whole cluster for large blocks
+// (factorization of twelve problems of up to 16,384 points / of 65,536 points:
+// QR clusters from p l = 2^17 386 and 331 ms, from 2^16 402 and 332, from 2^15
+// 413 and 331; Jacobi clusters from l = 128 386 and 338 ms, from 96 462 and 359)
 bool hqrCluster(int64_t p, int64_t l) { return p * l >= (int64_t)1 << 17; }
 bool jacobiCluster(int64_t l) { return l >= 160; }
 
@@ -1390,7 +1393,7 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
         }
         continue;
       }
-      rep->groups += 1;
+      (b.p < kSketchCounted ? rep->smallGroups : rep->groups) += 1;
       int64_t sumN = 0;
       for (auto const &d : gr.mem) sumN += d.n;
       if (sumN > b.p) {
@@ -1424,6 +1427,7 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
         gx.push_back(GemmDesc{S + b.oB2, S + m.oC, arena + m.arenaOff, nullptr, b.p, b.l, b.p, b.p,
                               m.n, b.l, 0, nullptr});
       }
+      if (b.p < kSketchCounted) continue;
       ++rep->blocks;
       rep->maxWidth = std::max<int64_t>(rep->maxWidth, b.l);
       rep->sumWidth += b.l;

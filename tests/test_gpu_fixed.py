@@ -121,3 +121,34 @@ def test_factorization_products_match_the_full_path(k):
                                     sketch=s, context=B.default_context(0)).apply(X)
          for s in (True, False)]
     assert torch.linalg.norm(y[0] - y[1]) < 2e-9 * torch.linalg.norm(y[1])
+
+
+def test_small_rank_blocks_solve_the_reexpansion_least_squares():
+    """Ranks 8 to 31, which the QR-preconditioned Jacobi at full width takes
+    too, against the oracle's pseudo-inverse (the bounds of the sketch tests)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from conftest import rel_err
+    from oracle import bf_oracle as O
+    n, k, tol = 2048, 24.0, 1e-7
+    src, tgt = B.uniform_square_points(n, 4), B.curve_points("ellipse", n)
+    fac = B.FacHelm2.make_multilevel(B.Helm2(k), B.Quadtree(src, leaf_size=64),
+                                     B.Quadtree(tgt, leaf_size=64), rank_eps=tol, pinv_tol=tol,
+                                     context=B.default_context(0))
+    of = O.Factorization(O.Helm2(k), src, tgt, leaf_size=64, eps=tol, rcut="relative", fill=False)
+    tab, ent = fac.blocks()
+    ranks = set()
+    for (kind, m, nb, off), ob in zip(tab, of.blocks()):
+        if kind not in (0, 1) or not 8 <= m < 32 or (m in ranks and len(ranks) < 12):
+            continue
+        Z = ent[off:off + m * nb].reshape(nb, m).T
+        eq, chk = O.circle_points(ob.ceq, m)[0], O.circle_points(ob.cchk, m)[0]
+        orig = (of.src_tree_pts[ob.src_range[0]:ob.src_range[1]] if ob.kind == "first"
+                else O.circle_points(ob.corig, nb)[0])
+        Ze, Zo = (O.kernel_matrix(O.Helm2(k), p, chk) for p in (eq, orig))
+        Xo = O.lstsq_pinv(Ze, Zo, "relative", tol)
+        assert (np.linalg.norm(Ze @ Z - Zo) < 2 * np.linalg.norm(Ze @ Xo - Zo)
+                + 1e-12 * np.linalg.norm(Zo))
+        assert rel_err(Z, Xo) < 1e-6
+        ranks.add(m)
+    assert len(ranks) >= 6
