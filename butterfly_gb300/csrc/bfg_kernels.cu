@@ -9,7 +9,7 @@
 //                          least-squares solve (mat_dense_complex.c:1768-1849)
 //                          by a one-sided Jacobi SVD (details at the kernel).
 //  * applyGemvKernel /     one stage of the staged FP32 apply (single / many
-//    applyTileKernel       RHS), each item a row chunk of one block row summing
+//    applyRhsKernel        RHS), each item a row chunk of one block row summing
 //                          its blocks in order; no atomics, so results are
 //                          reproducible bit for bit.
 //  * applyReduceKernel     sums the per-product outputs into Y in a fixed
@@ -20,10 +20,7 @@
 
 #include <cooperative_groups.h>
 
-#include <atomic>
 #include <cstdint>
-#include <cstdlib>
-#include <cstring>
 
 #include "bfg_device.cuh"
 #include "bfg_kernels.cuh"
@@ -764,266 +761,217 @@ __device__ __forceinline__ T2 mk2(typename Real<T2>::T a, typename Real<T2>::T b
 // fixed order.
 constexpr int kGemvWarps = 8;
 
-template <typename T2>
 __global__ void __launch_bounds__(32 * kGemvWarps)
 applyGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restrict__ contribs,
-                T2 const *__restrict__ arena, T2 const *__restrict__ X, int64_t ldx,
-                T2 *__restrict__ W) {
-  using T = typename Real<T2>::T;
-  __shared__ T2 part[kGemvWarps][32];
+                float2 const *__restrict__ arena, float2 const *__restrict__ X, int64_t ldx,
+                float2 *__restrict__ W) {
+  __shared__ float2 part[kGemvWarps][32];
   int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   ApplyItem const it = items[blockIdx.x];
   bool const active = lane < it.rows;
-  T accr = 0, acci = 0;
+  float accr = 0, acci = 0;
   for (int c = 0; c < it.nContrib; ++c) {
     ApplyContrib const cb = contribs[it.contrib0 + c];
-    T2 const *a = arena + cb.aOff + lane;
-    T2 const *x = cb.inIsX ? X + cb.inRow * ldx : W + cb.inRow;
+    float2 const *a = arena + cb.aOff + lane;
+    float2 const *x = cb.inIsX ? X + cb.inRow * ldx : W + cb.inRow;
     int64_t const xs = cb.inIsX ? ldx : 1;
     int const n = cb.n;
     int64_t const lda = cb.lda;
     int j = warp;
     constexpr int S = kGemvWarps;
     for (; j + 3 * S < n; j += 4 * S) {
-      T2 a0, a1, a2, a3;
+      float2 a0, a1, a2, a3;
       if (active) {
         a0 = a[(int64_t)(j + 0 * S) * lda];
         a1 = a[(int64_t)(j + 1 * S) * lda];
         a2 = a[(int64_t)(j + 2 * S) * lda];
         a3 = a[(int64_t)(j + 3 * S) * lda];
       } else {
-        a0 = a1 = a2 = a3 = mk2<T2>(0, 0);
+        a0 = a1 = a2 = a3 = make_float2(0, 0);
       }
-      T2 const x0 = x[(j + 0 * S) * xs], x1 = x[(j + 1 * S) * xs];
-      T2 const x2 = x[(j + 2 * S) * xs], x3 = x[(j + 3 * S) * xs];
+      float2 const x0 = x[(j + 0 * S) * xs], x1 = x[(j + 1 * S) * xs];
+      float2 const x2 = x[(j + 2 * S) * xs], x3 = x[(j + 3 * S) * xs];
       cmacc(accr, acci, a0, x0);
       cmacc(accr, acci, a1, x1);
       cmacc(accr, acci, a2, x2);
       cmacc(accr, acci, a3, x3);
     }
     for (; j < n; j += S) {
-      T2 const a0 = active ? a[(int64_t)j * lda] : mk2<T2>(0, 0);
-      T2 const x0 = x[j * xs];
+      float2 const a0 = active ? a[(int64_t)j * lda] : make_float2(0, 0);
+      float2 const x0 = x[j * xs];
       cmacc(accr, acci, a0, x0);
     }
   }
-  part[warp][lane] = mk2<T2>(accr, acci);
+  part[warp][lane] = make_float2(accr, acci);
   __syncthreads();
   if (warp == 0 && active) {
-    T sr = 0, si = 0;
+    float sr = 0, si = 0;
 #pragma unroll
     for (int w = 0; w < kGemvWarps; ++w) {
       sr += part[w][lane].x;
       si += part[w][lane].y;
     }
-    W[it.outRow + lane] = mk2<T2>(sr, si);
+    W[it.outRow + lane] = make_float2(sr, si);
   }
 }
 
-// two adjacent complex values from shared memory (16-byte aligned)
-__device__ __forceinline__ void load2(float2 const *p, float2 &a, float2 &b) {
-  float4 const v = *reinterpret_cast<float4 const *>(p);
-  a = make_float2(v.x, v.y);
-  b = make_float2(v.z, v.w);
+// R > 1 (FP32): one CTA of 4 warps per (item, tile of RT right-hand sides),
+// lane = row; warp w multiplies columns w, w + 4, ... of every block.  The
+// input rows are copied into shared memory a chunk ahead (cp.async) and read
+// as broadcasts, two complex values a load; the factor entries go from global
+// memory to registers, a batch of four columns a warp ahead over chunk and
+// block ends.  A complex product is two packed FMAs (fma.rn.f32x2):
+// (p, q) += a.re (x.re, x.im) and (u, v) += a.im (x.re, x.im), and y =
+// (p - v, q + u) at the end, so nothing is swapped or negated on the way.
+// Bound by issue and load latency together (at 8 right-hand sides HBM 32 %,
+// FMA pipe 49 % busy; at 64 the FMA pipe 65 %).  Measured at 32,768 points
+// (us; before: synchronous tiles up to 8 right-hand sides, a shared-memory
+// pipeline with a 4 x 4 register tile above): R = 2 375 -> 161, R = 4 378 ->
+// 177, R = 8 385 -> 220, R = 16 408 -> 317, R = 64 1,290 -> 1,020.  Two batches
+// ahead (more registers) 237 and 367 us at R = 8 and 16; 64 registers for more
+// warps 223 and, at 96, 430.
+constexpr int kRhsWarps = 4, kRhsCols = 64, kRhsAhead = 4;
+
+__device__ __forceinline__ void fma2(uint64_t &acc, uint64_t a, uint64_t x) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(x));
+}
+__device__ __forceinline__ uint64_t dup2(float a) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
 }
 
-// Asynchronous global -> shared copies (LDGSTS) of one complex entry
-__device__ __forceinline__ void cpAsyncEntry(float2 *dst, float2 const *src) {
-  unsigned const d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cpAsyncCommit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cpAsyncWait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
-// R > 1, pipelined: one CTA of NW warps per (item, tile of 16 RHS).  The
-// item's contributions are walked in chunks of up to KC columns; each chunk's
-// A panel (rows x columns) and X panel (columns x 16 RHS) are copied into
-// shared memory with cp.async, one chunk ahead of the one being multiplied,
-// so every load of a chunk is in flight at once instead of one column per
-// round trip.  Warp w multiplies the columns w, w+NW, ... of each chunk; a
-// lane owns 4 rows x 4 RHS of the 32 x 16 tile (4 vector shared loads per
-// 16 complex MACs) in 16 register accumulators; the NW partial 32 x 16 tiles
-// are summed in shared memory in a fixed order.  Rows >= item rows and RHS
-// >= R are never copied: they only reach accumulators that are not stored.
-template <typename T2>
-struct PipeShape {
-  static constexpr int KC = 32;   // 12 KB (FP32) / 24 KB (FP64) per stage
-  static constexpr int RT = 16;
-  static constexpr size_t stageBytes = (size_t)KC * (32 + RT) * sizeof(T2);
-};
-constexpr int kPipeWarps = 4;
-
-template <typename T2, int NW, int S>
-__global__ void __launch_bounds__(32 * NW, sizeof(T2) == 8 ? 8 : 4) applyPipeKernel(
+template <int RT>
+__global__ void __launch_bounds__(32 * kRhsWarps) applyRhsKernel(
     ApplyItem const *__restrict__ items, ApplyContrib const *__restrict__ contribs,
-    T2 const *__restrict__ arena, T2 const *__restrict__ X, int64_t ldx,
-    T2 *__restrict__ W, int64_t R) {
-  using T = typename Real<T2>::T;
-  constexpr int KC = PipeShape<T2>::KC, RT = PipeShape<T2>::RT, TH = 32 * NW;
-  static_assert((size_t)NW * RT * 32 <= (size_t)S * KC * 32, "partials must fit in sA");
-  extern __shared__ __align__(16) unsigned char pipeSmem[];
-  T2 *const sA = reinterpret_cast<T2 *>(pipeSmem);   // [S][KC][32]
-  T2 *const sX = sA + S * KC * 32;                   // [S][KC][RT]
-  int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int const rg = lane & 7, cg = lane >> 3;   // lane's rows 4rg.., RHS 4cg..
-  ApplyItem const it = items[blockIdx.x];
-  int64_t const r0 = (int64_t)blockIdx.y * RT;
+    float2 const *__restrict__ arena, float2 const *X, int64_t ldx, float2 *W, int64_t R,
+    unsigned tiles) {
+  constexpr int S = kRhsWarps, KC = kRhsCols, U = kRhsAhead, TH = 32 * S;
+  constexpr int kPanel = 2 * KC * RT, kPart = S * 32 * (RT + 1);
+  __shared__ __align__(16) float2 smem[kPanel > kPart ? kPanel : kPart];
+  int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // the tiles of an item run side by side and read its blocks from HBM once
+  ApplyItem const it = items[blockIdx.x / tiles];
+  int64_t const r0 = (int64_t)(blockIdx.x % tiles) * RT;
   int const nr = (R - r0) < RT ? (int)(R - r0) : RT;
-  int const rows = it.rows;
+  int const row = lane < it.rows ? lane : 0;   // inactive lanes re-read row 0
 
-  // issue cursor over (contribution, first column); uniform across the CTA
-  int ci = 0, cj = 0;
-  ApplyContrib icb{};
-  if (it.nContrib > 0) icb = contribs[it.contrib0];
-  int ncBuf[S];
-  int issued = 0;
-  // copies the next chunk (if any) into stage `slot`, then commits a group
-  // (an empty one at the end, so that group counts stay in step)
-  auto tryIssue = [&](int slot) {
-    if (ci < it.nContrib) {
-      int const nc = min(KC, icb.n - cj);
-      T2 const *a = arena + icb.aOff + (int64_t)cj * icb.lda;
-      int64_t const lda = icb.lda;
-      for (int e = threadIdx.x; e < nc * 32; e += TH) {
-        int const col = e >> 5, row = e & 31;
-        if (row < rows) cpAsyncEntry(&sA[(slot * KC + col) * 32 + row], a + col * lda + row);
-      }
-      int64_t const xld = icb.inIsX ? ldx : R;
-      T2 const *x =
-          (icb.inIsX ? X + icb.inRow * ldx : W + icb.inRow * R) + r0 + (int64_t)cj * xld;
-      for (int e = threadIdx.x; e < nc * RT; e += TH) {
-        int const col = e / RT, q = e % RT;
-        if (q < nr) cpAsyncEntry(&sX[(slot * KC + col) * RT + q], x + col * xld + q);
-      }
-      ncBuf[slot] = nc;
-      ++issued;
-      cj += nc;
-      if (cj >= icb.n) {
-        ++ci;
-        cj = 0;
-        if (ci < it.nContrib) icb = contribs[it.contrib0 + ci];
+  // the chunk being fetched: columns [j0, j0 + n) of contribution c
+  int c = 0, j0 = 0, n = 0, lda = 0;
+  float2 const *a = nullptr, *x = nullptr;
+  int64_t xld = 0;
+  ApplyContrib cb{};
+  auto begin = [&]() {   // the next chunk (c < nContrib)
+    if (j0 == 0) {
+      cb = contribs[it.contrib0 + c];
+      lda = cb.lda;
+      xld = cb.inIsX ? ldx : R;
+      x = (cb.inIsX ? X + cb.inRow * ldx : W + cb.inRow * R) + r0;
+      a = arena + cb.aOff + row;
+    } else {
+      x += KC * xld;
+      a += (int64_t)KC * lda;
+    }
+    n = min(KC, cb.n - j0);
+    j0 += KC;
+    if (j0 >= cb.n) {
+      j0 = 0;
+      ++c;
+    }
+  };
+  // the chunk's input rows; zeros for the columns that fill its last batch
+  auto copyX = [&](float2 *panel) {
+    int const full = (n + S * U - 1) / (S * U) * (S * U);
+    for (int e = tid; e < full * RT; e += TH) {
+      int const col = e / RT, q = e % RT;
+      if (col < n && q < nr) {
+        unsigned const d = (unsigned)__cvta_generic_to_shared(panel + e);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(x + col * xld + q)
+                     : "memory");
+      } else {
+        panel[e] = make_float2(0.f, 0.f);
       }
     }
-    cpAsyncCommit();
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  // this warp's entries of the batch at column b of the chunk (a column past
+  // the end re-reads the last one, against zeros)
+  float2 av[U];
+  auto loadA = [&](int b) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      av[u] = a[(int64_t)min(b + warp + u * S, n - 1) * lda];
   };
 
-  T accr[RT], acci[RT];
+  uint64_t p[RT], w[RT];
 #pragma unroll
-  for (int q = 0; q < RT; ++q) accr[q] = acci[q] = 0;
-
-#pragma unroll
-  for (int sl = 0; sl < S - 1; ++sl) tryIssue(sl);
-  for (int i = 0; i < issued; ++i) {
-    tryIssue((i + S - 1) % S);   // the stage multiplied in the previous pass
-    cpAsyncWait<S - 1>();         // chunk i has landed
-    __syncthreads();
-    int const slot = i % S;
-    int const nc = ncBuf[slot];
-    T2 const *pa = sA + slot * KC * 32 + 4 * rg;
-    T2 const *px = sX + slot * KC * RT + 4 * cg;
-    for (int col = warp; col < nc; col += NW) {
-      T2 a[4], x[4];
-      load2(pa + col * 32, a[0], a[1]);
-      load2(pa + col * 32 + 2, a[2], a[3]);
-      load2(px + col * RT, x[0], x[1]);
-      load2(px + col * RT + 2, x[2], x[3]);
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          cmacc(accr[4 * u + q], acci[4 * u + q], a[u], x[q]);
-        }
-    }
-    __syncthreads();
+  for (int q = 0; q < RT; ++q) p[q] = w[q] = 0ull;
+  int slot = 0;
+  bool more = it.nContrib > 0;
+  if (more) {
+    begin();
+    copyX(smem);
+    loadA(0);
   }
-  cpAsyncWait<0>();
-
-  T2 *const part = sA;   // [NW][RT][32], reuses the drained stage buffers
+  while (more) {
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();   // the chunk has landed, and every warp has left the other panel
+    float2 const *panel = smem + slot * KC * RT + warp * RT;
+    int const nNow = n;
+    for (int b = 0; b < nNow; b += S * U) {
+      float2 now[U];
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < U; ++u) now[u] = av[u];
+      if (b + S * U < nNow) {
+        loadA(b + S * U);
+      } else if ((more = c < it.nContrib)) {
+        begin();
+        copyX(smem + (slot ^ 1) * KC * RT);
+        loadA(0);
+      }
+      float2 const *xs = panel + b * RT;
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      part[(warp * RT + 4 * cg + q) * 32 + 4 * rg + u] =
-          mk2<T2>(accr[4 * u + q], acci[4 * u + q]);
+      for (int u = 0; u < U; ++u) {
+        uint64_t const re = dup2(now[u].x), im = dup2(now[u].y);
+        ulonglong2 const *xv = reinterpret_cast<ulonglong2 const *>(xs + u * S * RT);
+#pragma unroll
+        for (int q = 0; q < RT; q += 2) {
+          ulonglong2 const v = xv[q / 2];
+          fma2(p[q], re, v.x);
+          fma2(w[q], im, v.x);
+          fma2(p[q + 1], re, v.y);
+          fma2(w[q + 1], im, v.y);
+        }
+      }
+    }
+    slot ^= 1;
+  }
   __syncthreads();
-  for (int e = threadIdx.x; e < 32 * RT; e += TH) {
-    int const row = e & 31, q = e >> 5;
-    if (row >= rows || q >= nr) continue;
-    T sr = 0, si = 0;
+  float2 *const part = smem;   // [warp][row][RT + 1]
 #pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      T2 const v = part[(w * RT + q) * 32 + row];
-      sr += v.x;
-      si += v.y;
+  for (int q = 0; q < RT; ++q) {
+    float2 const s = unpack2(p[q]), t = unpack2(w[q]);
+    part[(warp * 32 + lane) * (RT + 1) + q] = make_float2(s.x - t.y, s.y + t.x);
+  }
+  __syncthreads();
+  for (int e = tid; e < it.rows * RT; e += TH) {
+    int const i = e / RT, q = e % RT;
+    if (q >= nr) continue;
+    float sr = 0.f, si = 0.f;
+#pragma unroll
+    for (int v = 0; v < S; ++v) {
+      float2 const t = part[(v * 32 + i) * (RT + 1) + q];
+      sr += t.x;
+      si += t.y;
     }
-    W[(it.outRow + row) * R + r0 + q] = mk2<T2>(sr, si);
+    W[(it.outRow + i) * R + r0 + q] = make_float2(sr, si);
   }
 }
-
-// R > 1: one CTA per (item, RHS tile of RT columns); 32 rows x RT outputs,
-// A and X staged through shared memory in chunks of KC columns.
-template <typename T2, int RT>
-__global__ void __launch_bounds__(256) applyTileKernel(
-    ApplyItem const *__restrict__ items, ApplyContrib const *__restrict__ contribs,
-    T2 const *__restrict__ arena, T2 const *__restrict__ X, int64_t ldx,
-    T2 *__restrict__ W, int64_t R) {
-  using T = typename Real<T2>::T;
-  constexpr int KC = 32;
-  constexpr int NT = 256;
-  constexpr int PER = 32 * RT / NT;      // outputs per thread
-  static_assert(PER >= 1, "tile too small");
-  __shared__ T2 As[KC][32];
-  __shared__ T2 Bs[KC][RT];
-  ApplyItem const it = items[blockIdx.x];
-  int64_t const r0 = (int64_t)blockIdx.y * RT;
-  int const tid = threadIdx.x;
-  // thread -> (row, first rhs); rhs columns strided by NT/32
-  int const row = tid & 31;
-  int const c0 = tid >> 5;               // 0..7
-  T accr[PER], acci[PER];
-#pragma unroll
-  for (int q = 0; q < PER; ++q) accr[q] = acci[q] = 0;
-  for (int cbi = 0; cbi < it.nContrib; ++cbi) {
-    ApplyContrib const cb = contribs[it.contrib0 + cbi];
-    T2 const *xin = cb.inIsX ? X + cb.inRow * ldx : W + cb.inRow * R;
-    int64_t const xld = cb.inIsX ? ldx : R;
-    for (int k0 = 0; k0 < cb.n; k0 += KC) {
-      int const kc = (cb.n - k0) < KC ? (cb.n - k0) : KC;
-      for (int e = tid; e < KC * 32; e += NT) {
-        int const kk = e >> 5, rr = e & 31;
-        As[kk][rr] = (kk < kc && rr < it.rows) ? arena[cb.aOff + (int64_t)(k0 + kk) * cb.lda + rr]
-                                              : mk2<T2>(0, 0);
-      }
-      for (int e = tid; e < KC * RT; e += NT) {
-        int const kk = e / RT, cc = e % RT;
-        Bs[kk][cc] = (kk < kc && r0 + cc < R) ? xin[(int64_t)(k0 + kk) * xld + r0 + cc]
-                                             : mk2<T2>(0, 0);
-      }
-      __syncthreads();
-#pragma unroll 4
-      for (int kk = 0; kk < kc; ++kk) {
-        T2 const a = As[kk][row];
-#pragma unroll
-        for (int q = 0; q < PER; ++q) {
-          T2 const b = Bs[kk][c0 + q * (NT / 32)];
-          cmacc(accr[q], acci[q], a, b);
-        }
-      }
-      __syncthreads();
-    }
-  }
-  if (row < it.rows) {
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      int64_t const col = r0 + c0 + q * (NT / 32);
-      if (col < R) W[(it.outRow + row) * R + col] = mk2<T2>(accr[q], acci[q]);
-    }
-  }
-}
-
 
 template <typename T2>
 __global__ void applyReduceKernel(int32_t const *__restrict__ rowSeg,
@@ -1068,16 +1016,15 @@ __global__ void gatherRowsKernel(T2 const *X, int64_t ldx, int64_t const *perm,
   }
 }
 
-// Multi-RHS kernel choice: the pipelined kernel above 8 RHS, the shared-memory
-// tile kernel up to 8 (the pipelined kernel computes 16 RHS per CTA); the
-// environment variable BFG_APPLY_KERNEL=tile forces the tile kernel for every
-// R > 1 (for A/B measurements).
-bool forceTileKernel() {
-  static bool v = [] {
-    char const *e = std::getenv("BFG_APPLY_KERNEL");
-    return e && std::strcmp(e, "tile") == 0;
-  }();
-  return v;
+template <int RT>
+cudaError_t launchRhs(ApplyItem const *items, int64_t nItems, ApplyContrib const *contribs,
+                      float2 const *arena, float2 const *X, int64_t ldx, float2 *W, int64_t R,
+                      cudaStream_t stream) {
+  int64_t const tiles = (R + RT - 1) / RT;
+  if (tiles > 0x7fffffff / nItems) return cudaErrorInvalidConfiguration;
+  applyRhsKernel<RT><<<(unsigned)(nItems * tiles), 32 * kRhsWarps, 0, stream>>>(
+      items, contribs, arena, X, ldx, W, R, (unsigned)tiles);
+  return cudaGetLastError();
 }
 
 int gridFor(int64_t total, int threads) {
@@ -1233,40 +1180,17 @@ cudaError_t launchApplyStage(ApplyItem const *items, int64_t nItems,
                              ApplyContrib const *contribs, float2 const *arena,
                              float2 const *X, int64_t ldx, float2 *W, int64_t R,
                              cudaStream_t stream) {
-  using T2 = float2;
   if (nItems == 0) return cudaSuccess;
   if (R == 1) {
-    applyGemvKernel<T2><<<(unsigned)nItems, 32 * kGemvWarps, 0, stream>>>(items, contribs,
-                                                                          arena, X, ldx, W);
-  } else if (R > 8 && !forceTileKernel()) {
-    size_t const smem = 2 * PipeShape<T2>::stageBytes;
-    // the shared-memory limit is a per-device function attribute: set it once
-    // per device, so that applies enqueue nothing else (stream capture)
-    static std::atomic<uint64_t> attrSet{0};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    uint64_t const bit = 1ull << (dev & 63);
-    if (!(attrSet.load() & bit)) {
-      e = cudaFuncSetAttribute(applyPipeKernel<T2, kPipeWarps, 2>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      attrSet.fetch_or(bit);
-    }
-    dim3 grid((unsigned)nItems, (unsigned)((R + 15) / 16));
-    applyPipeKernel<T2, kPipeWarps, 2><<<grid, 32 * kPipeWarps, smem, stream>>>(
-        items, contribs, arena, X, ldx, W, R);
-  } else if (R <= 8) {
-    dim3 grid((unsigned)nItems, 1);
-    applyTileKernel<T2, 8><<<grid, 256, 0, stream>>>(items, contribs, arena, X, ldx, W, R);
-  } else if (R <= 16) {
-    dim3 grid((unsigned)nItems, 1);
-    applyTileKernel<T2, 16><<<grid, 256, 0, stream>>>(items, contribs, arena, X, ldx, W, R);
-  } else {
-    dim3 grid((unsigned)nItems, (unsigned)((R + 31) / 32));
-    applyTileKernel<T2, 32><<<grid, 256, 0, stream>>>(items, contribs, arena, X, ldx, W, R);
+    applyGemvKernel<<<(unsigned)nItems, 32 * kGemvWarps, 0, stream>>>(items, contribs, arena, X,
+                                                                      ldx, W);
+    return cudaGetLastError();
   }
-  return cudaGetLastError();
+  // the narrowest tile that holds the right-hand sides
+  if (R <= 2) return launchRhs<2>(items, nItems, contribs, arena, X, ldx, W, R, stream);
+  if (R <= 4) return launchRhs<4>(items, nItems, contribs, arena, X, ldx, W, R, stream);
+  if (R <= 8) return launchRhs<8>(items, nItems, contribs, arena, X, ldx, W, R, stream);
+  return launchRhs<16>(items, nItems, contribs, arena, X, ldx, W, R, stream);
 }
 
 template <typename T2>

@@ -152,3 +152,22 @@ def test_small_rank_blocks_solve_the_reexpansion_least_squares():
         assert rel_err(Z, Xo) < 1e-6
         ranks.add(m)
     assert len(ranks) >= 6
+
+
+@pytest.mark.parametrize("m,n", [(9, 31), (131, 127), (130, 257), (70, 515)])
+def test_fp32_tiles_are_within_their_bound(m, n):
+    """The FP32 apply of several right-hand sides (bfg_kernels.cu): every
+    tile width and its remainders, against extended precision.  FP32 entries
+    and inputs are off by 2^-24 of themselves and every product and sum rounds
+    to FP32: less than 2^-22 sum |a||x| (n + 8) / 4 a block of n columns."""
+    fac, blocks = _problem(m, n)
+    X = B.Rng(n).complex_randn(n * 33).reshape(n, 33).astype(np.complex64)
+    Y = np.zeros((m, 33), LD)
+    bound = np.zeros((m, 33))
+    for r, c, A in blocks:
+        x = X[c:c + A.shape[1]]
+        Y[r:r + A.shape[0]] += A.astype(LD) @ x.astype(LD)
+        bound[r:r + A.shape[0]] += 2.0 ** -22 * (A.shape[1] + 8) / 4 * (np.abs(A) @ np.abs(x))
+    for R in (2, 3, 4, 5, 8, 9, 16, 17, 33):
+        y = fac.apply(torch.from_numpy(X[:, :R].copy()).cuda(), precision="fp32").cpu().numpy()
+        assert np.all(np.abs(y.astype(LD) - Y[:, :R]) <= bound[:, :R])
