@@ -641,7 +641,8 @@ void fillStats(bfgFac f) {
 
 template <typename T2>
 void runApply(bfgFac f, T2 const *arena, T2 const *X, int64_t ldx, int64_t R, T2 *Y,
-              int64_t ldy, uint32_t flags, std::vector<cudaEvent_t> *events) {
+              int64_t ldy, uint32_t flags, std::vector<cudaEvent_t> *events,
+              bfg::SystemTerms const *sys = nullptr) {
   cudaStream_t s = f->ctx->stream;
   bfg::ApplyProgram const &p = f->prog;
   ck(f->ws.ensure((size_t)std::max<int64_t>(1, p.wsRows) * R * sizeof(T2)), "workspace");
@@ -655,9 +656,15 @@ void runApply(bfgFac f, T2 const *arena, T2 const *X, int64_t ldx, int64_t R, T2
   mark();
   if (flags & BFG_APPLY_ORIGINAL_ORDER) {
     ck(f->xbuf.ensure((size_t)p.numCols * R * sizeof(T2)), "gather buffer");
-    ck(bfg::launchGatherRows<T2>(X, ldx, f->srcPerm.as<int64_t>(), p.numCols, R,
-                                 f->xbuf.as<T2>(), s),
-       "gather");
+    if constexpr (std::is_same_v<T2, double2>) {
+      if (sys)
+        ck(bfg::launchGatherScaled(*sys, f->srcPerm.as<int64_t>(), p.numCols, f->xbuf.as<T2>(), s),
+           "gather");
+    }
+    if (!sys)
+      ck(bfg::launchGatherRows<T2>(X, ldx, f->srcPerm.as<int64_t>(), p.numCols, R,
+                                   f->xbuf.as<T2>(), s),
+         "gather");
     Xt = f->xbuf.as<T2>();
     ldxt = R;
     mark();
@@ -667,12 +674,12 @@ void runApply(bfgFac f, T2 const *arena, T2 const *X, int64_t ldx, int64_t R, T2
     ck(launchStage(f, st, arena, Xt, ldxt, W, R), "apply stage");
     mark();
   }
-  ck(bfg::launchApplyReduce<T2>(f->rowSeg.as<int32_t>(), f->segStart.as<int64_t>(),
-                                f->segContrib0.as<int64_t>(), f->segBase.as<int64_t>(), W, R, Y,
-                                ldy, p.numRows,
-                                (flags & BFG_APPLY_ORIGINAL_ORDER) ? f->tgtPerm.as<int64_t>()
-                                                                  : nullptr,
-                                s),
+  ck(bfg::launchApplyReduce(f->rowSeg.as<int32_t>(), f->segStart.as<int64_t>(),
+                            f->segContrib0.as<int64_t>(), f->segBase.as<int64_t>(),
+                            p.sumRows, W, R, Y, ldy, p.numRows,
+                            (flags & BFG_APPLY_ORIGINAL_ORDER) ? f->tgtPerm.as<int64_t>()
+                                                              : nullptr,
+                            s, 0, 0, sys),
      "apply reduce");
   mark();
 }
@@ -719,7 +726,7 @@ void ensureArenaDf(bfgFac f) {
 // Y.  Same launch count as runApply (the split stands in for its gather;
 // without BFG_APPLY_ORIGINAL_ORDER it is timed with the first stage).
 void runApplyDf(bfgFac f, double2 const *X, int64_t ldx, double2 *Y, int64_t ldy, uint32_t flags,
-                std::vector<cudaEvent_t> *events) {
+                std::vector<cudaEvent_t> *events, bfg::SystemTerms const *sys = nullptr) {
   cudaStream_t s = f->ctx->stream;
   bfg::ApplyProgram const &p = f->prog;
   ck(f->ws.ensure((size_t)std::max<int64_t>(1, p.wsRows) * sizeof(float4)), "workspace");
@@ -731,7 +738,9 @@ void runApplyDf(bfgFac f, double2 const *X, int64_t ldx, double2 *Y, int64_t ldy
   };
   bool const orig = (flags & BFG_APPLY_ORIGINAL_ORDER) != 0;
   mark();
-  ck(bfg::launchGatherToDf(X, ldx, orig ? f->srcPerm.as<int64_t>() : nullptr, p.numCols, Xd, s),
+  ck(sys ? bfg::launchGatherScaled(*sys, f->srcPerm.as<int64_t>(), p.numCols, Xd, s)
+         : bfg::launchGatherToDf(X, ldx, orig ? f->srcPerm.as<int64_t>() : nullptr, p.numCols, Xd,
+                                 s),
      "split X");
   if (orig) mark();
   size_t const nStages = f->stageItem0.size() - 1;
@@ -743,9 +752,10 @@ void runApplyDf(bfgFac f, double2 const *X, int64_t ldx, double2 *Y, int64_t ldy
        "apply stage");
     mark();
   }
-  ck(bfg::launchApplyReduceDf(f->rowSeg.as<int32_t>(), f->segStart.as<int64_t>(),
-                              f->segContrib0.as<int64_t>(), f->segBase.as<int64_t>(), W, Y, ldy,
-                              p.numRows, orig ? f->tgtPerm.as<int64_t>() : nullptr, s),
+  ck(bfg::launchApplyReduce(f->rowSeg.as<int32_t>(), f->segStart.as<int64_t>(),
+                            f->segContrib0.as<int64_t>(), f->segBase.as<int64_t>(),
+                            p.sumRows, W, 1, Y, ldy, p.numRows,
+                            orig ? f->tgtPerm.as<int64_t>() : nullptr, s, 0, 0, sys),
      "apply reduce");
   mark();
 }
@@ -915,12 +925,12 @@ void runApplyTc(bfgFac f, int terms, float2 const *X, int64_t ldx, int64_t R, fl
        "tensor-core apply stage");
     mark();
   }
-  ck(bfg::launchApplyReduce<float2>(f->rowSeg.as<int32_t>(), f->segStart.as<int64_t>(),
-                                    f->segContrib0.as<int64_t>(), f->segBase.as<int64_t>(), W, R,
-                                    Y, ldy, p.numRows,
-                                    (flags & BFG_APPLY_ORIGINAL_ORDER) ? f->tgtPerm.as<int64_t>()
-                                                                      : nullptr,
-                                    s, tiled ? rt : 0, tiled ? wTs : 0),
+  ck(bfg::launchApplyReduce(f->rowSeg.as<int32_t>(), f->segStart.as<int64_t>(),
+                            f->segContrib0.as<int64_t>(), f->segBase.as<int64_t>(),
+                            p.sumRows, W, R, Y, ldy, p.numRows,
+                            (flags & BFG_APPLY_ORIGINAL_ORDER) ? f->tgtPerm.as<int64_t>()
+                                                              : nullptr,
+                            s, tiled ? rt : 0, tiled ? wTs : 0),
      "apply reduce");
   mark();
 }
@@ -1002,6 +1012,23 @@ int64_t noAllocWorkspaceEntries(bfgFac f, int64_t R, uint32_t flags) {
   return e;
 }
 
+// A system's apply (SystemTerms) in FP64 or double-float: two launches fewer
+// than the scaling, the apply and the sum of the other terms one by one
+bfgStatus facApplySystem(bfgFac f, bfgPrecision prec, SystemTerms const &sys, double2 *Y) {
+  return guarded(f->ctx, [&]() -> bfgStatus {
+    if (prec == BFG_PRECISION_FP64) {
+      runApply<double2>(f, f->arena64.as<double2>(), nullptr, 1, 1, Y, 1,
+                        BFG_APPLY_ORIGINAL_ORDER, nullptr, &sys);
+    } else if (prec == BFG_PRECISION_DF64) {
+      ensureArenaDf(f);
+      runApplyDf(f, nullptr, 1, Y, 1, BFG_APPLY_ORIGINAL_ORDER, nullptr, &sys);
+    } else {
+      return fail(f->ctx, BFG_ERROR_NOT_IMPLEMENTED, "system apply: FP64 or DF64 only");
+    }
+    return BFG_OK;
+  });
+}
+
 int noAllocDevice(bfgFac f) { return f->ctx->device; }
 
 bfgStatus noAllocFail(bfgFac f, bfgStatus st, char const *msg) { return fail(f->ctx, st, msg); }
@@ -1024,9 +1051,9 @@ bfgStatus noAllocApplyFp64(bfgFac f, double2 const *X, int64_t ldx, int64_t R, d
     size_t const nStages = f->stageItem0.size() - 1;
     for (size_t st = 0; st < nStages; ++st)
       ck(launchStage(f, st, f->arena64.as<double2>(), Xt, ldxt, W, R), "apply stage");
-    ck(bfg::launchApplyReduce<double2>(
+    ck(bfg::launchApplyReduce(
            f->rowSeg.as<int32_t>(), f->segStart.as<int64_t>(), f->segContrib0.as<int64_t>(),
-           f->segBase.as<int64_t>(), W, R, Y, ldy, p.numRows,
+           f->segBase.as<int64_t>(), p.sumRows, W, R, Y, ldy, p.numRows,
            (flags & BFG_APPLY_ORIGINAL_ORDER) ? f->tgtPerm.as<int64_t>() : nullptr, s),
        "apply reduce");
     return BFG_OK;

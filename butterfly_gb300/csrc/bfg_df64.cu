@@ -149,29 +149,6 @@ applyGemvDfKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__res
   }
 }
 
-// Y row i (outPerm[i] if given) = sum over the row's segment terms, in FP64
-__global__ void applyReduceDfKernel(int32_t const *__restrict__ rowSeg,
-                                    int64_t const *__restrict__ segStart,
-                                    int64_t const *__restrict__ segContrib0,
-                                    int64_t const *__restrict__ segBase,
-                                    float4 const *__restrict__ W, double2 *__restrict__ Y,
-                                    int64_t ldy, int64_t nRows,
-                                    int64_t const *__restrict__ outPerm) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nRows;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    int const s = rowSeg[i];
-    int64_t const di = i - segStart[s];
-    double sr = 0, si = 0;
-    for (int64_t c = segContrib0[s]; c < segContrib0[s + 1]; ++c) {
-      float4 const v = W[segBase[c] + di];
-      sr += (double)v.x + (double)v.y;
-      si += (double)v.z + (double)v.w;
-    }
-    int64_t const oi = outPerm ? outPerm[i] : i;
-    Y[oi * ldy] = make_double2(sr, si);
-  }
-}
-
 int gridDf(int64_t n) {
   int64_t g = (n + 255) / 256;
   return (int)(g < 1 ? 1 : (g > 152 * 32 ? 152 * 32 : g));
@@ -197,15 +174,6 @@ cudaError_t launchApplyStageDf(ApplyItem const *items, int64_t nItems,
                                float4 const *X, float4 *W, cudaStream_t stream) {
   if (nItems == 0) return cudaSuccess;
   applyGemvDfKernel<<<(unsigned)nItems, 32 * kDfWarps, 0, stream>>>(items, contribs, arena, X, W);
-  return cudaGetLastError();
-}
-
-cudaError_t launchApplyReduceDf(int32_t const *rowSeg, int64_t const *segStart,
-                                int64_t const *segContrib0, int64_t const *segBase,
-                                float4 const *W, double2 *Y, int64_t ldy, int64_t nRows,
-                                int64_t const *outPerm, cudaStream_t stream) {
-  applyReduceDfKernel<<<gridDf(nRows), 256, 0, stream>>>(rowSeg, segStart, segContrib0, segBase,
-                                                         W, Y, ldy, nRows, outPerm);
   return cudaGetLastError();
 }
 

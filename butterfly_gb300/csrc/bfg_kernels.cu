@@ -973,46 +973,135 @@ __global__ void __launch_bounds__(32 * kRhsWarps) applyRhsKernel(
   }
 }
 
-template <typename T2>
-__global__ void applyReduceKernel(int32_t const *__restrict__ rowSeg,
-                                  int64_t const *__restrict__ segStart,
-                                  int64_t const *__restrict__ segContrib0,
-                                  int64_t const *__restrict__ segBase,
-                                  T2 const *__restrict__ W, int64_t R,
-                                  T2 *__restrict__ Y, int64_t ldy, int64_t nRows,
-                                  int64_t const *__restrict__ outPerm, int64_t wTile,
-                                  int64_t wTileStride) {
+__device__ __forceinline__ void addTerm(double &sr, double &si, double2 v) {
+  sr += v.x;
+  si += v.y;
+}
+__device__ __forceinline__ void addTerm(float &sr, float &si, float2 v) {
+  sr += v.x;
+  si += v.y;
+}
+__device__ __forceinline__ void addTerm(double &sr, double &si, float4 v) {   // double-float
+  sr += (double)v.x + (double)v.y;
+  si += (double)v.z + (double)v.w;
+}
+
+// The last sum and the input copy run with threadIdx.x over right-hand sides
+// (a power of two of them) and threadIdx.y over rows, so that nothing is
+// divided per element.  A row's terms (of type TW) are read four at a time,
+// and where the rows alone leave the chip idle (kSplit) eight warps share
+// them: one after the other, each waits for its base's load and its own
+// (2,073 rows, one right-hand side: 13.7 -> 6.6 us).  kSys adds a
+// boundary-integral system's other terms to the sum of the one right-hand
+// side, a row's corrections shared by the eight warps too (as a kernel of
+// its own, 9.4 us more).
+template <typename TW, typename T2, bool kSplit, bool kSys>
+__global__ void __launch_bounds__(256)
+    applyReduceKernel(int32_t const *__restrict__ rowSeg, int64_t const *__restrict__ segStart,
+                      int64_t const *__restrict__ segContrib0,
+                      int64_t const *__restrict__ segBase, TW const *__restrict__ W, int64_t R,
+                      T2 *Y, int64_t ldy, int64_t nRows, int64_t const *__restrict__ outPerm,
+                      int64_t wTile, int64_t wTileStride, SystemTerms sys) {
   using T = typename Real<T2>::T;
-  int64_t const total = nRows * R;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    int64_t const i = e / R, r = e % R;
-    int const s = rowSeg[i];
-    int64_t const di = i - segStart[s];
-    // W row-major (ld R), or tile-major: panels of wTile columns
-    T2 const *Wc = wTile ? W + (r / wTile) * wTileStride + r % wTile : W + r;
-    int64_t const ldw = wTile ? wTile : R;
-    T sr = 0, si = 0;
-    for (int64_t c = segContrib0[s]; c < segContrib0[s + 1]; ++c) {
-      T2 const v = Wc[(segBase[c] + di) * ldw];
-      sr += v.x;
-      si += v.y;
+  constexpr int U = 4, kParts = kSplit ? 8 : 1;
+  __shared__ T2 part[kParts][32];
+  int const z = kSplit ? threadIdx.z : 0;
+  int64_t const ld = wTile ? wTile : R;
+  int64_t const step = (int64_t)gridDim.x * blockDim.y;
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.y; i0 < nRows; i0 += step) {
+    int64_t const i = i0 + threadIdx.y;
+    bool const live = i < nRows;
+    int64_t di = 0, c0 = 0, c1 = 0, o = i;
+    if (live) {
+      int const s = rowSeg[i];
+      di = i - segStart[s];
+      c0 = segContrib0[s];
+      c1 = segContrib0[s + 1];
+      if (outPerm) o = outPerm[i];
     }
-    int64_t const oi = outPerm ? outPerm[i] : i;
-    Y[oi * ldy + r] = mk2<T2>(sr, si);
+    for (int64_t r0 = 0; r0 < R; r0 += blockDim.x) {
+      int64_t const r = r0 + threadIdx.x;
+      bool const mine = live && r < R;
+      T sr = 0, si = 0;
+      if (mine) {
+        // W row-major (ld R), or tile-major: panels of wTile (16 or 32) columns
+        TW const *Wc = (wTile ? W + (r >> (wTile == 16 ? 4 : 5)) * wTileStride + (r & (wTile - 1))
+                              : W + r) + di * ld;
+        for (int64_t c = c0 + z; c < c1; c += U * kParts) {
+          TW v[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            int64_t const cu = c + u * kParts;
+            v[u] = Wc[segBase[cu < c1 ? cu : c] * ld];
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (c + u * kParts < c1) addTerm(sr, si, v[u]);
+        }
+        if constexpr (kSys) {
+          for (int q = z; q < sys.nc; q += kParts) {
+            double2 const c = sys.val[o * sys.nc + q], v = sys.xw[sys.col[o * sys.nc + q]];
+            sr += c.x * v.x - c.y * v.y;
+            si += c.x * v.y + c.y * v.x;
+          }
+          if (z == 0) {
+            double2 const v = sys.x[o];
+            sr += sys.shift * v.x;
+            si += sys.shift * v.y;
+          }
+        }
+      }
+      if (kSplit) {
+        int const l = threadIdx.y * blockDim.x + threadIdx.x;
+        part[z][l] = mk2<T2>(sr, si);
+        __syncthreads();
+        if (z == 0) {
+#pragma unroll
+          for (int q = 1; q < kParts; ++q) {
+            sr += part[q][l].x;
+            si += part[q][l].y;
+          }
+        }
+        __syncthreads();
+      }
+      if (z == 0 && mine) Y[o * ldy + r] = mk2<T2>(sr, si);
+    }
+  }
+}
+
+__device__ __forceinline__ void storeAs(double2 v, double2 *out) { *out = v; }
+__device__ __forceinline__ void storeAs(double2 v, float4 *out) {
+  float const xh = (float)v.x, yh = (float)v.y;
+  *out = make_float4(xh, (float)(v.x - (double)xh), yh, (float)(v.y - (double)yh));
+}
+
+// the input of a system's apply: xw = w x, and the same in tree order
+template <typename TO>
+__global__ void gatherScaledKernel(SystemTerms sys, int64_t const *__restrict__ perm, int64_t n,
+                                   TO *__restrict__ out) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    int64_t const p = perm[i];
+    double const w = sys.w[p];
+    double2 const x = sys.x[p], v = make_double2(w * x.x, w * x.y);
+    sys.xw[p] = v;
+    storeAs(v, out + i);
   }
 }
 
 template <typename T2>
-__global__ void gatherRowsKernel(T2 const *X, int64_t ldx, int64_t const *perm,
-                                 int64_t nRows, int64_t R, T2 *out, int64_t outTile,
-                                 int64_t outTileStride) {
-  int64_t const total = nRows * R;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    int64_t const i = e / R, r = e % R;
-    int64_t const o = outTile ? (r / outTile) * outTileStride + i * outTile + r % outTile : e;
-    out[o] = X[(perm ? perm[i] : i) * ldx + r];
+__global__ void gatherRowsKernel(T2 const *__restrict__ X, int64_t ldx,
+                                 int64_t const *__restrict__ perm, int64_t nRows, int64_t R,
+                                 T2 *__restrict__ out, int64_t outTile, int64_t outTileStride) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.y + threadIdx.y; i < nRows;
+       i += (int64_t)gridDim.x * blockDim.y) {
+    T2 const *x = X + (perm ? perm[i] : i) * ldx;
+    for (int64_t r = threadIdx.x; r < R; r += blockDim.x) {
+      int64_t const o = outTile ? (r >> (outTile == 16 ? 4 : 5)) * outTileStride + i * outTile +
+                                      (r & (outTile - 1))
+                                : i * R + r;
+      out[o] = x[r];
+    }
   }
 }
 
@@ -1025,6 +1114,18 @@ cudaError_t launchRhs(ApplyItem const *items, int64_t nItems, ApplyContrib const
   applyRhsKernel<RT><<<(unsigned)(nItems * tiles), 32 * kRhsWarps, 0, stream>>>(
       items, contribs, arena, X, ldx, W, R, (unsigned)tiles);
   return cudaGetLastError();
+}
+
+// Eight warps share a row's terms where the rows have eight of them on
+// average and are few: 15,346 points on 64 circles 19 us, 26 unshared; but
+// 65,536 points with three terms a row 13 us, 5.5 unshared
+constexpr int64_t kReduceSplitOut = 1 << 17, kReduceSplitTerms = 8;
+
+// 128 threads over (right-hand sides, rows): all right-hand sides up to 64
+dim3 rowBlock(int64_t R) {
+  unsigned x = 1;
+  while (x < 64 && x < R) x *= 2;
+  return dim3(x, 128 / x);
 }
 
 int gridFor(int64_t total, int threads) {
@@ -1193,34 +1294,70 @@ cudaError_t launchApplyStage(ApplyItem const *items, int64_t nItems,
   return launchRhs<16>(items, nItems, contribs, arena, X, ldx, W, R, stream);
 }
 
-template <typename T2>
+template <typename TW, typename T2>
 cudaError_t launchApplyReduce(int32_t const *rowSeg, int64_t const *segStart,
                               int64_t const *segContrib0, int64_t const *segBase,
-                              T2 const *W, int64_t R, T2 *Y, int64_t ldy,
+                              int64_t nTerms, TW const *W, int64_t R, T2 *Y, int64_t ldy,
                               int64_t nRows, int64_t const *outPerm,
-                              cudaStream_t stream, int64_t wTile, int64_t wTileStride) {
-  applyReduceKernel<T2><<<gridFor(nRows * R, 256), 256, 0, stream>>>(
-      rowSeg, segStart, segContrib0, segBase, W, R, Y, ldy, nRows, outPerm, wTile, wTileStride);
+                              cudaStream_t stream, int64_t wTile, int64_t wTileStride,
+                              SystemTerms const *sys) {
+  if (wTile != 0 && wTile != 16 && wTile != 32) return cudaErrorInvalidValue;
+  if (sys && R != 1) return cudaErrorInvalidValue;
+  bool const split = nRows * R < kReduceSplitOut && nTerms >= kReduceSplitTerms * nRows;
+  dim3 block = rowBlock(R);
+  if (split) {
+    unsigned const x = block.x < 32 ? block.x : 32;
+    block = dim3(x, 32 / x, 8);
+  }
+  auto run = [&](auto kernel) {
+    kernel<<<gridFor(nRows, block.y), block, 0, stream>>>(
+        rowSeg, segStart, segContrib0, segBase, W, R, Y, ldy, nRows, outPerm, wTile, wTileStride,
+        sys ? *sys : SystemTerms{});
+  };
+  if constexpr (std::is_same_v<T2, double2>) {
+    if (sys) {
+      if (split) run(applyReduceKernel<TW, T2, true, true>);
+      else run(applyReduceKernel<TW, T2, false, true>);
+      return cudaGetLastError();
+    }
+  }
+  if (split) run(applyReduceKernel<TW, T2, true, false>);
+  else run(applyReduceKernel<TW, T2, false, false>);
   return cudaGetLastError();
 }
+
+template <typename TO>
+cudaError_t launchGatherScaled(SystemTerms const &sys, int64_t const *perm, int64_t n, TO *out,
+                               cudaStream_t stream) {
+  if (n == 0) return cudaSuccess;
+  gatherScaledKernel<TO><<<gridFor(n, 64), 64, 0, stream>>>(sys, perm, n, out);
+  return cudaGetLastError();
+}
+template cudaError_t launchGatherScaled<double2>(SystemTerms const &, int64_t const *, int64_t,
+                                                 double2 *, cudaStream_t);
+template cudaError_t launchGatherScaled<float4>(SystemTerms const &, int64_t const *, int64_t,
+                                                float4 *, cudaStream_t);
 
 template <typename T2>
 cudaError_t launchGatherRows(T2 const *X, int64_t ldx, int64_t const *perm,
                              int64_t nRows, int64_t R, T2 *out, cudaStream_t stream,
                              int64_t outTile, int64_t outTileStride) {
-  gatherRowsKernel<T2><<<gridFor(nRows * R, 256), 256, 0, stream>>>(X, ldx, perm, nRows, R,
-                                                                    out, outTile, outTileStride);
+  if (outTile != 0 && outTile != 16 && outTile != 32) return cudaErrorInvalidValue;
+  dim3 const block = rowBlock(R);
+  gatherRowsKernel<T2><<<gridFor(nRows, block.y), block, 0, stream>>>(X, ldx, perm, nRows, R, out,
+                                                                      outTile, outTileStride);
   return cudaGetLastError();
 }
 
-template cudaError_t launchApplyReduce<double2>(int32_t const *, int64_t const *, int64_t const *,
-                                                int64_t const *, double2 const *, int64_t,
-                                                double2 *, int64_t, int64_t, int64_t const *,
-                                                cudaStream_t, int64_t, int64_t);
-template cudaError_t launchApplyReduce<float2>(int32_t const *, int64_t const *, int64_t const *,
-                                               int64_t const *, float2 const *, int64_t, float2 *,
-                                               int64_t, int64_t, int64_t const *, cudaStream_t,
-                                               int64_t, int64_t);
+template cudaError_t launchApplyReduce<double2, double2>(
+    int32_t const *, int64_t const *, int64_t const *, int64_t const *, int64_t, double2 const *, int64_t,
+    double2 *, int64_t, int64_t, int64_t const *, cudaStream_t, int64_t, int64_t, SystemTerms const *);
+template cudaError_t launchApplyReduce<float2, float2>(
+    int32_t const *, int64_t const *, int64_t const *, int64_t const *, int64_t, float2 const *, int64_t,
+    float2 *, int64_t, int64_t, int64_t const *, cudaStream_t, int64_t, int64_t, SystemTerms const *);
+template cudaError_t launchApplyReduce<float4, double2>(
+    int32_t const *, int64_t const *, int64_t const *, int64_t const *, int64_t, float4 const *, int64_t,
+    double2 *, int64_t, int64_t, int64_t const *, cudaStream_t, int64_t, int64_t, SystemTerms const *);
 template cudaError_t launchGatherRows<double2>(double2 const *, int64_t, int64_t const *, int64_t,
                                                int64_t, double2 *, cudaStream_t, int64_t, int64_t);
 template cudaError_t launchGatherRows<float2>(float2 const *, int64_t, int64_t const *, int64_t,

@@ -122,17 +122,13 @@ cudaError_t launchBessel01(double const *x, int64_t n, double *out, cudaStream_t
 // FP64 -> FP32 arena conversion (same layout)
 cudaError_t launchArenaToF32(double2 const *a64, float2 *a32, int64_t n, cudaStream_t stream);
 // double-float apply of one right-hand side (bfg_df64.cu): arena split, input split (and gather),
-// stage, final sum into complex128
+// stage
 cudaError_t launchArenaToDf(double2 const *a64, float4 *adf, int64_t n, cudaStream_t stream);
 cudaError_t launchGatherToDf(double2 const *X, int64_t ldx, int64_t const *perm, int64_t nRows,
                              float4 *out, cudaStream_t stream);
 cudaError_t launchApplyStageDf(ApplyItem const *items, int64_t nItems,
                                ApplyContrib const *contribs, float4 const *arena,
                                float4 const *X, float4 *W, cudaStream_t stream);
-cudaError_t launchApplyReduceDf(int32_t const *rowSeg, int64_t const *segStart,
-                                int64_t const *segContrib0, int64_t const *segBase,
-                                float4 const *W, double2 *Y, int64_t ldy, int64_t nRows,
-                                int64_t const *outPerm, cudaStream_t stream);
 
 // complex128 <-> complex64 matrix conversion (row-major, leading dims)
 // (bTile > 0: b tile-major, panel t of bTile columns at b + t bTileStride,
@@ -158,14 +154,35 @@ cudaError_t launchApplyStageFixed(ApplyItem const *items, int64_t nItems,
                                   double2 const *arena, double2 const *X, int64_t ldx, double2 *W,
                                   int64_t R, cudaStream_t stream);
 
-// W row-major with leading dimension R, or (wTile > 0) tile-major: panel t
-// of wTile columns at W + t wTileStride, leading dimension wTile
-template <typename T2>
+// A boundary-integral system around one FP64 or double-float apply of one
+// right-hand side in original point order (y = shift x + K xw + C xw with
+// xw = diag(w) x): the gather forms xw, the last sum adds the other terms.
+// C has nc entries a row.  y may be x.
+struct SystemTerms {
+  double const *w = nullptr;
+  double2 const *x = nullptr;
+  double2 *xw = nullptr;
+  double shift = 0.0;
+  double2 const *val = nullptr;
+  int64_t const *col = nullptr;
+  int nc = 0;
+};
+// out[i] = xw[perm[i]] = w x (TO = float4: split into double-float)
+template <typename TO>
+cudaError_t launchGatherScaled(SystemTerms const &sys, int64_t const *perm, int64_t n, TO *out,
+                               cudaStream_t stream);
+
+// The final sum.  W row-major with leading dimension R, or (wTile > 0)
+// tile-major: panel t of wTile columns at W + t wTileStride, leading dimension
+// wTile; of type T2, or double-float (float4, R = 1) with T2 = double2.
+// nTerms: the rows' terms, all told.
+template <typename TW, typename T2>
 cudaError_t launchApplyReduce(int32_t const *rowSeg, int64_t const *segStart,
                               int64_t const *segContrib0, int64_t const *segBase,
-                              T2 const *W, int64_t R, T2 *Y, int64_t ldy,
+                              int64_t nTerms, TW const *W, int64_t R, T2 *Y, int64_t ldy,
                               int64_t nRows, int64_t const *outPerm,
-                              cudaStream_t stream, int64_t wTile = 0, int64_t wTileStride = 0);
+                              cudaStream_t stream, int64_t wTile = 0, int64_t wTileStride = 0,
+                              SystemTerms const *sys = nullptr);
 
 // Split-BF16 tensor-core apply (terms = 2 or 3 bf16 planes).
 // sets the kernels' shared-memory limit; returns resident CTAs per SM

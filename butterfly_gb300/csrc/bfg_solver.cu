@@ -123,28 +123,6 @@ __global__ void krEntriesKernel(int64_t n, int64_t const *curveOf, int64_t const
   }
 }
 
-__global__ void scaleKernel(int64_t n, double const *w, double2 const *x, double2 *xw) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    xw[i] = make_double2(w[i] * x[i].x, w[i] * x[i].y);
-}
-
-// y = shift x + Kxw + C xw
-__global__ void systemPostKernel(int64_t n, double shift, double2 const *x, double2 const *xw,
-                                 double2 const *kxw, double2 const *val, int64_t const *col,
-                                 int nc, double2 *y) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    double sr = shift * x[i].x + kxw[i].x, si = shift * x[i].y + kxw[i].y;
-    for (int q = 0; q < nc; ++q) {
-      double2 const c = val[i * nc + q], v = xw[col[i * nc + q]];
-      sr += c.x * v.x - c.y * v.y;
-      si += c.x * v.y + c.y * v.x;
-    }
-    y[i] = make_double2(sr, si);
-  }
-}
-
 // dense diagonal block of A for every curve, row-major n_b x n_b at blkOff[b]
 __global__ void diagBlocksKernel(int64_t const *offsets, int64_t const *blkOff, double const *x,
                                  double const *y, double const *nx, double const *ny,
@@ -702,7 +680,6 @@ bfgStatus bfgSystemCreate(bfgContext ctx, bfgFac fac, bfgHelm2 const *helm, doub
     SYS_CK(sys->dX.alloc(4 * n * 8));
     SYS_CK(sys->dW.alloc(n * 8));
     SYS_CK(sys->tmpXw.alloc(n * 16));
-    SYS_CK(sys->tmpK.alloc(n * 16));
     SYS_CK(cudaMemcpyAsync(sys->dOffsets.p, curveOffsets, (numCurves + 1) * 8, cudaMemcpyHostToDevice, s));
     SYS_CK(cudaMemcpyAsync(sys->dCurveOf.p, curveOf.data(), n * 8, cudaMemcpyHostToDevice, s));
     SYS_CK(cudaMemcpyAsync(sys->dX.p, planes.data(), 4 * n * 8, cudaMemcpyHostToDevice, s));
@@ -758,19 +735,16 @@ bfgStatus bfgSystemSetApplyPrecision(bfgSystem sys, bfgPrecision prec) {
 
 namespace {
 bfgStatus systemApply(bfgSystem sys, bfgPrecision prec, void const *X, void *Y) {
-  cudaStream_t s = sys->stream();
-  int64_t const n = sys->n;
-  double2 const *x = static_cast<double2 const *>(X);
-  double2 *xw = sys->tmpXw.as<double2>(), *kxw = sys->tmpK.as<double2>();
-  scaleKernel<<<gridFor(n, 256), 256, 0, s>>>(n, sys->dW.as<double>(), x, xw);
-  SYS_CK(cudaGetLastError());
-  bfgStatus st = bfgFacApply(sys->fac, prec, xw, 1, 1, kxw, 1, BFG_APPLY_ORIGINAL_ORDER);
+  bfg::SystemTerms t;
+  t.w = sys->dW.as<double>();
+  t.x = static_cast<double2 const *>(X);
+  t.xw = sys->tmpXw.as<double2>();
+  t.shift = sys->shift;
+  t.val = sys->dKrVal.as<double2>();
+  t.col = sys->dKrCol.as<int64_t>();
+  t.nc = 2 * sys->order;
+  bfgStatus st = bfg::facApplySystem(sys->fac, prec, t, static_cast<double2 *>(Y));
   if (st != BFG_OK) return sysFail(sys, st, "system apply: butterfly apply failed");
-  systemPostKernel<<<gridFor(n, 256), 256, 0, s>>>(n, sys->shift, x, xw, kxw,
-                                                   sys->dKrVal.as<double2>(),
-                                                   sys->dKrCol.as<int64_t>(), 2 * sys->order,
-                                                   static_cast<double2 *>(Y));
-  SYS_CK(cudaGetLastError());
   return BFG_OK;
 }
 }  // namespace

@@ -53,7 +53,7 @@ struct bfgSystem_s {
   std::vector<int64_t> offsets;
   std::vector<double> weights;                   // host copy (coarse mode counts)
   Dev dOffsets, dCurveOf, dX, dW, dKrVal, dKrCol;
-  Dev tmpXw, tmpK;
+  Dev tmpXw;
   // block-Jacobi
   bool haveBj = false, haveBj64 = false;   // the FP32 inverses; the FP64 ones (on first use)
   std::vector<int64_t> blkOff;
@@ -76,6 +76,8 @@ struct bfgSystem_s {
 };
 
 namespace bfg {
+// one apply of a factorization inside a system (bfg_api.cpp)
+bfgStatus facApplySystem(bfgFac f, bfgPrecision prec, SystemTerms const &sys, double2 *Y);
 // A X for one device complex128 vector with the butterfly part in `prec`
 bfgStatus systemApplyPrec(bfgSystem sys, bfgPrecision prec, void const *X, void *Y);
 // z = M_bj r from the FP32 block inverses (block-Jacobi built)

@@ -171,3 +171,31 @@ def test_fp32_tiles_are_within_their_bound(m, n):
     for R in (2, 3, 4, 5, 8, 9, 16, 17, 33):
         y = fac.apply(torch.from_numpy(X[:, :R].copy()).cuda(), precision="fp32").cpu().numpy()
         assert np.all(np.abs(y.astype(LD) - Y[:, :R]) <= bound[:, :R])
+
+
+@pytest.mark.parametrize("n,onto_itself", [(33, False), (1153, False), (1153, True)])
+def test_wide_and_narrow_applies_agree(n, onto_itself):
+    """The input copy and the final sum (bfg_kernels.cu) share a row's terms
+    between warps or not by the number of outputs and of terms (many for a
+    curve onto itself), with every width of their thread blocks: both against the FP64 apply of single columns, whose
+    results FP64 repeats to a few units of 2^-51 of the sums of moduli (1e-12
+    of the norm with the multi-level factors' growth) and FP32 and three bf16
+    planes to a few 1e-6."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from conftest import rel_err
+    tgt = B.curve_points("ellipse", n)
+    fac = B.FacHelm2.make_multilevel(
+        B.Helm2(9.0),
+        B.Quadtree(tgt if onto_itself else B.uniform_square_points(n, 3), leaf_size=32),
+        B.Quadtree(tgt, leaf_size=32), context=B.default_context(0))
+    X = torch.from_numpy(B.Rng(n).complex_randn(n * 130).reshape(n, 130)).cuda()
+    for orig in (False, True):
+        cols = [fac.apply(X[:, i].contiguous(), original_order=orig).cpu().numpy()
+                for i in range(130)]
+        exact = np.stack(cols, 1)
+        for R in (1, 2, 3, 7, 16, 33, 64, 113, 114, 130):
+            for prec, tol in (("fp64", 1e-11), ("fp32", 2e-5), ("bf16x3", 2e-5)):
+                x = X[:, :R].to(torch.complex128 if prec == "fp64" else torch.complex64)
+                y = fac.apply(x.contiguous(), precision=prec, original_order=orig)
+                assert rel_err(y.cpu().numpy().astype(complex), exact[:, :R]) < tol
