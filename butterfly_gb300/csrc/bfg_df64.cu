@@ -26,7 +26,7 @@
 namespace bfg {
 namespace {
 
-constexpr int kDfWarps = 8;
+constexpr int kDfWarps = 4;
 
 // The _rn intrinsics are never contracted into FMAs, which would break the
 // error-free transformations.
@@ -84,8 +84,14 @@ __global__ void gatherToDfKernel(double2 const *__restrict__ X, int64_t ldx,
     out[i] = dfSplit(X[(perm ? perm[i] : i) * ldx]);
 }
 
-// One CTA per item: lane = item row, the 8 warps take every 8th column with 4
-// entries in flight each; the warps' sums are combined in a fixed order.
+// One CTA per item: lane = item row, the 4 warps take every 4th column with 4
+// entries in flight each, read past the caches (the input rows stay); the
+// warps' sums are combined in a fixed order.  Bound by the latency of the
+// loads: an item lasts about 7 us of which a few are its descriptors' chain,
+// so that 8 warps with half the columns each took 79 us where this takes 73
+// (a product of 15,346 points on 64 circles, 4 launches of 1.2 GB in all;
+// HBM alone 44).  Fetching a batch ahead cost more registers than it hid
+// (93 us).
 __global__ void __launch_bounds__(32 * kDfWarps)
 applyGemvDfKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restrict__ contribs,
                   float4 const *__restrict__ arena, float4 const *__restrict__ X,
@@ -113,10 +119,10 @@ applyGemvDfKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__res
     for (; j + 3 * S < n; j += 4 * S) {
       float4 a0, a1, a2, a3;
       if (active) {
-        a0 = a[(int64_t)(j + 0 * S) * lda];
-        a1 = a[(int64_t)(j + 1 * S) * lda];
-        a2 = a[(int64_t)(j + 2 * S) * lda];
-        a3 = a[(int64_t)(j + 3 * S) * lda];
+        a0 = __ldcs(a + (int64_t)(j + 0 * S) * lda);
+        a1 = __ldcs(a + (int64_t)(j + 1 * S) * lda);
+        a2 = __ldcs(a + (int64_t)(j + 2 * S) * lda);
+        a3 = __ldcs(a + (int64_t)(j + 3 * S) * lda);
       } else {
         a0 = a1 = a2 = a3 = make_float4(0.f, 0.f, 0.f, 0.f);
       }
@@ -128,7 +134,7 @@ applyGemvDfKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__res
       mac(a3, x3);
     }
     for (; j < n; j += S) {
-      float4 const a0 = active ? a[(int64_t)j * lda] : make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 const a0 = active ? __ldcs(a + (int64_t)j * lda) : make_float4(0.f, 0.f, 0.f, 0.f);
       mac(a0, x[j]);
     }
   }
