@@ -331,38 +331,75 @@ __global__ void putRowsKernel(float2 *A, int64_t D, int64_t c0, int m, float2 co
   }
 }
 
-// ---- per-iteration kernels
-// cin[c0 + m] = sum_j conj(Phi_b[j, m]) r[off_b + j]  (one CTA per curve)
-__global__ void coarseRestrictKernel(int64_t const *offsets, int64_t const *cStart,
-                                     int64_t const *tabOff, float2 const *tab, double2 const *r,
-                                     float2 *cin) {
-  int const b = blockIdx.x;
-  int64_t const o = offsets[b], n = offsets[b + 1] - o, c0 = cStart[b];
-  int const M = (int)(cStart[b + 1] - c0);
-  float2 const *t = tab + tabOff[b];
-  for (int m = threadIdx.x; m < M; m += blockDim.x) {
-    double sr = 0.0, si = 0.0;
-    for (int64_t j = 0; j < n; ++j) {
-      float2 const p = t[j * M + m];
-      double2 const v = r[o + j];
-      sr += (double)p.x * v.x + (double)p.y * v.y;
-      si += (double)p.x * v.y - (double)p.y * v.x;
+constexpr int kModeTile = 8, kRestrictWarps = 4;
+
+// A float's double by moving its bits: the conversion instruction runs at the
+// rate of the few FP64 units, which bound the kernels below.  Zeros,
+// subnormals, infinities and NaNs are converted.
+__device__ __forceinline__ double widen(float f) {
+  uint32_t const u = __float_as_uint(f);
+  if (((u >> 23) + 1 & 0xFFu) < 2u) return f;
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7FFFFFFFu) >> 3) + 0x38000000u)),
+                          (int)(u << 29));
+}
+
+// cin[c0 + m] = sum_j conj(Phi_b[j, m]) r[off_b + j]: a CTA takes 8 modes of
+// one curve (whole sectors of the table), its quarter warps every 16th point.
+// Bound by the FP64 units (4 FMAs a table entry); one thread a mode over all points was a
+// serial chain of loads (64 circles, 15,346 points: 22 us, 193 before).
+__global__ void __launch_bounds__(32 * kRestrictWarps)
+    coarseRestrictKernel(int64_t const *offsets, int64_t const *cStart, int64_t const *tabOff,
+                         float2 const *tab, double2 const *r, float2 *cin, int tiles) {
+  constexpr int kSlices = 32 * kRestrictWarps / kModeTile;
+  __shared__ double2 part[kSlices][kModeTile];
+  int const b = blockIdx.x / tiles, tile = blockIdx.x % tiles;
+  int const lm = threadIdx.x % kModeTile, sl = threadIdx.x / kModeTile;
+  int64_t const o = offsets[b], c0 = cStart[b];
+  int const n = (int)(offsets[b + 1] - o), M = (int)(cStart[b + 1] - c0);
+  int const m = tile * kModeTile + lm;
+  if (tile * kModeTile >= M) return;
+  float2 const *t = tab + tabOff[b] + min(m, M - 1);
+  double sr = 0.0, si = 0.0;
+#pragma unroll 4
+  for (int j = sl; j < n; j += kSlices) {
+    float2 const p = t[(int64_t)j * M];
+    double2 const v = r[o + j];
+    double const px = widen(p.x), py = widen(p.y);
+    sr = fma(py, v.y, fma(px, v.x, sr));
+    si = fma(-py, v.x, fma(px, v.y, si));
+  }
+  part[sl][lm] = make_double2(sr, si);
+  __syncthreads();
+  if (sl == 0 && m < M) {
+    sr = si = 0.0;
+#pragma unroll
+    for (int q = 0; q < kSlices; ++q) {
+      sr += part[q][lm].x;
+      si += part[q][lm].y;
     }
     cin[c0 + m] = make_float2((float)sr, (float)si);
   }
 }
 
-// cout = Ainv cin (D x D row-major): one warp per row
+// cout = Ainv cin (D x D row-major): one warp per row, 8 loads in flight
 __global__ void coarseGemvKernel(int64_t D, float2 const *Ainv, float2 const *cin, float2 *cout) {
+  constexpr int U = 8;
   int64_t const row = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
   int const lane = threadIdx.x & 31;
   if (row >= D) return;
   float2 const *a = Ainv + row * D;
   float sr = 0.f, si = 0.f;
-  for (int64_t c = lane; c < D; c += 32) {
-    float2 const v = a[c], x = cin[c];
-    sr = fmaf(v.x, x.x, fmaf(-v.y, x.y, sr));
-    si = fmaf(v.x, x.y, fmaf(v.y, x.x, si));
+  for (int64_t c0 = lane; c0 < D; c0 += 32 * U) {
+    float2 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = __ldcs(a + (c0 + 32 * u < D ? c0 + 32 * u : c0));
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c0 + 32 * u < D) {
+        float2 const x = cin[c0 + 32 * u];
+        sr = fmaf(v[u].x, x.x, fmaf(-v[u].y, x.y, sr));
+        si = fmaf(v[u].x, x.y, fmaf(v[u].y, x.x, si));
+      }
   }
   for (int o = 16; o > 0; o >>= 1) {
     sr += __shfl_down_sync(0xffffffffu, sr, o);
@@ -371,29 +408,43 @@ __global__ void coarseGemvKernel(int64_t D, float2 const *Ainv, float2 const *ci
   if (lane == 0) cout[row] = make_float2(sr, si);
 }
 
-// z[off_b + j] = sum_m Phi_b[j, m] cout[c0 + m]  (one CTA per curve)
-__global__ void coarseProlongKernel(int64_t const *offsets, int64_t const *cStart,
-                                    int64_t const *tabOff, float2 const *tab, float2 const *cout,
-                                    double2 *z) {
-  int const b = blockIdx.x;
+// z[off_b + j] = sum_m Phi_b[j, m] cout[c0 + m]: a CTA takes 32 points of one
+// curve, four lanes a point (whole sectors of the table), every fourth mode
+// each; the curve's coefficients are converted once (64 circles, 15,346
+// points: 22.5 us, 97 with one thread a point).
+constexpr int kProlongRows = 32, kProlongTiles = 256;
+__global__ void __launch_bounds__(4 * kProlongRows)
+    coarseProlongKernel(int64_t const *offsets, int64_t const *cStart, int64_t const *tabOff,
+                        float2 const *tab, float2 const *cout, double2 *z, int tiles) {
+  __shared__ double2 y[kMaxModes];
+  int const b = blockIdx.x / tiles, tile = blockIdx.x % tiles;
   int64_t const o = offsets[b], n = offsets[b + 1] - o, c0 = cStart[b];
   int const M = (int)(cStart[b + 1] - c0);
-  float2 const *t = tab + tabOff[b];
-  for (int64_t j = threadIdx.x; j < n; j += blockDim.x) {
-    double sr = 0.0, si = 0.0;
-    for (int m = 0; m < M; ++m) {
-      float2 const p = t[j * M + m], y = cout[c0 + m];
-      sr += (double)p.x * y.x - (double)p.y * y.y;
-      si += (double)p.x * y.y + (double)p.y * y.x;
-    }
-    z[o + j] = make_double2(sr, si);
+  if ((int64_t)tile * kProlongRows >= n) return;
+  for (int m = threadIdx.x; m < M; m += blockDim.x) {
+    float2 const v = cout[c0 + m];
+    y[m] = make_double2(v.x, v.y);
   }
-}
-
-__global__ void addToKernel(int64_t n, double2 const *x, double2 *y) {   // y += x
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = make_double2(y[i].x + x[i].x, y[i].y + x[i].y);
+  __syncthreads();
+  int const q = threadIdx.x % 4;
+  for (int64_t j0 = (int64_t)tile * kProlongRows; j0 < n; j0 += (int64_t)tiles * kProlongRows) {
+    int64_t const j = j0 + threadIdx.x / 4;
+    float2 const *t = tab + tabOff[b] + (j < n ? j : n - 1) * M;
+    double sr = 0.0, si = 0.0;
+#pragma unroll 4
+    for (int m = q; m < M; m += 4) {
+      float2 const p = t[m];
+      double const px = widen(p.x), py = widen(p.y);
+      sr = fma(-py, y[m].y, fma(px, y[m].x, sr));
+      si = fma(py, y[m].x, fma(px, y[m].y, si));
+    }
+#pragma unroll
+    for (int s = 1; s < 4; s *= 2) {
+      sr += __shfl_xor_sync(0xffffffffu, sr, s);
+      si += __shfl_xor_sync(0xffffffffu, si, s);
+    }
+    if (q == 0 && j < n) z[o + j] = make_double2(sr, si);
+  }
 }
 
 unsigned gridOf(int64_t n, int t) {
@@ -415,15 +466,19 @@ cudaError_t runGemm(CGemm const *host, int nb, int maxM, int maxN, Dev &dDesc, c
 void coarseCorrection(bfgSystem sys, double2 const *r, double2 *z, cudaStream_t s) {
   int const nb = (int)sys->numCurves;
   int64_t const D = sys->coarseDim;
-  coarseRestrictKernel<<<nb, 128, 0, s>>>(sys->dOffsets.as<int64_t>(), sys->dCStart.as<int64_t>(),
-                                          sys->dTabOff.as<int64_t>(), sys->dTab.as<float2>(), r,
-                                          sys->dCoarseIn.as<float2>());
+  int64_t maxM = 1;
+  for (int b = 0; b < nb; ++b) maxM = std::max(maxM, sys->cStart[b + 1] - sys->cStart[b]);
+  int const mTiles = (int)((maxM + kModeTile - 1) / kModeTile);
+  int const jTiles = (int)std::min<int64_t>((sys->maxCurve + kProlongRows - 1) / kProlongRows, kProlongTiles);
+  coarseRestrictKernel<<<(unsigned)nb * mTiles, 32 * kRestrictWarps, 0, s>>>(
+      sys->dOffsets.as<int64_t>(), sys->dCStart.as<int64_t>(), sys->dTabOff.as<int64_t>(),
+      sys->dTab.as<float2>(), r, sys->dCoarseIn.as<float2>(), mTiles);
   coarseGemvKernel<<<(unsigned)((D + 7) / 8), 256, 0, s>>>(D, sys->dAcInv.as<float2>(),
                                                           sys->dCoarseIn.as<float2>(),
                                                           sys->dCoarseOut.as<float2>());
-  coarseProlongKernel<<<nb, 256, 0, s>>>(sys->dOffsets.as<int64_t>(), sys->dCStart.as<int64_t>(),
-                                         sys->dTabOff.as<int64_t>(), sys->dTab.as<float2>(),
-                                         sys->dCoarseOut.as<float2>(), z);
+  coarseProlongKernel<<<(unsigned)nb * jTiles, 4 * kProlongRows, 0, s>>>(
+      sys->dOffsets.as<int64_t>(), sys->dCStart.as<int64_t>(), sys->dTabOff.as<int64_t>(),
+      sys->dTab.as<float2>(), sys->dCoarseOut.as<float2>(), z, jTiles);
 }
 
 }  // namespace
@@ -431,16 +486,13 @@ void coarseCorrection(bfgSystem sys, double2 const *r, double2 *z, cudaStream_t 
 namespace bfg {
 bfgStatus applyTwoLevel(bfgSystem sys, double2 const *r, double2 *z) {
   cudaStream_t s = sys->stream();
-  int64_t const n = sys->n;
   double2 *z1 = sys->dZ1.as<double2>(), *t = sys->dT1.as<double2>();
   coarseCorrection(sys, r, z1, s);
   CO_CK(cudaGetLastError());
-  // t = r - A z1, z = M_bj t + z1
+  // t = A z1, z = M_bj (r - t) + z1
   bfgStatus st = systemApplyPrec(sys, sys->applyPrec, z1, t);
   if (st != BFG_OK) return st;
-  launchSubFrom(n, r, t, s);
-  applyBlockJacobi32(sys, t, z, s);
-  addToKernel<<<gridOf(n, 256), 256, 0, s>>>(n, z1, z);
+  applyBlockJacobi32(sys, r, t, z1, z, s);
   CO_CK(cudaGetLastError());
   return BFG_OK;
 }

@@ -45,7 +45,7 @@ struct bfgSystem_s {
   using Dev = bfg::Dev;
   bfgContext ctx = nullptr;
   bfgFac fac = nullptr;
-  int64_t n = 0, numCurves = 0;
+  int64_t n = 0, numCurves = 0, maxCurve = 1;   // maxCurve: points of the largest
   int32_t order = 0;
   double shift = 0.5;
   bfgPrecision applyPrec = BFG_PRECISION_FP64;   // of the butterfly part
@@ -80,10 +80,9 @@ namespace bfg {
 bfgStatus facApplySystem(bfgFac f, bfgPrecision prec, SystemTerms const &sys, double2 *Y);
 // A X for one device complex128 vector with the butterfly part in `prec`
 bfgStatus systemApplyPrec(bfgSystem sys, bfgPrecision prec, void const *X, void *Y);
-// z = M_bj r from the FP32 block inverses (block-Jacobi built)
-void applyBlockJacobi32(bfgSystem sys, double2 const *r, double2 *z, cudaStream_t s);
+// z = M_bj (r - sub) + add from the FP32 block inverses (block-Jacobi built)
+void applyBlockJacobi32(bfgSystem sys, double2 const *r, double2 const *sub, double2 const *add,
+                        double2 *z, cudaStream_t s);
 // the two-level preconditioner z = z1 + M_bj (r - A z1), z1 = Phi A_c^-1 Phi^H r
 bfgStatus applyTwoLevel(bfgSystem sys, double2 const *r, double2 *z);
-// kernels shared with bfg_coarse.cu
-void launchSubFrom(int64_t n, double2 const *x, double2 *y, cudaStream_t s);   // y = x - y
 }  // namespace bfg
