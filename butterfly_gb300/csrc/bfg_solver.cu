@@ -510,105 +510,158 @@ __global__ void c128ToC64FlatKernel(int64_t n, double2 const *a, float2 *b) {
     b[i] = make_float2((float)a[i].x, (float)a[i].y);
 }
 
-// h[i] = sum_r conj(V_i[r]) w[r], i < k, in two steps: CTA (c, i) sums the
-// products of vector i over row chunk c (1,024 rows, 4 per thread) into one
-// partial; then each vector's partials are added over the chunks in order.
-// One CTA per (chunk, vector) keeps every SM busy: the FP64 work of
-// classical Gram-Schmidt needs all of GB300's FP64 units.
-constexpr int kDotThreads = 256, kDotRows = 4 * kDotThreads;
-__global__ void __launch_bounds__(kDotThreads)
-multiDotPartKernel(int64_t n, double2 const *V, int64_t ldv, int k, double2 const *w,
-                   double2 *part, int32_t const *gate) {
-  if (gate && !*gate) return;   // a skipped reorthogonalisation pass
-  __shared__ double red[2][kDotThreads / 32];
-  int64_t const r0 = blockIdx.x * (int64_t)kDotRows;
-  int const i = blockIdx.y;
-  double2 const *v = V + (int64_t)i * ldv;
-  double sr = 0, si = 0;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    int64_t const r = r0 + q * kDotThreads + threadIdx.x;
-    if (r < n) {
-      double2 const a = v[r], b = w[r];
-      sr += a.x * b.x + a.y * b.y;
-      si += a.x * b.y - a.y * b.x;
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    sr += __shfl_xor_sync(0xffffffffu, sr, o);
-    si += __shfl_xor_sync(0xffffffffu, si, o);
-  }
-  int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) {
-    red[0][warp] = sr;
-    red[1][warp] = si;
-  }
+// Classical Gram-Schmidt of w against k basis vectors, by kernels that end in
+// their own last CTA (the one that draws a counter's last ticket adds the
+// partial sums in order, so results are reproducible, and resets it):
+//   arnoldiDots  h = V^H w, and ||w||^2
+//   arnoldiAxpy  w -= V h, ||w||^2 again and whether a second pass is due
+// Twice, then the scaling: 5 launches an iteration.  A finishing kernel for
+// every reduction and one for the criterion took 13, each a few microseconds
+// of latency at 2,073 unknowns (1.8 ms of a
+// solve's 49 iterations more than these).
+
+// draws a ticket; true in every thread of the CTA that drew the last of `total`
+__device__ __forceinline__ bool lastOf(uint32_t *counter, uint32_t total) {
+  __shared__ bool last;
+  __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
-    double a = 0, c = 0;
-    for (int q = 0; q < kDotThreads / 32; ++q) {
-      a += red[0][q];
-      c += red[1][q];
-    }
-    part[blockIdx.x * (int64_t)k + i] = make_double2(a, c);
+    last = atomicAdd(counter, 1u) == total - 1;
+    if (last) *counter = 0;
   }
+  __syncthreads();
+  __threadfence();
+  return last;
 }
-__global__ void multiDotFinishKernel(int nChunks, int k, double2 const *part, double2 *h,
-                                     int32_t const *gate) {
-  int const i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= k) return;
-  if (gate && !*gate) {
-    h[i] = make_double2(0, 0);
-    return;
+// the sum of a double2 over the CTA, in every thread of warp 0
+template <int kWarps>
+__device__ __forceinline__ double2 ctaSum(double2 v) {
+  __shared__ double2 red[kWarps];
+  for (int o = 16; o > 0; o >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+  }
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = make_double2(0.0, 0.0);
+  for (int w = 0; w < kWarps; ++w) {
+    v.x += red[w].x;
+    v.y += red[w].y;
+  }
+  return v;
+}
+
+// h[i] = sum_r conj(V_i[r]) w[r], i < k (CTA (c, i): row chunk c of vector i),
+// and for i = k, if the grid has it, *self = ||w||^2.  gate: nothing to do if
+// it is closed.
+constexpr int kDotThreads = 128, kDotRows = 8 * kDotThreads;
+__global__ void __launch_bounds__(kDotThreads)
+arnoldiDotsKernel(int64_t n, double2 const *V, int64_t ldv, int k, double2 const *w,
+                  double2 *part, uint32_t *counters, double2 *h, double2 *self,
+                  int32_t const *gate) {
+  if (gate && !*gate) return;
+  constexpr int U = kDotRows / kDotThreads, kWarps = kDotThreads / 32;
+  int const i = blockIdx.y;
+  double2 const *v = i < k ? V + (int64_t)i * ldv : w;
+  int64_t const r0 = blockIdx.x * (int64_t)kDotRows + threadIdx.x;
+  double2 a[U], b[U];
+#pragma unroll
+  for (int q = 0; q < U; ++q) {
+    bool const in = r0 + q * kDotThreads < n;
+    a[q] = in ? v[r0 + q * kDotThreads] : make_double2(0.0, 0.0);
+    b[q] = in ? w[r0 + q * kDotThreads] : make_double2(0.0, 0.0);
   }
   double sr = 0, si = 0;
-  for (int c = 0; c < nChunks; ++c) {
-    double2 const v = part[(int64_t)c * k + i];
-    sr += v.x;
-    si += v.y;
+#pragma unroll
+  for (int q = 0; q < U; ++q) {
+    sr = fma(a[q].y, b[q].y, fma(a[q].x, b[q].x, sr));
+    si = fma(-a[q].y, b[q].x, fma(a[q].x, b[q].y, si));
   }
-  h[i] = make_double2(sr, si);
+  double2 t = ctaSum<kWarps>(make_double2(sr, si));
+  if (gridDim.x > 1) {
+    double2 *p = part + (int64_t)i * gridDim.x;
+    if (threadIdx.x == 0) p[blockIdx.x] = t;
+    if (!lastOf(counters + i, gridDim.x)) return;
+    t = make_double2(0.0, 0.0);
+    for (unsigned c = threadIdx.x; c < gridDim.x; c += kDotThreads) {
+      double2 const u = __ldcg(p + c);
+      t.x += u.x;
+      t.y += u.y;
+    }
+    t = ctaSum<kWarps>(t);
+  }
+  if (threadIdx.x == 0) *(i < k ? h + i : self) = t;
 }
 int dotChunks(int64_t n) { return (int)((n + kDotRows - 1) / kDotRows); }
 
-// w += sign * sum_{i<k} V_i h_i.  A CTA takes 32 rows; its 16 warps split
-// the k basis vectors (warp s takes i = s, s + 16, ...), each warp reading
-// 32 consecutive rows of a vector, and the 16 partial sums are added in a
-// fixed order.
-constexpr int kAxpyRows = 32, kAxpySlices = 16;
+// w += sign * sum_{i<k} V_i h_i.  A CTA takes 16 rows; its 16 half warps split
+// the k basis vectors (slice s takes i = s, s + 16, ...), and the 16 partial
+// sums are added in a fixed order.
+// With `norm`: ||w||^2 to *norm (the partial sums in `part`), and, on the
+// first pass of two (before = ||w||^2 ahead of it), the DGKS criterion: the
+// second pass is due when the first removed more than half of the squared
+// norm (||w_after|| < ||w_before|| / sqrt 2); if not, its coefficients h2 = 0.
+constexpr int kAxpyRows = 16, kAxpySlices = 16;
 __global__ void __launch_bounds__(kAxpyRows * kAxpySlices)
-multiAxpyKernel(int64_t n, double2 const *V, int64_t ldv, int k, double2 const *h, double sign,
-                double2 *w, int32_t const *gate) {
+arnoldiAxpyKernel(int64_t n, double2 const *V, int64_t ldv, int k, double2 const *h, double sign,
+                  double2 *w, int32_t const *gate, double2 *norm, double2 *part,
+                  uint32_t *counter, double2 const *before, int32_t *gateOut, double2 *h2) {
   if (gate && !*gate) return;
-  __shared__ double2 part[kAxpySlices][kAxpyRows];
+  constexpr int kThreads = kAxpyRows * kAxpySlices, U = 4;
+  __shared__ double2 sum[kAxpySlices][kAxpyRows];
   int const lr = threadIdx.x % kAxpyRows, sl = threadIdx.x / kAxpyRows;
   int64_t const r = blockIdx.x * (int64_t)kAxpyRows + lr;
+  double2 const old = sl == 0 && r < n ? w[r] : make_double2(0.0, 0.0);
   double sr = 0, si = 0;
   if (r < n)
-    for (int i = sl; i < k; i += kAxpySlices) {
-      double2 const a = V[(int64_t)i * ldv + r], c = h[i];
-      sr += a.x * c.x - a.y * c.y;
-      si += a.x * c.y + a.y * c.x;
+    for (int i0 = sl; i0 < k; i0 += U * kAxpySlices) {
+      double2 a[U], c[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        int const i = min(i0 + u * kAxpySlices, k - 1);
+        a[u] = V[(int64_t)i * ldv + r];
+        c[u] = h[i];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (i0 + u * kAxpySlices < k) {
+          sr = fma(-a[u].y, c[u].y, fma(a[u].x, c[u].x, sr));
+          si = fma(a[u].y, c[u].x, fma(a[u].x, c[u].y, si));
+        }
     }
-  part[sl][lr] = make_double2(sr, si);
+  sum[sl][lr] = make_double2(sr, si);
   __syncthreads();
+  double2 q = make_double2(0.0, 0.0);   // |w[r]|^2 after
   if (sl == 0 && r < n) {
     double tr = 0, ti = 0;
 #pragma unroll
-    for (int q = 0; q < kAxpySlices; ++q) {
-      tr += part[q][lr].x;
-      ti += part[q][lr].y;
+    for (int s = 0; s < kAxpySlices; ++s) {
+      tr += sum[s][lr].x;
+      ti += sum[s][lr].y;
     }
-    w[r] = make_double2(w[r].x + sign * tr, w[r].y + sign * ti);
+    double2 const v = make_double2(old.x + sign * tr, old.y + sign * ti);
+    w[r] = v;
+    q.x = v.x * v.x + v.y * v.y;
+  }
+  if (!norm) return;
+  if (threadIdx.x < 32) {
+    for (int o = kAxpyRows / 2; o > 0; o >>= 1) q.x += __shfl_xor_sync(0xffffffffu, q.x, o);
+    if (threadIdx.x == 0) part[blockIdx.x] = q;
+  }
+  if (!lastOf(counter, gridDim.x)) return;
+  double2 t = make_double2(0.0, 0.0);
+  for (unsigned c = threadIdx.x; c < gridDim.x; c += kThreads) t.x += __ldcg(&part[c].x);
+  t = ctaSum<kThreads / 32>(t);
+  if (threadIdx.x == 0) *norm = t;
+  if (before) {
+    bool const again = t.x < 0.5 * before->x;
+    if (threadIdx.x == 0) *gateOut = again ? 1 : 0;
+    if (!again)
+      for (int i = threadIdx.x; i < k; i += kThreads) h2[i] = make_double2(0.0, 0.0);
   }
 }
 int axpyGrid(int64_t n) { return (int)((n + kAxpyRows - 1) / kAxpyRows); }
-
-// DGKS criterion: a second Gram-Schmidt pass when the first removed more
-// than half of w's squared norm (||w_after|| < ||w_before|| / sqrt 2)
-__global__ void reorthGateKernel(double2 const *before, double2 const *after, int32_t *gate) {
-  *gate = after->x < 0.5 * before->x ? 1 : 0;
-}
 
 // y = x / sqrt(nrm2->x) (0 if the norm is 0), the norm read on the device
 __global__ void scaleByNormKernel(int64_t n, double2 const *nrm2, double2 const *x, double2 *y) {
@@ -972,19 +1025,25 @@ bfgStatus bfgSolveGmres(bfgSystem sys, void const *B, void *X, double tol, int64
   SYS_CK(w.alloc(n * 16));
   SYS_CK(r.alloc(n * 16));
   SYS_CK(h.alloc((2 * m + 4) * 16));
-  Dev dotPart;
+  // partial sums of the two reductions, their counters (m + 1 of dots, one of
+  // the vector update) and the second pass's gate
+  Dev part, flags;
   int const nChunks = dotChunks(n);
-  SYS_CK(dotPart.alloc((size_t)nChunks * (m + 1) * 16));
-  // h_out[i] = (V_i, w) for i < k
-  Dev gateBuf;
-  SYS_CK(gateBuf.alloc(4));
-  int32_t *gate = gateBuf.as<int32_t>();
-  auto dots = [&](double2 const *Vm, int k, double2 const *wv, double2 *hOut,
+  SYS_CK(part.alloc(std::max<size_t>((size_t)nChunks * (m + 1), (size_t)axpyGrid(n)) * 16));
+  SYS_CK(flags.alloc((size_t)(m + 3) * 4));
+  SYS_CK(cudaMemsetAsync(flags.p, 0, (size_t)(m + 3) * 4, s));
+  uint32_t *counters = flags.as<uint32_t>(), *axpyCounter = counters + m + 1;
+  int32_t *gate = flags.as<int32_t>() + m + 2;
+  // hOut[i] = (V_i, w) for i < k; self: ||w||^2
+  auto dots = [&](double2 const *Vm, int k, double2 const *wv, double2 *hOut, double2 *self,
                   int32_t const *g = nullptr) {
-    multiDotPartKernel<<<dim3((unsigned)nChunks, (unsigned)k), kDotThreads, 0, s>>>(
-        n, Vm, n, k, wv, dotPart.as<double2>(), g);
-    multiDotFinishKernel<<<(k + 127) / 128, 128, 0, s>>>(nChunks, k, dotPart.as<double2>(), hOut,
-                                                         g);
+    bool const apart = self && k >= 65535;   // the grid's limit in y
+    if (apart)
+      arnoldiDotsKernel<<<dim3((unsigned)nChunks, 1), kDotThreads, 0, s>>>(
+          n, nullptr, n, 0, wv, part.as<double2>(), counters, nullptr, self, g);
+    arnoldiDotsKernel<<<dim3((unsigned)nChunks, (unsigned)(k + (self && !apart ? 1 : 0))),
+                        kDotThreads, 0, s>>>(n, Vm, n, k, wv, part.as<double2>(), counters, hOut,
+                                             self, g);
   };
   double2 *Vp = V.as<double2>(), *Zp = Z.as<double2>(), *wp = w.as<double2>(), *rp = r.as<double2>();
   double2 *hp = h.as<double2>();
@@ -992,7 +1051,7 @@ bfgStatus bfgSolveGmres(bfgSystem sys, void const *B, void *X, double tol, int64
   double2 const *bp = static_cast<double2 const *>(B);
 
   auto norm = [&](double2 const *v, double *out) -> bfgStatus {
-    dots(v, 1, v, hp);
+    dots(nullptr, 0, v, nullptr, hp);
     SYS_CK(cudaGetLastError());
     double2 hv;
     SYS_CK(cudaMemcpyAsync(&hv, hp, 16, cudaMemcpyDeviceToHost, s));
@@ -1058,20 +1117,18 @@ bfgStatus bfgSolveGmres(bfgSystem sys, void const *B, void *X, double tol, int64
     // classical Gram-Schmidt with a second pass where the DGKS criterion
     // asks for it, the norm and the next basis vector, all on the device;
     // one read of the Hessenberg column per iteration (h: passes 1 and 2 in
-    // slots [0, k) and [k, 2k), ||w||^2 in slot 2k, before / after pass 1
-    // in slots 2k+1, 2k+2)
+    // slots [0, k) and [k, 2k), ||w||^2 in slot 2k, before pass 1 in slot
+    // 2k+1)
     int const k = (int)(j + 1);
     std::vector<cd> hcol(k + 1, cd(0));
-    dots(wp, 1, wp, hp + 2 * k + 1);
-    dots(Vp, k, wp, hp);
-    multiAxpyKernel<<<axpyGrid(n), kAxpyRows * kAxpySlices, 0, s>>>(n, Vp, n, k, hp, -1.0, wp,
-                                                                    nullptr);
-    dots(wp, 1, wp, hp + 2 * k + 2);
-    reorthGateKernel<<<1, 1, 0, s>>>(hp + 2 * k + 1, hp + 2 * k + 2, gate);
-    dots(Vp, k, wp, hp + k, gate);
-    multiAxpyKernel<<<axpyGrid(n), kAxpyRows * kAxpySlices, 0, s>>>(n, Vp, n, k, hp + k, -1.0,
-                                                                    wp, gate);
-    dots(wp, 1, wp, hp + 2 * k);
+    dots(Vp, k, wp, hp, hp + 2 * k + 1);
+    arnoldiAxpyKernel<<<axpyGrid(n), kAxpyRows * kAxpySlices, 0, s>>>(
+        n, Vp, n, k, hp, -1.0, wp, nullptr, hp + 2 * k, part.as<double2>(), axpyCounter,
+        hp + 2 * k + 1, gate, hp + k);
+    dots(Vp, k, wp, hp + k, nullptr, gate);
+    arnoldiAxpyKernel<<<axpyGrid(n), kAxpyRows * kAxpySlices, 0, s>>>(
+        n, Vp, n, k, hp + k, -1.0, wp, gate, hp + 2 * k, part.as<double2>(), axpyCounter, nullptr,
+        nullptr, nullptr);
     scaleByNormKernel<<<gridFor(n, 256), 256, 0, s>>>(n, hp + 2 * k, wp, Vp + (j + 1) * n);
     SYS_CK(cudaGetLastError());
     SYS_CK(cudaMemcpyAsync(hh.data(), hp, (2 * k + 1) * 16, cudaMemcpyDeviceToHost, s));
@@ -1113,8 +1170,9 @@ bfgStatus bfgSolveGmres(bfgSystem sys, void const *B, void *X, double tol, int64
     std::vector<double2> yd(j);
     for (int64_t i = 0; i < j; ++i) yd[i] = make_double2(yv[i].real(), yv[i].imag());
     SYS_CK(cudaMemcpyAsync(hp, yd.data(), j * 16, cudaMemcpyHostToDevice, s));
-    multiAxpyKernel<<<axpyGrid(n), kAxpyRows * kAxpySlices, 0, s>>>(n, Zp, n, (int)j, hp, 1.0, xp,
-                                                                    nullptr);
+    arnoldiAxpyKernel<<<axpyGrid(n), kAxpyRows * kAxpySlices, 0, s>>>(
+        n, Zp, n, (int)j, hp, 1.0, xp, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+        nullptr);
     SYS_CK(cudaGetLastError());
   }
   // true residual, with the FP64 apply whatever the iterations used

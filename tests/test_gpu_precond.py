@@ -77,3 +77,27 @@ def test_fp32_block_jacobi_of_every_curve_size(problem):
     x64, info64 = B.solve_gmres(s, b, tol=1e-10, max_num_iter=100, precond=fp64_inverses)
     assert info["converged"] and abs(info["iterations"] - info64["iterations"]) <= 1
     assert rel_err(x.cpu().numpy(), x64.cpu().numpy()) < 1e-8
+
+
+@pytest.mark.parametrize("n", [15, 16, 17, 1023, 1024, 1025, 2081])
+def test_arnoldi_residual_is_the_true_one(n):
+    """One to three row chunks of the Gram-Schmidt kernels and remainders of
+    their 16 rows: wrong coefficients or norms would part the residual of the
+    Arnoldi relation from that of the solution (both FP64, a few hundred
+    roundings of 2^-53 and products within 1e-12)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    k, t = 9.0, 2 * np.pi * np.arange(n) / n
+    pts = np.stack([np.cos(t), np.sin(t)], 1)
+    helm = B.Helm2(k, B.LayerPot.CombinedField, alpha=-1j * k, beta=1.0)
+    fac = B.FacHelm2.make_multilevel(helm, B.Quadtree(pts, pts, leaf_size=64),
+                                     B.Quadtree(pts, leaf_size=64), rank_eps=1e-13,
+                                     pinv_tol=1e-13, context=B.default_context(0))
+    s = B.System(fac, pts, pts, np.full(n, 2 * np.pi / n), [0, n], kr_order=6, diag_shift=0.5)
+    b = torch.from_numpy(B.Rng(n).complex_randn(n)).cuda()
+    for iters in (3, n):
+        x, info = B.solve_gmres(s, b, tol=1e-9, max_num_iter=iters, precond="none")
+        res = torch.linalg.norm(b - s.apply(x)).item() / torch.linalg.norm(b).item()
+        assert abs(info["trueRelResidual"] - res) < 1e-10
+        assert abs(info["relResidual"] - res) < 1e-10
+        assert iters == 3 or info["converged"]
