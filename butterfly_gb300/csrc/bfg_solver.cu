@@ -1019,34 +1019,42 @@ bfgStatus bfgSolveGmres(bfgSystem sys, void const *B, void *X, double tol, int64
   auto t0 = std::chrono::steady_clock::now();
   cudaStream_t s = sys->stream();
   int64_t const n = sys->n, m = maxIter;
-  Dev V, Z, w, r, h;
-  SYS_CK(V.alloc((size_t)(m + 1) * n * 16));
-  SYS_CK(Z.alloc((size_t)m * n * 16));
-  SYS_CK(w.alloc(n * 16));
-  SYS_CK(r.alloc(n * 16));
-  SYS_CK(h.alloc((2 * m + 4) * 16));
+  // one allocation: the basis V, Z = M V, w, r, the Hessenberg column's slots,
   // partial sums of the two reductions, their counters (m + 1 of dots, one of
   // the vector update) and the second pass's gate
-  Dev part, flags;
   int const nChunks = dotChunks(n);
-  SYS_CK(part.alloc(std::max<size_t>((size_t)nChunks * (m + 1), (size_t)axpyGrid(n)) * 16));
-  SYS_CK(flags.alloc((size_t)(m + 3) * 4));
-  SYS_CK(cudaMemsetAsync(flags.p, 0, (size_t)(m + 3) * 4, s));
-  uint32_t *counters = flags.as<uint32_t>(), *axpyCounter = counters + m + 1;
-  int32_t *gate = flags.as<int32_t>() + m + 2;
+  size_t bytes = 0;
+  auto place = [&](size_t b) {
+    size_t const at = bytes;
+    bytes += (b + 255) / 256 * 256;
+    return at;
+  };
+  size_t const oV = place((size_t)(m + 1) * n * 16), oZ = place((size_t)m * n * 16);
+  size_t const oW = place(n * 16), oR = place(n * 16), oH = place((size_t)(2 * m + 4) * 16);
+  size_t const oPart =
+      place(std::max<size_t>((size_t)nChunks * (m + 1), (size_t)axpyGrid(n)) * 16);
+  size_t const oFlags = place((size_t)(m + 3) * 4);
+  Dev work;
+  SYS_CK(work.alloc(bytes));
+  char *base = work.as<char>();
+  double2 *part = reinterpret_cast<double2 *>(base + oPart);
+  SYS_CK(cudaMemsetAsync(base + oFlags, 0, (size_t)(m + 3) * 4, s));
+  uint32_t *counters = reinterpret_cast<uint32_t *>(base + oFlags), *axpyCounter = counters + m + 1;
+  int32_t *gate = reinterpret_cast<int32_t *>(base + oFlags) + m + 2;
   // hOut[i] = (V_i, w) for i < k; self: ||w||^2
   auto dots = [&](double2 const *Vm, int k, double2 const *wv, double2 *hOut, double2 *self,
                   int32_t const *g = nullptr) {
     bool const apart = self && k >= 65535;   // the grid's limit in y
     if (apart)
       arnoldiDotsKernel<<<dim3((unsigned)nChunks, 1), kDotThreads, 0, s>>>(
-          n, nullptr, n, 0, wv, part.as<double2>(), counters, nullptr, self, g);
+          n, nullptr, n, 0, wv, part, counters, nullptr, self, g);
     arnoldiDotsKernel<<<dim3((unsigned)nChunks, (unsigned)(k + (self && !apart ? 1 : 0))),
-                        kDotThreads, 0, s>>>(n, Vm, n, k, wv, part.as<double2>(), counters, hOut,
+                        kDotThreads, 0, s>>>(n, Vm, n, k, wv, part, counters, hOut,
                                              self, g);
   };
-  double2 *Vp = V.as<double2>(), *Zp = Z.as<double2>(), *wp = w.as<double2>(), *rp = r.as<double2>();
-  double2 *hp = h.as<double2>();
+  double2 *Vp = reinterpret_cast<double2 *>(base + oV), *Zp = reinterpret_cast<double2 *>(base + oZ);
+  double2 *wp = reinterpret_cast<double2 *>(base + oW), *rp = reinterpret_cast<double2 *>(base + oR);
+  double2 *hp = reinterpret_cast<double2 *>(base + oH);
   double2 *xp = static_cast<double2 *>(X);
   double2 const *bp = static_cast<double2 const *>(B);
 
@@ -1104,35 +1112,48 @@ bfgStatus bfgSolveGmres(bfgSystem sys, void const *B, void *X, double tol, int64
   if ((st = norm(rp, &beta)) != BFG_OK) return st;
   scaleCopyKernel<<<gridFor(n, 256), 256, 0, s>>>(n, 1.0 / beta, rp, Vp);
 
-  std::vector<cd> H((size_t)(m + 1) * m, cd(0)), g(m + 1, cd(0)), cs(m), sn(m);
-  g[0] = beta;
-  std::vector<double2> hh(2 * m + 4);
+  // column j of the rotated Hessenberg matrix from entry j (j + 1) / 2 on; all
+  // grow with the iterations, which are mostly far fewer than m
+  std::vector<cd> H, g(1, cd(beta)), cs, sn, hcol;
   int64_t j = 0;
-  double res = beta / bnorm;
-  bool converged = res < tol;
+  double res = beta / bnorm, before = 0;   // residuals after this iteration, the one before
+  bool converged = res < tol, ahead = false;
+  auto product = [&](int64_t i) {   // w = A z_i, z_i = M v_i
+    bfgStatus const e = applyM(Vp + i * n, Zp + i * n);
+    return e != BFG_OK ? e : bfgSystemApply(sys, Zp + i * n, wp);
+  };
   for (; j < m && !converged; ++j) {
-    double2 *vj = Vp + j * n, *zj = Zp + j * n;
-    if ((st = applyM(vj, zj)) != BFG_OK) return st;
-    if ((st = bfgSystemApply(sys, zj, wp)) != BFG_OK) return st;
+    if (!ahead && (st = product(j)) != BFG_OK) return st;
     // classical Gram-Schmidt with a second pass where the DGKS criterion
     // asks for it, the norm and the next basis vector, all on the device;
     // one read of the Hessenberg column per iteration (h: passes 1 and 2 in
     // slots [0, k) and [k, 2k), ||w||^2 in slot 2k, before pass 1 in slot
     // 2k+1)
     int const k = (int)(j + 1);
-    std::vector<cd> hcol(k + 1, cd(0));
     dots(Vp, k, wp, hp, hp + 2 * k + 1);
     arnoldiAxpyKernel<<<axpyGrid(n), kAxpyRows * kAxpySlices, 0, s>>>(
-        n, Vp, n, k, hp, -1.0, wp, nullptr, hp + 2 * k, part.as<double2>(), axpyCounter,
+        n, Vp, n, k, hp, -1.0, wp, nullptr, hp + 2 * k, part, axpyCounter,
         hp + 2 * k + 1, gate, hp + k);
     dots(Vp, k, wp, hp + k, nullptr, gate);
     arnoldiAxpyKernel<<<axpyGrid(n), kAxpyRows * kAxpySlices, 0, s>>>(
-        n, Vp, n, k, hp + k, -1.0, wp, gate, hp + 2 * k, part.as<double2>(), axpyCounter, nullptr,
+        n, Vp, n, k, hp + k, -1.0, wp, gate, hp + 2 * k, part, axpyCounter, nullptr,
         nullptr, nullptr);
     scaleByNormKernel<<<gridFor(n, 256), 256, 0, s>>>(n, hp + 2 * k, wp, Vp + (j + 1) * n);
     SYS_CK(cudaGetLastError());
-    SYS_CK(cudaMemcpyAsync(hh.data(), hp, (2 * k + 1) * 16, cudaMemcpyDeviceToHost, s));
-    SYS_CK(cudaStreamSynchronize(s));
+    double2 *hh = sys->column.ensure(2 * (size_t)k + 1);
+    if (!hh) return sysFail(sys, BFG_ERROR_CUDA, "GMRES: no pinned memory");
+    SYS_CK(cudaMemcpyAsync(hh, hp, (2 * k + 1) * 16, cudaMemcpyDeviceToHost, s));
+    SYS_CK(cudaEventRecord(sys->column.ready, s));
+    // The device waits ~30 us for the read, the rotations and the next
+    // launches (99 us of kernels in a 130 us iteration at 2,073 unknowns), so
+    // the next product is launched ahead of the read unless the residual's
+    // last reduction, repeated, would end the solve here (within a factor of
+    // 4; a product too many costs more than the wait saves).  A user's
+    // preconditioner is called for the iterations only.
+    ahead = precond != BFG_PRECOND_USER && j > 0 && j + 1 < m && res * (res / before) > 4 * tol;
+    if (ahead && (st = product(j + 1)) != BFG_OK) return st;
+    SYS_CK(cudaEventSynchronize(sys->column.ready));
+    hcol.assign(k + 1, cd(0));
     for (int i = 0; i < k; ++i) hcol[i] = cd(hh[i].x + hh[k + i].x, hh[i].y + hh[k + i].y);
     double const wn = std::sqrt(std::max(0.0, hh[2 * k].x));
     hcol[k] = wn;
@@ -1144,18 +1165,14 @@ bfgStatus bfgSolveGmres(bfgSystem sys, void const *B, void *X, double tol, int64
     }
     cd const a = hcol[j], b = hcol[j + 1];
     double const den = std::sqrt(std::norm(a) + std::norm(b));
-    if (den == 0) {
-      cs[j] = 1;
-      sn[j] = 0;
-    } else {
-      cs[j] = a / den;
-      sn[j] = b / den;
-    }
+    cs.push_back(den == 0 ? cd(1) : a / den);
+    sn.push_back(den == 0 ? cd(0) : b / den);
     hcol[j] = std::conj(cs[j]) * a + std::conj(sn[j]) * b;
     hcol[j + 1] = 0;
-    g[j + 1] = -sn[j] * g[j];
+    g.push_back(-sn[j] * g[j]);
     g[j] = std::conj(cs[j]) * g[j];
-    for (int i = 0; i <= j; ++i) H[(size_t)i * m + j] = hcol[i];
+    H.insert(H.end(), hcol.begin(), hcol.begin() + k);
+    before = res;
     res = std::abs(g[j + 1]) / bnorm;
     if (res < tol || wn == 0) converged = res < tol || wn == 0;
   }
@@ -1163,8 +1180,8 @@ bfgStatus bfgSolveGmres(bfgSystem sys, void const *B, void *X, double tol, int64
   std::vector<cd> yv(j, cd(0));
   for (int64_t i = j - 1; i >= 0; --i) {
     cd acc = g[i];
-    for (int64_t q = i + 1; q < j; ++q) acc -= H[(size_t)i * m + q] * yv[q];
-    yv[i] = acc / H[(size_t)i * m + i];
+    for (int64_t q = i + 1; q < j; ++q) acc -= H[(size_t)q * (q + 1) / 2 + i] * yv[q];
+    yv[i] = acc / H[(size_t)i * (i + 1) / 2 + i];
   }
   if (j > 0) {
     std::vector<double2> yd(j);

@@ -39,6 +39,34 @@ struct Dev {
   template <typename T> T *as() const { return static_cast<T *>(p); }
 };
 
+// a pinned landing place for device reads, with the event that says they are in
+struct Landing {
+  double2 *p = nullptr;
+  size_t count = 0;
+  cudaEvent_t ready = nullptr;
+  Landing() = default;
+  Landing(Landing const &) = delete;
+  Landing &operator=(Landing const &) = delete;
+  ~Landing() {
+    if (p) cudaFreeHost(p);
+    if (ready) cudaEventDestroy(ready);
+  }
+  // room for n entries (the old contents are lost; none may be in flight), null on failure
+  double2 *ensure(size_t n) {
+    if (!ready && cudaEventCreateWithFlags(&ready, cudaEventDisableTiming) != cudaSuccess)
+      return nullptr;
+    if (n <= count) return p;
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    count = 0;
+    n = std::max<size_t>(2 * n, 256);
+    if (cudaMallocHost(reinterpret_cast<void **>(&p), n * sizeof(double2)) != cudaSuccess)
+      return p = nullptr;
+    count = n;
+    return p;
+  }
+};
+
 }  // namespace bfg
 
 struct bfgSystem_s {
@@ -54,6 +82,7 @@ struct bfgSystem_s {
   std::vector<double> weights;                   // host copy (coarse mode counts)
   Dev dOffsets, dCurveOf, dX, dW, dKrVal, dKrCol;
   Dev tmpXw;
+  bfg::Landing column;   // the solver's Hessenberg column
   // block-Jacobi
   bool haveBj = false, haveBj64 = false;   // the FP32 inverses; the FP64 ones (on first use)
   std::vector<int64_t> blkOff;
