@@ -22,6 +22,7 @@
 #include <cstdint>
 
 #include "bfg_kernels.cuh"
+#include "bfg_launch.cuh"
 
 namespace bfg {
 namespace {
@@ -76,9 +77,10 @@ __global__ void arenaToDfKernel(double2 const *__restrict__ a, float4 *__restric
 }
 
 // out[i] = X row perm[i] (or i), split
-__global__ void gatherToDfKernel(double2 const *__restrict__ X, int64_t ldx,
+__global__ void gatherToDfKernel(double2 const *X, int64_t ldx,
                                  int64_t const *__restrict__ perm, int64_t nRows,
                                  float4 *__restrict__ out) {
+  afterPrevious();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nRows;
        i += (int64_t)gridDim.x * blockDim.x)
     out[i] = dfSplit(X[(perm ? perm[i] : i) * ldx]);
@@ -94,12 +96,12 @@ __global__ void gatherToDfKernel(double2 const *__restrict__ X, int64_t ldx,
 // (93 us).
 __global__ void __launch_bounds__(32 * kDfWarps)
 applyGemvDfKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restrict__ contribs,
-                  float4 const *__restrict__ arena, float4 const *__restrict__ X,
-                  float4 *__restrict__ W) {
+                  float4 const *__restrict__ arena, float4 const *X, float4 *W) {
   __shared__ float4 part[kDfWarps][32];
   int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   ApplyItem const it = items[blockIdx.x];
   bool const active = lane < it.rows;
+  afterPrevious();
   float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
   auto mac = [&](float4 a, float4 x) {
     // re += ar xr - ai xi, im += ar xi + ai xr
@@ -171,16 +173,16 @@ cudaError_t launchArenaToDf(double2 const *a64, float4 *adf, int64_t n, cudaStre
 cudaError_t launchGatherToDf(double2 const *X, int64_t ldx, int64_t const *perm, int64_t nRows,
                              float4 *out, cudaStream_t stream) {
   if (nRows == 0) return cudaSuccess;
-  gatherToDfKernel<<<gridDf(nRows), 256, 0, stream>>>(X, ldx, perm, nRows, out);
-  return cudaGetLastError();
+  return launchAfter(gatherToDfKernel, dim3(gridDf(nRows)), dim3(256), 0, stream, X, ldx, perm, nRows,
+                     out);
 }
 
 cudaError_t launchApplyStageDf(ApplyItem const *items, int64_t nItems,
                                ApplyContrib const *contribs, float4 const *arena,
                                float4 const *X, float4 *W, cudaStream_t stream) {
   if (nItems == 0) return cudaSuccess;
-  applyGemvDfKernel<<<(unsigned)nItems, 32 * kDfWarps, 0, stream>>>(items, contribs, arena, X, W);
-  return cudaGetLastError();
+  return launchAfter(applyGemvDfKernel, dim3((unsigned)nItems), dim3(32 * kDfWarps), 0, stream,
+                     items, contribs, arena, X, W);
 }
 
 }  // namespace bfg

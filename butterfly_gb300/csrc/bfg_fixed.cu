@@ -41,6 +41,7 @@
 #include "bfg_device.cuh"
 #include "bfg_fixed.cuh"
 #include "bfg_kernels.cuh"
+#include "bfg_launch.cuh"
 
 namespace bfg {
 namespace {
@@ -389,7 +390,7 @@ fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restric
   int64_t step = 0, xs = 0, lda = 0;
   ApplyContrib cb{};
   double2 av[U], xv;
-  auto fetch = [&](int buf) {
+  auto fetch = [&](int buf, bool first) {
     if (j0 == 0) {
       cb = contribs[it.contrib0 + c];
       ea = active ? rowExp[(it.contrib0 + c) * 32 + lane] : 1023;
@@ -403,18 +404,22 @@ fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restric
       a += KC * lda;
     }
     n = min(KC, cb.n - j0);
-    xv = tid < n ? x[(int64_t)tid * xs] : make_double2(0.0, 0.0);
     // this warp's columns warp, warp + 4, ... in whole batches: a column past
     // the end re-reads the last one (or column 0) against a zero input
     last = (n - 1 - warp) / S;
     double2 const *aw = a + (n > warp ? warp * lda : 0);
 #pragma unroll
     for (int u = 0; u < U; ++u) av[u] = aw[min(u, last) * step];
+    // the inputs come from the kernel before; the factors and their scales were
+    // complete before any apply (the host waited for them)
+    if (first) afterPrevious();
+    xv = tid < n ? x[(int64_t)tid * xs] : make_double2(0.0, 0.0);
     int const code = __reduce_max_sync(0xffffffffu, fixCode(xv));
     if (lane == 0) sMax[buf][warp] = code;
   };
   int buf = 0;
-  if (it.nContrib > 0) fetch(0);
+  if (it.nContrib > 0) fetch(0, true);
+  else afterPrevious();
   while (c < it.nContrib) {
     __syncthreads();
     int code = sMax[buf][0];
@@ -475,7 +480,7 @@ fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restric
       ++c;
     }
     buf ^= 1;
-    if (c < it.nContrib) fetch(buf);
+    if (c < it.nContrib) fetch(buf, false);
     if (!special) {
       __syncthreads();
       if (warp >= S - 2) {
@@ -534,9 +539,8 @@ cudaError_t launchApplyStageFixed(ApplyItem const *items, int64_t nItems,
                                   int64_t R, cudaStream_t stream) {
   if (nItems == 0) return cudaSuccess;
   if (R == 1) {
-    fixGemvKernel<<<(unsigned)nItems, 32 * kGemvWarps, 0, stream>>>(items, contribs, rowExp, arena,
-                                                                    X, ldx, W);
-    return cudaGetLastError();
+    return launchAfter(fixGemvKernel, dim3((unsigned)nItems), dim3(32 * kGemvWarps), 0, stream,
+                       items, contribs, rowExp, arena, X, ldx, W);
   }
   // the narrowest tile that holds the right-hand sides: a tile's empty
   // columns cost as much as full ones (32,768 points: 515 us with 4 columns,

@@ -24,6 +24,7 @@
 
 #include "bfg_device.cuh"
 #include "bfg_kernels.cuh"
+#include "bfg_launch.cuh"
 #include "hankel.cuh"
 
 namespace bfg {
@@ -999,8 +1000,8 @@ template <typename TW, typename T2, bool kSplit, bool kSys>
 __global__ void __launch_bounds__(256)
     applyReduceKernel(int32_t const *__restrict__ rowSeg, int64_t const *__restrict__ segStart,
                       int64_t const *__restrict__ segContrib0,
-                      int64_t const *__restrict__ segBase, TW const *__restrict__ W, int64_t R,
-                      T2 *Y, int64_t ldy, int64_t nRows, int64_t const *__restrict__ outPerm,
+                      int64_t const *__restrict__ segBase, TW const *W, int64_t R, T2 *Y,
+                      int64_t ldy, int64_t nRows, int64_t const *__restrict__ outPerm,
                       int64_t wTile, int64_t wTileStride, SystemTerms sys) {
   using T = typename Real<T2>::T;
   constexpr int U = 4, kParts = kSplit ? 8 : 1;
@@ -1019,6 +1020,7 @@ __global__ void __launch_bounds__(256)
       c1 = segContrib0[s + 1];
       if (outPerm) o = outPerm[i];
     }
+    if (i0 == blockIdx.x * (int64_t)blockDim.y) afterPrevious();
     for (int64_t r0 = 0; r0 < R; r0 += blockDim.x) {
       int64_t const r = r0 + threadIdx.x;
       bool const mine = live && r < R;
@@ -1079,6 +1081,7 @@ __device__ __forceinline__ void storeAs(double2 v, float4 *out) {
 template <typename TO>
 __global__ void gatherScaledKernel(SystemTerms sys, int64_t const *__restrict__ perm, int64_t n,
                                    TO *__restrict__ out) {
+  afterPrevious();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     int64_t const p = perm[i];
@@ -1090,9 +1093,10 @@ __global__ void gatherScaledKernel(SystemTerms sys, int64_t const *__restrict__ 
 }
 
 template <typename T2>
-__global__ void gatherRowsKernel(T2 const *__restrict__ X, int64_t ldx,
+__global__ void gatherRowsKernel(T2 const *X, int64_t ldx,
                                  int64_t const *__restrict__ perm, int64_t nRows, int64_t R,
                                  T2 *__restrict__ out, int64_t outTile, int64_t outTileStride) {
+  afterPrevious();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.y + threadIdx.y; i < nRows;
        i += (int64_t)gridDim.x * blockDim.y) {
     T2 const *x = X + (perm ? perm[i] : i) * ldx;
@@ -1310,28 +1314,26 @@ cudaError_t launchApplyReduce(int32_t const *rowSeg, int64_t const *segStart,
     block = dim3(x, 32 / x, 8);
   }
   auto run = [&](auto kernel) {
-    kernel<<<gridFor(nRows, block.y), block, 0, stream>>>(
-        rowSeg, segStart, segContrib0, segBase, W, R, Y, ldy, nRows, outPerm, wTile, wTileStride,
-        sys ? *sys : SystemTerms{});
+    return launchAfter(kernel, dim3(gridFor(nRows, block.y)), block, 0, stream, rowSeg, segStart,
+                       segContrib0, segBase, W, R, Y, ldy, nRows, outPerm, wTile, wTileStride,
+                       sys ? *sys : SystemTerms{});
   };
   if constexpr (std::is_same_v<T2, double2>) {
     if (sys) {
-      if (split) run(applyReduceKernel<TW, T2, true, true>);
-      else run(applyReduceKernel<TW, T2, false, true>);
-      return cudaGetLastError();
+      return split ? run(applyReduceKernel<TW, T2, true, true>)
+                   : run(applyReduceKernel<TW, T2, false, true>);
     }
   }
-  if (split) run(applyReduceKernel<TW, T2, true, false>);
-  else run(applyReduceKernel<TW, T2, false, false>);
-  return cudaGetLastError();
+  return split ? run(applyReduceKernel<TW, T2, true, false>)
+               : run(applyReduceKernel<TW, T2, false, false>);
 }
 
 template <typename TO>
 cudaError_t launchGatherScaled(SystemTerms const &sys, int64_t const *perm, int64_t n, TO *out,
                                cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
-  gatherScaledKernel<TO><<<gridFor(n, 64), 64, 0, stream>>>(sys, perm, n, out);
-  return cudaGetLastError();
+  return launchAfter(gatherScaledKernel<TO>, dim3(gridFor(n, 64)), dim3(64), 0, stream, sys, perm, n,
+                     out);
 }
 template cudaError_t launchGatherScaled<double2>(SystemTerms const &, int64_t const *, int64_t,
                                                  double2 *, cudaStream_t);
@@ -1344,9 +1346,8 @@ cudaError_t launchGatherRows(T2 const *X, int64_t ldx, int64_t const *perm,
                              int64_t outTile, int64_t outTileStride) {
   if (outTile != 0 && outTile != 16 && outTile != 32) return cudaErrorInvalidValue;
   dim3 const block = rowBlock(R);
-  gatherRowsKernel<T2><<<gridFor(nRows, block.y), block, 0, stream>>>(X, ldx, perm, nRows, R, out,
-                                                                      outTile, outTileStride);
-  return cudaGetLastError();
+  return launchAfter(gatherRowsKernel<T2>, dim3(gridFor(nRows, block.y)), block, 0, stream, X, ldx,
+                     perm, nRows, R, out, outTile, outTileStride);
 }
 
 template cudaError_t launchApplyReduce<double2, double2>(

@@ -31,6 +31,7 @@
 
 #include "../../include/bfg.h"
 #include "bfg_kernels.cuh"
+#include "bfg_launch.cuh"
 #include "bfg_mlp.cuh"
 #include "bfg_system.hpp"
 #include "hankel.cuh"
@@ -276,6 +277,7 @@ __global__ void __launch_bounds__(32 * kBjWarps)
   constexpr int Q = kBjRows, U = 4, kRows = kBjRows * kBjWarps;
   int const b = blockIdx.x / tiles, tile = blockIdx.x % tiles, lane = threadIdx.x & 31;
   int64_t const i0 = offsets[b], m = offsets[b + 1] - i0, blk = blkOff[b];
+  bfg::afterPrevious();
   for (int64_t row = (int64_t)tile * kRows + (threadIdx.x >> 5) * Q; row < m;
        row += (int64_t)tiles * kRows) {
     float2 const *a[Q];   // a row past the end repeats the last one
@@ -560,6 +562,7 @@ __global__ void __launch_bounds__(kDotThreads)
 arnoldiDotsKernel(int64_t n, double2 const *V, int64_t ldv, int k, double2 const *w,
                   double2 *part, uint32_t *counters, double2 *h, double2 *self,
                   int32_t const *gate) {
+  bfg::afterPrevious();
   if (gate && !*gate) return;
   constexpr int U = kDotRows / kDotThreads, kWarps = kDotThreads / 32;
   int const i = blockIdx.y;
@@ -607,6 +610,7 @@ __global__ void __launch_bounds__(kAxpyRows * kAxpySlices)
 arnoldiAxpyKernel(int64_t n, double2 const *V, int64_t ldv, int k, double2 const *h, double sign,
                   double2 *w, int32_t const *gate, double2 *norm, double2 *part,
                   uint32_t *counter, double2 const *before, int32_t *gateOut, double2 *h2) {
+  bfg::afterPrevious();
   if (gate && !*gate) return;
   constexpr int kThreads = kAxpyRows * kAxpySlices, U = 4;
   __shared__ double2 sum[kAxpySlices][kAxpyRows];
@@ -665,6 +669,7 @@ int axpyGrid(int64_t n) { return (int)((n + kAxpyRows - 1) / kAxpyRows); }
 
 // y = x / sqrt(nrm2->x) (0 if the norm is 0), the norm read on the device
 __global__ void scaleByNormKernel(int64_t n, double2 const *nrm2, double2 const *x, double2 *y) {
+  bfg::afterPrevious();
   double const q = nrm2->x;
   double const s = q > 0 ? 1.0 / sqrt(q) : 0.0;
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n;
@@ -923,7 +928,8 @@ void applyBj32(bfgSystem sys, double2 const *r, double2 *z, cudaStream_t s,
                double2 const *sub = nullptr, double2 const *add = nullptr) {
   constexpr int kRows = kBjRows * kBjWarps;
   int const tiles = (int)std::min<int64_t>((sys->maxCurve + kRows - 1) / kRows, kBjTiles);
-  blockDiagApply32Kernel<<<(unsigned)(sys->numCurves * tiles), 32 * kBjWarps, 0, s>>>(
+  bfg::launchAfter(blockDiagApply32Kernel, dim3((unsigned)(sys->numCurves * tiles)),
+                   dim3(32 * kBjWarps), 0, s,
       sys->dOffsets.as<int64_t>(), sys->dBlkOff.as<int64_t>(), sys->dInv32.as<float2>(), r, sub,
       add, z, tiles);
 }
@@ -1046,11 +1052,11 @@ bfgStatus bfgSolveGmres(bfgSystem sys, void const *B, void *X, double tol, int64
                   int32_t const *g = nullptr) {
     bool const apart = self && k >= 65535;   // the grid's limit in y
     if (apart)
-      arnoldiDotsKernel<<<dim3((unsigned)nChunks, 1), kDotThreads, 0, s>>>(
-          n, nullptr, n, 0, wv, part, counters, nullptr, self, g);
-    arnoldiDotsKernel<<<dim3((unsigned)nChunks, (unsigned)(k + (self && !apart ? 1 : 0))),
-                        kDotThreads, 0, s>>>(n, Vm, n, k, wv, part, counters, hOut,
-                                             self, g);
+      bfg::launchAfter(arnoldiDotsKernel, dim3((unsigned)nChunks, 1), dim3(kDotThreads), 0,
+                       s, n, nullptr, n, 0, wv, part, counters, nullptr, self, g);
+    bfg::launchAfter(arnoldiDotsKernel,
+                     dim3((unsigned)nChunks, (unsigned)(k + (self && !apart ? 1 : 0))),
+                     dim3(kDotThreads), 0, s, n, Vm, n, k, wv, part, counters, hOut, self, g);
   };
   double2 *Vp = reinterpret_cast<double2 *>(base + oV), *Zp = reinterpret_cast<double2 *>(base + oZ);
   double2 *wp = reinterpret_cast<double2 *>(base + oW), *rp = reinterpret_cast<double2 *>(base + oR);
@@ -1131,14 +1137,17 @@ bfgStatus bfgSolveGmres(bfgSystem sys, void const *B, void *X, double tol, int64
     // 2k+1)
     int const k = (int)(j + 1);
     dots(Vp, k, wp, hp, hp + 2 * k + 1);
-    arnoldiAxpyKernel<<<axpyGrid(n), kAxpyRows * kAxpySlices, 0, s>>>(
+    bfg::launchAfter(arnoldiAxpyKernel, dim3(axpyGrid(n)),
+                     dim3(kAxpyRows * kAxpySlices), 0, s,
         n, Vp, n, k, hp, -1.0, wp, nullptr, hp + 2 * k, part, axpyCounter,
         hp + 2 * k + 1, gate, hp + k);
     dots(Vp, k, wp, hp + k, nullptr, gate);
-    arnoldiAxpyKernel<<<axpyGrid(n), kAxpyRows * kAxpySlices, 0, s>>>(
+    bfg::launchAfter(arnoldiAxpyKernel, dim3(axpyGrid(n)),
+                     dim3(kAxpyRows * kAxpySlices), 0, s,
         n, Vp, n, k, hp + k, -1.0, wp, gate, hp + 2 * k, part, axpyCounter, nullptr,
         nullptr, nullptr);
-    scaleByNormKernel<<<gridFor(n, 256), 256, 0, s>>>(n, hp + 2 * k, wp, Vp + (j + 1) * n);
+    bfg::launchAfter(scaleByNormKernel, dim3(gridFor(n, 256)), dim3(256), 0, s, n, hp + 2 * k, wp,
+                     Vp + (j + 1) * n);
     SYS_CK(cudaGetLastError());
     double2 *hh = sys->column.ensure(2 * (size_t)k + 1);
     if (!hh) return sysFail(sys, BFG_ERROR_CUDA, "GMRES: no pinned memory");
@@ -1187,7 +1196,8 @@ bfgStatus bfgSolveGmres(bfgSystem sys, void const *B, void *X, double tol, int64
     std::vector<double2> yd(j);
     for (int64_t i = 0; i < j; ++i) yd[i] = make_double2(yv[i].real(), yv[i].imag());
     SYS_CK(cudaMemcpyAsync(hp, yd.data(), j * 16, cudaMemcpyHostToDevice, s));
-    arnoldiAxpyKernel<<<axpyGrid(n), kAxpyRows * kAxpySlices, 0, s>>>(
+    bfg::launchAfter(arnoldiAxpyKernel, dim3(axpyGrid(n)),
+                     dim3(kAxpyRows * kAxpySlices), 0, s,
         n, Zp, n, (int)j, hp, 1.0, xp, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
         nullptr);
     SYS_CK(cudaGetLastError());

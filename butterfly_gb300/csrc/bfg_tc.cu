@@ -24,6 +24,7 @@
 #include <cstdint>
 
 #include "bfg_kernels.cuh"
+#include "bfg_launch.cuh"
 
 namespace bfg {
 namespace {
@@ -345,7 +346,7 @@ __global__ void __launch_bounds__(256) tcFillKernel(TcFill const *__restrict__ f
 template <int TERMS, int RT>
 __global__ void __launch_bounds__(TcLayout<TERMS, RT>::kThreads, 1) applyTcKernel(
     TcChunk const *__restrict__ chunks, int64_t const *__restrict__ ctaChunk0,
-    uint8_t const *__restrict__ tarena, float2 const *__restrict__ X, int64_t ldx, int64_t xTs,
+    uint8_t const *__restrict__ tarena, float2 const *X, int64_t ldx, int64_t xTs,
     float2 *__restrict__ W, int64_t ldw, int64_t wTs, int64_t R, int32_t rhsTiles, int32_t xBulk,
     uint64_t waitLimitNs, int32_t *status) {
   using L = TcLayout<TERMS, RT>;
@@ -364,13 +365,16 @@ __global__ void __launch_bounds__(TcLayout<TERMS, RT>::kThreads, 1) applyTcKerne
   int const tile = (int)(blockIdx.x % (unsigned)rhsTiles);
   int64_t const c0 = ctaChunk0[stream];
   int64_t const nCh = ctaChunk0[stream + 1] - c0;
-  if (nCh <= 0) return;
+  if (nCh <= 0) {
+    afterPrevious();
+    return;
+  }
   int64_t const r0 = (int64_t)tile * RT;
   int const nr = (R - r0) < RT ? (int)(R - r0) : RT;
   // this tile's right-hand sides: row i at Xt + i ldx (inputs), Wt + i ldw
   // (intermediates and outputs); the tile stride is RT for row-major
   // operands and rows x RT for tile-major ones
-  float2 const *__restrict__ Xt = X + tile * xTs;
+  float2 const *Xt = X + tile * xTs;
   float2 *__restrict__ Wt = W + tile * wTs;
   TcChunk const *ch = chunks + c0;
   // a chunk's right-hand sides arrive by one bulk copy with its A planes when
@@ -407,6 +411,7 @@ __global__ void __launch_bounds__(TcLayout<TERMS, RT>::kThreads, 1) applyTcKerne
   __syncthreads();
   tcFenceAfter();
   uint32_t const tmem = *tmemSlot;
+  afterPrevious();   // from here on X and W are read
 
   // what each role has in flight, for the drains after an abort: the
   // producer's issued bulk copies, each MMA thread's last committed chunk
@@ -788,9 +793,9 @@ void launchOne(dim3 grid, cudaStream_t stream, TcChunk const *chunks, int64_t co
                uint8_t const *tarena, float2 const *X, int64_t ldx, int64_t xTs, float2 *W,
                int64_t ldw, int64_t wTs, int64_t R, int32_t tiles, int32_t xBulk,
                uint64_t waitLimitNs, int32_t *status) {
-  applyTcKernel<TERMS, RT><<<grid, TcLayout<TERMS, RT>::kThreads, TcLayout<TERMS, RT>::smemBytes,
-                             stream>>>(
-      chunks, ctaChunk0, tarena, X, ldx, xTs, W, ldw, wTs, R, tiles, xBulk, waitLimitNs, status);
+  launchAfter(applyTcKernel<TERMS, RT>, grid, dim3(TcLayout<TERMS, RT>::kThreads),
+              TcLayout<TERMS, RT>::smemBytes, stream, chunks, ctaChunk0, tarena, X, ldx, xTs, W, ldw,
+              wTs, R, tiles, xBulk, waitLimitNs, status);
 }
 }  // namespace
 
