@@ -65,11 +65,18 @@ struct TcLayout {
   // warp roles: builders (B planes), extractors (TMEM partial sums and
   // stores; 16 RHS of one TMEM lane quarter each), one bulk-copy warp and
   // the two MMA warps (the even and the odd chunks: one thread's waits and
-  // descriptor work overlap the other's MMAs).  RT = 16: 4 + 4 + 1 + 2
-  // warps; RT = 32: 4 + 8 + 1 + 2 warps (the extractors' accumulators of 32
-  // RHS would not fit one thread's registers; measured at 256 RHS, two
-  // builder warps were 12 % and one MMA warp 7 % slower)
-  static constexpr int kBuilders = 128;
+  // descriptor work overlap the other's MMAs).  The builders are two groups
+  // of 4 warps, one for the even and one for the odd chunks, for the same
+  // reason: a chunk's waits, conversions and hand-off are one chain (at 256
+  // RHS, 65,536 points: one group 4,455 us, two 3,978, four groups of 2 warps
+  // 4,150).  RT = 16: 8 + 4 + 1 + 2 warps; RT = 32: 8 + 8 + 1 + 2 warps (the
+  // extractors' accumulators of 32 RHS would not fit one thread's registers;
+  // measured at 256 RHS, one MMA warp was 7 % slower).
+  // What bounds a chunk (~1,200 cycles at RT = 32) is that chain of hand-offs:
+  // the tensor pipe is busy a third of the time, and leaving out two thirds
+  // of the A copies, of the conversions or of the MMAs changes 0 to 3 %.
+  static constexpr int kBuildGroups = 2, kBuildThreads = 128;
+  static constexpr int kBuilders = kBuildGroups * kBuildThreads;
   static constexpr int kExtractors = RT == 16 ? 128 : 256;
   static constexpr int kMmaWarps = 2;
   static constexpr int kProducerWarp = (kBuilders + kExtractors) / 32;
@@ -288,6 +295,25 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(o.x), "=f"(o.y) : "l"(r));
   return o;
 }
+// acc holds a lane's row of 16 complex values (real parts, then imaginary
+// ones) as 8 pieces of two.  Afterwards piece r of lane l is piece l % 8 of the
+// row of lane (l & ~7) + r.
+__device__ __forceinline__ void transposePieces(float (&acc)[32], int lane) {
+#pragma unroll
+  for (int s = 4; s > 0; s >>= 1) {
+    bool const hi = lane & s;
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {   // c = 16 part + 2 piece + which
+      if ((c >> 1) & s) continue;
+      int const d = c + 2 * s;
+      float const got = __shfl_xor_sync(0xffffffffu, hi ? acc[c] : acc[d], s);
+      if (hi)
+        acc[c] = got;
+      else
+        acc[d] = got;
+    }
+  }
+}
 __device__ __forceinline__ void tmemWaitLoads() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -396,7 +422,7 @@ __global__ void __launch_bounds__(TcLayout<TERMS, RT>::kThreads, 1) applyTcKerne
     for (int s = 0; s < S; ++s) {
       mbarInit(fullA + 8 * s, 1);
       mbarInit(fullX + 8 * s, 1);
-      mbarInit(fullB + 8 * s, kBuilders / 32);
+      mbarInit(fullB + 8 * s, L::kBuildThreads / 32);
       mbarInit(empty + 8 * s, 1);
     }
     for (int b = 0; b < NB; ++b) {
@@ -571,10 +597,12 @@ __global__ void __launch_bounds__(TcLayout<TERMS, RT>::kThreads, 1) applyTcKerne
       // path the thread that copies an element into the X stage is the one
       // that converts it, so the cp.async groups need no barrier.
       // Descriptors are loaded one iteration before their first use.
-      constexpr int kJgPass = kBuilders / RT;               // k-groups per pass
+      constexpr int kGT = L::kBuildThreads, G = L::kBuildGroups;
+      constexpr int kJgPass = kGT / RT;               // k-groups per pass
       constexpr int kPasses = (kTcChunkCols / 4) / kJgPass;
       static_assert(kPasses * kJgPass == kTcChunkCols / 4, "builder passes");
-      int const q = tid % RT, jgBase = tid / RT;
+      int const gt = tid % kGT, group = tid / kGT;
+      int const q = gt % RT, jgBase = gt / RT;
       auto issueX = [&](Cd const &d, int64_t i) {
         int64_t const xld = d.inIsX ? ldx : ldw;
         float2 const *src = (d.inIsX ? Xt : Wt) + d.inRow * xld + q;
@@ -589,18 +617,16 @@ __global__ void __launch_bounds__(TcLayout<TERMS, RT>::kThreads, 1) applyTcKerne
             }
       };
       auto bulkOf = [&](Cd const &d) { return d.inIsX ? bulkX : bulkW; };
-      Cd d0 = loadCd(0), d1 = loadCd(1), d2 = loadCd(2);
-      // inputs of chunks 0 and 1 in flight before the loop (two cp.async groups)
-      if (0 < nCh && !bulkOf(d0)) issueX(d0, 0);
+      Cd d0 = loadCd(group), d1 = loadCd(group + G);
+      // the inputs of the group's first chunk in flight before the loop
+      if (group < nCh && !bulkOf(d0)) issueX(d0, group);
       cpAsyncCommit();
-      if (1 < nCh && !bulkOf(d1)) issueX(d1, 1);
-      cpAsyncCommit();
-      for (int64_t i = 0; i < nCh; ++i) {
+      for (int64_t i = group; i < nCh; i += G) {
         int const s = (int)(i % S);
-        Cd const d3 = loadCd(i + 3);   // used from the next iteration on
-        // inputs of chunk i+2 into its stage: that stage's X area last held
-        // chunk i+2-S, which this thread has converted
-        if (i + 2 < nCh && !bulkOf(d2)) issueX(d2, i + 2);
+        Cd const d2 = loadCd(i + 2 * G);   // used from the next iteration on
+        // inputs of the group's next chunk into its stage: that stage's X area
+        // last held chunk i+G-S, which this thread has converted
+        if (i + G < nCh && !bulkOf(d1)) issueX(d1, i + G);
         cpAsyncCommit();
         // bulk inputs land on fullX, which the producer arrives on only once
         // the MMAs of chunk i-S are done; the empty wait then returns at once.
@@ -619,7 +645,7 @@ __global__ void __launch_bounds__(TcLayout<TERMS, RT>::kThreads, 1) applyTcKerne
           *abortFlag = 1;
           break;
         }
-        cpAsyncWait<2>();   // this thread's elements of chunk i have landed
+        cpAsyncWait<1>();   // this thread's elements of chunk i have landed
         uint8_t *stage = smem + s * L::stageBytes;
         uint8_t *bsm = stage + L::aBytes;
         float2 const *xs = reinterpret_cast<float2 const *>(stage + L::aBytes + L::bBytes);
@@ -656,7 +682,7 @@ __global__ void __launch_bounds__(TcLayout<TERMS, RT>::kThreads, 1) applyTcKerne
         // in A: zero it (B is zero there, but stale shared memory may hold NaNs)
         if (d0.kg & 1) {
           uint32_t const padOff = (uint32_t)d0.kg * d0.mg * 128, padBytes = (uint32_t)d0.mg * 128;
-          for (uint32_t e = (uint32_t)tid * 16; e < padBytes; e += kBuilders * 16)
+          for (uint32_t e = (uint32_t)gt * 16; e < padBytes; e += kGT * 16)
 #pragma unroll
             for (int t = 0; t < TERMS; ++t)
               *reinterpret_cast<uint4 *>(stage + t * kAPlaneBytes + padOff + e) =
@@ -667,7 +693,6 @@ __global__ void __launch_bounds__(TcLayout<TERMS, RT>::kThreads, 1) applyTcKerne
         if (lane == 0) mbarArrive(fullB + 8 * s);
         d0 = d1;
         d1 = d2;
-        d2 = d3;
       }
       cpAsyncWait<0>();
     } else {
@@ -732,12 +757,28 @@ __global__ void __launch_bounds__(TcLayout<TERMS, RT>::kThreads, 1) applyTcKerne
         if (lane == 0) mbarArrive(accEmpty + 8 * b);
         if (d.flags & kTcLast) {
           // M = 64 chunks (items of <= 64 rows): lanes 16..31 hold no row
-          int const row = d.rows <= 64 ? (lane < 16 ? e * 16 + lane : kTcRows) : e * 32 + lane;
-          if (row < d.rows) {
-            float2 *out = Wt + (d.outRow + row) * ldw + 16 * h;
+          bool const half = d.rows <= 64;
+          if (bulkW) {
+            // whole lines: eight lanes exchange their rows' eight 16-byte
+            // pieces, so that each store writes four full rows of 128 bytes
+            // (a row a lane, 8 bytes a store touched 32 lines: 11 % of the
+            // apply at 256 RHS, 65,536 points)
+            transposePieces(acc, lane);
+            int const row0 = half ? e * 16 + (lane & 8) : e * 32 + (lane & 24);
+            float2 *out = Wt + (d.outRow + row0) * RT + 16 * h + 2 * (lane & 7);
 #pragma unroll
-            for (int c = 0; c < 16; ++c)
-              if (16 * h + c < nr) out[c] = make_float2(acc[c], acc[16 + c]);
+            for (int r = 0; r < 8; ++r)
+              if (row0 + r < d.rows && !(half && lane >= 16))
+                *reinterpret_cast<float4 *>(out + r * RT) =
+                    make_float4(acc[2 * r], acc[16 + 2 * r], acc[2 * r + 1], acc[17 + 2 * r]);
+          } else {
+            int const row = half ? (lane < 16 ? e * 16 + lane : kTcRows) : e * 32 + lane;
+            if (row < d.rows) {
+              float2 *out = Wt + (d.outRow + row) * ldw + 16 * h;
+#pragma unroll
+              for (int c = 0; c < 16; ++c)
+                if (16 * h + c < nr) out[c] = make_float2(acc[c], acc[16 + c]);
+            }
           }
 #pragma unroll
           for (int c = 0; c < 32; ++c) acc[c] = 0.f;
