@@ -94,4 +94,14 @@ __device__ __forceinline__ double warpSum4(double a, double b, double c, double 
   return v;
 }
 
+// two sums the same way: a's in lanes 0 .. 15, b's in lanes 16 .. 31
+__device__ __forceinline__ double warpSum2(double a, double b) {
+  bool const hi = threadIdx.x & 16;
+  double v = hi ? b : a;
+  v += __shfl_xor_sync(0xffffffffu, hi ? a : b, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 }  // namespace bfg

@@ -621,7 +621,11 @@ __global__ void __launch_bounds__(512) hqrKernel(HqrDesc const *__restrict__ des
 // (square roots, divisions), more than the products of a pair of 50-row
 // columns: so a round goes in three steps -- every warp's dot products, the
 // angles of up to kJacSlots pairs with one thread a pair, the rotations --
-// and the angles cost one pair's instructions for 32 pairs.  Measured: the
+// and the angles cost one pair's instructions for 32 pairs.  The squared norms
+// are formed once a sweep and follow the rotations (|x|^2 - t |<x, y>|,
+// |y|^2 + t |<x, y>|): they only choose angles and say which pairs are done,
+// the rotation is orthogonal whatever they are (make: 331 -> 319 ms at 65,536
+// points, 387 -> 363 for the twelve problems).  Measured: the
 // sweeps of the re-expansions 436 -> 234 ms at 65,536 points (k = 512), 762 ->
 // 416 ms for twelve problems of up to 16,384 points, 21 -> 11 ms at 4,096 (and
 // less again after the FP32 sweeps below).
@@ -637,20 +641,19 @@ __global__ void __launch_bounds__(512) sketchJacobiKernel(JacobiDesc const *__re
   int const rank = kMode == 2 ? (int)(blockIdx.x % kSketchCluster) : 0;
   JacobiDesc const d = descs[blk];
   int const nc = d.cols, rd = d.rowsDot, LD = d.ld;
-  int const tid = threadIdx.x, nthr = blockDim.x;
-  int const lane = tid & 31, warp = tid >> 5, nWarps = nthr >> 5;
+  int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nWarps = blockDim.x >> 5;
   int const gWarp = rank * nWarps + warp, gWarps = ctas * nWarps;
   double2 *M = d.M;
   __shared__ int sRotated;
-  // pair k nWarps + w of a step: warp w's k-th; (|x|^2, |y|^2, <x, y>), then
+  // pair k nWarps + w of a step: warp w's k-th; (-, -, <x, y>), then
   // the rotation (c, s, exp(-i phi)), c = 2 for none
   __shared__ double4 sPair[kJacSlots];
+  static_assert(kJacSlots <= 512, "one thread a pair");
 
   int const P = nc + (nc & 1), nPairs = P / 2;
   double const tolRot = kEpsS * sqrt((double)rd);
   // the columns of pair pr of a round (false: the bye of an odd count)
-  auto columns = [&](int round, int pr, double2 *&ci, double2 *&cj) {
-    int i, j;
+  auto columns = [&](int round, int pr, int &i, int &j) {
     if (pr == 0) {
       i = round;
       j = P - 1;
@@ -660,37 +663,53 @@ __global__ void __launch_bounds__(512) sketchJacobiKernel(JacobiDesc const *__re
       j = round - pr;
       if (j < 0) j += P - 1;
     }
-    ci = M + (int64_t)i * LD;
-    cj = M + (int64_t)j * LD;
     return i < nc && j < nc;
+  };
+  // |column|^2 over the first rowsDot rows of every column into d.s2
+  auto norms = [&]() {
+    for (int a = gWarp; a < nc; a += gWarps) {
+      double2 const *ca = M + (int64_t)a * LD;
+      double s2 = 0;
+      for (int r = lane; r < rd; r += 32) {
+        double2 const v = Mem::ld(ca + r);
+        s2 += v.x * v.x + v.y * v.y;
+      }
+      s2 = warpSum(s2);
+      if (lane == 0) __stcg(d.s2 + a, s2);
+    }
   };
   bool converged = nc < 2;
   for (int sweep = 0; sweep < kSketchMaxSweeps && !converged; ++sweep) {
     if (tid == 0) sRotated = 0;
-    __syncthreads();
+    norms();
+    Mem::sync();
     for (int round = 0; round < P - 1; ++round) {
       for (int pr0 = 0; pr0 < nPairs; pr0 += gWarps * kJacPer) {
+        // the pair whose angle this thread finds, its norms fetched ahead
+        int const mine = pr0 + rank * nWarps + (tid / nWarps) * gWarps + tid % nWarps;
+        bool const angle = tid < kJacPer * nWarps && mine < nPairs;
+        int mi = 0, mj = 0;
+        if (angle && !columns(round, mine, mi, mj)) mi = mj = 0;
+        double const al = __ldcg(d.s2 + mi), be = __ldcg(d.s2 + mj);
         for (int k = 0, pr = pr0 + gWarp; k < kJacPer && pr < nPairs; ++k, pr += gWarps) {
-          double2 *ci, *cj;
-          double al = 0, be = 0, gr = 0, gi = 0;
-          if (columns(round, pr, ci, cj))
+          int i, j;
+          double gr = 0, gi = 0;
+          if (columns(round, pr, i, j)) {
+            double2 const *ci = M + (int64_t)i * LD, *cj = M + (int64_t)j * LD;
             for (int r = lane; r < rd; r += 32) {
               double2 const x = Mem::ld(ci + r), y = Mem::ld(cj + r);
-              al = fma(x.x, x.x, fma(x.y, x.y, al));
-              be = fma(y.x, y.x, fma(y.y, y.y, be));
               gr = fma(x.x, y.x, fma(x.y, y.y, gr));
               gi = fma(x.x, y.y, fma(-x.y, y.x, gi));
             }
+          }
           // (a bye's zeros do not rotate)
-          double const v = warpSum4(al, be, gr, gi);
-          if ((lane & 7) == 0)
-            reinterpret_cast<double *>(sPair + k * nWarps + warp)[lane >> 3] = v;
+          double const v = warpSum2(gr, gi);
+          if ((lane & 15) == 0)
+            reinterpret_cast<double *>(sPair + k * nWarps + warp)[2 + (lane >> 4)] = v;
         }
         __syncthreads();
-        int const left = nPairs - pr0 - rank * nWarps;   // pairs from this CTA's first on
-        for (int q = tid; q < kJacPer * nWarps; q += nthr) {
-          if ((q / nWarps) * gWarps + q % nWarps >= left) continue;
-          double const al = sPair[q].x, be = sPair[q].y, gr = sPair[q].z, gi = sPair[q].w;
+        if (angle) {
+          double const gr = sPair[tid].z, gi = sPair[tid].w;
           double4 rot = make_double4(2.0, 0.0, 0.0, 0.0);
           double const ag = sqrt(gr * gr + gi * gi);
           if (ag > tolRot * sqrt(al * be) && ag > 0.0) {
@@ -698,17 +717,20 @@ __global__ void __launch_bounds__(512) sketchJacobiKernel(JacobiDesc const *__re
             double const t = (zeta >= 0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
             double const c = 1.0 / sqrt(1.0 + t * t);
             rot = make_double4(c, c * t, gr / ag, -gi / ag);
+            __stcg(d.s2 + mi, fmax(al - t * ag, 0.0));
+            __stcg(d.s2 + mj, fmax(be + t * ag, 0.0));
             sRotated = 1;
           }
-          sPair[q] = rot;
+          sPair[tid] = rot;
         }
         __syncthreads();
         for (int k = 0, pr = pr0 + gWarp; k < kJacPer && pr < nPairs; ++k, pr += gWarps) {
           double4 const rot = sPair[k * nWarps + warp];
           if (rot.x > 1.5) continue;
           double const c = rot.x, s = rot.y, er = rot.z, ei = rot.w;
-          double2 *ci, *cj;
-          columns(round, pr, ci, cj);
+          int i, j;
+          columns(round, pr, i, j);
+          double2 *ci = M + (int64_t)i * LD, *cj = M + (int64_t)j * LD;
           for (int r = lane; r < LD; r += 32) {
             double2 const x = Mem::ld(ci + r), y = Mem::ld(cj + r);
             double const ytr = y.x * er - y.y * ei, yti = y.x * ei + y.y * er;
@@ -732,16 +754,7 @@ __global__ void __launch_bounds__(512) sketchJacobiKernel(JacobiDesc const *__re
     if (!rotated) converged = true;
   }
   if (!converged && tid == 0 && rank == 0) atomicOr(status, kStatusJacobiNotConverged);
-  for (int a = gWarp; a < nc; a += gWarps) {
-    double2 const *ca = M + (int64_t)a * LD;
-    double s2 = 0;
-    for (int r = lane; r < rd; r += 32) {
-      double2 const v = Mem::ld(ca + r);
-      s2 += v.x * v.x + v.y * v.y;
-    }
-    s2 = warpSum(s2);
-    if (lane == 0) d.s2[a] = s2;
-  }
+  norms();
 }
 
 // ---------------------------------------------------------------------------
