@@ -760,16 +760,22 @@ __global__ void __launch_bounds__(512) sketchJacobiKernel(JacobiDesc const *__re
 // ---------------------------------------------------------------------------
 // The first sweeps of the Jacobi in FP32: one-sided Jacobi on [X ; I], X the
 // top half of M scaled to FP32's range, one CTA per block; M's bottom half
-// receives the rotations' product V (unitary to ~1e-5).  Two Newton-Schulz
-// steps make V unitary to FP64 (products on the tensor cores), and the FP64
-// sweeps then run on [X V ; V], whose columns are orthogonal to ~1e-6: three
-// sweeps with half their pairs rotating instead of seven or eight, at FP32's 64
-// times higher rate for the rest (mixed-precision Jacobi: Zhang, Gao and Bai,
-// SIAM J. Matrix Anal. Appl. 2022).  The FP64 sweeps' stopping rule is
-// unchanged, and so is the accuracy of what they leave.
+// receives the rotations' product V (unitary to ~1e-5).  On the tensor cores
+// follow a Newton-Schulz step V <- V (3/2 I - 1/2 V^H V), a first-order step
+// V <- V (I + S) from the Gram matrix of X V (jacRefineKernel), and
+// Newton-Schulz again, which leaves V unitary to FP64.  The FP64 sweeps then
+// run on [X V ; V]: two, the second of which rotates next to nothing, instead
+// of seven or eight, at FP32's 64 times higher rate for the rest
+// (mixed-precision Jacobi: Zhang, Gao and Bai, SIAM J. Matrix Anal. Appl.
+// 2022).  The first rotates nearly every pair whatever was done before: X V
+// has an error of 2^-53 |X|, which shows in every column shorter than that.
+// The FP64 sweeps' stopping rule is unchanged, and so is the accuracy of what
+// they leave.
 // [X ; I] lives in shared memory where it fits (l <= 118), else in `scr`.
-// Measured, all sweeps: 234 -> 117 ms at 65,536 points (k = 512), 416 -> 195 ms
-// for twelve problems of up to 16,384 points, 11.9 -> 6.8 ms at 4,096.
+// Measured, FP32 sweeps: all sweeps 234 -> 117 ms at 65,536 points (k = 512),
+// 416 -> 195 ms for twelve problems of up to 16,384 points, 11.9 -> 6.8 ms at
+// 4,096; the first-order step: FP64 sweeps of the twelve 146 -> 91 ms for 15 ms
+// of products (make 363 -> 347, 319 -> 310 and 15.2 -> 14.5 ms).
 // ---------------------------------------------------------------------------
 struct Jac32Desc {
   double2 *M;    // 2 l x l, ld 2 l
@@ -876,6 +882,31 @@ __global__ void __launch_bounds__(512) jac32Kernel(Jac32Desc const *__restrict__
     int64_t const o = (int64_t)(e / l) * LD + l + e % l;
     float2 const v = A[o];
     d.M[o] = make_double2((double)v.x, (double)v.y);
+  }
+}
+
+// I + S into M's bottom half from Y^H Y in `scr` (l x l FP64, ld l): the
+// first-order step S_ij = G_ij / (G_jj - G_ii) that orthogonalises Y's columns,
+// S anti-Hermitian.  An entry above 1e-5 (two singular values close together,
+// or columns of rounding errors) is left to the sweeps, so that I + S is
+// unitary to l 1e-10 and one Newton-Schulz step makes it so to FP64.  The
+// quotient needs no more than FP32: its error is of the second order.
+__global__ void __launch_bounds__(256) jacRefineKernel(Jac32Desc const *__restrict__ descs) {
+  constexpr float kMost = 1e-5f;
+  Jac32Desc const d = descs[blockIdx.x];
+  int const l = d.l;
+  double2 const *G = reinterpret_cast<double2 const *>(d.scr);
+  double2 *T = d.M + l;
+  for (int e = threadIdx.x; e < l * l; e += blockDim.x) {
+    int const i = e % l, j = e / l;
+    double2 t = make_double2(i == j ? 1.0 : 0.0, 0.0);
+    if (i != j) {
+      double2 const v = G[e];
+      float const inv = 1.f / (float)(G[(int64_t)j * l + j].x - G[(int64_t)i * l + i].x);
+      float const sx = (float)v.x * inv, sy = (float)v.y * inv;
+      if (sx * sx + sy * sy <= kMost * kMost) t = make_double2(sx, sy);
+    }
+    T[(int64_t)j * 2 * l + i] = t;
   }
 }
 
@@ -1288,9 +1319,8 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
     }
     if ((err = launchHqr<1>(h1, dHqr1, s)) != cudaSuccess) return err;
     if ((err = launchHqr<2>(h2, dHqr2, s)) != cudaSuccess) return err;
-    // Jacobi on [R2^H ; I]: FP32 sweeps give V (M's bottom half), two
-    // Newton-Schulz steps V <- V (3/2 I - 1/2 V^H V) by way of Z's and G's
-    // buffers, then FP64 sweeps on [R2^H V ; V]
+    // Jacobi on [R2^H ; I]: FP32 sweeps give V (M's bottom half), products by
+    // way of Z's and G's buffers refine it, then FP64 sweeps on [R2^H V ; V]
     mark(5);
     {
       // by shared memory: four, two and one CTA an SM, and in global memory
@@ -1320,33 +1350,39 @@ cudaError_t runSketchReexpansion(std::vector<SketchInput> const &in, PointsDev s
         jac32Kernel<<<(unsigned)(at[c + 1] - at[c]), 512, (size_t)smem[c], s>>>(jd + at[c], c < 3);
         if ((err = cudaGetLastError()) != cudaSuccess) return err;
       }
-      // what 0: S = 3/2 I - 1/2 V^H V; 1: V S; 2: R2^H V
-      auto products = [&](int what, bool second) {
+      // C = op(A) B (kGram: A^H B, kNewton: 3/2 I - 1/2 A^H B) over every
+      // block's l x l matrices: M's halves, Z's and G's buffers
+      enum Where { kTop, kLow, kInZ, kInG };
+      enum What { kPlain, kGram, kNewton };
+      auto product = [&](What what, Where wa, Where wb, Where wc) {
         g.clear();
         for (auto const &b : blks) {
-          double2 *top = S + b.oM, *low = S + b.oM + b.l, *z = S + b.oZ, *sb = S + b.oB1;
-          int64_t const l = b.l;
+          auto at = [&](Where w) {
+            return w == kTop ? S + b.oM : w == kLow ? S + b.oM + b.l : w == kInZ ? S + b.oZ : S + b.oB1;
+          };
+          auto ld = [&](Where w) { return (w == kTop || w == kLow ? 2 : 1) * (int64_t)b.l; };
           GemmDesc d{};
           d.M = d.N = d.K = b.l;
-          double2 *v = second ? z : low;
-          int64_t const ldv = second ? l : 2 * l;
-          if (what == 0) {
-            d.A = v; d.lda = ldv; d.B = v; d.ldb = ldv; d.C = sb; d.ldc = l; d.opA = 1; d.newton = 1;
-          } else if (what == 1) {
-            d.A = v; d.lda = ldv; d.B = sb; d.ldb = l;
-            d.C = second ? low : z; d.ldc = second ? 2 * l : l;
-          } else {
-            d.A = top; d.lda = 2 * l; d.B = low; d.ldb = 2 * l; d.C = z; d.ldc = l;
-          }
+          d.A = at(wa); d.lda = ld(wa);
+          d.B = at(wb); d.ldb = ld(wb);
+          d.C = at(wc); d.ldc = ld(wc);
+          d.opA = what != kPlain;
+          d.newton = what == kNewton;
           g.push_back(d);
         }
         return launchGemms(g, gemmBufs, s);
       };
-      if ((err = products(0, false)) != cudaSuccess) return err;
-      if ((err = products(1, false)) != cudaSuccess) return err;
-      if ((err = products(0, true)) != cudaSuccess) return err;
-      if ((err = products(1, true)) != cudaSuccess) return err;
-      if ((err = products(2, false)) != cudaSuccess) return err;
+      // V to FP64 unitarity, its refinement, and the same again
+      if ((err = product(kNewton, kLow, kLow, kInG)) != cudaSuccess) return err;
+      if ((err = product(kPlain, kLow, kInG, kInZ)) != cudaSuccess) return err;
+      if ((err = product(kPlain, kTop, kInZ, kLow)) != cudaSuccess) return err;   // Y = X V
+      if ((err = product(kGram, kLow, kLow, kInG)) != cudaSuccess) return err;    // Y^H Y
+      jacRefineKernel<<<(unsigned)js.size(), 256, 0, s>>>(jd);                    // I + S
+      if ((err = cudaGetLastError()) != cudaSuccess) return err;
+      if ((err = product(kPlain, kInZ, kLow, kInG)) != cudaSuccess) return err;   // V (I + S)
+      if ((err = product(kNewton, kInG, kInG, kInZ)) != cudaSuccess) return err;
+      if ((err = product(kPlain, kInG, kInZ, kLow)) != cudaSuccess) return err;
+      if ((err = product(kPlain, kTop, kLow, kInZ)) != cudaSuccess) return err;
       jacTopKernel<<<(unsigned)js.size(), 256, 0, s>>>(jd, static_cast<double2 const *const *>(dTops.p));
       if ((err = cudaGetLastError()) != cudaSuccess) return err;
     }
