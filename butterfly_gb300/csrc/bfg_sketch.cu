@@ -731,11 +731,25 @@ __global__ void __launch_bounds__(512) sketchJacobiKernel(JacobiDesc const *__re
           int i, j;
           columns(round, pr, i, j);
           double2 *ci = M + (int64_t)i * LD, *cj = M + (int64_t)j * LD;
+          // x <- c x - w y, y <- c y + conj(w) x (a column's phase is free)
+          double const wr = s * er, wi = s * ei;
+          if (c == 1.0) {
+            // most of the rotations after the first-order step: a third fewer FMAs
+            for (int r = lane; r < LD; r += 32) {
+              double2 const x = Mem::ld(ci + r), y = Mem::ld(cj + r);
+              Mem::st(ci + r, make_double2(fma(-wr, y.x, fma(wi, y.y, x.x)),
+                                           fma(-wr, y.y, fma(-wi, y.x, x.y))));
+              Mem::st(cj + r, make_double2(fma(wr, x.x, fma(wi, x.y, y.x)),
+                                           fma(wr, x.y, fma(-wi, x.x, y.y))));
+            }
+            continue;
+          }
           for (int r = lane; r < LD; r += 32) {
             double2 const x = Mem::ld(ci + r), y = Mem::ld(cj + r);
-            double const ytr = y.x * er - y.y * ei, yti = y.x * ei + y.y * er;
-            Mem::st(ci + r, make_double2(c * x.x - s * ytr, c * x.y - s * yti));
-            Mem::st(cj + r, make_double2(s * x.x + c * ytr, s * x.y + c * yti));
+            Mem::st(ci + r, make_double2(fma(-wr, y.x, fma(wi, y.y, c * x.x)),
+                                         fma(-wr, y.y, fma(-wi, y.x, c * x.y))));
+            Mem::st(cj + r, make_double2(fma(wr, x.x, fma(wi, x.y, c * y.x)),
+                                         fma(wr, x.y, fma(-wi, x.x, c * y.y))));
           }
         }
         if (pr0 + gWarps * kJacPer < nPairs) __syncthreads();   // sPair is rewritten
