@@ -130,7 +130,7 @@ struct bfgFac_s {
     if (upStream) cudaStreamDestroy(upStream);
     if (downStream) cudaStreamDestroy(downStream);
   }
-  std::vector<int64_t> stageItem0;
+  std::vector<int64_t> stageItem0, stagePasses;   // passes: see launchApplyStageFixed
   // split-BF16 tensor-core apply, per plane count (index terms - 2): the
   // chunk schedule of the 128-row program and the bf16 planes of the factors
   struct Tc {
@@ -607,6 +607,18 @@ void buildApply(bfgFac f) {
   upload(f->segContrib0, p.segContrib0, s, "apply program");
   upload(f->segBase, p.segBase, s, "apply program");
   f->stageItem0 = p.stageItem0;
+  f->stagePasses.assign(p.stageItem0.empty() ? 0 : p.stageItem0.size() - 1, 0);
+  for (size_t st = 0; st < f->stagePasses.size(); ++st)
+    for (int64_t i = p.stageItem0[st]; i < p.stageItem0[st + 1]; ++i) {
+      bfg::ApplyItem const &it = p.items[(size_t)i];
+      if (it.nContrib > 32) {
+        f->stagePasses[st] = 0;
+        break;
+      }
+      for (int32_t c = 0; c < it.nContrib; ++c)
+        f->stagePasses[st] +=
+            (p.contribs[(size_t)(it.contrib0 + c)].n + bfg::kGemvCols - 1) / bfg::kGemvCols;
+    }
   // the FP64 apply's row scales: here, once, and not in the applies, so that
   // these launch and allocate nothing for it (a pass over the factors: 0.6 ms
   // for 3.3 GB)
@@ -625,7 +637,7 @@ cudaError_t launchStage(bfgFac f, size_t st, double2 const *arena, double2 const
   int64_t const a = f->stageItem0[st], b = f->stageItem0[st + 1];
   return bfg::launchApplyStageFixed(f->items.as<bfg::ApplyItem>() + a, b - a,
                                     f->contribs.as<bfg::ApplyContrib>(), f->rowExp.as<int16_t>(),
-                                    arena, X, ldx, W, R, f->ctx->stream);
+                                    arena, X, ldx, W, R, f->ctx->stream, f->stagePasses[st]);
 }
 cudaError_t launchStage(bfgFac f, size_t st, float2 const *arena, float2 const *X, int64_t ldx,
                         float2 *W, int64_t R) {

@@ -34,6 +34,7 @@
 // (g = lane / 4, t = lane % 4) holds the entries (g, t), (g + 8, t),
 // (g, t + 4), (g + 8, t + 4) of A, one register each, and the results of rows
 // g and g + 8 in columns 2t, 2t + 1: one complex value each.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -341,8 +342,15 @@ __global__ void __launch_bounds__(kFixThreads, NT == 1 ? 3 : 2) fixTileKernel(
 // into FP64: one rounding a pass.  The next pass's input rows and first
 // entries are fetched while a pass is multiplied, so a pass costs two
 // barriers and no exposed latency.
+//
+// Few items leave most of the chip idle while each walks its passes (4,096
+// points: 264 items of 8 passes, 356 of 3): then a cluster of 2 or 4 CTAs
+// shares an item's passes (kSplit), whose sums meet in rank 0 through
+// distributed shared memory.  An apply from HBM: 2,048 points 44 -> 34 us,
+// 4,096 65 -> 47, 8,192 94 -> 84, 16,384 184 -> 167, 32,768 unchanged at 348.
 // ---------------------------------------------------------------------------
-constexpr int kGemvCols = 120, kGemvAhead = 3, kGemvWarps = 4;
+constexpr int kGemvAhead = 3, kGemvWarps = 4;
+constexpr int64_t kGemvCtas = 152 * 16;
 static_assert(kGemvCols <= 127, "4 products of 2^54 a column below 2^63");
 static_assert(kGemvCols <= 32 * kGemvWarps, "one input row per thread");
 static_assert(kGemvCols % (kGemvWarps * kGemvAhead) == 0, "whole batches of columns");
@@ -368,6 +376,7 @@ __device__ __forceinline__ void fixMad(int64_t &acc, int32_t a, int32_t b) {
   acc += (int64_t)a * b;
 }
 
+template <int kSplit>
 __global__ void __launch_bounds__(32 * kGemvWarps, 6)
 fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restrict__ contribs,
               int16_t const *__restrict__ rowExp, double2 const *__restrict__ arena,
@@ -378,20 +387,32 @@ fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restric
   // sums of the real part (high, mixed, low) and of the imaginary part
   __shared__ int64_t part[6][S][32];
   int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  ApplyItem const it = items[blockIdx.x];
+  int const rank = blockIdx.x % kSplit;   // in the item's cluster
+  ApplyItem const it = items[blockIdx.x / kSplit];
   bool const active = lane < it.rows;
   double acc = 0.0;   // the last two warps: real and imaginary part of row lane
   double spr = 0.0, spi = 0.0;   // plain FP64 sums of this lane's columns
   bool anySpecial = false;
 
-  // the pass being fetched: columns [j0, j0 + n) of contribution c
-  int c = 0, j0 = 0, n = 0, last = 0, ea = 1023;
+  // the pass being fetched: columns [j0, j0 + n) of contribution c, of which
+  // this CTA takes every kSplit-th pass: pass b of contribution c if b + c is
+  // its rank modulo kSplit
+  int c = 0, j0 = rank * KC, n = 0, last = 0, ea = 1023, have = -1;
+  int const cols = kSplit > 1 && lane < it.nContrib ? contribs[it.contrib0 + lane].n : 0;
+  auto seek = [&]() {   // from (c, j0) on to a pass that there is
+    while (c < it.nContrib && j0 >= __shfl_sync(0xffffffffu, cols, c)) {
+      ++c;
+      j0 = ((rank - c) & (kSplit - 1)) * KC;
+    }
+  };
+  if (kSplit > 1) seek();
   double2 const *a = nullptr, *x = nullptr;
   int64_t step = 0, xs = 0, lda = 0;
   ApplyContrib cb{};
   double2 av[U], xv;
   auto fetch = [&](int buf, bool first) {
-    if (j0 == 0) {
+    if (kSplit > 1 ? c != have : j0 == 0) {
+      have = c;
       cb = contribs[it.contrib0 + c];
       ea = active ? rowExp[(it.contrib0 + c) * 32 + lane] : 1023;
       lda = cb.lda;
@@ -399,9 +420,13 @@ fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restric
       xs = cb.inIsX ? ldx : 1;
       x = cb.inIsX ? X + cb.inRow * ldx : W + cb.inRow;
       a = arena + cb.aOff + (active ? lane : 0);   // inactive lanes re-read row 0
+      if (kSplit > 1) {
+        x += j0 * xs;
+        a += j0 * lda;
+      }
     } else {
-      x += KC * xs;
-      a += KC * lda;
+      x += kSplit * KC * xs;
+      a += kSplit * KC * lda;
     }
     n = min(KC, cb.n - j0);
     // this warp's columns warp, warp + 4, ... in whole batches: a column past
@@ -418,7 +443,7 @@ fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restric
     if (lane == 0) sMax[buf][warp] = code;
   };
   int buf = 0;
-  if (it.nContrib > 0) fetch(0, true);
+  if (c < it.nContrib) fetch(0, true);
   else afterPrevious();
   while (c < it.nContrib) {
     __syncthreads();
@@ -474,8 +499,10 @@ fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restric
       anySpecial = true;
       for (int j = warp; j < n; j += S) cmacc(spr, spi, a[j * lda], x[j * xs]);
     }
-    j0 += KC;
-    if (j0 >= cb.n) {
+    j0 += kSplit * KC;
+    if (kSplit > 1) {
+      seek();
+    } else if (j0 >= cb.n) {
       j0 = 0;
       ++c;
     }
@@ -510,6 +537,18 @@ fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restric
     if (warp >= S - 2)
       for (int w = 0; w < S; ++w) acc += p[((warp - (S - 2)) * S + w) * 32 + lane];
   }
+  if constexpr (kSplit > 1) {
+    // the ranks' sums, in order, through the cluster's shared memory
+    __shared__ double sums[2][32];
+    auto cluster = cooperative_groups::this_cluster();
+    if (warp >= S - 2) sums[warp - (S - 2)][lane] = acc;
+    cluster.sync();
+    if (rank == 0 && warp >= S - 2)
+      for (int q = 1; q < kSplit; ++q)
+        acc += *cluster.map_shared_rank(&sums[warp - (S - 2)][lane], q);
+    cluster.sync();
+    if (rank) return;
+  }
   if (warp >= S - 2 && active) reinterpret_cast<double *>(W + it.outRow + lane)[warp - (S - 2)] = acc;
 }
 
@@ -536,11 +575,19 @@ cudaError_t launchRowExp(ApplyItem const *items, int64_t nItems, ApplyContrib co
 cudaError_t launchApplyStageFixed(ApplyItem const *items, int64_t nItems,
                                   ApplyContrib const *contribs, int16_t const *rowExp,
                                   double2 const *arena, double2 const *X, int64_t ldx, double2 *W,
-                                  int64_t R, cudaStream_t stream) {
+                                  int64_t R, cudaStream_t stream, int64_t nPasses) {
   if (nItems == 0) return cudaSuccess;
   if (R == 1) {
-    return launchAfter(fixGemvKernel, dim3((unsigned)nItems), dim3(32 * kGemvWarps), 0, stream,
-                       items, contribs, rowExp, arena, X, ldx, W);
+    // CTAs an item: as many as have two passes each, while the grid stays below
+    // 16 CTAs an SM (6 are resident, but they end at different times: at
+    // 4,096 points 57 us with a limit of 8, 46.5 with 12, 45 with 16, 53 with
+    // 24; up to 8 CTAs an item or one and a half passes each gained nothing)
+    int split = 1;
+    while (split < 4 && nItems * split * 2 <= kGemvCtas && nPasses >= 2 * split * nItems) split *= 2;
+    auto kernel = split == 4 ? fixGemvKernel<4> : split == 2 ? fixGemvKernel<2> : fixGemvKernel<1>;
+    return launchAfterClusters(kernel, split, dim3((unsigned)(nItems * split)),
+                               dim3(32 * kGemvWarps), 0, stream, items, contribs, rowExp, arena, X,
+                               ldx, W);
   }
   // the narrowest tile that holds the right-hand sides: a tile's empty
   // columns cost as much as full ones (32,768 points: 515 us with 4 columns,
