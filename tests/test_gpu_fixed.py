@@ -199,3 +199,23 @@ def test_wide_and_narrow_applies_agree(n, onto_itself):
                 x = X[:, :R].to(torch.complex128 if prec == "fp64" else torch.complex64)
                 y = fac.apply(x.contiguous(), precision=prec, original_order=orig)
                 assert rel_err(y.cpu().numpy().astype(complex), exact[:, :R]) < tol
+
+
+@pytest.mark.parametrize("n", [485, 1001, 2101, 4321])
+def test_plain_sums_of_shared_items(n):
+    """One right-hand side whose items' passes clusters of 2 and 4 CTAs share
+    (from 2 and 4 passes of 120 columns a block): plain FP64 sums in every
+    CTA's passes, and an infinity in the first, a middle and the last column.
+    Bounds as above."""
+    fac, blocks = _problem(40, n)
+    X = B.Rng(n).complex_randn(n).reshape(n, 1)
+    Y, bound = _exact_and_bound(fac, blocks, X)
+    clean = _apply(fac, X)
+    assert np.all(np.abs(clean.astype(LD) - Y) <= bound)
+    tiny = _apply(fac, X * 2.0 ** -1010) * 2.0 ** 1000 * 2.0 ** 10
+    assert np.all(np.abs(tiny.astype(LD) - Y) <= bound + np.abs(Y).max() * 2.0 ** -40)
+    for at in (0, n // 2, n - 1):
+        Z = X.copy()
+        Z[at] = complex(0.0, np.inf)
+        assert not np.any(np.isfinite(_apply(fac, Z)))
+    assert np.array_equal(_apply(fac, X), clean)
