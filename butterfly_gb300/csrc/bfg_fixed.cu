@@ -148,7 +148,10 @@ __device__ __forceinline__ void fixNextBlock(FixCursor &k, ApplyItem const &it, 
 // 16 right-hand sides): splitting the entries and the inputs takes about 45
 // instructions each.  Wider CTAs (8 warps on 128 rows, 8 right-hand sides a
 // tile, the next step split under the MMAs) were slower: 2,330 against 1,650
-// us at 32,768 points and 16 right-hand sides.
+// us at 32,768 points and 16 right-hand sides.  So was copying a chunk's inputs
+// to shared memory (cp.async) during the chunk before: 5,158 against 4,819 us at
+// 65,536 points and 16 right-hand sides (the addresses cost registers there
+// are none left of).
 template <int NT>
 __global__ void __launch_bounds__(kFixThreads, NT == 1 ? 3 : 2) fixTileKernel(
     ApplyItem const *__restrict__ items, ApplyContrib const *__restrict__ contribs,
