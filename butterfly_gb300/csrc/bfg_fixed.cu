@@ -15,8 +15,8 @@
 //
 // Measured (GB300; microseconds an apply; before: the FP64-unit kernels):
 //   32,768 points, k = 256, 6.0e7 entries   R = 1: 526 -> 350
-//     R = 2..4: 4,000 -> 515   R = 8: 4,018 -> 870   R = 16: 7,650 -> 1,650
-//     R = 64: 27,950 -> 6,200
+//     R = 2..4: 4,000 -> 515   R = 8: 4,018 -> 787   R = 16: 7,650 -> 1,455
+//     R = 64: 27,950 -> 5,470
 //   65,536 points, k = 512, 2.1e8 entries   R = 1: 1,583 -> 912
 // Error against extended precision on the same blocks: 4,096 points at
 // tolerance 1e-8, R = 1 4.4e-16 -> 2.0e-16, R = 2 1.1e-15 -> 2.1e-16, R = 9
@@ -141,26 +141,28 @@ __device__ __forceinline__ void fixNextBlock(FixCursor &k, ApplyItem const &it, 
 // digits in shared memory in the B fragments' order, the factor entries
 // (fetched a k-step ahead) in the registers of the lane that loaded them.
 // The digit sums are flushed into FP64 accumulators at the end of a block,
-// after fixMaxSteps k-steps and when a chunk's inputs pass their scale by more
-// than a binade; the chunk after a flush sets the scale.  The warps that share rows
-// add their FP64 sums at the end, in order.
-// Bound by instruction issue and latency, not by the tensor pipe (30 % busy at
-// 16 right-hand sides): splitting the entries and the inputs takes about 45
-// instructions each.  Wider CTAs (8 warps on 128 rows, 8 right-hand sides a
-// tile, the next step split under the MMAs) were slower: 2,330 against 1,650
-// us at 32,768 points and 16 right-hand sides.  So was copying a chunk's inputs
-// to shared memory (cp.async) during the chunk before: 5,158 against 4,819 us at
-// 65,536 points and 16 right-hand sides (the addresses cost registers there
-// are none left of).
+// after kFixMaxSteps k-steps and when a chunk's inputs pass their scale; the
+// chunk after a flush sets the scale.  The warps that share rows add their FP64
+// sums at the end, in order.
+// Bound by instruction issue and latency, not by the tensor pipe: splitting the
+// entries and the inputs takes about 45 instructions each.  So resident warps
+// count: 8 right-hand sides a tile with 168 registers and 3 CTAs an SM (16 of
+// them: 255 and 2, the tensor pipe 30 % busy) take 2,076 us where 2 CTAs took
+// 2,332 (65,536 points, 8 right-hand sides), and two such tiles 3,980 us for 16
+// where one of 16 took 4,782 although the entries are split twice; 32,768
+// points 882 -> 787 and 1,680 -> 1,455, 4,096 points 98 -> 100 and 187 -> 155.
+// 4 right-hand sides a tile at 4 CTAs an SM: 1,366 -> 1,330 us at 65,536 points,
+// 69 -> 76 at 4,096.  Wider CTAs (8 warps on 128 rows, the next step split under
+// the MMAs) were slower, 2,330 against 1,650 us at 32,768 points and 16
+// right-hand sides, and so was copying a chunk's inputs to shared memory
+// (cp.async) during the chunk before, by 7 %.
 template <int NT>
-__global__ void __launch_bounds__(kFixThreads, NT == 1 ? 3 : 2) fixTileKernel(
+__global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
     ApplyItem const *__restrict__ items, ApplyContrib const *__restrict__ contribs,
     int16_t const *__restrict__ rowExp, double2 const *__restrict__ arena, double2 const *X,
     int64_t ldx, double2 *W, int64_t R, unsigned tiles) {
   constexpr int RT = 4 * NT, KC = 128 / NT, D = kFixDigits;
-  // chunks of 32 columns flush less often with room for growth
-  constexpr int kGrow = NT == 4 ? 1 : 0;
-  static_assert(KC / 8 / (kFixWarps / 2) <= fixMaxSteps(kGrow), "a chunk between flushes");
+  static_assert(KC / 8 / (kFixWarps / 2) <= kFixMaxSteps, "a chunk between flushes");
   // B fragments: word ((st D + digit) NT + n tile) 64 + 2 lane + register
   __shared__ __align__(16) uint32_t sB[(KC / 8) * D * NT * 64];
   __shared__ int sMax[2][RT];
@@ -229,12 +231,12 @@ __global__ void __launch_bounds__(kFixThreads, NT == 1 ? 3 : 2) fixTileKernel(
     __syncthreads();
     int const cm = lane < RT ? sMax[buf][lane] : 0;
     bool const first = k.j0 == 0;
-    // a scale stays until an entry passes it by more than kGrow binades.
+    // a scale stays until an entry passes it.
     // Every warp holds the same codes and row scales, so these decisions are
     // the same in the whole CTA.
     int const mySteps = (KC / 8 + role.ks - 1) / role.ks;
-    bool const grown = code == 0 ? cm != 0 : cm > code + kGrow || cm >= kFixSpecial;
-    if (steps > 0 && (first || steps + mySteps > fixMaxSteps(kGrow) || __any_sync(0xffffffffu, grown)))
+    bool const grown = code == 0 ? cm != 0 : cm > code || cm >= kFixSpecial;
+    if (steps > 0 && (first || steps + mySteps > kFixMaxSteps || __any_sync(0xffffffffu, grown)))
       flush();
     if (steps == 0) code = cm;
     ea0 = k.ea0;
@@ -248,7 +250,7 @@ __global__ void __launch_bounds__(kFixThreads, NT == 1 ? 3 : 2) fixTileKernel(
       for (int i = 0; i < 4; ++i) {
         int const col = colX + i * (kFixThreads / RT);
         uint32_t d[D];
-        fixSplit<kGrow>(xv[i], exq, d);
+        fixSplit(xv[i], exq, d);
         // column col = 8 st + c8: lane t = c8 % 4, register c8 / 4; result
         // columns 2 (q % 4) and 2 (q % 4) + 1 of n tile q / 4
         uint32_t *w = sB + ((col >> 3) * D * NT + (q >> 2)) * 64 +
@@ -592,12 +594,11 @@ cudaError_t launchApplyStageFixed(ApplyItem const *items, int64_t nItems,
                                dim3(32 * kGemvWarps), 0, stream, items, contribs, rowExp, arena, X,
                                ldx, W);
   }
-  // the narrowest tile that holds the right-hand sides: a tile's empty
-  // columns cost as much as full ones (32,768 points: 515 us with 4 columns,
-  // 870 with 8, 1,650 with 16, whatever part of them is used)
+  // the narrowest tile that holds the right-hand sides (an empty column costs as
+  // much as a full one: 32,768 points 527 us with 4 columns, 787 with 8,
+  // whatever part of them is used), several of 8 for more
   if (R <= 4) return launchTile<1>(items, nItems, contribs, rowExp, arena, X, ldx, W, R, stream);
-  if (R <= 8) return launchTile<2>(items, nItems, contribs, rowExp, arena, X, ldx, W, R, stream);
-  return launchTile<4>(items, nItems, contribs, rowExp, arena, X, ldx, W, R, stream);
+  return launchTile<2>(items, nItems, contribs, rowExp, arena, X, ldx, W, R, stream);
 }
 
 }  // namespace bfg

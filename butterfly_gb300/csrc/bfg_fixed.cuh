@@ -29,12 +29,9 @@ namespace bfg {
 
 constexpr int kFixDigits = 7, kFixSums = 8;
 // k-steps (8 complex columns) between flushes: a step adds seven digit
-// products of 16 * 129^2 to the sum s = 6, which stays below 2^24; with
-// entries of B up to a binade above their scale (top digit 257) one of the
-// seven is 16 * 129 * 257
-__host__ __device__ constexpr int fixMaxSteps(bool grown) { return grown ? 6 : 8; }
-static_assert(7 * fixMaxSteps(false) * 16 * 129 * 129 < 1 << 24 &&
-              (6 * 129 * 129 + 129 * 257) * fixMaxSteps(true) * 16 < 1 << 24, "exact FP32 sums");
+// products of 16 * 129^2 to the sum s = 6, which stays below 2^24
+constexpr int kFixMaxSteps = 8;
+static_assert(7 * kFixMaxSteps * 16 * 129 * 129 < 1 << 24, "exact FP32 sums");
 constexpr int kFixSpecial = 2047;   // exponent code: not for fixed point
 // V 2^56 2^(Ea - 1077) 2^(Ex - 1077) as a power of two: exponent field of the
 // scale Ea + Ex - 1075, a normal number (and 2^-24 of it) in this range
@@ -68,23 +65,21 @@ __device__ __forceinline__ double fixScale(int sumE) {
 
 // t + 0x0200808080808080: its bytes are the digits + 128, its top 16 bits the
 // top digit + 512.  v at scale E: kFixMinCode <= E < kFixSpecial,
-// |v| < 2^(E - 1022 + kGrow).
-template <int kGrow = 0>
+// |v| < 2^(E - 1022).
 __device__ __forceinline__ uint64_t fixInt(double v, int E) {
   uint32_t const h = (uint32_t)__double2hiint(v), l = (uint32_t)__double2loint(v);
   uint32_t const mh = (h & 0xFFFFFu) | 0x100000u;
-  uint32_t const sh = (uint32_t)(E + kGrow) - ((h >> 20) & 0x7FFu);
+  uint32_t const sh = (uint32_t)E - ((h >> 20) & 0x7FFu);
   int32_t const s = (int32_t)h >> 31;
-  uint64_t y = ((uint64_t)__funnelshift_l(l, mh, 2 + kGrow) << 32) | (l << (2 + kGrow));
+  uint64_t y = ((uint64_t)__funnelshift_l(l, mh, 2) << 32) | (l << 2);
   asm("shr.u64 %0, %0, %1;" : "+l"(y) : "r"(sh));   // 0 from 64 on
   // the bias, and the 1 of a two's complement negation
   uint64_t const c = ((uint64_t)0x02008080u << 32) | (uint32_t)(0x80808080 - s);
   return (y ^ (uint64_t)(int64_t)s) + c;
 }
 // the digits of a complex entry, most significant first, as half pairs (re, im)
-template <int kGrow = 0>
 __device__ __forceinline__ void fixSplit(double2 v, int E, uint32_t (&d)[kFixDigits]) {
-  uint64_t const r = fixInt<kGrow>(v.x, E), i = fixInt<kGrow>(v.y, E);
+  uint64_t const r = fixInt(v.x, E), i = fixInt(v.y, E);
   uint32_t const rl = (uint32_t)r, rh = (uint32_t)(r >> 32);
   uint32_t const il = (uint32_t)i, ih = (uint32_t)(i >> 32);
   // bytes interleaved (re, im, re, im), then each pair under the exponent of

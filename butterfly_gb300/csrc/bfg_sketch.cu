@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(256) sketchFillKernel(SketchDev const *__restr
 // each thread splits two entries of A and one of B into shared memory in the
 // fragments' order -- while the MMAs of the step before run from the other
 // buffer -- and fetches the ones after.  34 MMAs of 16 x 8 x 16 per four
-// columns; the exact sums go to FP64 every fixMaxSteps k-steps.
+// columns; the exact sums go to FP64 every kFixMaxSteps k-steps.
 // Bound by the tensor pipe and by splitting the entries.  Measured, against the
 // FP64-FMA form (64 x 64 tiles, FP64 pipe 99.9 % busy): all products of the
 // 65,536-point factorization 296 -> 52 ms (the output products 225 -> 41), of
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(256, 1) zgemmKernel(GemmDesc const *__restrict
             fixMma(sum[u][i + j], a.x, a.y, a.z, a.w, b.x, b.y);
           }
       }
-      if (++steps == fixMaxSteps(false)) {
+      if (++steps == kFixMaxSteps) {
         flush();
         steps = 0;
       }
