@@ -987,7 +987,7 @@ bfgStatus applyDispatch(bfgFac f, bfgPrecision prec, void const *X, int64_t ldx,
     // the FP64 apply's fixed-point products are both more exact than
     // double-float ones and faster from two right-hand sides on, where those
     // cost as much a right-hand side as for one (32,768 points: 262 us each;
-    // the FP64 apply takes 515 for 2 and 1,650 for 16)
+    // the FP64 apply takes 515 for 2 and 1,455 for 16)
     if (R > 65535) ck(cudaErrorInvalidConfiguration, "apply stage");   // refused as ever
     runApply<double2>(f, f->arena64.as<double2>(), static_cast<double2 const *>(X), ldx, R,
                       static_cast<double2 *>(Y), ldy, flags, ev);

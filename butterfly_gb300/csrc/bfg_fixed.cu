@@ -153,7 +153,7 @@ __device__ __forceinline__ void fixNextBlock(FixCursor &k, ApplyItem const &it, 
 // points 882 -> 787 and 1,680 -> 1,455, 4,096 points 98 -> 100 and 187 -> 155.
 // 4 right-hand sides a tile at 4 CTAs an SM: 1,366 -> 1,330 us at 65,536 points,
 // 69 -> 76 at 4,096.  Wider CTAs (8 warps on 128 rows, the next step split under
-// the MMAs) were slower, 2,330 against 1,650 us at 32,768 points and 16
+// the MMAs) were slower than tiles of 16, 2,330 against 1,650 us at 32,768 points and 16
 // right-hand sides, and so was copying a chunk's inputs to shared memory
 // (cp.async) during the chunk before, by 7 %.
 template <int NT>
