@@ -140,10 +140,11 @@ __device__ __forceinline__ void fixNextBlock(FixCursor &k, ApplyItem const &it, 
 // chunk's input rows (fetched a chunk ahead, into registers) are split into
 // digits in shared memory in the B fragments' order, the factor entries
 // (fetched a k-step ahead) in the registers of the lane that loaded them.
-// The digit sums are flushed into FP64 accumulators at the end of a block,
-// after kFixMaxSteps k-steps and when a chunk's inputs pass their scale; the
-// chunk after a flush sets the scale.  The warps that share rows add their FP64
-// sums at the end, in order.
+// The digit sums are flushed into FP64 accumulators at the end of every chunk,
+// whose inputs have a scale of their own, and a right-hand side that fixed point
+// does not cover is summed in plain FP64 in that chunk: a right-hand side's
+// result depends on nothing but its own entries.  The warps that share rows add
+// their FP64 sums at the end, in order.
 // Bound by instruction issue and latency, not by the tensor pipe: splitting the
 // entries and the inputs takes about 45 instructions each.  So resident warps
 // count: 8 right-hand sides a tile with 168 registers and 3 CTAs an SM (16 of
@@ -213,58 +214,39 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
   if (tid < 2 * RT) sMax[tid / RT][tid % RT] = 0;
   __syncthreads();
 
-  int buf = 0, steps = 0;   // k-steps summed since the last flush (any warp's most)
-  int code = 0;             // lane l: scale code of right-hand side l
-  int ea0 = 1023, ea1 = 1023;
-  auto flush = [&]() {
-#pragma unroll
-    for (int u = 0; u < NT; ++u) {
-      int const ex = fixScaleOf(__shfl_sync(0xffffffffu, code, 4 * u + t));
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-        acc[u][r] = fma((double)fixTake(sum[u], r), fixScale((r < 2 ? ea0 : ea1) + ex), acc[u][r]);
-    }
-    steps = 0;
-  };
+  int buf = 0;
   if (it.nContrib > 0) fetch(0);
   while (k.c < it.nContrib) {
     __syncthreads();
-    int const cm = lane < RT ? sMax[buf][lane] : 0;
-    bool const first = k.j0 == 0;
-    // a scale stays until an entry passes it.
-    // Every warp holds the same codes and row scales, so these decisions are
-    // the same in the whole CTA.
-    int const mySteps = (KC / 8 + role.ks - 1) / role.ks;
-    bool const grown = code == 0 ? cm != 0 : cm > code || cm >= kFixSpecial;
-    if (steps > 0 && (first || steps + mySteps > kFixMaxSteps || __any_sync(0xffffffffu, grown)))
-      flush();
-    if (steps == 0) code = cm;
-    ea0 = k.ea0;
-    ea1 = k.ea1;
+    // lane q: the scale code of right-hand side q's rows in hand
+    int const code = lane < RT ? sMax[buf][lane] : 0;
     int const ex = fixScaleOf(code);
-    bool const plain = !__all_sync(0xffffffffu, fixCovers(k.eaMin, k.eaMax, ex));
     int const exq = __shfl_sync(0xffffffffu, ex, q);
+    int const ea0 = k.ea0, ea1 = k.ea1;
     if (tid < RT) sMax[buf ^ 1][tid] = 0;   // read by every warp a chunk ago
-    if (!plain) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        int const col = colX + i * (kFixThreads / RT);
-        uint32_t d[D];
-        fixSplit(xv[i], exq, d);
-        // column col = 8 st + c8: lane t = c8 % 4, register c8 / 4; result
-        // columns 2 (q % 4) and 2 (q % 4) + 1 of n tile q / 4
-        uint32_t *w = sB + ((col >> 3) * D * NT + (q >> 2)) * 64 +
-                      2 * (8 * (q & 3) + (col & 3)) + ((col >> 2) & 1);
+    for (int i = 0; i < 4; ++i) {
+      int const col = colX + i * (kFixThreads / RT);
+      uint32_t d[D];
+      fixSplit(xv[i], exq, d);
+      // column col = 8 st + c8: lane t = c8 % 4, register c8 / 4; result
+      // columns 2 (q % 4) and 2 (q % 4) + 1 of n tile q / 4
+      uint32_t *w = sB + ((col >> 3) * D * NT + (q >> 2)) * 64 +
+                    2 * (8 * (q & 3) + (col & 3)) + ((col >> 2) & 1);
 #pragma unroll
-        for (int j = 0; j < D; ++j, w += NT * 64) {
-          w[0] = d[j] ^ 0x80000000u;                   // (Re x, -Im x)
-          w[8] = __byte_perm(d[j], 0, 0x1032);         // (Im x, Re x)
-        }
+      for (int j = 0; j < D; ++j, w += NT * 64) {
+        w[0] = d[j] ^ 0x80000000u;                   // (Re x, -Im x)
+        w[8] = __byte_perm(d[j], 0, 0x1032);         // (Im x, Re x)
       }
     }
     __syncthreads();
+    // the right-hand sides that fixed point covers, each by its own rows alone
+    // (bit q; every warp finds the same)
+    unsigned const fixed =
+        __ballot_sync(0xffffffffu, lane < RT && fixCovers(k.eaMin, k.eaMax, ex));
+    unsigned const rhs = (1u << nr) - 1u;
     int const nSteps = (k.n + 7) >> 3;
-    if (!plain) {
+    if (fixed & rhs) {
 #pragma unroll 1
       for (int st = role.kp; st < nSteps; st += role.ks) {
         uint32_t d[4][D];
@@ -284,14 +266,25 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
               fixMma(sum[u][i + j], d[0][i], d[1][i], d[2][i], d[3][i], bv[u].x, bv[u].y);
         }
       }
-      steps += mySteps;
-    } else {
+#pragma unroll
+      for (int u = 0; u < NT; ++u) {
+        int const exu = __shfl_sync(0xffffffffu, ex, 4 * u + t);
+        bool const mine = (fixed >> (4 * u + t)) & 1u;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          double const v =
+              fma((double)fixTake(sum[u], r), fixScale((r < 2 ? ea0 : ea1) + exu), acc[u][r]);
+          if (mine) acc[u][r] = v;
+        }
+      }
+    }
+    if (~fixed & rhs) {
       for (int st = role.kp; st < nSteps; st += role.ks)
         for (int col = 8 * st; col < min(8 * st + 8, k.n); ++col) {
           double2 const a0 = k.a[col * k.lda + role.row0], a1 = k.a[col * k.lda + role.row1];
 #pragma unroll
           for (int u = 0; u < NT; ++u)
-            if (4 * u + t < nr) {
+            if (((~fixed & rhs) >> (4 * u + t)) & 1u) {
               double2 const x = k.x[col * k.xld + 4 * u + t];
               cmacc(acc[u][0], acc[u][1], a0, x);
               cmacc(acc[u][2], acc[u][3], a1, x);
@@ -306,7 +299,6 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
     buf ^= 1;
     if (k.c < it.nContrib) fetch(buf);
   }
-  if (steps > 0) flush();
   __syncthreads();
   double *const part = reinterpret_cast<double *>(sB);   // [warp][u][r][lane]
 #pragma unroll
