@@ -1,6 +1,6 @@
 // FP64 apply of the butterfly factors (complex128 factors and vectors) with
 // the products formed exactly from fixed-point parts: integer digits on the
-// tensor cores for several right-hand sides (bfg_fixed.cuh), 28-bit halves on
+// tensor cores for several right-hand sides (bfg_fixed.cuh), 31-bit halves on
 // the integer units for one.  GB300's FP64 units (2 FMAs a clock and SM) made
 // the plain form 3 to 40 times slower than HBM delivers the factors.  Same
 // apply program and workspace as the other precisions
@@ -10,22 +10,23 @@
 // of the factors, computed once when the factors are stored (rowExpKernel),
 // and one per right-hand side of the input rows in hand, found as they are
 // read.  Rows that fixed point does not cover (NaN, infinities, subnormals,
-// products beyond the exponent range) are multiplied in plain FP64 by the
-// same kernels.
+// products beyond the exponent range, operands graded in opposite directions:
+// fixCovers, fixEven) are multiplied in plain FP64 by the same kernels.
 //
 // Measured (GB300; microseconds an apply; before: the FP64-unit kernels):
-//   32,768 points, k = 256, 6.0e7 entries   R = 1: 526 -> 350
-//     R = 2..4: 4,000 -> 515   R = 8: 4,018 -> 787   R = 16: 7,650 -> 1,455
-//     R = 64: 27,950 -> 5,470
-//   65,536 points, k = 512, 2.1e8 entries   R = 1: 1,583 -> 912
-// Error against extended precision on the same blocks: 4,096 points at
-// tolerance 1e-8, R = 1 4.4e-16 -> 2.0e-16, R = 2 1.1e-15 -> 2.1e-16, R = 9
-// 6.4e-16 -> 2.2e-16; 1,500 points at the reference's settings 2.0e-15 ->
-// 1.9e-15, 5.5e-15 -> 1.9e-15, 3.7e-15 -> 2.2e-15.
+//   32,768 points, k = 256, 6.0e7 entries   R = 1: 526 -> 345
+//     R = 2..4: 4,000 -> 576   R = 8: 4,018 -> 940   R = 16: 7,650 -> 1,766
+//   65,536 points, k = 512, 2.1e8 entries   R = 1: 1,583 -> 905
+//     R = 8: 2,484   R = 16: 23,853 -> 4,808
+// Largest error against extended precision, in units of each result's sum of
+// moduli, blocks of 20 to 120 columns: R = 1 5e-17 -> 1e-17, R = 2 1.6e-16 ->
+// 4e-17, R = 16 8e-17 -> 4e-17 for entries of like size; operands graded in
+// opposite directions by 2^10 5e-17 -> 6e-17, 2.3e-16 -> 1.9e-16, 8e-17 ->
+// 1.3e-16 and by 2^30 5e-17 -> 5e-17, 1.7e-16 -> 9e-17, 7e-17 -> 1.2e-16.
 //
 // Why not `tcgen05` for the digits: a lane forms an entry's digits from the
 // 16 bytes it loaded, in the registers `mma.sync` reads them from; `tcgen05`
-// needs them in shared memory, and precomputed in HBM they would be 28 bytes
+// needs them in shared memory, and precomputed in HBM they would be 32 bytes
 // an entry beside the stored 16.
 //
 // Complex to real: A (16 rows x 16) holds row m = Re a_m0, Im a_m0, Re a_m1,
@@ -50,10 +51,11 @@ namespace {
 static_assert(kItemRows == 32, "two 16-row MMA tiles per item");
 
 // Row scales of every contribution of every item: rowExp[32 (contribution) +
-// row].  One CTA per item, the warps split a contribution's columns.  HBM
-// bound: reads the stored factors once.
+// row], and the most small columns of a row (fixEven).  One CTA per item, the
+// warps split a contribution's columns.  HBM bound: reads the stored factors
+// once (a piece's second pass finds them in the caches).
 __global__ void __launch_bounds__(256) rowExpKernel(ApplyItem const *__restrict__ items,
-                                                    ApplyContrib const *__restrict__ contribs,
+                                                    ApplyContrib *contribs,
                                                     double2 const *__restrict__ arena,
                                                     int16_t *__restrict__ rowExp) {
   __shared__ int red[8][32];
@@ -62,15 +64,26 @@ __global__ void __launch_bounds__(256) rowExpKernel(ApplyItem const *__restrict_
   for (int c = 0; c < it.nContrib; ++c) {
     ApplyContrib const cb = contribs[it.contrib0 + c];
     double2 const *a = arena + cb.aOff + lane;
-    int code = 0;
+    int code = 0, small = 0;
     if (lane < it.rows)
       for (int j = warp; j < cb.n; j += 8) code = max(code, fixCode(a[(int64_t)j * cb.lda]));
     red[warp][lane] = code;
     __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) code = max(code, red[w][lane]);
+    __syncthreads();
+    if (code > 0) {   // (a row of zeros is exact)
+      int const least = code - fixRowGap(cb.n);
+      for (int j = warp; j < cb.n; j += 8) small += fixCode(a[(int64_t)j * cb.lda]) < least;
+    }
+    red[warp][lane] = small;
+    __syncthreads();
     if (warp == 0) {
 #pragma unroll
-      for (int w = 1; w < 8; ++w) code = max(code, red[w][lane]);
+      for (int w = 1; w < 8; ++w) small += red[w][lane];
+      small = __reduce_max_sync(0xffffffffu, small);
       rowExp[(it.contrib0 + c) * 32 + lane] = (int16_t)fixScaleOf(code);
+      if (lane == 0) contribs[it.contrib0 + c].graded = small;
     }
     __syncthreads();
   }
@@ -142,16 +155,19 @@ __device__ __forceinline__ void fixNextBlock(FixCursor &k, ApplyItem const &it, 
 // (fetched a k-step ahead) in the registers of the lane that loaded them.
 // The digit sums are flushed into FP64 accumulators at the end of every chunk,
 // whose inputs have a scale of their own, and a right-hand side that fixed point
-// does not cover is summed in plain FP64 in that chunk: a right-hand side's
-// result depends on nothing but its own entries.  The warps that share rows add
-// their FP64 sums at the end, in order.
+// does not cover (fixCovers, fixEven) is summed in plain FP64 in that chunk: a
+// right-hand side's result depends on nothing but its own entries.  The warps
+// that share rows add their FP64 sums at the end, in order.
 // Bound by instruction issue and latency, not by the tensor pipe: splitting the
-// entries and the inputs takes about 45 instructions each.  So resident warps
-// count: 8 right-hand sides a tile with 168 registers and 3 CTAs an SM (16 of
-// them: 255 and 2, the tensor pipe 30 % busy) take 2,076 us where 2 CTAs took
-// 2,332 (65,536 points, 8 right-hand sides), and two such tiles 3,980 us for 16
-// where one of 16 took 4,782 although the entries are split twice; 32,768
-// points 882 -> 787 and 1,680 -> 1,455, 4,096 points 98 -> 100 and 187 -> 155.
+// entries and the inputs takes about 50 instructions each.  So resident warps
+// count.  (65,536 points, 8 and 16 right-hand sides: 2,484 and 4,808 us.  With
+// seven digits and without the gradings 2,225 and 4,290; with seven digits and
+// flushes a block also the tiles' shape was chosen:) 8 right-hand sides a tile
+// with 168 registers and 3 CTAs an SM (16 of them: 255 and 2, the tensor pipe
+// 30 % busy) took 2,076 us where 2 CTAs took 2,332, and two such tiles 3,980
+// us for 16 where one of 16 took 4,782 although the entries are split twice;
+// 32,768 points 882 -> 787 and 1,680 -> 1,455, 4,096 points 98 -> 100 and 187
+// -> 155.
 // 4 right-hand sides a tile at 4 CTAs an SM: 1,366 -> 1,330 us at 65,536 points,
 // 69 -> 76 at 4,096.  Wider CTAs (8 warps on 128 rows, the next step split under
 // the MMAs) were slower than tiles of 16, 2,330 against 1,650 us at 32,768 points and 16
@@ -166,7 +182,7 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
   static_assert(KC / 8 / (kFixWarps / 2) <= kFixMaxSteps, "a chunk between flushes");
   // B fragments: word ((st D + digit) NT + n tile) 64 + 2 lane + register
   __shared__ __align__(16) uint32_t sB[(KC / 8) * D * NT * 64];
-  __shared__ int sMax[2][RT];
+  __shared__ int sMax[2][RT], sBig[kFixWarps][RT];
   static_assert(sizeof(sB) >= kFixWarps * NT * 4 * 32 * sizeof(double), "partial sums");
   int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t = lane & 3;
   int const q = tid % RT, colX = tid / RT;   // the input entries this thread splits
@@ -222,11 +238,14 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
     int const code = lane < RT ? sMax[buf][lane] : 0;
     int const ex = fixScaleOf(code);
     int const exq = __shfl_sync(0xffffffffu, ex, q);
+    int const leastq = __shfl_sync(0xffffffffu, code, q) - kFixInputGap;
     int const ea0 = k.ea0, ea1 = k.ea1;
     if (tid < RT) sMax[buf ^ 1][tid] = 0;   // read by every warp a chunk ago
+    int big = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       int const col = colX + i * (kFixThreads / RT);
+      big += col < k.n && fixCode(xv[i]) >= leastq;
       uint32_t d[D];
       fixSplit(xv[i], exq, d);
       // column col = 8 st + c8: lane t = c8 % 4, register c8 / 4; result
@@ -239,12 +258,20 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
         w[8] = __byte_perm(d[j], 0, 0x1032);         // (Im x, Re x)
       }
     }
+#pragma unroll
+    for (int o = RT; o < 32; o *= 2) big += __shfl_xor_sync(0xffffffffu, big, o);
+    if (lane < RT) sBig[warp][lane] = big;
     __syncthreads();
     // the right-hand sides that fixed point covers, each by its own rows alone
     // (bit q; every warp finds the same)
-    unsigned const fixed =
-        __ballot_sync(0xffffffffu, lane < RT && fixCovers(k.eaMin, k.eaMax, ex));
-    unsigned const rhs = (1u << nr) - 1u;
+    bool ok = false;
+    if (lane < RT) {
+      int all = 0;
+#pragma unroll
+      for (int w = 0; w < kFixWarps; ++w) all += sBig[w][lane];
+      ok = fixCovers(k.eaMin, k.eaMax, ex) && (code == 0 || fixEven(k.n, all, cb.graded));
+    }
+    unsigned const fixed = __ballot_sync(0xffffffffu, ok), rhs = (1u << nr) - 1u;
     int const nSteps = (k.n + 7) >> 3;
     if (fixed & rhs) {
 #pragma unroll 1
@@ -272,8 +299,7 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
         bool const mine = (fixed >> (4 * u + t)) & 1u;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-          double const v =
-              fma((double)fixTake(sum[u], r), fixScale((r < 2 ? ea0 : ea1) + exu), acc[u][r]);
+          double const v = fixAdd(acc[u][r], sum[u], r, (r < 2 ? ea0 : ea1) + exu);
           if (mine) acc[u][r] = v;
         }
       }
@@ -325,11 +351,18 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
 
 // ---------------------------------------------------------------------------
 // One right-hand side.  A matrix tile of 8 columns would be nearly empty, so
-// the products are formed from two 28-bit halves on the integer units
-// instead: t (the scaled entry, |t| <= 2^55) = hi 2^28 + lo, and
-//   t t' = 2^56 hi hi' + 2^28 (hi lo' + lo hi') + lo lo',
-// each sum carried in 64 bits without rounding: 16 widening multiply-adds a
-// complex entry (32 lanes of them a clock and SM, against 2 FP64 FMAs).
+// the products are formed from two 31-bit halves on the integer units
+// instead: t (the scaled entry, rounded, |t| <= 2^61) = hi 2^31 + lo, and
+//   t t' = 2^62 hi hi' + 2^31 (hi lo' + lo hi') + lo lo',
+// of which the last, below 2^60 = 2^-60 of the largest t t', is left out: 12
+// widening multiply-adds a complex entry (32 lanes of them a clock and SM,
+// against 2 FP64 FMAs).  The sums of a batch of columns fit 64 bits; they are
+// then added to wider ones.  A real product is off by less than 2^-59 of the
+// largest (typically 2^-62).  An apply at 65,536 points: 936 us with 28-bit
+// halves, whose four products a real one and 2^-55 were neither as fast nor
+// as exact, 905 so; 866 with 30-bit halves, whose sums of a pass fit 64 bits,
+// but which left opposite gradings of 2^12 with 8e-16 of the sum of moduli
+// (FP64 sums 5e-17, these 9e-17).
 //
 // One CTA of 4 warps per item, lane = row.  A block's columns are walked in
 // passes of at most 120: the pass's input rows are brought to one scale in
@@ -337,33 +370,38 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
 // entries in registers with the next three columns' loads in flight, and the
 // warps' integer sums are added exactly before two threads a row turn them
 // into FP64: one rounding a pass.  The next pass's input rows and first
-// entries are fetched while a pass is multiplied, so a pass costs two
-// barriers and no exposed latency.
+// entries are fetched while a pass is multiplied, so a pass costs three
+// barriers and no exposed latency.  A pass that fixed point does not cover
+// (fixCovers, fixEven) is summed in plain FP64.
 //
 // Few items leave most of the chip idle while each walks its passes (4,096
 // points: 264 items of 8 passes, 356 of 3): then a cluster of 2 or 4 CTAs
 // shares an item's passes (kSplit), whose sums meet in rank 0 through
 // distributed shared memory.  An apply from HBM: 2,048 points 44 -> 34 us,
-// 4,096 65 -> 47, 8,192 94 -> 84, 16,384 184 -> 167, 32,768 unchanged at 348.
+// 4,096 65 -> 47, 8,192 94 -> 84, 16,384 184 -> 167, 32,768 unchanged (348).
 // ---------------------------------------------------------------------------
 constexpr int kGemvAhead = 3, kGemvWarps = 4;
 constexpr int64_t kGemvCtas = 152 * 16;
-static_assert(kGemvCols <= 127, "4 products of 2^54 a column below 2^63");
+static_assert(2 * kGemvAhead < 8, "two products of 2^60 a column and sum: below 2^63");
 static_assert(kGemvCols <= 32 * kGemvWarps, "one input row per thread");
 static_assert(kGemvCols % (kGemvWarps * kGemvAhead) == 0, "whole batches of columns");
 
-// (hi, lo) of v at scale E, rounded: |hi| <= 2^27, |lo| <= 2^27
+__device__ __forceinline__ void fixUnpack(uint64_t v, uint32_t &lo, uint32_t &hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
+}
+// (hi, lo) of v at scale E: t = v 2^(1083 - E) rounded, |hi|, |lo| <= 2^30
 __device__ __forceinline__ int2 fixHalves(double v, int E) {
   uint32_t const h = (uint32_t)__double2hiint(v), l = (uint32_t)__double2loint(v);
   uint32_t const mh = (h & 0xFFFFFu) | 0x100000u, sh = (uint32_t)E - ((h >> 20) & 0x7FFu);
   int32_t const s = (int32_t)h >> 31;
   // twice t, truncated (its last bit rounds lo); shr.u64 gives 0 from 64 on
-  uint64_t y = ((uint64_t)__funnelshift_l(l, mh, 3) << 32) | (l << 3);
+  uint64_t y = ((uint64_t)__funnelshift_l(l, mh, 9) << 32) | (l << 9);
   asm("shr.u64 %0, %0, %1;" : "+l"(y) : "r"(sh));
-  uint64_t const u = (y ^ (uint64_t)(int64_t)s) + (uint32_t)((1 << 28) - s);
-  uint32_t const ul = (uint32_t)u, uh = (uint32_t)(u >> 32);
-  return make_int2((int32_t)__funnelshift_r(ul, uh, 29),
-                   ((int32_t)(ul & 0x1FFFFFFFu) - ((1 << 28) - 1)) >> 1);
+  // 2 t + 1 + 2^31: the upper word is hi, the lower one 2 (lo + 2^30) and a bit
+  // (unpacked by hand: a shift by 32 would be taken into 64-bit multiplications)
+  uint32_t lo, hi;
+  fixUnpack((y ^ (uint64_t)(int64_t)s) + (uint32_t)(0x80000001 - s), lo, hi);
+  return make_int2((int32_t)hi, (int32_t)(lo >> 1) - (1 << 30));
 }
 __device__ __forceinline__ int4 fixHalves(double2 v, int E) {
   int2 const a = fixHalves(v.x, E), b = fixHalves(v.y, E);
@@ -373,6 +411,28 @@ __device__ __forceinline__ void fixMad(int64_t &acc, int32_t a, int32_t b) {
   acc += (int64_t)a * b;
 }
 
+// A sum of products in units of 2^62 (96 bits: low word and the rest) and of
+// 2^39 (m).
+struct FixWide {
+  uint32_t low = 0;
+  int64_t rest = 0, m = 0;
+  __device__ __forceinline__ void add(int64_t hh, int64_t hl, int64_t lh) {
+    uint32_t a, b, c, d;
+    fixUnpack((uint64_t)hh, a, b);
+    fixUnpack((uint64_t)rest, c, d);
+    asm("add.cc.u32 %0, %0, %3; addc.cc.u32 %1, %1, %4; addc.u32 %2, %2, %5;"
+        : "+&r"(low), "+&r"(c), "+&r"(d) : "r"(a), "r"(b), "r"((uint32_t)((int32_t)b >> 31)));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(rest) : "r"(c), "r"(d));
+    m += (hl >> 8) + (lh >> 8);
+  }
+  // m's whole units of 2^62 into the rest (rounded)
+  __device__ __forceinline__ void settle() {
+    int64_t const v = (int64_t)low + ((m + (1 << 22)) >> 23);
+    low = (uint32_t)v;
+    rest += v >> 32;
+  }
+};
+
 template <int kSplit>
 __global__ void __launch_bounds__(32 * kGemvWarps, 6)
 fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restrict__ contribs,
@@ -380,9 +440,10 @@ fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restric
               double2 const *X, int64_t ldx, double2 *W) {
   constexpr int S = kGemvWarps, U = kGemvAhead, KC = kGemvCols;
   __shared__ int4 sx[KC];
-  __shared__ int sMax[2][S];
-  // sums of the real part (high, mixed, low) and of the imaginary part
-  __shared__ int64_t part[6][S][32];
+  __shared__ int sMax[2][S], sBig[S];
+  // sums of the real and of the imaginary part: the rest and the low word
+  __shared__ int64_t part[2][S][32];
+  __shared__ uint32_t partLow[2][S][32];
   int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int const rank = blockIdx.x % kSplit;   // in the item's cluster
   ApplyItem const it = items[blockIdx.x / kSplit];
@@ -448,11 +509,18 @@ fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restric
 #pragma unroll
     for (int w = 1; w < S; ++w) code = max(code, sMax[buf][w]);
     int const ex = fixScaleOf(code);
-    // the same in every warp: all hold the scales of the same 32 rows
-    bool const special = !__all_sync(0xffffffffu, fixCovers(ea, ea, ex));
-    if (!special && tid < KC) sx[tid] = tid < n ? fixHalves(xv, ex) : make_int4(0, 0, 0, 0);
+    if (tid < KC) sx[tid] = tid < n ? fixHalves(xv, ex) : make_int4(0, 0, 0, 0);
+    int const big =
+        __popc(__ballot_sync(0xffffffffu, tid < n && fixCode(xv) >= code - kFixInputGap));
+    if (lane == 0) sBig[warp] = big;
     __syncthreads();
-    int64_t hr = 0, mr = 0, lr = 0, hi = 0, mi = 0, li = 0;
+    int all = 0;
+#pragma unroll
+    for (int w = 0; w < S; ++w) all += sBig[w];
+    // the same in every warp: all hold the scales of the same 32 rows
+    bool const special = !__all_sync(0xffffffffu, fixCovers(ea, ea, ex)) ||
+                         !(code == 0 || fixEven(n, all, cb.graded));
+    FixWide re, im;
     int const eaNow = ea;
     if (!special) {
       double2 const *aw = a + (n > warp ? warp * lda : 0);
@@ -462,36 +530,35 @@ fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restric
         double2 nv[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) nv[u] = aw[min(i + U + u, last) * step];
+        int64_t hr = 0, hlr = 0, lhr = 0, hi = 0, hli = 0, lhi = 0;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           int4 const f = fixHalves(av[u], eaNow), y = xw[u * S];
           int const nh = -f.z, nl = -f.w;
           fixMad(hr, f.x, y.x);
           fixMad(hi, f.x, y.z);
-          fixMad(mr, f.x, y.y);
-          fixMad(mi, f.x, y.w);
-          fixMad(lr, f.y, y.y);
-          fixMad(li, f.y, y.w);
+          fixMad(hlr, f.x, y.y);
+          fixMad(hli, f.x, y.w);
+          fixMad(lhr, f.y, y.x);
+          fixMad(lhi, f.y, y.z);
           fixMad(hr, nh, y.z);
           fixMad(hi, f.z, y.x);
-          fixMad(mr, f.y, y.x);
-          fixMad(mi, f.y, y.z);
-          fixMad(lr, nl, y.w);
-          fixMad(li, f.w, y.y);
-          fixMad(mr, nh, y.w);
-          fixMad(mi, f.z, y.y);
-          fixMad(mr, nl, y.z);
-          fixMad(mi, f.w, y.x);
+          fixMad(hlr, nh, y.w);
+          fixMad(hli, f.z, y.y);
+          fixMad(lhr, nl, y.z);
+          fixMad(lhi, f.w, y.x);
         }
+        re.add(hr, hlr, lhr);
+        im.add(hi, hli, lhi);
 #pragma unroll
         for (int u = 0; u < U; ++u) av[u] = nv[u];
       }
-      part[0][warp][lane] = hr;
-      part[1][warp][lane] = mr;
-      part[2][warp][lane] = lr;
-      part[3][warp][lane] = hi;
-      part[4][warp][lane] = mi;
-      part[5][warp][lane] = li;
+      re.settle();
+      im.settle();
+      part[0][warp][lane] = re.rest;
+      partLow[0][warp][lane] = re.low;
+      part[1][warp][lane] = im.rest;
+      partLow[1][warp][lane] = im.low;
     } else {
       anySpecial = true;
       for (int j = warp; j < n; j += S) cmacc(spr, spi, a[j * lda], x[j * xs]);
@@ -508,19 +575,17 @@ fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restric
     if (!special) {
       __syncthreads();
       if (warp >= S - 2) {
-        int const q = 3 * (warp - (S - 2));
-        int64_t h = 0, m = 0, l = 0;
+        int const q = warp - (S - 2);
+        // units of 2^62
+        int64_t h = 0, l = 0;
 #pragma unroll
         for (int w = 0; w < S; ++w) {
           h += part[q][w][lane];
-          m += part[q + 1][w][lane];
-          l += part[q + 2][w][lane];
+          l += partLow[q][w][lane];
         }
-        m += l >> 28;
-        h += m >> 28;
+        h += l >> 32;
         int const e = eaNow + ex;
-        acc = fma((double)h, fixScale(e),
-                  fma((double)(int)(m & 0xFFFFFFF), fixScale(e) * 0x1.0p-28, acc));
+        acc = fma((double)h, fixPow(e - 1049), fma((double)(uint32_t)l, fixPow(e - 1081), acc));
       }
     }
   }
@@ -562,7 +627,7 @@ cudaError_t launchTile(ApplyItem const *items, int64_t nItems, ApplyContrib cons
 
 }  // namespace
 
-cudaError_t launchRowExp(ApplyItem const *items, int64_t nItems, ApplyContrib const *contribs,
+cudaError_t launchRowExp(ApplyItem const *items, int64_t nItems, ApplyContrib *contribs,
                          double2 const *arena, int16_t *rowExp, cudaStream_t stream) {
   if (nItems == 0) return cudaSuccess;
   rowExpKernel<<<(unsigned)nItems, 256, 0, stream>>>(items, contribs, arena, rowExp);
@@ -587,7 +652,7 @@ cudaError_t launchApplyStageFixed(ApplyItem const *items, int64_t nItems,
                                ldx, W);
   }
   // the narrowest tile that holds the right-hand sides (an empty column costs as
-  // much as a full one: 32,768 points 527 us with 4 columns, 787 with 8,
+  // much as a full one: 32,768 points 576 us with 4 columns, 940 with 8,
   // whatever part of them is used), several of 8 for more
   if (R <= 4) return launchTile<1>(items, nItems, contribs, rowExp, arena, X, ldx, W, R, stream);
   return launchTile<2>(items, nItems, contribs, rowExp, arena, X, ldx, W, R, stream);

@@ -7,17 +7,25 @@
 // Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59, 2012): with E the
 // largest biased exponent of a row's (or of a right-hand side's) entries, an
 // entry v becomes
-//   t = trunc(v 2^(1077 - E)),  |t| <= 2^55,  t = sum_k d_k 256^(6 - k),
-// seven digits |d_k| <= 129 held as halves, and
-//   t t' = sum_s 256^(12 - s) sum_{i + j = s} d_i d'_j,  s = 0 .. 7
-// (34 of the 49 digit products; the others are below 2^-66 of the largest
-// t t').  The sum of each s is exact, and the eight are put together in
-// 64-bit integers, in units of 2^56: a right-hand side costs 34 of the 1,000
-// multiply-adds a real product, 0.14 clocks an SM for a complex one against
-// 2.2 for its four FP64 FMAs.  An entry is off by less than 2^-55 of the
-// largest one, a quarter of an FP64 rounding (2^-53), and the sum rounds once
-// per flush instead of once per term, so the error against exact arithmetic
-// is below that of the FP64 sum.
+//   t = trunc(v 2^(1084 - E)),  |t| < 2^62,  t = sum_k d_k 256^(7 - k),
+// eight digits |d_k| <= 128 (|d_0| <= 65) held as halves, and
+//   t t' = sum_s 256^(14 - s) sum_{i + j = s} d_i d'_j,  s = 0 .. 7
+// (36 of the 64 digit products).  The sum of each s is exact, and the eight
+// are put together in an integer, which is rounded once: a right-hand side
+// costs 36 of the 1,000 multiply-adds a real product, 0.15 clocks an SM for a
+// complex one against 2.2 for its four FP64 FMAs.  (The factorization's
+// products, whose operands are unitary or scaled by column, take seven digits:
+// bfg_sketch.cu.)
+//
+// Error.  With m the product of the largest part of the row and the largest
+// part of the right-hand side (the largest t is at least 2^61, so m at least
+// 2^122): the digit products left out, s = 8 above all, are below 7 2^14
+// 2^48 2^1.01 < 2^65 = 2^-57 m, and truncation is below 2^-61 of the largest
+// part on either side: a real product is off by less than 2^-56.8 m, and
+// typically (digits of either sign) by 2^-60 m.  That is an error against m,
+// not against the product itself: an FP64 sum's error is about 2^-53 sum |a x|,
+// which for operands graded in opposite directions may be far below m.  So the
+// applies look at the gradings: see fixEven.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -27,15 +35,17 @@
 
 namespace bfg {
 
-constexpr int kFixDigits = 7, kFixSums = 8;
-// k-steps (8 complex columns) between flushes: a step adds seven digit
-// products of 16 * 129^2 to the sum s = 6, which stays below 2^24
+constexpr int kFixDigits = 8, kFixSums = 8;
+// k-steps (8 complex columns) between flushes: a step adds eight digit
+// products, two of them with a first digit, of 16 columns each to the sum
+// s = 7, which stays below 2^24
 constexpr int kFixMaxSteps = 8;
-static_assert(7 * kFixMaxSteps * 16 * 129 * 129 < 1 << 24, "exact FP32 sums");
+static_assert((6 * 128 * 128 + 2 * 65 * 128) * 16 * kFixMaxSteps < 1 << 24, "exact FP32 sums");
 constexpr int kFixSpecial = 2047;   // exponent code: not for fixed point
-// V 2^56 2^(Ea - 1077) 2^(Ex - 1077) as a power of two: exponent field of the
-// scale Ea + Ex - 1075, a normal number (and 2^-24 of it) in this range
-constexpr int kFixMinSum = 1100, kFixMaxSum = 3121;
+// the scales of the sums' units, 2^56 2^(Ea - 1084) 2^(Ex - 1084) (exponent
+// field Ea + Ex - 1089) and 2^60 2^(Ea - 1081) 2^(Ex - 1081) (Ea + Ex - 1079),
+// and 2^32 times these are normal numbers in this range
+constexpr int kFixMinSum = 1100, kFixMaxSum = 3090;
 // smallest usable code: below it an entry that is zero (whose implicit bit
 // fixInt sets all the same) would not be shifted out
 constexpr int kFixMinCode = 64;
@@ -58,62 +68,85 @@ __device__ __forceinline__ bool fixCovers(int eaMin, int eaMax, int ex) {
   return eaMax < kFixSpecial && ex < kFixSpecial && eaMin + ex >= kFixMinSum &&
          eaMax + ex <= kFixMaxSum;
 }
-// 2^56 2^(Ea - 1077) 2^(Ex - 1077) for a covered pair of scales
-__device__ __forceinline__ double fixScale(int sumE) {
-  return __hiloint2double((sumE - 1075) << 20, 0);
+// the power of two with this exponent field
+__device__ __forceinline__ double fixPow(int field) { return __hiloint2double(field << 20, 0); }
+
+// Gradings.  A column counts as small in a row of n columns where its entry's
+// code is more than fixRowGap(n) below the row's largest, and as small in a
+// right-hand side where it is more than kFixInputGap below.  `graded`: the most
+// small columns that a row of the block piece has.  If an eighth of the columns
+// in hand are small in neither, every row's sum of |a||x| over these n of N
+// columns is at least n / 8 2^-(fixRowGap(N) + 1) 2^-(kFixInputGap + 1) m
+// >= (n / N) 2^-11 m, and the fixed-point sum is within N 2^-43 of it whatever
+// the entries (typically, as in opposite geometric gradings of up to 2^10, at
+// or below FP64's own 2^-53).  Otherwise the columns are summed in plain FP64.
+// The gaps: wide enough for the factors' natural gradings (equivalent points
+// near and far from a source: up to 2^9 within a row), so that of the products
+// of circles, ellipses and stars none and of scattering operators 0.2 % take
+// the plain form; an input gap of 3 would send 1 % there and a quarter instead
+// of an eighth with it 3 %, at three to four times the cost.
+constexpr int kFixInputGap = 4;
+__device__ __forceinline__ int fixRowGap(int n) { return 33 - __clz(n - 1); }   // ceil(log2 n) + 1
+__device__ __forceinline__ bool fixEven(int n, int big, int graded) {
+  return 8 * (big - graded) >= n;
 }
 
-// t + 0x0200808080808080: its bytes are the digits + 128, its top 16 bits the
-// top digit + 512.  v at scale E: kFixMinCode <= E < kFixSpecial,
-// |v| < 2^(E - 1022).
+// t and a bias that makes its bytes the digits + 128.  Eight digits: t + 2^7
+// (1 + 256 + ... + 256^7).  Seven (t = trunc(v 2^(1077 - E)), |t| <= 2^55):
+// six such bytes, and the top 16 bits the first digit + 512.  v at scale E:
+// kFixMinCode <= E < kFixSpecial, |v| < 2^(E - 1022).
+template <int D>
 __device__ __forceinline__ uint64_t fixInt(double v, int E) {
+  static_assert(D == 7 || D == 8, "digits");
+  constexpr int L = D == 8 ? 9 : 2;
   uint32_t const h = (uint32_t)__double2hiint(v), l = (uint32_t)__double2loint(v);
   uint32_t const mh = (h & 0xFFFFFu) | 0x100000u;
   uint32_t const sh = (uint32_t)E - ((h >> 20) & 0x7FFu);
   int32_t const s = (int32_t)h >> 31;
-  uint64_t y = ((uint64_t)__funnelshift_l(l, mh, 2) << 32) | (l << 2);
+  uint64_t y = ((uint64_t)__funnelshift_l(l, mh, L) << 32) | (l << L);
   asm("shr.u64 %0, %0, %1;" : "+l"(y) : "r"(sh));   // 0 from 64 on
   // the bias, and the 1 of a two's complement negation
-  uint64_t const c = ((uint64_t)0x02008080u << 32) | (uint32_t)(0x80808080 - s);
+  uint64_t const c = ((uint64_t)(D == 8 ? 0x80808080u : 0x02008080u) << 32) |
+                     (uint32_t)(0x80808080 - s);
   return (y ^ (uint64_t)(int64_t)s) + c;
 }
 // the digits of a complex entry, most significant first, as half pairs (re, im)
-__device__ __forceinline__ void fixSplit(double2 v, int E, uint32_t (&d)[kFixDigits]) {
-  uint64_t const r = fixInt(v.x, E), i = fixInt(v.y, E);
+template <int D>
+__device__ __forceinline__ void fixSplit(double2 v, int E, uint32_t (&d)[D]) {
+  uint64_t const r = fixInt<D>(v.x, E), i = fixInt<D>(v.y, E);
   uint32_t const rl = (uint32_t)r, rh = (uint32_t)(r >> 32);
   uint32_t const il = (uint32_t)i, ih = (uint32_t)(i >> 32);
   // bytes interleaved (re, im, re, im), then each pair under the exponent of
-  // 1024 (halves 1024 + byte), less 1024 + 128 (512 for the top digit)
-  uint32_t const p0 = __byte_perm(rl, il, 0x5140), p1 = __byte_perm(rl, il, 0x7362);
-  uint32_t const p2 = __byte_perm(rh, ih, 0x5140);
-  uint32_t const k = 0x64646464u;
-  d[6] = __byte_perm(p0, k, 0x4140);
-  d[5] = __byte_perm(p0, k, 0x4342);
-  d[4] = __byte_perm(p1, k, 0x4140);
-  d[3] = __byte_perm(p1, k, 0x4342);
-  d[2] = __byte_perm(p2, k, 0x4140);
-  d[1] = __byte_perm(p2, k, 0x4342);
-  d[0] = __byte_perm(rh, ih, 0x7632) | 0x64006400u;
+  // 1024 (halves 1024 + byte), less 1024 + 128 (512 for seven digits' first)
+  uint32_t const p[4] = {__byte_perm(rl, il, 0x5140), __byte_perm(rl, il, 0x7362),
+                         __byte_perm(rh, ih, 0x5140), __byte_perm(rh, ih, 0x7362)};
 #pragma unroll
-  for (int q = 0; q < kFixDigits; ++q) {
-    __half2 const off = __half2half2(__ushort_as_half(q == 0 ? 0xE600 : 0xE480));   // -1536, -1152
-    __half2 const x = __hadd2(*reinterpret_cast<__half2 const *>(&d[q]), off);
-    d[q] = *reinterpret_cast<uint32_t const *>(&x);
+  for (int q = 0; q < D; ++q) {   // q: from the last digit on
+    bool const wide = D == 7 && q == 6;
+    uint32_t const b = wide ? __byte_perm(rh, ih, 0x7632) | 0x64006400u
+                            : __byte_perm(p[q / 2], 0x64646464u, q % 2 ? 0x4342 : 0x4140);
+    __half2 const off = __half2half2(__ushort_as_half(wide ? 0xE600 : 0xE480));   // -1536, -1152
+    __half2 const x = __hadd2(*reinterpret_cast<__half2 const *>(&b), off);
+    d[D - 1 - q] = *reinterpret_cast<uint32_t const *>(&x);
   }
 }
 
-// the exact sum put together from the digit sums' element r, in units of 2^56
-// (rounded), which are cleared
-__device__ __forceinline__ int64_t fixTake(float (&sum)[kFixSums][4], int r) {
+// acc + the sum put together from the digit sums' element r, which are
+// cleared; sumE: the scales' sum Ea + Ex
+__device__ __forceinline__ double fixAdd(double acc, float (&sum)[kFixSums][4], int r, int sumE) {
   int v[kFixSums];
 #pragma unroll
   for (int s = 0; s < kFixSums; ++s) {
     v[s] = __float2int_rn(sum[s][r]);
     sum[s][r] = 0.f;
   }
-  return ((int64_t)v[0] << 40) + ((int64_t)v[1] << 32) + ((int64_t)v[2] << 24) +
-         ((int64_t)v[3] << 16) + ((int64_t)v[4] << 8) +
-         (v[5] + ((v[6] + (v[7] >> 8) + 128) >> 8));
+  int64_t const hi = ((int64_t)v[0] << 24) + ((int64_t)v[1] << 16) + ((int64_t)v[2] << 8) + v[3];
+  int64_t const lo = ((int64_t)v[4] << 24) + ((int64_t)v[5] << 16) + ((int64_t)v[6] << 8) + v[7];
+  // hi 2^32 + lo in 63 bits: one conversion and one FMA on the FP64 pipe, not
+  // two (an apply of 16 right-hand sides at 65,536 points 5,141 -> 4,808 us)
+  int const top = (int)(hi >> 12), sh = max(14 - __clz(top ^ (top >> 31)), 0);
+  int64_t const t = (int64_t)((uint64_t)hi << (32 - sh)) + (lo >> sh);
+  return fma((double)t, fixPow(sumE - 1089 + sh), acc);
 }
 
 // D += A B, 16 x 8 x 16, halves in, FP32 sums (of integers: exact)

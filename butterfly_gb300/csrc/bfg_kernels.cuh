@@ -146,11 +146,12 @@ cudaError_t launchApplyStage(ApplyItem const *items, int64_t nItems,
                              cudaStream_t stream);
 
 // FP64 apply (bfg_fixed.cu): the factors' row scales, kItemRows per
-// contribution of the program, and one stage of items.  nPasses: the stage's
+// contribution of the program, and their gradings (into the contributions);
+// and one stage of items.  nPasses: the stage's
 // blocks in passes of at most kGemvCols columns, all told; 0 (also if an item
 // has more than 32 blocks) shares no item between thread blocks.
 constexpr int kGemvCols = 120;
-cudaError_t launchRowExp(ApplyItem const *items, int64_t nItems, ApplyContrib const *contribs,
+cudaError_t launchRowExp(ApplyItem const *items, int64_t nItems, ApplyContrib *contribs,
                          double2 const *arena, int16_t *rowExp, cudaStream_t stream);
 cudaError_t launchApplyStageFixed(ApplyItem const *items, int64_t nItems,
                                   ApplyContrib const *contribs, int16_t const *rowExp,

@@ -167,7 +167,7 @@ struct ApplyContrib {
   int32_t lda;                  // column stride of the block (its m)
   int32_t n;                    // columns
   int32_t inIsX;                // 1: input rows are in X, 0: in the workspace
-  int32_t pad;
+  int32_t graded;               // FP64 apply: see fixEven (set on the device)
 };
 
 struct ApplyProgram {

@@ -232,7 +232,26 @@ __global__ void __launch_bounds__(256) sketchFillKernel(SketchDev const *__restr
 // 65,536-point factorization 296 -> 52 ms (the output products 225 -> 41), of
 // twelve problems of up to 16,384 points 257 -> 45 ms.
 // ---------------------------------------------------------------------------
-constexpr int kGemmStageWords = kFixDigits * (4 * 32 * 4 + 8 * 32 * 2);
+// Seven digits: t = trunc(v 2^(1077 - E)), |t| <= 2^55, |d_k| <= 129, and the
+// products of digits i + j <= 7 (34 of 49): an entry is off by less than 2^-54
+// of the largest of its row or column, and so is a product.
+constexpr int kGemmDigits = 7;
+constexpr int kGemmStageWords = kGemmDigits * (4 * 32 * 4 + 8 * 32 * 2);
+static_assert(7 * kFixMaxSteps * 16 * 129 * 129 < 1 << 24, "exact FP32 sums");
+
+// the exact sum put together from the digit sums' element r, in units of 2^56
+// (rounded), which are cleared
+__device__ __forceinline__ int64_t gemmTake(float (&sum)[kFixSums][4], int r) {
+  int v[kFixSums];
+#pragma unroll
+  for (int s = 0; s < kFixSums; ++s) {
+    v[s] = __float2int_rn(sum[s][r]);
+    sum[s][r] = 0.f;
+  }
+  return ((int64_t)v[0] << 40) + ((int64_t)v[1] << 32) + ((int64_t)v[2] << 24) +
+         ((int64_t)v[3] << 16) + ((int64_t)v[4] << 8) +
+         (v[5] + ((v[6] + (v[7] >> 8) + 128) >> 8));
+}
 
 __device__ __forceinline__ double2 gemmA(GemmDesc const &g, int i, int k) {
   if (i >= g.M || k >= g.K) return make_double2(0.0, 0.0);
@@ -274,7 +293,7 @@ __global__ void __launch_bounds__(256) gemmCodeKernel(GemmDesc const *__restrict
 
 __global__ void __launch_bounds__(256, 1) zgemmKernel(GemmDesc const *__restrict__ descs,
                                                       int4 const *__restrict__ tiles) {
-  constexpr int D = kFixDigits;
+  constexpr int D = kGemmDigits;
   extern __shared__ __align__(16) uint32_t gemmSmem[];   // two stages
   __shared__ int16_t sRow[kGM], sCol[kGN];
   int4 const tile = tiles[blockIdx.x];
@@ -344,7 +363,8 @@ __global__ void __launch_bounds__(256, 1) zgemmKernel(GemmDesc const *__restrict
         int const ec = sCol[16 * nh + 4 * u + t];
 #pragma unroll
         for (int r = 0; r < 4; ++r)
-          acc[u][r] = fma((double)fixTake(sum[u], r), fixScale((r < 2 ? ea0 : ea1) + ec), acc[u][r]);
+          acc[u][r] = fma((double)gemmTake(sum[u], r),
+                          fixPow((r < 2 ? ea0 : ea1) + ec - 1075), acc[u][r]);
       }
     };
     fetch(0);

@@ -46,7 +46,13 @@ typedef enum bfgLayerPotential {
 
 /* Arithmetic of an apply. */
 typedef enum bfgPrecision {
-  BFG_PRECISION_FP64 = 0,   /* complex128 factors and vectors */
+  /* complex128 factors and vectors.  Products are formed from integer parts
+   * where the operands' magnitudes allow it, else from FP64 multiply-adds: a
+   * result differs from its exact sum by about what an FP64 sum would (2^-53
+   * of the sum of moduli of its products), and never by more than N 2^-43 of
+   * it for blocks of N columns.  It depends on nothing but its own
+   * right-hand side and their number. */
+  BFG_PRECISION_FP64 = 0,
   BFG_PRECISION_FP32 = 1,   /* complex64 factors and vectors, FP32 accumulate */
   /* Tensor-core products with complex64 vectors: factors and right-hand sides
    * split into bf16 planes (hi + lo, or hi + lo + lo2), FP32 accumulate.
