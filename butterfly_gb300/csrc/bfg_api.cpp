@@ -131,6 +131,7 @@ struct bfgFac_s {
     if (downStream) cudaStreamDestroy(downStream);
   }
   std::vector<int64_t> stageItem0, stagePasses;   // passes: see launchApplyStageFixed
+  std::vector<int64_t> stageCols, stageLongest;   // columns of the items: all, the longest
   // split-BF16 tensor-core apply, per plane count (index terms - 2): the
   // chunk schedule of the 128-row program and the bf16 planes of the factors
   struct Tc {
@@ -607,18 +608,26 @@ void buildApply(bfgFac f) {
   upload(f->segContrib0, p.segContrib0, s, "apply program");
   upload(f->segBase, p.segBase, s, "apply program");
   f->stageItem0 = p.stageItem0;
-  f->stagePasses.assign(p.stageItem0.empty() ? 0 : p.stageItem0.size() - 1, 0);
-  for (size_t st = 0; st < f->stagePasses.size(); ++st)
+  size_t const nStages = p.stageItem0.empty() ? 0 : p.stageItem0.size() - 1;
+  f->stagePasses.assign(nStages, 0);
+  f->stageCols.assign(nStages, 0);
+  f->stageLongest.assign(nStages, 0);
+  for (size_t st = 0; st < nStages; ++st) {
+    bool share = true;
     for (int64_t i = p.stageItem0[st]; i < p.stageItem0[st + 1]; ++i) {
       bfg::ApplyItem const &it = p.items[(size_t)i];
-      if (it.nContrib > 32) {
-        f->stagePasses[st] = 0;
-        break;
+      if (it.nContrib > 32) share = false;
+      int64_t cols = 0;
+      for (int32_t c = 0; c < it.nContrib; ++c) {
+        int64_t const n = p.contribs[(size_t)(it.contrib0 + c)].n;
+        cols += n;
+        f->stagePasses[st] += (n + bfg::kGemvCols - 1) / bfg::kGemvCols;
       }
-      for (int32_t c = 0; c < it.nContrib; ++c)
-        f->stagePasses[st] +=
-            (p.contribs[(size_t)(it.contrib0 + c)].n + bfg::kGemvCols - 1) / bfg::kGemvCols;
+      f->stageCols[st] += cols;
+      f->stageLongest[st] = std::max(f->stageLongest[st], cols);
     }
+    if (!share) f->stagePasses[st] = 0;
+  }
   // the FP64 apply's row scales: here, once, and not in the applies, so that
   // these launch and allocate nothing for it (a pass over the factors: 0.6 ms
   // for 3.3 GB)
@@ -748,16 +757,17 @@ void ensureArenaDf(bfgFac f) {
   f->arenaDfReady = true;
 }
 
-// the double-float apply of one right-hand side: input split (and gathered)
-// into the X buffer, stages on double-float rows, final sum into complex128
-// Y.  Same launch count as runApply (the split stands in for its gather;
-// without BFG_APPLY_ORIGINAL_ORDER it is timed with the first stage).
-void runApplyDf(bfgFac f, double2 const *X, int64_t ldx, double2 *Y, int64_t ldy, uint32_t flags,
-                std::vector<cudaEvent_t> *events, bfg::SystemTerms const *sys = nullptr) {
+// the double-float apply of a few right-hand sides: input split (and
+// gathered) into the X buffer, stages on double-float rows, final sum into
+// complex128 Y.  Same launch count as runApply (the split stands in for its
+// gather; without BFG_APPLY_ORIGINAL_ORDER it is timed with the first stage).
+void runApplyDf(bfgFac f, double2 const *X, int64_t ldx, int R, double2 *Y, int64_t ldy,
+                uint32_t flags, std::vector<cudaEvent_t> *events,
+                bfg::SystemTerms const *sys = nullptr) {
   cudaStream_t s = f->ctx->stream;
   bfg::ApplyProgram const &p = f->prog;
-  ck(f->ws.ensure((size_t)std::max<int64_t>(1, p.wsRows) * sizeof(float4)), "workspace");
-  ck(f->xbuf.ensure((size_t)std::max<int64_t>(1, p.numCols) * sizeof(float4)), "input buffer");
+  ck(f->ws.ensure((size_t)std::max<int64_t>(1, p.wsRows) * R * sizeof(float4)), "workspace");
+  ck(f->xbuf.ensure((size_t)std::max<int64_t>(1, p.numCols) * R * sizeof(float4)), "input buffer");
   float4 *W = f->ws.as<float4>(), *Xd = f->xbuf.as<float4>();
   size_t ev = 0;
   auto mark = [&]() {
@@ -766,8 +776,8 @@ void runApplyDf(bfgFac f, double2 const *X, int64_t ldx, double2 *Y, int64_t ldy
   bool const orig = (flags & BFG_APPLY_ORIGINAL_ORDER) != 0;
   mark();
   ck(sys ? bfg::launchGatherScaled(*sys, f->srcPerm.as<int64_t>(), p.numCols, Xd, s)
-         : bfg::launchGatherToDf(X, ldx, orig ? f->srcPerm.as<int64_t>() : nullptr, p.numCols, Xd,
-                                 s),
+         : bfg::launchGatherToDf(X, ldx, orig ? f->srcPerm.as<int64_t>() : nullptr, p.numCols, R,
+                                 Xd, s),
      "split X");
   if (orig) mark();
   size_t const nStages = f->stageItem0.size() - 1;
@@ -775,13 +785,13 @@ void runApplyDf(bfgFac f, double2 const *X, int64_t ldx, double2 *Y, int64_t ldy
     int64_t a = f->stageItem0[st], b = f->stageItem0[st + 1];
     ck(bfg::launchApplyStageDf(f->items.as<bfg::ApplyItem>() + a, b - a,
                                f->contribs.as<bfg::ApplyContrib>(), f->arenaDf.as<float4>(), Xd,
-                               W, s),
+                               W, R, f->stageCols[st], f->stageLongest[st], s),
        "apply stage");
     mark();
   }
   ck(bfg::launchApplyReduce(f->rowSeg.as<int32_t>(), f->segStart.as<int64_t>(),
                             f->segContrib0.as<int64_t>(), f->segBase.as<int64_t>(),
-                            p.sumRows, W, 1, Y, ldy, p.numRows,
+                            p.sumRows, W, R, Y, ldy, p.numRows,
                             orig ? f->tgtPerm.as<int64_t>() : nullptr, s, 0, 0, sys),
      "apply reduce");
   mark();
@@ -962,6 +972,10 @@ void runApplyTc(bfgFac f, int terms, float2 const *X, int64_t ldx, int64_t R, fl
   mark();
 }
 
+// Which BFG_PRECISION_DF64 applies run in double-float: of one right-hand side.
+// The others take the FP64 apply, whose fixed-point products are more exact.
+bool doubleFloat(bfgFac, int64_t R) { return R == 1; }
+
 // one-time preparation of a precision's copy of the factors
 void preparePrecision(bfgFac f, bfgPrecision prec) {
   if (prec == BFG_PRECISION_FP32) ensureArena32(f);
@@ -983,17 +997,14 @@ bfgStatus applyDispatch(bfgFac f, bfgPrecision prec, void const *X, int64_t ldx,
     ensureArena32(f);
     runApply<float2>(f, f->arena32.as<float2>(), static_cast<float2 const *>(X), ldx, R,
                      static_cast<float2 *>(Y), ldy, flags, ev);
-  } else if (prec == BFG_PRECISION_DF64 && R > 1) {
-    // the FP64 apply's fixed-point products are both more exact than
-    // double-float ones and faster from two right-hand sides on, where those
-    // cost as much a right-hand side as for one (32,768 points: 262 us each;
-    // the FP64 apply takes 515 for 2 and 1,455 for 16)
+  } else if (prec == BFG_PRECISION_DF64 && !doubleFloat(f, R)) {
     if (R > 65535) ck(cudaErrorInvalidConfiguration, "apply stage");   // refused as ever
     runApply<double2>(f, f->arena64.as<double2>(), static_cast<double2 const *>(X), ldx, R,
                       static_cast<double2 *>(Y), ldy, flags, ev);
   } else if (prec == BFG_PRECISION_DF64) {
     ensureArenaDf(f);
-    runApplyDf(f, static_cast<double2 const *>(X), ldx, static_cast<double2 *>(Y), ldy, flags, ev);
+    runApplyDf(f, static_cast<double2 const *>(X), ldx, (int)R, static_cast<double2 *>(Y), ldy, flags,
+               ev);
   } else if (isTcPrecision(prec)) {
     int const terms = prec == BFG_PRECISION_BF16X3 ? 3 : 2;
     ensureTc(f, terms);
@@ -1048,7 +1059,7 @@ bfgStatus facApplySystem(bfgFac f, bfgPrecision prec, SystemTerms const &sys, do
                         BFG_APPLY_ORIGINAL_ORDER, nullptr, &sys);
     } else if (prec == BFG_PRECISION_DF64) {
       ensureArenaDf(f);
-      runApplyDf(f, nullptr, 1, Y, 1, BFG_APPLY_ORIGINAL_ORDER, nullptr, &sys);
+      runApplyDf(f, nullptr, 1, 1, Y, 1, BFG_APPLY_ORIGINAL_ORDER, nullptr, &sys);
     } else {
       return fail(f->ctx, BFG_ERROR_NOT_IMPLEMENTED, "system apply: FP64 or DF64 only");
     }

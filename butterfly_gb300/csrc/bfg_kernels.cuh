@@ -121,14 +121,16 @@ cudaError_t launchBessel01(double const *x, int64_t n, double *out, cudaStream_t
 
 // FP64 -> FP32 arena conversion (same layout)
 cudaError_t launchArenaToF32(double2 const *a64, float2 *a32, int64_t n, cudaStream_t stream);
-// double-float apply of one right-hand side (bfg_df64.cu): arena split, input split (and gather),
-// stage
+// double-float apply of a few right-hand sides (bfg_df64.cu): arena split,
+// input split (and gather), stage; X and W with leading dimension R.  cols,
+// longest: the columns of the stage's items, all told and of the longest.
 cudaError_t launchArenaToDf(double2 const *a64, float4 *adf, int64_t n, cudaStream_t stream);
 cudaError_t launchGatherToDf(double2 const *X, int64_t ldx, int64_t const *perm, int64_t nRows,
-                             float4 *out, cudaStream_t stream);
+                             int R, float4 *out, cudaStream_t stream);
 cudaError_t launchApplyStageDf(ApplyItem const *items, int64_t nItems,
                                ApplyContrib const *contribs, float4 const *arena,
-                               float4 const *X, float4 *W, cudaStream_t stream);
+                               float4 const *X, float4 *W, int R, int64_t cols, int64_t longest,
+                               cudaStream_t stream);
 
 // complex128 <-> complex64 matrix conversion (row-major, leading dims)
 // (bTile > 0: b tile-major, panel t of bTile columns at b + t bTileStride,
@@ -178,7 +180,7 @@ cudaError_t launchGatherScaled(SystemTerms const &sys, int64_t const *perm, int6
 
 // The final sum.  W row-major with leading dimension R, or (wTile > 0)
 // tile-major: panel t of wTile columns at W + t wTileStride, leading dimension
-// wTile; of type T2, or double-float (float4, R = 1) with T2 = double2.
+// wTile; of type T2, or double-float (float4) with T2 = double2.
 // nTerms: the rows' terms, all told.
 template <typename TW, typename T2>
 cudaError_t launchApplyReduce(int32_t const *rowSeg, int64_t const *segStart,
