@@ -972,9 +972,23 @@ void runApplyTc(bfgFac f, int terms, float2 const *X, int64_t ldx, int64_t R, fl
   mark();
 }
 
-// Which BFG_PRECISION_DF64 applies run in double-float: of one right-hand side.
-// The others take the FP64 apply, whose fixed-point products are more exact.
-bool doubleFloat(bfgFac, int64_t R) { return R == 1; }
+// Which BFG_PRECISION_DF64 applies run in double-float: the others take the
+// FP64 apply, whose fixed-point products are more exact and cost the same for
+// one right-hand side as for four, where double-float costs as much for each
+// (us for 2, 3 and 4, double-float against FP64: 4,096 points 57, 75 and 84
+// against 83; 10,007 117, 143 and 171 against 153; 32,768 497, 700 and 895
+// against 580).  So two run in double-float (at every size measured, 1,024 to
+// 65,536 points, faster by up to 30 %), and three where the columns are few
+// and much of the time goes by in the longest items: 2,048 to 10,007 points 5
+// to 15 % faster, but slower at 16,384, at 1,024 (one dense stage) and for
+// batches.
+bool doubleFloat(bfgFac f, int64_t R) {
+  if (R != 3) return R < 3;
+  int64_t cols = 0, longest = 0;
+  for (int64_t c : f->stageCols) cols += c;
+  for (int64_t c : f->stageLongest) longest += c;
+  return cols <= 500000 && 456 * longest >= cols;
+}
 
 // one-time preparation of a precision's copy of the factors
 void preparePrecision(bfgFac f, bfgPrecision prec) {
