@@ -990,10 +990,11 @@ bool doubleFloat(bfgFac f, int64_t R) {
   return cols <= 500000 && 456 * longest >= cols;
 }
 
-// one-time preparation of a precision's copy of the factors
-void preparePrecision(bfgFac f, bfgPrecision prec) {
+// one-time preparation of the copy of the factors that applies of R
+// right-hand sides read (R = 1: what bfgFacPrepare prepares)
+void preparePrecision(bfgFac f, bfgPrecision prec, int64_t R) {
   if (prec == BFG_PRECISION_FP32) ensureArena32(f);
-  if (prec == BFG_PRECISION_DF64) ensureArenaDf(f);
+  if (prec == BFG_PRECISION_DF64 && doubleFloat(f, R)) ensureArenaDf(f);
   if (prec == BFG_PRECISION_BF16X2) ensureTc(f, 2);
   if (prec == BFG_PRECISION_BF16X3) ensureTc(f, 3);
 }
@@ -1619,7 +1620,7 @@ bfgStatus bfgFacApplyTimed(bfgFac f, bfgPrecision prec, void const *X, int64_t l
     size_t const n = numApplyLaunches(f, flags, prec, R);
     *numLaunches = (int32_t)n;
     if (!ms || cap < (int32_t)n) return fail(f->ctx, BFG_ERROR_OUT_OF_RANGE, "timed apply: buffer too small");
-    preparePrecision(f, prec);
+    preparePrecision(f, prec, R);
     Events ev(n + 1, "event");
     bfgStatus st = applyDispatch(f, prec, X, ldx, R, Y, ldy, flags, &ev.v);
     if (st == BFG_OK) {
@@ -1848,7 +1849,7 @@ bfgStatus bfgFacPrepare(bfgFac f, bfgPrecision prec) {
   if (prec < BFG_PRECISION_FP64 || prec > BFG_PRECISION_DF64)
     return fail(f->ctx, BFG_ERROR_INVALID_ARGUMENTS, "prepare: unknown precision");
   return guarded(f->ctx, [&]() -> bfgStatus {
-    preparePrecision(f, prec);
+    preparePrecision(f, prec, 1);
     ck(cudaStreamSynchronize(f->ctx->stream), "prepare");
     return BFG_OK;
   });
@@ -1863,7 +1864,7 @@ bfgStatus bfgFacApplyHostAsync(bfgFac f, bfgPrecision prec, double const *X, int
     bool const c128 = prec == BFG_PRECISION_FP64 || prec == BFG_PRECISION_DF64;
     if (!c128 && prec != BFG_PRECISION_FP32 && !isTcPrecision(prec))
       return fail(f->ctx, BFG_ERROR_NOT_IMPLEMENTED, "apply: unknown precision");
-    preparePrecision(f, prec);
+    preparePrecision(f, prec, R);
     if (!f->upStream) {
       ck(cudaStreamCreateWithFlags(&f->upStream, cudaStreamNonBlocking), "copy streams");
       ck(cudaStreamCreateWithFlags(&f->downStream, cudaStreamNonBlocking), "copy streams");

@@ -61,10 +61,13 @@ typedef enum bfgPrecision {
    * computes in complex128 only; these are GB300 additions. */
   BFG_PRECISION_BF16X2 = 2,
   BFG_PRECISION_BF16X3 = 3,
-  /* complex128 vectors in and out, factors and intermediates as pairs of
-   * FP32 numbers (hi + lo, ~48 significant bits, 16 bytes per complex
-   * entry) with error-free FP32 products: within ~1e-13 of FP64 at FP32
-   * rates.  A GB300 addition (its FP64 units run at 1/64 of FP32). */
+  /* complex128 vectors in and out.  One or two right-hand sides (three of
+   * small problems): factors and intermediates as pairs of FP32 numbers (hi +
+   * lo, ~48 significant bits, 16 bytes per complex entry, a copy of the
+   * factors beside the FP64 ones) with error-free FP32 products, within ~1e-13
+   * of FP64 at FP32 rates.  More right-hand sides run as BFG_PRECISION_FP64,
+   * which is as fast for them, and need no copy.  A GB300 addition (its FP64
+   * units run at 1/64 of FP32). */
   BFG_PRECISION_DF64 = 4
 } bfgPrecision;
 
