@@ -988,9 +988,9 @@ __device__ __forceinline__ void addTerm(double &sr, double &si, float4 v) {   //
 }
 
 // The last sum and the input copy run with threadIdx.x over right-hand sides
-// (a power of two of them) and threadIdx.y over rows, so that nothing is
-// divided per element.  A row's terms (of type TW) are read four at a time,
-// and where the rows alone leave the chip idle (kSplit) eight warps share
+// (a power of two of them; blockIdx.y over the rest of them where the rows are
+// few) and threadIdx.y over rows, so that nothing is divided per element.  A
+// row's terms (of type TW) are read four at a time, and where the rows alone leave the chip idle (kSplit) eight warps share
 // them: one after the other, each waits for its base's load and its own
 // (2,073 rows, one right-hand side: 13.7 -> 6.6 us).  kSys adds a
 // boundary-integral system's other terms to the sum of the one right-hand
@@ -1021,7 +1021,8 @@ __global__ void __launch_bounds__(256)
       if (outPerm) o = outPerm[i];
     }
     if (i0 == blockIdx.x * (int64_t)blockDim.y) afterPrevious();
-    for (int64_t r0 = 0; r0 < R; r0 += blockDim.x) {
+    for (int64_t r0 = blockIdx.y * (int64_t)blockDim.x; r0 < R;
+         r0 += (int64_t)gridDim.y * blockDim.x) {
       int64_t const r = r0 + threadIdx.x;
       bool const mine = live && r < R;
       T sr = 0, si = 0;
@@ -1100,7 +1101,8 @@ __global__ void gatherRowsKernel(T2 const *X, int64_t ldx,
   for (int64_t i = blockIdx.x * (int64_t)blockDim.y + threadIdx.y; i < nRows;
        i += (int64_t)gridDim.x * blockDim.y) {
     T2 const *x = X + (perm ? perm[i] : i) * ldx;
-    for (int64_t r = threadIdx.x; r < R; r += blockDim.x) {
+    for (int64_t r = blockIdx.y * (int64_t)blockDim.x + threadIdx.x; r < R;
+         r += (int64_t)gridDim.y * blockDim.x) {
       int64_t const o = outTile ? (r >> (outTile == 16 ? 4 : 5)) * outTileStride + i * outTile +
                                       (r & (outTile - 1))
                                 : i * R + r;
@@ -1130,6 +1132,14 @@ dim3 rowBlock(int64_t R) {
   unsigned x = 1;
   while (x < 64 && x < R) x *= 2;
   return dim3(x, 128 / x);
+}
+
+// the grid for that: thread blocks over rows, and over right-hand sides as far
+// as the rows alone leave the chip idle (40 points, 65,536 right-hand sides in
+// points' order and FP32: 1,350 us with 20 thread blocks a kernel, 246 so)
+dim3 rowGrid(int64_t rowBlocks, int64_t R, dim3 block) {
+  int64_t const cols = (R + block.x - 1) / block.x, want = (152 * 16 + rowBlocks - 1) / rowBlocks;
+  return dim3((unsigned)rowBlocks, (unsigned)(cols < want ? cols : want));
 }
 
 int gridFor(int64_t total, int threads) {
@@ -1314,7 +1324,8 @@ cudaError_t launchApplyReduce(int32_t const *rowSeg, int64_t const *segStart,
     block = dim3(x, 32 / x, 8);
   }
   auto run = [&](auto kernel) {
-    return launchAfter(kernel, dim3(gridFor(nRows, block.y)), block, 0, stream, rowSeg, segStart,
+    return launchAfter(kernel, rowGrid(gridFor(nRows, block.y), R, block), block, 0, stream, rowSeg,
+                       segStart,
                        segContrib0, segBase, W, R, Y, ldy, nRows, outPerm, wTile, wTileStride,
                        sys ? *sys : SystemTerms{});
   };
@@ -1346,8 +1357,8 @@ cudaError_t launchGatherRows(T2 const *X, int64_t ldx, int64_t const *perm,
                              int64_t outTile, int64_t outTileStride) {
   if (outTile != 0 && outTile != 16 && outTile != 32) return cudaErrorInvalidValue;
   dim3 const block = rowBlock(R);
-  return launchAfter(gatherRowsKernel<T2>, dim3(gridFor(nRows, block.y)), block, 0, stream, X, ldx,
-                     perm, nRows, R, out, outTile, outTileStride);
+  return launchAfter(gatherRowsKernel<T2>, rowGrid(gridFor(nRows, block.y), R, block), block, 0,
+                     stream, X, ldx, perm, nRows, R, out, outTile, outTileStride);
 }
 
 template cudaError_t launchApplyReduce<double2, double2>(
