@@ -348,16 +348,16 @@ __device__ __forceinline__ double widen(float f) {
 // Bound by the FP64 units (4 FMAs a table entry); one thread a mode over all points was a
 // serial chain of loads (64 circles, 15,346 points: 22 us, 193 before).
 __global__ void __launch_bounds__(32 * kRestrictWarps)
-    coarseRestrictKernel(int64_t const *offsets, int64_t const *cStart, int64_t const *tabOff,
-                         float2 const *tab, double2 const *r, float2 *cin, int tiles) {
+    coarseRestrictKernel(bfg::CurveTile const *tiles, int64_t const *offsets, int64_t const *cStart,
+                         int64_t const *tabOff, float2 const *tab, double2 const *r, float2 *cin) {
   constexpr int kSlices = 32 * kRestrictWarps / kModeTile;
   __shared__ double2 part[kSlices][kModeTile];
-  int const b = blockIdx.x / tiles, tile = blockIdx.x % tiles;
+  bfg::CurveTile const tile = tiles[blockIdx.x];
+  int const b = tile.curve;
   int const lm = threadIdx.x % kModeTile, sl = threadIdx.x / kModeTile;
   int64_t const o = offsets[b], c0 = cStart[b];
   int const n = (int)(offsets[b + 1] - o), M = (int)(cStart[b + 1] - c0);
-  int const m = tile * kModeTile + lm;
-  if (tile * kModeTile >= M) return;
+  int const m = tile.first + lm;
   float2 const *t = tab + tabOff[b] + min(m, M - 1);
   double sr = 0.0, si = 0.0;
 #pragma unroll 4
@@ -412,39 +412,37 @@ __global__ void coarseGemvKernel(int64_t D, float2 const *Ainv, float2 const *ci
 // curve, four lanes a point (whole sectors of the table), every fourth mode
 // each; the curve's coefficients are converted once (64 circles, 15,346
 // points: 22.5 us, 97 with one thread a point).
-constexpr int kProlongRows = 32, kProlongTiles = 256;
+constexpr int kProlongRows = 32;
 __global__ void __launch_bounds__(4 * kProlongRows)
-    coarseProlongKernel(int64_t const *offsets, int64_t const *cStart, int64_t const *tabOff,
-                        float2 const *tab, float2 const *cout, double2 *z, int tiles) {
+    coarseProlongKernel(bfg::CurveTile const *tiles, int64_t const *offsets, int64_t const *cStart,
+                        int64_t const *tabOff, float2 const *tab, float2 const *cout, double2 *z) {
   __shared__ double2 y[kMaxModes];
-  int const b = blockIdx.x / tiles, tile = blockIdx.x % tiles;
+  bfg::CurveTile const tile = tiles[blockIdx.x];
+  int const b = tile.curve;
   int64_t const o = offsets[b], n = offsets[b + 1] - o, c0 = cStart[b];
   int const M = (int)(cStart[b + 1] - c0);
-  if ((int64_t)tile * kProlongRows >= n) return;
   for (int m = threadIdx.x; m < M; m += blockDim.x) {
     float2 const v = cout[c0 + m];
     y[m] = make_double2(v.x, v.y);
   }
   __syncthreads();
   int const q = threadIdx.x % 4;
-  for (int64_t j0 = (int64_t)tile * kProlongRows; j0 < n; j0 += (int64_t)tiles * kProlongRows) {
-    int64_t const j = j0 + threadIdx.x / 4;
-    float2 const *t = tab + tabOff[b] + (j < n ? j : n - 1) * M;
-    double sr = 0.0, si = 0.0;
+  int64_t const j = tile.first + threadIdx.x / 4;
+  float2 const *t = tab + tabOff[b] + (j < n ? j : n - 1) * M;
+  double sr = 0.0, si = 0.0;
 #pragma unroll 4
-    for (int m = q; m < M; m += 4) {
-      float2 const p = t[m];
-      double const px = widen(p.x), py = widen(p.y);
-      sr = fma(-py, y[m].y, fma(px, y[m].x, sr));
-      si = fma(py, y[m].x, fma(px, y[m].y, si));
-    }
-#pragma unroll
-    for (int s = 1; s < 4; s *= 2) {
-      sr += __shfl_xor_sync(0xffffffffu, sr, s);
-      si += __shfl_xor_sync(0xffffffffu, si, s);
-    }
-    if (q == 0 && j < n) z[o + j] = make_double2(sr, si);
+  for (int m = q; m < M; m += 4) {
+    float2 const p = t[m];
+    double const px = widen(p.x), py = widen(p.y);
+    sr = fma(-py, y[m].y, fma(px, y[m].x, sr));
+    si = fma(py, y[m].x, fma(px, y[m].y, si));
   }
+#pragma unroll
+  for (int s = 1; s < 4; s *= 2) {
+    sr += __shfl_xor_sync(0xffffffffu, sr, s);
+    si += __shfl_xor_sync(0xffffffffu, si, s);
+  }
+  if (q == 0 && j < n) z[o + j] = make_double2(sr, si);
 }
 
 unsigned gridOf(int64_t n, int t) {
@@ -464,21 +462,16 @@ cudaError_t runGemm(CGemm const *host, int nb, int maxM, int maxN, Dev &dDesc, c
 
 // z = Phi A_c^-1 Phi^H r
 void coarseCorrection(bfgSystem sys, double2 const *r, double2 *z, cudaStream_t s) {
-  int const nb = (int)sys->numCurves;
   int64_t const D = sys->coarseDim;
-  int64_t maxM = 1;
-  for (int b = 0; b < nb; ++b) maxM = std::max(maxM, sys->cStart[b + 1] - sys->cStart[b]);
-  int const mTiles = (int)((maxM + kModeTile - 1) / kModeTile);
-  int const jTiles = (int)std::min<int64_t>((sys->maxCurve + kProlongRows - 1) / kProlongRows, kProlongTiles);
-  coarseRestrictKernel<<<(unsigned)nb * mTiles, 32 * kRestrictWarps, 0, s>>>(
-      sys->dOffsets.as<int64_t>(), sys->dCStart.as<int64_t>(), sys->dTabOff.as<int64_t>(),
-      sys->dTab.as<float2>(), r, sys->dCoarseIn.as<float2>(), mTiles);
+  coarseRestrictKernel<<<(unsigned)sys->modeTiles, 32 * kRestrictWarps, 0, s>>>(
+      sys->dModeTiles.as<bfg::CurveTile>(), sys->dOffsets.as<int64_t>(), sys->dCStart.as<int64_t>(),
+      sys->dTabOff.as<int64_t>(), sys->dTab.as<float2>(), r, sys->dCoarseIn.as<float2>());
   coarseGemvKernel<<<(unsigned)((D + 7) / 8), 256, 0, s>>>(D, sys->dAcInv.as<float2>(),
                                                           sys->dCoarseIn.as<float2>(),
                                                           sys->dCoarseOut.as<float2>());
-  coarseProlongKernel<<<(unsigned)nb * jTiles, 4 * kProlongRows, 0, s>>>(
-      sys->dOffsets.as<int64_t>(), sys->dCStart.as<int64_t>(), sys->dTabOff.as<int64_t>(),
-      sys->dTab.as<float2>(), sys->dCoarseOut.as<float2>(), z, jTiles);
+  coarseProlongKernel<<<(unsigned)sys->pointTiles, 4 * kProlongRows, 0, s>>>(
+      sys->dPointTiles.as<bfg::CurveTile>(), sys->dOffsets.as<int64_t>(), sys->dCStart.as<int64_t>(),
+      sys->dTabOff.as<int64_t>(), sys->dTab.as<float2>(), sys->dCoarseOut.as<float2>(), z);
 }
 
 }  // namespace
@@ -527,6 +520,16 @@ bfgStatus bfgSystemBuildCoarse(bfgSystem sys, int32_t extraModes, int64_t *dimOu
   int64_t const D = sys->cStart.back();
   sys->coarseDim = D;
   if (D > 0x7fffffff / kCT) return coarseFail(sys, BFG_ERROR_OUT_OF_RANGE, "coarse space too large");
+  std::vector<bfg::CurveTile> const modeTiles = bfg::curveTiles(sys->cStart, kModeTile);
+  std::vector<bfg::CurveTile> const pointTiles = bfg::curveTiles(sys->offsets, kProlongRows);
+  sys->modeTiles = (int64_t)modeTiles.size();
+  sys->pointTiles = (int64_t)pointTiles.size();
+  CO_CK(sys->dModeTiles.alloc(modeTiles.size() * sizeof(bfg::CurveTile)));
+  CO_CK(sys->dPointTiles.alloc(pointTiles.size() * sizeof(bfg::CurveTile)));
+  CO_CK(cudaMemcpyAsync(sys->dModeTiles.p, modeTiles.data(), modeTiles.size() * sizeof(bfg::CurveTile),
+                        cudaMemcpyHostToDevice, s));
+  CO_CK(cudaMemcpyAsync(sys->dPointTiles.p, pointTiles.data(), pointTiles.size() * sizeof(bfg::CurveTile),
+                        cudaMemcpyHostToDevice, s));
   CO_CK(sys->dCStart.alloc((nb + 1) * 8));
   CO_CK(sys->dTabOff.alloc((nb + 1) * 8));
   CO_CK(sys->dTab.alloc((size_t)sys->tabOff.back() * 8));

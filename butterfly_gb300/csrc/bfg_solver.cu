@@ -269,17 +269,18 @@ __global__ void blockDiagApplyKernel(int64_t n, int64_t const *curveOf, int64_t 
 // four rows, so that a residual entry is read and converted once for four
 // products and four times the loads are in flight (15,346 points on 64
 // curves: 22 us, 45 with a row a warp; 2,073 on 16: 5.4 and 5.5).
-constexpr int kBjRows = 4, kBjWarps = 4, kBjTiles = 1024;
+constexpr int kBjRows = 4, kBjWarps = 4;
 __global__ void __launch_bounds__(32 * kBjWarps)
-    blockDiagApply32Kernel(int64_t const *offsets, int64_t const *blkOff, float2 const *inv,
-                           double2 const *r, double2 const *sub, double2 const *add, double2 *z,
-                           int tiles) {
-  constexpr int Q = kBjRows, U = 4, kRows = kBjRows * kBjWarps;
-  int const b = blockIdx.x / tiles, tile = blockIdx.x % tiles, lane = threadIdx.x & 31;
-  int64_t const i0 = offsets[b], m = offsets[b + 1] - i0, blk = blkOff[b];
+    blockDiagApply32Kernel(bfg::CurveTile const *tiles, int64_t const *offsets,
+                           int64_t const *blkOff, float2 const *inv, double2 const *r,
+                           double2 const *sub, double2 const *add, double2 *z) {
+  constexpr int Q = kBjRows, U = 4;
+  bfg::CurveTile const tile = tiles[blockIdx.x];
+  int const lane = threadIdx.x & 31;
+  int64_t const i0 = offsets[tile.curve], m = offsets[tile.curve + 1] - i0;
+  int64_t const blk = blkOff[tile.curve], row = tile.first + (threadIdx.x >> 5) * Q;
   bfg::afterPrevious();
-  for (int64_t row = (int64_t)tile * kRows + (threadIdx.x >> 5) * Q; row < m;
-       row += (int64_t)tiles * kRows) {
+  if (row < m) {
     float2 const *a[Q];   // a row past the end repeats the last one
 #pragma unroll
     for (int q = 0; q < Q; ++q) a[q] = inv + blk + min(row + q, m - 1) * m;
@@ -759,8 +760,6 @@ bfgStatus bfgSystemCreate(bfgContext ctx, bfgFac fac, bfgHelm2 const *helm, doub
   cudaStream_t s = sys->stream();
   std::vector<int64_t> curveOf(n);
   for (int64_t b = 0; b < numCurves; ++b)
-    sys->maxCurve = std::max(sys->maxCurve, curveOffsets[b + 1] - curveOffsets[b]);
-  for (int64_t b = 0; b < numCurves; ++b)
     for (int64_t i = curveOffsets[b]; i < curveOffsets[b + 1]; ++i) curveOf[i] = b;
   std::vector<double> planes(4 * n, 0.0);
   for (int64_t i = 0; i < n; ++i) {
@@ -863,6 +862,11 @@ bfgStatus bfgSystemBuildBlockJacobi(bfgSystem sys) {
   SYS_CK(sys->dPerm.alloc(sys->n * 4));
   SYS_CK(sys->dFlag.alloc(4));
   SYS_CK(cudaMemcpyAsync(sys->dBlkOff.p, sys->blkOff.data(), (nb + 1) * 8, cudaMemcpyHostToDevice, s));
+  std::vector<bfg::CurveTile> const tiles = bfg::curveTiles(sys->offsets, kBjRows * kBjWarps);
+  sys->bjTiles = (int64_t)tiles.size();
+  SYS_CK(sys->dBjTiles.alloc(tiles.size() * sizeof(bfg::CurveTile)));
+  SYS_CK(cudaMemcpyAsync(sys->dBjTiles.p, tiles.data(), tiles.size() * sizeof(bfg::CurveTile),
+                         cudaMemcpyHostToDevice, s));
   SYS_CK(cudaMemsetAsync(sys->dFlag.p, 0, 4, s));
   double const *X = sys->dX.as<double>();
   int64_t const n = sys->n;
@@ -926,12 +930,9 @@ namespace {
 // z = M_bj (r - sub) + add from the FP32 inverses
 void applyBj32(bfgSystem sys, double2 const *r, double2 *z, cudaStream_t s,
                double2 const *sub = nullptr, double2 const *add = nullptr) {
-  constexpr int kRows = kBjRows * kBjWarps;
-  int const tiles = (int)std::min<int64_t>((sys->maxCurve + kRows - 1) / kRows, kBjTiles);
-  bfg::launchAfter(blockDiagApply32Kernel, dim3((unsigned)(sys->numCurves * tiles)),
-                   dim3(32 * kBjWarps), 0, s,
-      sys->dOffsets.as<int64_t>(), sys->dBlkOff.as<int64_t>(), sys->dInv32.as<float2>(), r, sub,
-      add, z, tiles);
+  bfg::launchAfter(blockDiagApply32Kernel, dim3((unsigned)sys->bjTiles), dim3(32 * kBjWarps), 0, s,
+                   sys->dBjTiles.as<bfg::CurveTile>(), sys->dOffsets.as<int64_t>(),
+                   sys->dBlkOff.as<int64_t>(), sys->dInv32.as<float2>(), r, sub, add, z);
 }
 }  // namespace
 

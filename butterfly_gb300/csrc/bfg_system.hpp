@@ -67,13 +67,29 @@ struct Landing {
   }
 };
 
+// Pieces of `step` rows of the curves' ranges [start[b], start[b + 1]), one
+// thread block each: their number follows the rows, however uneven the curves.
+// (One curve of 2,000 points among 4,000 of 8, an iteration of GMRES with
+// block-Jacobi: 1,256 us; with a grid of curves x the largest one's pieces,
+// most of them empty, 1,734.)
+struct CurveTile {
+  int32_t curve, first;
+};
+inline std::vector<CurveTile> curveTiles(std::vector<int64_t> const &start, int step) {
+  std::vector<CurveTile> t;
+  for (size_t b = 0; b + 1 < start.size(); ++b)
+    for (int64_t i = 0; i < start[b + 1] - start[b]; i += step)
+      t.push_back(CurveTile{(int32_t)b, (int32_t)i});
+  return t;
+}
+
 }  // namespace bfg
 
 struct bfgSystem_s {
   using Dev = bfg::Dev;
   bfgContext ctx = nullptr;
   bfgFac fac = nullptr;
-  int64_t n = 0, numCurves = 0, maxCurve = 1;   // maxCurve: points of the largest
+  int64_t n = 0, numCurves = 0;
   int32_t order = 0;
   double shift = 0.5;
   bfgPrecision applyPrec = BFG_PRECISION_FP64;   // of the butterfly part
@@ -86,6 +102,8 @@ struct bfgSystem_s {
   // block-Jacobi
   bool haveBj = false, haveBj64 = false;   // the FP32 inverses; the FP64 ones (on first use)
   std::vector<int64_t> blkOff;
+  int64_t bjTiles = 0;
+  Dev dBjTiles;   // CurveTile
   Dev dBlkOff, dInv, dInv32, dWork, dColBuf, dPerm, dFlag;
   // learned preconditioner: chunks of consecutive points of a curve
   bfgMlp mlp = nullptr;
@@ -99,6 +117,8 @@ struct bfgSystem_s {
   bool haveCoarse = false;
   int64_t coarseDim = 0;
   std::vector<int64_t> cStart, tabOff;
+  int64_t modeTiles = 0, pointTiles = 0;
+  Dev dModeTiles, dPointTiles;   // CurveTile
   Dev dCStart, dTabOff, dTab, dAc, dAcInv, dCoarseIn, dCoarseOut, dZ1, dT1, dT2;
   std::string err;
   cudaStream_t stream() const;
