@@ -89,7 +89,10 @@ def factorization_work(table, st):
     the same Z_equiv share one SVD, and blocks of large rank take the
     randomized path.  The rate is therefore this work over the time of both
     re-expansion paths, a reference-equivalent rate and not a fraction of a
-    hardware peak."""
+    hardware peak.
+
+    Where the fill ran beside the randomized path neither time is that of the
+    work alone: there is no rate then but the whole factorization's."""
     kind = table[:, 0]
     m = table[:, 1].astype(np.float64)
     n = table[:, 2].astype(np.float64)
@@ -98,15 +101,23 @@ def factorization_work(table, st):
     proxy = float(np.sum(m[fm] * m[fm] + m[fm] * n[fm]))
     svd = float(np.sum(22.0 * m[fm] ** 3 + 16.0 * m[fm] ** 2 * n[fm]))
     reexp_s = (st["reexpSmemMs"] + st["reexpGlobalMs"] + st.get("sketchMs", 0.0)) / 1e3
+    # the parts' sum passes the whole by what ran side by side (device time
+    # that is in no part hides a little of it)
+    overlap = max(0.0, st["fillMs"] + 1e3 * reexp_s - st["factorMs"]) if "factorMs" in st else 0.0
+    rated_s = reexp_s if overlap == 0.0 else st["factorMs"] / 1e3
     return {"kernel_evals": fill + proxy, "fill_evals": fill, "proxy_evals": proxy,
-            "fill_evals_per_s": fill / (st["fillMs"] / 1e3) if st["fillMs"] > 0 else None,
+            "fill_evals_per_s": fill / (st["fillMs"] / 1e3)
+            if st["fillMs"] > 0 and overlap == 0.0 else None,
+            "kernel_evals_per_s": (fill + proxy) / (st["factorMs"] / 1e3)
+            if st.get("factorMs") else None,
+            "fill_overlap_ms": overlap,
             "first_middle_blocks": int(np.sum(fm)),
             "full_path_svds": st.get("reexpSvds"),
             "sketched_blocks": st.get("numSketched"),
             "reexp_s": reexp_s,
             "svd_flops_reference_equivalent": svd,
             "svd_model": "22 p^3 + 16 p^2 n per FIRST/MIDDLE block (rank p, n columns)",
-            "reference_equivalent_tflops": svd / reexp_s / 1e12 if reexp_s > 0 else None}
+            "reference_equivalent_tflops": svd / rated_s / 1e12 if rated_s > 0 else None}
 
 
 def gpu_local_cpus(dev=0):

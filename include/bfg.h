@@ -130,14 +130,19 @@ typedef struct bfgFacStats {
   int64_t jacobiNotConverged; /* 1 if any block's Jacobi SVD hit the sweep cap */
   double factorMs;            /* device time of the factorization kernels */
   double flopsPerRhs;         /* 8 * sum over blocks of m*n */
-  double fillMs;              /* evaluation and dense blocks */
+  double fillMs;              /* evaluation and dense blocks.  They run beside
+                                 the randomized path where there is one: then
+                                 neither part's time is its time alone, and
+                                 the parts add up to more than factorMs */
   double reexpSmemMs;         /* re-expansions held in shared memory */
   double reexpGlobalMs;       /* re-expansions held in global memory */
-  int64_t numSketched;        /* re-expansions by the randomized path */
+  int64_t numSketched;        /* re-expansions by the randomized path, of rank
+                                 32 and more */
   int64_t sketchRetries;      /* sketches redone wider (rank not captured) */
   int64_t sketchFallbacks;    /* blocks handed back to the full path */
   int64_t sketchMaxWidth;     /* widest accepted sketch */
-  double sketchMs;            /* device time of the randomized path */
+  double sketchMs;            /* device time of the randomized path, the
+                                 blocks of rank 8 to 31 that take it included */
   double sketchMeanWidth;     /* mean accepted sketch width */
   int64_t applyBufferBytes;   /* device bytes the allocating applies have
                                  allocated so far (workspace and gather
@@ -145,10 +150,11 @@ typedef struct bfgFacStats {
   double sketchPhaseMs[8];    /* randomized path by phase: fills, Z Omega,
                                  qr(Y), Z^H Q, qr(G), Jacobi, weights and
                                  capture test, output products */
-  int64_t reexpSvds;          /* SVDs of the full path: its blocks with the
-                                 same Z_equiv share one */
-  int64_t sketchGroups;       /* SVDs of the randomized path, shared the same
-                                 way */
+  int64_t reexpSvds;          /* SVDs of the full path, and of the blocks of
+                                 rank 8 to 31 in the randomized one: blocks
+                                 with the same Z_equiv share one */
+  int64_t sketchGroups;       /* SVDs of the randomized path for rank 32 and
+                                 more, shared the same way */
 } bfgFacStats;
 
 /* Contexts: one CUDA device and one stream; calls on a context are
