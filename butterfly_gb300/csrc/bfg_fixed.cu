@@ -183,7 +183,6 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
   // B fragments: word ((st D + digit) NT + n tile) 64 + 2 lane + register
   __shared__ __align__(16) uint32_t sB[(KC / 8) * D * NT * 64];
   __shared__ int sMax[2][RT], sBig[kFixWarps][RT];
-  static_assert(sizeof(sB) >= kFixWarps * NT * 4 * 32 * sizeof(double), "partial sums");
   int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t = lane & 3;
   int const q = tid % RT, colX = tid / RT;   // the input entries this thread splits
   // the tiles of an item run side by side and read its blocks from HBM once
@@ -192,13 +191,24 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
   int const nr = (R - r0) < RT ? (int)(R - r0) : RT;
   FixRole const role(it.rows, warp, lane);
 
-  double acc[NT][4];   // (row0 re, im, row1 re, im) of right-hand side 4 nt + t
+  // (row0 re, im, row1 re, im) of right-hand side 4 nt + t.  Eight right-hand
+  // sides keep them in shared memory, where they are touched once a chunk: in
+  // registers they were spilled with others (16 right-hand sides at 65,536 points
+  // 4,824 -> 4,484 us; 4 a tile have the registers: 1,485 against 1,496)
+  __shared__ double sAcc[NT * 4][kFixThreads];
+  double rAcc[NT * 4];
+  auto acc = [&](int u, int r) -> double & {
+    if constexpr (NT > 1)
+      return sAcc[4 * u + r][tid];
+    else
+      return rAcc[4 * u + r];
+  };
   float sum[NT][kFixSums][4];
 #pragma unroll
   for (int u = 0; u < NT; ++u)
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      acc[u][r] = 0.0;
+      acc(u, r) = 0.0;
 #pragma unroll
       for (int s = 0; s < kFixSums; ++s) sum[u][s][r] = 0.f;
     }
@@ -245,7 +255,7 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       int const col = colX + i * (kFixThreads / RT);
-      big += col < k.n && fixCode(xv[i]) >= leastq;
+      big += col < k.n && fixLarge(xv[i], leastq);
       uint32_t d[D];
       fixSplit(xv[i], exq, d);
       // column col = 8 st + c8: lane t = c8 % 4, register c8 / 4; result
@@ -299,8 +309,8 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
         bool const mine = (fixed >> (4 * u + t)) & 1u;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-          double const v = fixAdd(acc[u][r], sum[u], r, (r < 2 ? ea0 : ea1) + exu);
-          if (mine) acc[u][r] = v;
+          double const v = fixAdd(acc(u, r), sum[u], r, (r < 2 ? ea0 : ea1) + exu);
+          if (mine) acc(u, r) = v;
         }
       }
     }
@@ -312,8 +322,8 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
           for (int u = 0; u < NT; ++u)
             if (((~fixed & rhs) >> (4 * u + t)) & 1u) {
               double2 const x = k.x[col * k.xld + 4 * u + t];
-              cmacc(acc[u][0], acc[u][1], a0, x);
-              cmacc(acc[u][2], acc[u][3], a1, x);
+              cmacc(acc(u, 0), acc(u, 1), a0, x);
+              cmacc(acc(u, 2), acc(u, 3), a1, x);
             }
         }
     }
@@ -325,26 +335,26 @@ __global__ void __launch_bounds__(kFixThreads, 3) fixTileKernel(
     buf ^= 1;
     if (k.c < it.nContrib) fetch(buf);
   }
-  __syncthreads();
-  double *const part = reinterpret_cast<double *>(sB);   // [warp][u][r][lane]
+  if constexpr (NT == 1) {
 #pragma unroll
-  for (int u = 0; u < NT; ++u)
-#pragma unroll
-    for (int r = 0; r < 4; ++r) part[((warp * NT + u) * 4 + r) * 32 + lane] = acc[u][r];
+    for (int r = 0; r < 4; ++r) sAcc[r][tid] = rAcc[r];
+  }
   __syncthreads();
   if (role.kp != 0) return;
   int const warpStep = kFixWarps / role.ks;   // warps of one row tile
 #pragma unroll
   for (int u = 0; u < NT; ++u) {
+    double v[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[r] = sAcc[4 * u + r][tid];
     for (int w = 1; w < role.ks; ++w)
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
-        acc[u][r] += part[(((warp + w * warpStep) * NT + u) * 4 + r) * 32 + lane];
+      for (int r = 0; r < 4; ++r) v[r] += sAcc[4 * u + r][tid + 32 * w * warpStep];
     int const rhs = 4 * u + t, row = 16 * role.mt + (lane >> 2);
     if (rhs < nr) {
       double2 *out = W + (it.outRow + row) * R + r0 + rhs;
-      if (row < it.rows) out[0] = make_double2(acc[u][0], acc[u][1]);
-      if (row + 8 < it.rows) out[8 * R] = make_double2(acc[u][2], acc[u][3]);
+      if (row < it.rows) out[0] = make_double2(v[0], v[1]);
+      if (row + 8 < it.rows) out[8 * R] = make_double2(v[2], v[3]);
     }
   }
 }
@@ -511,7 +521,7 @@ fixGemvKernel(ApplyItem const *__restrict__ items, ApplyContrib const *__restric
     int const ex = fixScaleOf(code);
     if (tid < KC) sx[tid] = tid < n ? fixHalves(xv, ex) : make_int4(0, 0, 0, 0);
     int const big =
-        __popc(__ballot_sync(0xffffffffu, tid < n && fixCode(xv) >= code - kFixInputGap));
+        __popc(__ballot_sync(0xffffffffu, tid < n && fixLarge(xv, code - kFixInputGap)));
     if (lane == 0) sBig[warp] = big;
     __syncthreads();
     int all = 0;

@@ -57,6 +57,10 @@ __device__ __forceinline__ int fixCode(double v) {
   return (e == 0 && (h | (uint32_t)__double2loint(v)) != 0u) ? 1 : e;
 }
 __device__ __forceinline__ int fixCode(double2 v) { return max(fixCode(v.x), fixCode(v.y)); }
+// code of v >= least, for least from 1 to 2046 (a subnormal's is below all)
+__device__ __forceinline__ bool fixLarge(double2 v, int least) {
+  return max(__double2hiint(v.x) & 0x7FFFFFFF, __double2hiint(v.y) & 0x7FFFFFFF) >= least << 20;
+}
 // the scale used for a largest code: any for all-zero data, the special one
 // for data whose range fixed point does not cover (subnormal, NaN, infinite)
 __device__ __forceinline__ int fixScaleOf(int code) {
