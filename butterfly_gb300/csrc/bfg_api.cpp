@@ -975,9 +975,9 @@ void runApplyTc(bfgFac f, int terms, float2 const *X, int64_t ldx, int64_t R, fl
 // Which BFG_PRECISION_DF64 applies run in double-float: the others take the
 // FP64 apply, whose fixed-point products are more exact and cost the same for
 // one right-hand side as for four, where double-float costs as much for each
-// (us for 2, 3 and 4, double-float against FP64: 4,096 points 57, 75 and 84
-// against 83; 10,007 117, 143 and 171 against 153; 32,768 497, 700 and 895
-// against 580).  So two run in double-float (at every size measured, 1,024 to
+// (us for 2, 3 and 4, double-float against FP64: 4,096 points 56, 76 and 84
+// against 82; 10,007 118, 144 and 171 against 151; 32,768 495, 700 and 895
+// against 571).  So two run in double-float (at every size measured, 1,024 to
 // 65,536 points, faster by up to 30 %), and three where the columns are few
 // and much of the time goes by in the longest items: 2,048 to 10,007 points 5
 // to 15 % faster, but slower at 16,384, at 1,024 (one dense stage) and for

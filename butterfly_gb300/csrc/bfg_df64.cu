@@ -3,11 +3,10 @@
 // significant bits) and multiplied with FP32 FMAs and their exact error terms.
 // The same 16 bytes per stored entry as FP64, within ~1e-13 of it, and fewer
 // instructions an entry than the FP64 apply's fixed-point products (32,768
-// points: 268 us against 345).  More right-hand sides take the FP64 apply,
+// points: 269 us against 351).  More right-hand sides take the FP64 apply,
 // which is both more exact and faster there.  Same apply program as the other
-// precisions
-// (mat_block_dense.c:512-572, mat_product.c:211-245, one item = rows of one
-// block row summing its blocks in order), no atomics, reproducible.
+// precisions (mat_block_dense.c:512-572, mat_product.c:211-245, one item =
+// rows of one block row summing its blocks in order), no atomics, reproducible.
 //
 // Arithmetic (error-free transformations, Dekker 1971 / Knuth TAOCP 4.2.2;
 // the FMA form of the product and the double-word sums of Joldes, Muller and

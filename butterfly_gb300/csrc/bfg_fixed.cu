@@ -14,10 +14,10 @@
 // fixCovers, fixEven) are multiplied in plain FP64 by the same kernels.
 //
 // Measured (GB300; microseconds an apply; before: the FP64-unit kernels):
-//   32,768 points, k = 256, 6.0e7 entries   R = 1: 526 -> 345
-//     R = 2..4: 4,000 -> 576   R = 8: 4,018 -> 940   R = 16: 7,650 -> 1,766
+//   32,768 points, k = 256, 6.0e7 entries   R = 1: 526 -> 351
+//     R = 2..4: 4,000 -> 571   R = 8: 4,018 -> 873   R = 16: 7,650 -> 1,647
 //   65,536 points, k = 512, 2.1e8 entries   R = 1: 1,583 -> 905
-//     R = 8: 2,484   R = 16: 23,853 -> 4,808
+//     R = 2..4: 1,467   R = 8: 2,302   R = 16: 23,853 -> 4,476
 // Largest error against extended precision, in units of each result's sum of
 // moduli, blocks of 20 to 120 columns: R = 1 5e-17 -> 1e-17, R = 2 1.6e-16 ->
 // 4e-17, R = 16 8e-17 -> 4e-17 for entries of like size; operands graded in
@@ -160,10 +160,10 @@ __device__ __forceinline__ void fixNextBlock(FixCursor &k, ApplyItem const &it, 
 // that share rows add their FP64 sums at the end, in order.
 // Bound by instruction issue and latency, not by the tensor pipe: splitting the
 // entries and the inputs takes about 50 instructions each.  So resident warps
-// count.  (65,536 points, 8 and 16 right-hand sides: 2,484 and 4,808 us.  With
-// seven digits and without the gradings 2,225 and 4,290; with seven digits and
-// flushes a block also the tiles' shape was chosen:) 8 right-hand sides a tile
-// with 168 registers and 3 CTAs an SM (16 of them: 255 and 2, the tensor pipe
+// count.  (65,536 points, 8 and 16 right-hand sides: 2,302 and 4,476 us.  With
+// seven digits, the gradings left out and the sums in registers 2,225 and
+// 4,290.  The tiles' shape was chosen with seven digits and flushes a block:)
+// 8 right-hand sides a tile with 168 registers and 3 CTAs an SM (16 of them: 255 and 2, the tensor pipe
 // 30 % busy) took 2,076 us where 2 CTAs took 2,332, and two such tiles 3,980
 // us for 16 where one of 16 took 4,782 although the entries are split twice;
 // 32,768 points 882 -> 787 and 1,680 -> 1,455, 4,096 points 98 -> 100 and 187
@@ -662,7 +662,7 @@ cudaError_t launchApplyStageFixed(ApplyItem const *items, int64_t nItems,
                                ldx, W);
   }
   // the narrowest tile that holds the right-hand sides (an empty column costs as
-  // much as a full one: 32,768 points 576 us with 4 columns, 940 with 8,
+  // much as a full one: 32,768 points 571 us with 4 columns, 873 with 8,
   // whatever part of them is used), several of 8 for more
   if (R <= 4) return launchTile<1>(items, nItems, contribs, rowExp, arena, X, ldx, W, R, stream);
   return launchTile<2>(items, nItems, contribs, rowExp, arena, X, ldx, W, R, stream);

@@ -147,7 +147,8 @@ __device__ __forceinline__ double fixAdd(double acc, float (&sum)[kFixSums][4], 
   int64_t const hi = ((int64_t)v[0] << 24) + ((int64_t)v[1] << 16) + ((int64_t)v[2] << 8) + v[3];
   int64_t const lo = ((int64_t)v[4] << 24) + ((int64_t)v[5] << 16) + ((int64_t)v[6] << 8) + v[7];
   // hi 2^32 + lo in 63 bits: one conversion and one FMA on the FP64 pipe, not
-  // two (an apply of 16 right-hand sides at 65,536 points 5,141 -> 4,808 us)
+  // two (an apply of 16 right-hand sides at 65,536 points 5,141 -> 4,808 us,
+  // with the FP64 sums still in registers)
   int const top = (int)(hi >> 12), sh = max(14 - __clz(top ^ (top >> 31)), 0);
   int64_t const t = (int64_t)((uint64_t)hi << (32 - sh)) + (lo >> sh);
   return fma((double)t, fixPow(sumE - 1089 + sh), acc);

@@ -12,8 +12,9 @@
 // reference's SVD spends O(p^3) on directions that the pseudo-inverse cut
 // then drops.  This path spends its work on the numerical rank instead
 // (a randomized range finder; Halko, Martinsson and Tropp, SIAM Review 53,
-// 2011, algorithms 4.1 and 5.1), in FP64 precision throughout
-// (the products by exact digit sums, bfg_fixed.cuh):
+// 2011, algorithms 4.1 and 5.1), its results in FP64 precision (only the
+// Jacobi's first sweeps run in FP32; the products are exact digit sums,
+// bfg_fixed.cuh):
 //
 //   Y  = Z_equiv Omega        Omega p x l with iid complex Gaussian entries
 //   Q  = qr(Y)                Householder (explicit Q, p x l)
