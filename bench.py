@@ -52,17 +52,17 @@ CONFIGS = {
 }
 METRIC = "Butterfly apply RHS/s at 1e-6 rel err vs plain FP64 GPU; GMRES time-to-1e-8"
 # DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) per algorithmic
-# byte of each stage launch of the 16-RHS apply (FP32 pipelined kernel, bf16x3
-# tensor-core kernel), from one ncu capture of the c2s workload each; the c2
-# workload (same geometry, kernels and stage structure at twice the size)
+# byte of each stage launch of the 16-RHS apply (applyRhsKernel in FP32,
+# applyTcKernel in bf16x3), from one ncu capture of the c2s workload each; the
+# c2 workload (same geometry, kernels and stage structure at twice the size)
 # reports its dominant launch's traffic as this ratio times its own
 # algorithmic bytes
-NCU_DRAM_PER_ALG = {("c2", "fp32", 16): [0.7973, 1.0266, 0.9855, 0.7925],
-                    ("c2", "bf16x3", 16): [0.8888, 1.0627, 1.0246, 1.0386],
-                    ("c2s", "fp32", 16): [0.7973, 1.0266, 0.9855, 0.7925],
-                    ("c2s", "bf16x3", 16): [0.8888, 1.0627, 1.0246, 1.0386],
-                    ("c2", "bf16x3", 256): [0.537, 1.057],
-                    ("c4", "bf16x3", 256): [0.537, 1.057]}
+NCU_DRAM_PER_ALG = {("c2", "fp32", 16): [0.7815, 1.0409, 0.9971, 0.9678],
+                    ("c2", "bf16x3", 16): [0.8900, 1.0609, 1.0256, 1.0369],
+                    ("c2s", "fp32", 16): [0.7815, 1.0409, 0.9971, 0.9678],
+                    ("c2s", "bf16x3", 16): [0.8900, 1.0609, 1.0256, 1.0369],
+                    ("c2", "bf16x3", 256): [0.538, 1.057],
+                    ("c4", "bf16x3", 256): [0.538, 1.057]}
 NCU_TRAFFIC_SOURCE = {
     ("c2", 16): "ncu DRAM bytes of the same stage in a capture of the 32,768-point workload, "
                 "scaled by algorithmic bytes",
